@@ -16,7 +16,7 @@ from typing import List, Optional, Tuple
 
 import numpy as np
 
-from . import _lib
+from . import _lib, _results
 
 
 def _ptr(a) -> C.c_void_p:
@@ -61,6 +61,7 @@ class Context:
         if self.h:
             self.lib.hl_b200_shutdown(self.h)
             self.h = None
+            _results.release()
 
     def label(self) -> str:
         return self.lib.hl_b200_label(self.h).decode()
@@ -154,7 +155,7 @@ class Context:
         gates, outputs = np.ascontiguousarray(gates, np.int64), np.ascontiguousarray(outputs, np.int64)
         ids = np.ascontiguousarray(group_ids, np.uint32)
         a, b, t = (np.array(v, dtype=np.uint64) for v in (alpha, beta, tag))
-        h = np.empty((gates.size, 2), dtype=np.uint64)
+        h = _results.empty((gates.size, 2), np.uint64)
         self.check(self.lib.hl_b200_act_helpers(self.h, _ptr(gates), _ptr(outputs), gates.size, f_pad, tokens, hidden, _ptr(ids), _ptr(a), _ptr(b),
                                                 _ptr(t), _ptr(h)))
         return h
@@ -163,7 +164,7 @@ class Context:
         """``accuracy_act::table`` (accuracy_act.rs:13-31) and its helper m / (alpha - t) (protocol.rs:1928): (compressed, ht)."""
         tables, mult = np.ascontiguousarray(tables, np.int64), _u64(mult)
         a, b, t = (np.array(v, dtype=np.uint64) for v in (alpha, beta, tag))
-        comp, ht = np.empty((length, 2), dtype=np.uint64), np.empty((length, 2), dtype=np.uint64)
+        comp, ht = _results.empty((length, 2), np.uint64), _results.empty((length, 2), np.uint64)
         self.check(self.lib.hl_b200_act_table(self.h, _ptr(tables), tables.size // 4096, length, _ptr(mult), _ptr(a), _ptr(b), _ptr(t), _ptr(comp), _ptr(ht)))
         return comp, ht
 
@@ -171,7 +172,7 @@ class Context:
         """``gpu::witness_product`` (metal.rs:4646-4680): the exact int16 x int8 -> int64 plane, or None when the CPU must take
         it (an activation outside int16, a shape outside the kernels' bounds)."""
         x, w = np.ascontiguousarray(x, np.int64), np.ascontiguousarray(w, np.int8)
-        out, taken = np.empty(out_len, dtype=np.int64), C.c_int(0)
+        out, taken = _results.empty(out_len, np.int64), C.c_int(0)
         self.check(self.lib.hl_b200_witness_product(self.h, t_rows, _ptr(x), x.size, xs, _ptr(w), w.size, inner, outer, os_, out_len,
                                                     1 if in_out else 0, _ptr(out), C.byref(taken)))
         return out if taken.value else None
@@ -187,7 +188,7 @@ class Context:
     def rng_fill(self, key32: bytes, first_word: int, count: int, as_fp: bool) -> np.ndarray:
         """`count` draws of the caller's ZkRng stream (rng.rs:279-417) from word position `first_word`, expanded on the
         device: u64 words, or field elements (two words each) when `as_fp`."""
-        out = np.zeros(count, dtype=np.uint64)
+        out = _results.empty(count, np.uint64)
         self.check(self.lib.hl_b200_rng_fill(self.h, key32, first_word, count, 1 if as_fp else 0, _ptr(out)))
         return out
 
@@ -197,14 +198,14 @@ class Context:
     def probe_field(self, a, b) -> np.ndarray:
         """metal_probe_field: (a+b, a-b, a*b) per pair, shape (n, 3)."""
         a, b = _u64(a), _u64(b)
-        out = np.empty((a.size, 3), dtype=np.uint64)
+        out = _results.empty((a.size, 3), np.uint64)
         self.check(self.lib.hl_b200_probe_field(self.h, _ptr(a), _ptr(b), a.size, _ptr(out)))
         return out
 
     def logup_histogram(self, idx, table_len: int) -> np.ndarray:
         """accuracy_act.rs:55-73: multiplicity of every table entry over all queries (padding included)."""
         idx = np.ascontiguousarray(idx, dtype=np.int32)
-        out = np.empty(table_len, dtype=np.uint64)
+        out = _results.empty(table_len, np.uint64)
         self.check(self.lib.hl_b200_logup_histogram(self.h, _ptr(idx), idx.size, table_len, _ptr(out)))
         return out
 
@@ -214,7 +215,7 @@ class Context:
         outv = np.ascontiguousarray(outv, dtype=np.int32)
         ix = np.ascontiguousarray(idx, dtype=np.int32) if idx is not None else None
         mu = _u64(mult) if mult is not None else None
-        h = np.empty((outv.size, 2), dtype=np.uint64)
+        h = _results.empty((outv.size, 2), np.uint64)
         a, b, t = (np.array([int(x[0]), int(x[1])], dtype=np.uint64) for x in (alpha, beta, tag))
         self.check(self.lib.hl_b200_logup_helpers(self.h, _ptr(ix), _ptr(outv), outv.size, _ptr(a), _ptr(b), _ptr(t), idx_off, _ptr(mu), _ptr(h)))
         return h
@@ -262,7 +263,7 @@ class Context:
         """salt_leaf_keyed + MerkleTree::build_keyed: all levels, (2 nn - 1, 32) bytes, root last."""
         leaves = np.ascontiguousarray(leaves, dtype=np.uint8)
         nn = leaves.shape[0]
-        out = np.empty((2 * nn - 1, 32), dtype=np.uint8)
+        out = _results.empty((2 * nn - 1, 32), np.uint8)
         s = np.ascontiguousarray(salts, dtype=np.uint8) if salts is not None else None
         self.check(self.lib.hl_b200_merkle(self.h, _ptr(leaves), _ptr(s), nn, _ptr(leaf_key), _ptr(node_key), _ptr(out)))
         return out
@@ -285,7 +286,7 @@ class B200Commit:
         """rho^T M over the message columns: (k, rows, 2) -> (k, n, 2)."""
         rhos = _u64(rhos)
         k = rhos.shape[0]
-        out = np.empty((k, self.n, 2), dtype=np.uint64)
+        out = _results.empty((k, self.n, 2), np.uint64)
         self.ctx.check(self.ctx.lib.hl_b200_store_fold(self.h, _ptr(rhos), k, 0, _ptr(out)))
         return out
 
@@ -293,14 +294,14 @@ class B200Commit:
         """backend.rs:56-59 ([A8]): rho^T [M | pads], (k, n + q, 2); the pads are the commit's, resident."""
         rhos = _u64(rhos)
         k = rhos.shape[0]
-        out = np.empty((k, self.n + self.q, 2), dtype=np.uint64)
+        out = _results.empty((k, self.n + self.q, 2), np.uint64)
         self.ctx.check(self.ctx.lib.hl_b200_store_fold(self.h, _ptr(rhos), k, 1, _ptr(out)))
         return out
 
     def columns(self, idx) -> np.ndarray:
         """The encoded columns at idx, (len(idx), rows), order of idx, duplicates repeated."""
         idx = _u64(idx)
-        out = np.empty((idx.size, self.rows), dtype=np.uint64)
+        out = _results.empty((idx.size, self.rows), np.uint64)
         self.ctx.check(self.ctx.lib.hl_b200_store_columns(self.h, _ptr(idx), idx.size, _ptr(out)))
         return out
 
@@ -308,7 +309,7 @@ class B200Commit:
         """All levels of the salted tree, (2 nn - 1, 32).  `out`: the caller's buffer for them (page-locked memory makes the read-back
         a direct copy)."""
         if out is None:
-            out = np.empty((2 * self.nn - 1, 32), dtype=np.uint8)
+            out = _results.empty((2 * self.nn - 1, 32), np.uint8)
         assert out.dtype == np.uint8 and out.size == (2 * self.nn - 1) * 32 and out.flags.c_contiguous
         s = np.ascontiguousarray(salts, dtype=np.uint8) if salts is not None else None
         self.ctx.check(self.ctx.lib.hl_b200_store_merkle(self.h, _ptr(s), _ptr(leaf_key), _ptr(node_key), _ptr(out)))
@@ -351,7 +352,7 @@ class B200Backend:
     def try_commit(self, log_cols: int, inv_rate: int, data, max_log: int, key: Optional[bytes] = None):
         data = _u64(data)
         rows = data.size >> log_cols
-        leaves = np.empty((inv_rate << log_cols, 32), dtype=np.uint8)
+        leaves = _results.empty((inv_rate << log_cols, 32), np.uint8)
         h = C.c_void_p()
         rc = self.ctx.lib.hl_b200_commit(self.ctx.h, log_cols, inv_rate, _ptr(data), rows, max_log, _ptr(key), C.byref(h), _ptr(leaves))
         if rc != 0:
@@ -366,7 +367,7 @@ class B200Backend:
         data, pads, pows = _u64(data), _u64(pads), _u64(pows)
         rows = data.size >> log_cols
         q = pads.size // rows if rows else 0
-        leaves = leaves_out if leaves_out is not None else np.empty((inv_rate << log_cols, 32), dtype=np.uint8)
+        leaves = leaves_out if leaves_out is not None else _results.empty((inv_rate << log_cols, 32), np.uint8)
         assert leaves.dtype == np.uint8 and leaves.size == (inv_rate << log_cols) * 32 and leaves.flags.c_contiguous
         h = C.c_void_p()
         rc = self.ctx.lib.hl_b200_commit_zk(self.ctx.h, log_cols, inv_rate, _ptr(data), rows, _ptr(pads), q, _ptr(pows), max_log,
@@ -385,8 +386,8 @@ class B200Backend:
         salts = np.ascontiguousarray(salts, dtype=np.uint8)
         rows, nn = data.size >> log_cols, inv_rate << log_cols
         q = pads.size // rows if rows else 0
-        leaves = None if not want_leaves else leaves_out if leaves_out is not None else np.empty((nn, 32), dtype=np.uint8)
-        levels = levels_out if levels_out is not None else np.empty((2 * nn - 1, 32), dtype=np.uint8)
+        leaves = None if not want_leaves else leaves_out if leaves_out is not None else _results.empty((nn, 32), np.uint8)
+        levels = levels_out if levels_out is not None else _results.empty((2 * nn - 1, 32), np.uint8)
         assert (leaves is None or leaves.size == nn * 32) and levels.size == (2 * nn - 1) * 32 and salts.size == nn * 32
         h = C.c_void_p()
         rc = self.ctx.lib.hl_b200_commit_zk_tree(self.ctx.h, log_cols, inv_rate, _ptr(data), rows, _ptr(pads), q, _ptr(pows), max_log, _ptr(key),
@@ -409,11 +410,11 @@ class B200Backend:
         q = pads.size // rows if rows else 0
         assert packed.size == int(row_width.astype(np.int64).sum()) << log_cols
         tree = salts is not None
-        leaves = np.empty((nn, 32), dtype=np.uint8) if (want_leaves or not tree) else None
+        leaves = _results.empty((nn, 32), np.uint8) if (want_leaves or not tree) else None
         levels = None
         if tree:
             salts = np.ascontiguousarray(salts, dtype=np.uint8)
-            levels = levels_out if levels_out is not None else np.empty((2 * nn - 1, 32), dtype=np.uint8)
+            levels = levels_out if levels_out is not None else _results.empty((2 * nn - 1, 32), np.uint8)
             assert salts.size == nn * 32 and levels.size == (2 * nn - 1) * 32
         h = C.c_void_p()
         rc = self.ctx.lib.hl_b200_commit_zk_packed(self.ctx.h, log_cols, inv_rate, _ptr(packed), _ptr(row_width), rows, _ptr(pads), q, _ptr(pows), max_log,
@@ -528,7 +529,7 @@ def mask_commit(ctx: Context, msgs: np.ndarray, coef_rows: np.ndarray, pows: np.
     msgs, coef_rows, pows = _u64(msgs), _u64(coef_rows), _u64(pows)
     m = 1 << log_msg
     n_msg, n_coef = msgs.size // m, coef_rows.size // (2 * m)
-    a_coefs = np.empty((n_msg, m), dtype=np.uint64)
+    a_coefs = _results.empty((n_msg, m), np.uint64)
     leaves = np.empty((1 << log_dom, 32), dtype=np.uint8)
     h = C.c_void_p()
     rc = ctx.lib.hl_b200_mask_commit(ctx.h, log_msg, log_dom, _ptr(msgs), n_msg, _ptr(coef_rows), n_coef, _ptr(pows), _ptr(col_key), C.byref(h),
@@ -636,7 +637,7 @@ class B200Tables:
         self.ctx.check(self.ctx.lib.hl_b200_tables_flush(self.h))
 
     def read(self, i: int) -> np.ndarray:
-        out = np.zeros((1 << self.n_vars, 2), dtype=np.uint64)
+        out = _results.empty((1 << self.n_vars, 2), np.uint64)
         self.ctx.check(self.ctx.lib.hl_b200_tables_read(self.h, i, _ptr(out)))
         return out
 

@@ -119,8 +119,7 @@ int hl_b200_act_histogram(hl_ctx* c, const int64_t* gates, const int64_t* output
     if (!shape_ok(n, f_pad, tokens, hidden) || groups < 1 || groups > 4) return fail(c, HL_B200_ERR_ARG, "act_histogram: query rows or table count");
     for (size_t j = 0; j < hidden; j++)
         if (group_ids[j] >= groups) return fail(c, HL_B200_ERR_ARG, "act_histogram: a group id outside the registered tables");
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     Bufs bufs{c, {}};
     long long *d_g = nullptr, *d_o = nullptr, *d_t = nullptr;
     u32* d_ids = nullptr;
@@ -156,8 +155,7 @@ int hl_b200_act_helpers(hl_ctx* c, const int64_t* gates, const int64_t* outputs,
     if (!c || !gates || !outputs || !group_ids || !alpha || !beta || !tag || !h) return fail(c, HL_B200_ERR_ARG, "act_helpers: null argument");
     if (!shape_ok(n, f_pad, tokens, hidden)) return fail(c, HL_B200_ERR_ARG, "act_helpers: query rows");
     if (n == 0) return HL_B200_OK;
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     Bufs bufs{c, {}};
     long long *d_g = nullptr, *d_o = nullptr;
     u32* d_ids = nullptr;
@@ -201,8 +199,7 @@ int hl_b200_act_table(hl_ctx* c, const int64_t* tables, size_t groups, size_t le
     if (groups < 1 || groups > 4 || len < entries || (len & (len - 1)) != 0) return fail(c, HL_B200_ERR_ARG, "act_table: one to four registered tables must fit in one row");
     for (size_t g = 0; g < groups; g++)
         if (tables[g * 4096 + 2048] != 0) return fail(c, HL_B200_ERR_ARG, "act_table: invalid generated table zero row");
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     Bufs bufs{c, {}};
     long long* d_t = nullptr;
     u64 *d_m = nullptr, *d_v = nullptr, *d_h = nullptr;

@@ -44,56 +44,6 @@ void dev_free(hl_ctx* c, void* p, size_t bytes) {
     c->alloc_live = c->alloc_live >= bytes ? c->alloc_live - bytes : 0;
 }
 
-int h2d(hl_ctx* c, void* d, const void* h, size_t bytes) {
-    if (!bytes) return HL_B200_OK;
-    cudaError_t e = cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, c->stream);
-    if (e != cudaSuccess) return fail(c, HL_B200_ERR_DEVICE, "copy to device", e);
-    c->stats.bytes_h2d += bytes;
-    return HL_B200_OK;
-}
-
-// An asynchronous copy out of page-locked caller memory reads the source when the DMA runs, not when the call is made: a call
-// that returns without synchronising would let the caller overwrite inputs that are still to be read.  Small inputs are
-// bounced through a page-locked area of the context (reused after a synchronisation when it wraps); large ones are copied
-// in place and waited for.
-constexpr size_t ARENA_BYTES = (size_t)4 << 20;
-int h2d_owned(hl_ctx* c, void* d, const void* h, size_t bytes) {
-    if (!bytes) return HL_B200_OK;
-    if (!c->arena && cudaHostAlloc((void**)&c->arena, ARENA_BYTES, cudaHostAllocDefault) != cudaSuccess) {
-        cudaGetLastError();
-        c->arena = nullptr;
-    }
-    if (c->arena && bytes <= ARENA_BYTES / 4) {
-        const size_t need = (bytes + 63) & ~(size_t)63;
-        if (c->arena_off + need > ARENA_BYTES) {
-            cudaError_t e = cudaStreamSynchronize(c->stream);
-            if (e != cudaSuccess) return fail(c, HL_B200_ERR_DEVICE, "staging area", e);
-            c->arena_off = 0;
-        }
-        char* slot = c->arena + c->arena_off;
-        c->arena_off += need;
-        memcpy(slot, h, bytes);
-        return h2d(c, d, slot, bytes);
-    }
-    int rc = h2d(c, d, h, bytes);
-    if (!rc) rc = sync(c, "copy to device");
-    return rc;
-}
-
-int d2h(hl_ctx* c, void* h, const void* d, size_t bytes) {
-    if (!bytes) return HL_B200_OK;
-    cudaError_t e = cudaMemcpyAsync(h, d, bytes, cudaMemcpyDeviceToHost, c->stream);
-    if (e != cudaSuccess) return fail(c, HL_B200_ERR_DEVICE, "copy from device", e);
-    c->stats.bytes_d2h += bytes;
-    return HL_B200_OK;
-}
-
-int sync(hl_ctx* c, const char* what) {
-    cudaError_t e = cudaStreamSynchronize(c->stream);
-    if (e != cudaSuccess) return fail(c, HL_B200_ERR_DEVICE, what, e);
-    return HL_B200_OK;
-}
-
 // w_nn^j for j < nn, w_nn = 7^((p-1)/2^32)^(2^(32-log nn)) (field.rs:86-91, ntt.rs:29-43);
 // built once per size on the host and kept on the device.
 int root_powers(hl_ctx* c, u32 lognn, const u64** out) {
@@ -162,8 +112,7 @@ int hl_b200_timing_enable(hl_ctx* c, int on) {
 
 int hl_b200_timing_read(hl_ctx* c, hl_timing* out, int reset) {
     if (!c || !out) return HL_B200_ERR_ARG;
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     int rc = sync(c, "timing_read");
     if (rc) return rc;
     for (auto& s : c->spans) {
@@ -202,6 +151,7 @@ int hl_b200_init(int device, hl_ctx** out) {
     snprintf(buf, sizeof buf, "hl_b200: %s (sm_%d%d, %d SMs, %.0f GB), device %d", prop.name, prop.major, prop.minor,
              prop.multiProcessorCount, (double)prop.totalGlobalMem / 1e9, device);
     c->label = buf;
+    host_copy_retain();
     *out = c;
     return HL_B200_OK;
 }
@@ -212,10 +162,7 @@ void hl_b200_shutdown(hl_ctx* c) {
     cudaStreamSynchronize(c->stream);
     for (auto& kv : c->tw) cudaFree(kv.second);
     if (c->d_wp_flag) cudaFree(c->d_wp_flag);
-    for (int i = 0; i < 2; i++) {
-        if (c->stage[i]) cudaFreeHost(c->stage[i]);
-        if (c->stage_ev[i]) cudaEventDestroy(c->stage_ev[i]);
-    }
+    host_copy_release(c);
     if (c->arena) cudaFreeHost(c->arena);
     for (auto& s : c->spans) { cudaEventDestroy(s.a); cudaEventDestroy(s.b); }
     for (auto e : c->ev_pool) cudaEventDestroy(e);
@@ -225,6 +172,7 @@ void hl_b200_shutdown(hl_ctx* c) {
     cudaStreamDestroy(c->copy_stream);
     cudaStreamDestroy(c->own_stream);
     delete c;
+    host_copy_drop();
 }
 
 const char* hl_b200_label(hl_ctx* c) { return c ? c->label.c_str() : "hl_b200: no context"; }
@@ -247,8 +195,7 @@ int hl_b200_set_stream(hl_ctx* c, void* s) {
 
 int hl_b200_sync(hl_ctx* c) {
     if (!c) return HL_B200_ERR_ARG;
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     return sync(c, "synchronize");
 }
 
@@ -281,8 +228,7 @@ int hl_b200_stats(hl_ctx* c, hl_stats* out) {
 
 int hl_b200_probe_field(hl_ctx* c, const uint64_t* a, const uint64_t* b, size_t n, uint64_t* out3n) {
     if (!c || (n && (!a || !b || !out3n))) return fail(c, HL_B200_ERR_ARG, "probe_field: null argument");
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     u64 *da = nullptr, *db = nullptr, *dout = nullptr;
     int rc = dev_alloc(c, (void**)&da, n * 8);
     if (!rc) rc = dev_alloc(c, (void**)&db, n * 8);
@@ -302,8 +248,7 @@ int hl_b200_probe_field(hl_ctx* c, const uint64_t* a, const uint64_t* b, size_t 
 
 int hl_b200_butterfly_peak(hl_ctx* c, uint32_t iters, double* butterflies_per_second) {
     if (!c || !butterflies_per_second || iters == 0) return fail(c, HL_B200_ERR_ARG, "butterfly_peak: argument");
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     std::vector<u64> seed(4096);
     u64 x = 88172645463325252ULL;
     for (auto& v : seed) { x ^= x << 13; x ^= x >> 7; x ^= x << 17; v = gl_canon(x); }
@@ -334,8 +279,7 @@ int hl_b200_butterfly_peak(hl_ctx* c, uint32_t iters, double* butterflies_per_se
 
 int hl_b200_compress_peak(hl_ctx* c, uint32_t iters, double* compressions_per_second) {
     if (!c || !compressions_per_second || iters == 0) return fail(c, HL_B200_ERR_ARG, "compress_peak: argument");
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     std::vector<u64> seed(4096);
     u64 x = 88172645463325252ULL;
     for (auto& v : seed) { x ^= x << 13; x ^= x >> 7; x ^= x << 17; v = gl_canon(x); }

@@ -11,6 +11,8 @@
 #include "../../include/hl_b200.h"
 #include "kernels.h"
 
+namespace hlapi { struct CopyRing; }
+
 struct hl_ctx {
     int device = 0;
     int sm_count = 0;
@@ -31,11 +33,11 @@ struct hl_ctx {
     std::vector<Span> spans;          // recorded, not yet read
     std::vector<cudaEvent_t> ev_pool;  // events ready for reuse
     hl_timing timing_acc{};
-    void* stage[2] = {nullptr, nullptr};       // page-locked staging for uploads from pageable host memory (lazily allocated)
-    size_t stage_bytes = 0;
-    cudaEvent_t stage_ev[2] = {nullptr, nullptr};  // the copy out of stage[i] has completed
-    char* arena = nullptr;     // page-locked bounce area for small caller-owned inputs of calls that return before their copies run
+    hlapi::CopyRing* ring = nullptr;  // page-locked slots for large copies of pageable host memory (host_copy.cu, made on first use)
+    char* arena = nullptr;     // page-locked bounce area for small copies in either direction, empty after every synchronisation
     size_t arena_off = 0;
+    struct Pending { void* to; const char* from; size_t bytes; };
+    std::vector<Pending> pending;  // small results in the bounce area, handed out by the next `sync`
     int* d_wp_flag = nullptr;  // the witness products' status word: zero between calls
     bool wp_attr = false;      // the product kernel's shared-memory size has been raised on this device
     std::set<const struct hl_store*> stores;  // the live commitment stores (a planned slot table that reads one checks it is still there when it is built)
@@ -62,11 +64,26 @@ namespace hlapi {
 int fail(hl_ctx* c, int code, const char* what, cudaError_t e = cudaSuccess);
 int dev_alloc(hl_ctx* c, void** p, size_t bytes);
 void dev_free(hl_ctx* c, void* p, size_t bytes);
+// host_copy.cu: uploads on the context's stream (h2d_on: on another one that the context's stream waits for before the call ends);
+// h2d_owned: the caller's bytes are no longer needed when it returns, whatever kind of host memory they live in;
+// d2h: the bytes are in place after the next `sync`
 int h2d(hl_ctx* c, void* d, const void* h, size_t bytes);
-int d2h(hl_ctx* c, void* h, const void* d, size_t bytes);
-// like h2d, but the caller's bytes are no longer needed when it returns, whatever kind of host memory they live in
+int h2d_on(hl_ctx* c, void* d, const void* h, size_t bytes, cudaStream_t s);
 int h2d_owned(hl_ctx* c, void* d, const void* h, size_t bytes);
+int d2h(hl_ctx* c, void* h, const void* d, size_t bytes);
 int sync(hl_ctx* c, const char* what);
+void host_copy_retain();
+void host_copy_release(hl_ctx* c);
+void host_copy_drop();
+
+// What every entry point that works on a context holds: its lock and its device.  Results that a failed call left in the bounce area
+// go with it: nothing may write to that caller's memory later.
+struct Call {
+    hl_ctx* c;
+    std::lock_guard<std::mutex> g;
+    explicit Call(hl_ctx* ctx) : c(ctx), g(ctx->mu) { cudaSetDevice(c->device); }
+    ~Call() { c->pending.clear(); }
+};
 int root_powers(hl_ctx* c, u32 lognn, const u64** out);
 int upload_key(hl_ctx* c, const uint8_t* key32, uint32_t** d_key);
 int log2_exact(size_t v);

@@ -17,8 +17,7 @@ extern "C" {
 
 int hl_b200_logup_histogram(hl_ctx* c, const int32_t* idx, size_t nq, size_t table_len, uint64_t* mult) {
     if (!c || !mult || (nq && !idx) || table_len == 0 || table_len > (1u << 30)) return fail(c, HL_B200_ERR_ARG, "logup_histogram: argument");
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     int *d_idx = nullptr, *d_err = nullptr, h_err = 0;
     u64* d_mult = nullptr;
     int rc = dev_alloc(c, (void**)&d_idx, nq * 4);
@@ -44,8 +43,7 @@ int hl_b200_logup_helpers(hl_ctx* c, const int32_t* idx, const int32_t* outv, si
                           const uint64_t beta[2], const uint64_t tag[2], int64_t idx_off, const uint64_t* mult, uint64_t* h) {
     if (!c || !outv || !alpha || !beta || !tag || !h) return fail(c, HL_B200_ERR_ARG, "logup_helpers: null argument");
     if (n == 0) return HL_B200_OK;
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     // alpha - (idx + off + beta out + tag) = (alpha - tag - off) - idx - beta out, every term formed in the field
     fp2 base = f2_sub(f2(alpha[0], alpha[1]), f2(tag[0], tag[1]));
     base.c0 = gl_sub(base.c0, gl_from_i64(idx_off));
@@ -80,8 +78,7 @@ int hl_b200_logup_helpers(hl_ctx* c, const int32_t* idx, const int32_t* outv, si
 
 static int fold_i8(hl_ctx* c, bool by_rows, const int8_t* m, size_t rows, size_t cols, const uint64_t* w, uint64_t* out) {
     if (!c || !m || !w || !out || rows == 0 || cols == 0 || rows > 0x7FFFFFFFu || cols > 0x7FFFFFFFu) return fail(c, HL_B200_ERR_ARG, "fold_i8: argument");
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     const size_t nw = by_rows ? rows : cols, no = by_rows ? cols : rows;
     signed char* d_m = nullptr;
     u64 *d_w = nullptr, *d_o = nullptr;

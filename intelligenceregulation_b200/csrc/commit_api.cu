@@ -1,6 +1,5 @@
 // C ABI: commitments (Backend::try_commit*), stores (EncodedStore), Merkle trees.
 #include <cstring>
-#include <thread>
 
 #include "api_internal.h"
 
@@ -121,34 +120,8 @@ int commit_on_device(hl_ctx* c, hl_store* st, const u64* d_pows, const uint8_t* 
         if (e == cudaSuccess) e = cudaStreamWaitEvent(c->copy_stream, c->ev_main, 0);
         if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "stream ordering", e);
     }
-    // Rows in ordinary pageable memory: the driver would stage them through its own buffer at about 10 GB/s, so the pieces go
-    // through two page-locked buffers of the context instead, filled by a few host threads while the previous piece is on the bus.
-    bool staged = false;
-    if (!rc && pieces) {
-        cudaPointerAttributes attr;
-        const bool pageable = cudaPointerGetAttributes(&attr, h_data) != cudaSuccess || attr.type == cudaMemoryTypeUnregistered;
-        cudaGetLastError();  // an unregistered pointer is not an error here
-        size_t need = 0;  // the largest piece
-        for (u32 r0 = 0, k = 0; k < piece_rows.size(); r0 += piece_rows[k++]) {
-            const size_t b = byte_at(r0 + piece_rows[k]) - byte_at(r0);
-            need = b > need ? b : need;
-        }
-        if (pageable) {
-            staged = true;
-            if (c->stage_bytes < need) {
-                for (int i = 0; i < 2; i++) {
-                    if (c->stage[i]) { cudaFreeHost(c->stage[i]); c->stage[i] = nullptr; }
-                    if (cudaHostAlloc(&c->stage[i], need, cudaHostAllocDefault) != cudaSuccess) { c->stage[i] = nullptr; staged = false; }
-                    if (!c->stage_ev[i] && cudaEventCreateWithFlags(&c->stage_ev[i], cudaEventDisableTiming) != cudaSuccess) staged = false;
-                }
-                c->stage_bytes = staged ? need : 0;
-                cudaGetLastError();
-            }
-        }
-    }
     if (!rc && !pieces && hr.pads) rc = h2d(c, st->d_pads, hr.pads, (size_t)st->rows * st->q * 8);
     if (!rc && !pieces && hr.tail_bytes) rc = h2d(c, hr.tail_dst, hr.tail_src, hr.tail_bytes);
-    size_t piece_i = 0;
     if (!rc) {
         Timed t(c, HL_T_ENCODE);
         size_t ev_i = 0;
@@ -159,32 +132,12 @@ int commit_on_device(hl_ctx* c, hl_store* st, const u64* d_pows, const uint8_t* 
             if (h_data) {
                 cudaStream_t cs = pieces ? c->copy_stream : c->stream;
                 const size_t b0 = byte_at(r0), bytes = byte_at(r0 + nr) - b0;
-                const void* from = (const char*)h_data + b0;
-                if (staged) {
-                    const int b = (int)(piece_i++ & 1);
-                    if (piece_i > 2) cudaEventSynchronize(c->stage_ev[b]);  // the copy that last read this buffer is done
-                    const unsigned hw = std::thread::hardware_concurrency();
-                    const int nth = bytes >= ((size_t)8 << 20) ? (int)(hw >= 8 ? 8 : hw >= 2 ? hw : 1) : 1;
-                    std::vector<std::thread> th;
-                    for (int k = 1; k < nth; k++)
-                        th.emplace_back([=] { memcpy((char*)c->stage[b] + bytes * k / nth, (const char*)from + bytes * k / nth, bytes * (k + 1) / nth - bytes * k / nth); });
-                    memcpy(c->stage[b], from, bytes / nth);
-                    for (auto& x : th) x.join();
-                    from = c->stage[b];
-                }
                 void* to = packed ? (void*)(d_narrow + b0) : (void*)(st->d_data + (size_t)r0 * n);
-                cudaError_t e = cudaMemcpyAsync(to, from, bytes, cudaMemcpyHostToDevice, cs);
-                if (staged && e == cudaSuccess) e = cudaEventRecord(c->stage_ev[(piece_i - 1) & 1], cs);
-                c->stats.bytes_h2d += bytes;
-                if (pieces && hr.pads && e == cudaSuccess) {
-                    const size_t pb = (size_t)nr * st->q * 8;
-                    e = cudaMemcpyAsync(st->d_pads + (size_t)r0 * st->q, hr.pads + (size_t)r0 * st->q, pb, cudaMemcpyHostToDevice, cs);
-                    c->stats.bytes_h2d += pb;
-                }
-                if (pieces && hr.tail_bytes && r0 + nr == st->rows && e == cudaSuccess) {
-                    e = cudaMemcpyAsync(hr.tail_dst, hr.tail_src, hr.tail_bytes, cudaMemcpyHostToDevice, cs);
-                    c->stats.bytes_h2d += hr.tail_bytes;
-                }
+                rc = h2d_on(c, to, (const char*)h_data + b0, bytes, cs);
+                if (!rc && pieces && hr.pads) rc = h2d_on(c, st->d_pads + (size_t)r0 * st->q, hr.pads + (size_t)r0 * st->q, (size_t)nr * st->q * 8, cs);
+                if (!rc && pieces && hr.tail_bytes && r0 + nr == st->rows) rc = h2d_on(c, hr.tail_dst, hr.tail_src, hr.tail_bytes, cs);
+                if (rc) break;
+                cudaError_t e = cudaSuccess;
                 if (e == cudaSuccess && cs != c->stream) {
                     if (ev_i == c->ev_chunks.size()) {
                         cudaEvent_t ev = nullptr;
@@ -349,8 +302,7 @@ extern "C" {
 int hl_b200_commit(hl_ctx* c, uint32_t log_cols, uint32_t inv_rate, const uint64_t* data, size_t rows, uint32_t max_log,
                    const uint8_t* key32, hl_store** store, uint8_t* leaves32) {
     if (!c || !data || !store || !leaves32) return fail(c, HL_B200_ERR_ARG, "commit: null argument");
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     Shape s;
     int rc = check_shape(c, log_cols, inv_rate, rows, 0, false, max_log, &s);
     if (rc) return rc;
@@ -363,8 +315,7 @@ int hl_b200_commit_zk(hl_ctx* c, uint32_t log_cols, uint32_t inv_rate, const uin
                       const uint64_t* pads, size_t q, const uint64_t* pows, uint32_t max_log, const uint8_t* key32,
                       hl_store** store, uint8_t* leaves32) {
     if (!c || !data || !pads || !pows || !store || !leaves32) return fail(c, HL_B200_ERR_ARG, "commit_zk: null argument");
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     Shape s;
     int rc = check_shape(c, log_cols, inv_rate, rows, q, true, max_log, &s);
     if (rc) return rc;
@@ -377,8 +328,7 @@ int hl_b200_commit_zk_tree(hl_ctx* c, uint32_t log_cols, uint32_t inv_rate, cons
                            const uint64_t* pows, uint32_t max_log, const uint8_t* key32, const uint8_t* salts32, const uint8_t* leaf_key32,
                            const uint8_t* node_key32, hl_store** store, uint8_t* leaves32, uint8_t* levels_out) {
     if (!c || !data || !pads || !pows || !salts32 || !store || !levels_out) return fail(c, HL_B200_ERR_ARG, "commit_zk_tree: null argument");
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     Shape s;
     int rc = check_shape(c, log_cols, inv_rate, rows, q, true, max_log, &s);
     if (rc) return rc;
@@ -408,8 +358,7 @@ int hl_b200_commit_zk_packed(hl_ctx* c, uint32_t log_cols, uint32_t inv_rate, co
         at += (u64)w << log_cols;
     }
     hr.off[rows] = at;
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     if (salts32) {
         const TreeAsk tree{salts32, leaf_key32, node_key32, levels_out};
         return commit_host(c, s, hr, pads, pows, key32, store, leaves32, &tree);
@@ -421,8 +370,7 @@ int hl_b200_commit_zk_dev(hl_ctx* c, uint32_t log_cols, uint32_t inv_rate, const
                           const uint64_t* d_pads, size_t q, const uint64_t* d_pows, const uint8_t* key32,
                           hl_store** store, uint8_t* d_leaves32) {
     if (!c || !d_data || !d_pads || !d_pows || !store) return fail(c, HL_B200_ERR_ARG, "commit_zk_dev: null argument");
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     return commit_resident(c, log_cols, inv_rate, (const u64*)d_data, rows, (const u64*)d_pads, q, (const u64*)d_pows, key32, store, d_leaves32);
 }
 
@@ -441,8 +389,7 @@ const uint8_t* hl_b200_store_leaves_dev(hl_store* st) { return st ? (const uint8
 void hl_b200_store_free(hl_store* st) {
     if (!st) return;
     hl_ctx* c = st->ctx;
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     free_store(st);
 }
 
@@ -453,8 +400,7 @@ int hl_b200_store_fold(hl_store* st, const uint64_t* rhos, size_t k, int with_pa
     if (with_pads && !st->zk) return fail(c, HL_B200_ERR_ARG, "store_fold: pads asked of a plain store");
     if (k == 0) return HL_B200_OK;
     if (k > 0xFFFFu * 8u) return fail(c, HL_B200_ERR_ARG, "store_fold: too many vectors");
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     const u32 n = (u32)st->n(), q = with_pads ? st->q : 0, w = n + q, rows = st->rows;
     // An opening's group vectors are zero outside their claims' rows (pcs.rs:851-891), its proximity vector is dense.
     // Vectors with few non-zero rows go to the list kernel, the others to the dense one; both write the caller's order.
@@ -546,8 +492,7 @@ int hl_b200_store_columns(hl_store* st, const uint64_t* idx, size_t nidx, uint64
     if (nidx > 65535) return fail(c, HL_B200_ERR_ARG, "store_columns: more than 65535 columns in one call");
     for (size_t i = 0; i < nidx; i++)
         if (idx[i] >= st->nn()) return fail(c, HL_B200_ERR_ARG, "store_columns: index out of range");
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     u64 *d_idx = nullptr, *d_out = nullptr;
     const size_t ob = nidx * (size_t)st->rows * 8;
     int rc = dev_alloc(c, (void**)&d_idx, nidx * 8);
@@ -596,8 +541,7 @@ static int merkle_common(hl_ctx* c, const uint32_t* d_leaves_in, const uint8_t* 
 int hl_b200_merkle(hl_ctx* c, const uint8_t* leaves32, const uint8_t* salts32, size_t nn, const uint8_t* leaf_key32,
                    const uint8_t* node_key32, uint8_t* levels_out) {
     if (!c || !leaves32 || !levels_out) return fail(c, HL_B200_ERR_ARG, "merkle: null argument");
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     return merkle_common(c, nullptr, leaves32, salts32, nn, leaf_key32, node_key32, levels_out);
 }
 
@@ -605,8 +549,7 @@ int hl_b200_store_merkle(hl_store* st, const uint8_t* salts32, const uint8_t* le
                          uint8_t* levels_out) {
     if (!st || !levels_out) return HL_B200_ERR_ARG;
     hl_ctx* c = st->ctx;
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     return merkle_common(c, st->d_leaves, nullptr, salts32, st->nn(), leaf_key32, node_key32, levels_out);
 }
 
@@ -616,8 +559,7 @@ int hl_b200_store_merkle_dev(hl_store* st, const uint8_t* d_salts32, const uint8
     hl_ctx* c = st->ctx;
     // the tree kernels move digests as 16-byte vectors: a misaligned caller pointer would be a device fault, not a status
     if (((uintptr_t)d_levels_out & 15) || ((uintptr_t)d_salts32 & 15)) return fail(c, HL_B200_ERR_ARG, "store_merkle_dev: device pointers must be 16-byte aligned");
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     int rc = merkle_on_device(c, st->d_leaves, (const uint32_t*)d_salts32, st->nn(), leaf_key32, node_key32, (uint32_t*)d_levels_out);
     if (!rc) c->stats.merkles++;
     return rc;

@@ -106,8 +106,7 @@ int hl_b200_lookup_inverse_table(hl_ctx* c, const uint64_t alpha[2], const uint6
     if (!c || !alpha || !g || !d_table) return fail(c, HL_B200_ERR_ARG, "lookup_inverse_table: null argument");
     if (int rc = check_log(c, log_len)) return rc;
     if ((uintptr_t)d_table & 15) return fail(c, HL_B200_ERR_ARG, "lookup_inverse_table: the table must be 16-byte aligned");
-    std::lock_guard<std::mutex> lk(c->mu);
-    cudaSetDevice(c->device);
+    Call lk(c);
     const u32 len = 1u << log_len;
     const fp2 amg = f2_sub(f2(alpha[0], alpha[1]), f2(g[0], g[1]));
     Timed t(c, HL_T_LOGUP);
@@ -127,8 +126,7 @@ int hl_b200_lookup_helpers_dev(hl_ctx* c, const int64_t* d_a, const uint64_t* d_
     if (n == 0) return HL_B200_OK;
     if (((uintptr_t)d_table_a & 15) || ((uintptr_t)d_table_b & 15) || ((uintptr_t)d_a & 7) || ((uintptr_t)d_b & 7) || ((uintptr_t)d_re & 7) || ((uintptr_t)d_im & 7))
         return fail(c, HL_B200_ERR_ARG, "lookup_helpers: tables must be 16-byte aligned, columns and planes 8-byte aligned");
-    std::lock_guard<std::mutex> lk(c->mu);
-    cudaSetDevice(c->device);
+    Call lk(c);
     int* d_err = nullptr;
     int rc = dev_alloc(c, (void**)&d_err, 4);
     if (!rc && cudaMemsetAsync(d_err, 0, 4, c->stream) != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "lookup_helpers: flag");

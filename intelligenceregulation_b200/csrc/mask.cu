@@ -130,8 +130,7 @@ int hl_b200_mask_commit(hl_ctx* c, uint32_t log_msg, uint32_t log_dom, const uin
     if (log_msg < 8 || log_msg > 11 || log_dom < log_msg + 1 || log_dom > log_msg + 6)
         return fail(c, HL_B200_ERR_UNSUPPORTED, "mask_commit: messages of 2^8 .. 2^11 words, domain 2 .. 64 times the message");
     if (n_msg_rows == 0 || n_msg_rows > 4096 || n_coef_rows == 0 || n_coef_rows > 64) return fail(c, HL_B200_ERR_ARG, "mask_commit: row counts");
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     const size_t m = (size_t)1 << log_msg, m2 = 2 * m, dom = (size_t)1 << log_dom, rows = n_msg_rows + n_coef_rows;
     hl_store* st = new hl_store();
     st->ctx = c; st->rows = (u32)rows; st->logn = log_msg + 1; st->logr = log_dom - log_msg - 1; st->q = 0; st->zk = false; st->fold_data = true;
@@ -199,8 +198,7 @@ int hl_b200_mask_open_q(hl_store* st, size_t n_masks, const uint64_t* ws, uint64
     hl_ctx* c = st->ctx;
     if (!ws || !q || n_masks == 0) return fail(c, HL_B200_ERR_ARG, "mask_open_q: null argument");
     if (!st->fold_data || !st->d_data || st->logn < 9 || 2 * n_masks + 2 > st->rows) return fail(c, HL_B200_ERR_ARG, "mask_open_q: not a masking commitment of that many masks");
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     const u32 logm = st->logn - 1, logdom = st->logn + st->logr;
     const size_t m = (size_t)1 << logm, m2 = 2 * m;
     const u64* tw = nullptr;

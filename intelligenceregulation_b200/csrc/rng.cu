@@ -78,16 +78,14 @@ extern "C" {
 
 int hl_b200_rng_fill_dev(hl_ctx* c, const uint8_t* key32, uint64_t first_word, uint64_t count, int as_fp, uint64_t* d_out) {
     if (!c || !key32 || (count && !d_out)) return fail(c, HL_B200_ERR_ARG, "rng_fill_dev: null argument");
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     return fill_dev(c, key32, first_word, count, as_fp, reinterpret_cast<u64*>(d_out));
 }
 
 int hl_b200_rng_fill(hl_ctx* c, const uint8_t* key32, uint64_t first_word, uint64_t count, int as_fp, uint64_t* out) {
     if (!c || !key32 || (count && !out)) return fail(c, HL_B200_ERR_ARG, "rng_fill: null argument");
     if (count == 0) return HL_B200_OK;
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     u64* d_out = nullptr;
     int rc = dev_alloc(c, (void**)&d_out, count * 8);
     if (!rc) rc = fill_dev(c, key32, first_word, count, as_fp, d_out);

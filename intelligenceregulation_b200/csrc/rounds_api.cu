@@ -128,8 +128,7 @@ struct GenAsk {  // a slot program's generated kernel, looked up by the caller
 
 int rounds_build(hl_ctx* c, int poly, size_t k, uint32_t n_vars, uint32_t degree, const uint64_t* tables, const uint64_t* coefs,
                  size_t ncoefs, const std::vector<u32>* plan, hl_rounds** out, hl_tables* built = nullptr, const GenAsk* gen = nullptr) {
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     if (built) {
         if (int rc = hl_tables_flush_locked(built)) return rc;
     }
@@ -289,8 +288,7 @@ int hl_b200_rounds_from_tables_ir(hl_ctx* c, uint32_t degree, hl_tables* t, cons
 void hl_b200_rounds_free(hl_rounds* r) {
     if (!r) return;
     hl_ctx* c = r->ctx;
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     free_rounds(r);
 }
 
@@ -298,8 +296,7 @@ int hl_b200_rounds_round(hl_rounds* r, uint32_t j, int eval_one, uint64_t* sums)
     if (!r || !sums) return HL_B200_ERR_ARG;
     hl_ctx* c = r->ctx;
     if (j != r->next || j >= r->n_vars) return fail(c, HL_B200_ERR_ARG, "rounds_round: round order (a round needs the preceding fold)");
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     int rc;
     {
         Timed t(c, HL_T_ROUNDS);
@@ -314,8 +311,7 @@ int hl_b200_rounds_fold(hl_rounds* r, const uint64_t rr[2]) {
     if (!r || !rr) return HL_B200_ERR_ARG;
     hl_ctx* c = r->ctx;
     if (r->next >= r->n_vars) return fail(c, HL_B200_ERR_ARG, "rounds_fold: every variable is already folded");
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     int rc = h2d(c, (char*)r->d_state + offsetof(hlk::ScState, r), rr, 16);
     if (!rc) {
         Timed t(c, HL_T_ROUNDS);
@@ -329,8 +325,7 @@ int hl_b200_rounds_finals(hl_rounds* r, uint64_t* out) {
     if (!r || !out) return HL_B200_ERR_ARG;
     hl_ctx* c = r->ctx;
     if (r->next != r->n_vars) return fail(c, HL_B200_ERR_ARG, "rounds_finals: finals need all folds");
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     int rc = HL_B200_OK;
     for (u32 t = 0; t < r->k && !rc; t++) rc = d2h(c, out + 2 * t, r->d_tables + 2 * (size_t)t * r->stride, 16);
     if (!rc) rc = sync(c, "rounds_finals");
@@ -351,8 +346,7 @@ int hl_b200_rounds_batched(hl_rounds* r, uint32_t nd, hl_fs_state* fs, const uin
     if (mask_coeffs && (r->next != 0 || !mask_c || mask_vars < r->n_vars || mask_vars > 63))
         return fail(c, HL_B200_ERR_ARG, "rounds_batched: a masked batch starts at round 0 and its mask covers every variable");
     if (fs->recover_one && r->degree < 1) return fail(c, HL_B200_ERR_ARG, "rounds_batched: claim recovery requires degree >= 1");
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     hlk::ScState st;
     memset(&st, 0, sizeof st);
     memcpy(st.state, fs->state, 32);

@@ -204,8 +204,7 @@ extern "C" {
 int hl_b200_tables_new(hl_ctx* c, size_t k, uint32_t n_vars, hl_tables** out) {
     if (!c || !out || k == 0) return fail(c, HL_B200_ERR_ARG, "tables_new: null argument or no table");
     if (n_vars > 30 || k > 64) return fail(c, HL_B200_ERR_UNSUPPORTED, "tables_new: more than 30 variables or 64 tables");
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     hl_tables* t = new hl_tables();
     t->ctx = c; t->k = (u32)k; t->n_vars = n_vars;
     int rc = dev_alloc(c, (void**)&t->d_tables, t->bytes());
@@ -227,8 +226,7 @@ int hl_b200_tables_new(hl_ctx* c, size_t k, uint32_t n_vars, hl_tables** out) {
 void hl_b200_tables_free(hl_tables* t) {
     if (!t) return;
     hl_ctx* c = t->ctx;
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     if (t->d_tables) dev_free(c, t->d_tables, t->bytes());
     dev_free(c, t->d_flag, 4);
     delete t;
@@ -237,8 +235,7 @@ void hl_b200_tables_free(hl_tables* t) {
 int hl_b200_tables_put(hl_tables* t, size_t i, const uint64_t* words) {
     if (!t || !words || !t->d_tables || i >= t->k) return HL_B200_ERR_ARG;
     hl_ctx* c = t->ctx;
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     if (int rc = launch_planned(t)) return rc;  // a planned table may be the one overwritten here: keep the caller's order
     return h2d_owned(c, t->d_tables + 2 * i * t->len(), words, t->len() * 16);
 }
@@ -307,16 +304,14 @@ int hl_b200_tables_plane(hl_tables* t, size_t i, const hl_store* store, const ui
 int hl_b200_tables_flush(hl_tables* t) {
     if (!t || !t->d_tables) return HL_B200_ERR_ARG;
     hl_ctx* c = t->ctx;
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     return hl_tables_flush_locked(t);
 }
 
 int hl_b200_tables_read(hl_tables* t, size_t i, uint64_t* out) {
     if (!t || !t->d_tables || i >= t->k || !out) return HL_B200_ERR_ARG;
     hl_ctx* c = t->ctx;
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     int rc = launch_planned(t);
     if (!rc) rc = d2h(c, out, t->d_tables + 2 * i * t->len(), t->len() * 16);
     if (!rc) rc = sync(c, "tables_read");

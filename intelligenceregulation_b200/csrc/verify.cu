@@ -186,8 +186,7 @@ extern "C" int hl_b200_verify_columns(hl_ctx* c, const uint64_t* cols, size_t ro
                                       const uint8_t* leaf_key32, const uint8_t* node_key32, const uint64_t* rhos, size_t k, const uint64_t* wants,
                                       const hl_store* vec_store, int32_t* verdict, int64_t* first_bad) {
     if (!c) return HL_B200_ERR_ARG;
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     return verify_columns_locked(c, cols, rows, ncols, idx, salts32, paths32, depth, root32, column_key32, leaf_key32, node_key32, rhos, k, wants, vec_store,
                                  verdict, first_bad);
 }
@@ -199,8 +198,7 @@ extern "C" int hl_b200_verify_opening(hl_ctx* c, uint32_t log_cols, uint32_t inv
     if (!c) return HL_B200_ERR_ARG;
     if (!pows || !vecs || k == 0 || q == 0) return fail(c, HL_B200_ERR_ARG, "verify_opening: null or empty argument");
     if (log_cols < 1 || log_cols > 16 || k > 0x7FFFu) return fail(c, HL_B200_ERR_ARG, "verify_opening: shape");
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     const size_t n = (size_t)1 << log_cols, nn = n * inv_rate, w = n + q;
     u64 *d_vecs = nullptr, *d_data = nullptr, *d_pads = nullptr, *d_pows = nullptr;
     hl_store* st = nullptr;

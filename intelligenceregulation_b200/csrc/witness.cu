@@ -366,8 +366,7 @@ int hl_b200_witness_product_dev(hl_ctx* c, size_t t_rows, const int64_t* d_x, si
     *taken = 0;
     if (!shape_fits(t_rows, x_len, xs, w_len, inner, outer, os, out_len)) return HL_B200_OK;
     if (!d_x || !d_w || !d_out) return fail(c, HL_B200_ERR_ARG, "witness_product: null argument");
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     return product_on_device(c, t_rows, d_x, xs, d_w, inner, outer, os, out_len, in_out, d_out, taken);
 }
 
@@ -377,8 +376,7 @@ int hl_b200_witness_product(hl_ctx* c, size_t t_rows, const int64_t* x, size_t x
     *taken = 0;
     if (!shape_fits(t_rows, x_len, xs, w_len, inner, outer, os, out_len)) return HL_B200_OK;
     if (!x || !w || !out) return fail(c, HL_B200_ERR_ARG, "witness_product: null argument");
-    std::lock_guard<std::mutex> g(c->mu);
-    cudaSetDevice(c->device);
+    Call g(c);
     const size_t xb = ((t_rows - 1) * xs + inner) * 8, wb = inner * outer, ob = out_len * 8;
     int64_t *d_x = nullptr, *d_out = nullptr;
     int8_t* d_w = nullptr;
