@@ -245,7 +245,11 @@ int hl_b200_rng_fill_dev(hl_ctx* ctx, const uint8_t* key32, uint64_t first_word,
  *                  Every address the maps can form is checked against the rows before the launch.
  * base_check != 0 declares the table base-valued; tables_flush (and rounds_from_tables) answer
  * HL_B200_ERR_MISMATCH if a word of such a table has a non-zero imaginary part (metal.rs:2649-2665).
- * tables_eq and tables_plane PLAN a table (MetalTables::plan_eq / plan_plane): the maps are copied during the call, and every planned
+ * tables_eq_point and tables_plane_coords are the same two from what a caller has before it makes the maps: the point itself (p Fp2),
+ * and the plane's coordinates (argument.rs:486-512; the first is the most significant index bit): k >= 0 reads cube variable k, -1 - k
+ * reads it complemented, HL_COORD_FIXED takes the next Fp2 of `fixed` (at most 16 of them, at most 32 coordinates).  A cube variable
+ * outside the cube or read twice is HL_B200_ERR_ARG.  The library makes the eq halves on the device and the maps in the call.
+ * The eq and plane calls PLAN a table (MetalTables::plan_eq / plan_plane): the maps are copied during the call, and every planned
  * table is written by one launch when the set is flushed, read or handed to an evaluator.  The commitment (or the device rows) a
  * planned plane reads must still be there then; a freed store is refused at that point (HL_B200_ERR_ARG), nothing is launched.
  * rounds_from_tables[_ir] takes the set over on success (the handle stays valid but empty; free it). */
@@ -253,6 +257,10 @@ typedef struct hl_tables hl_tables;
 int hl_b200_tables_new(hl_ctx* ctx, size_t k, uint32_t n_vars, hl_tables** out);
 int hl_b200_tables_put(hl_tables* t, size_t i, const uint64_t* words);
 int hl_b200_tables_eq(hl_tables* t, size_t i, uint32_t start, uint32_t p, const uint64_t* hi, const uint64_t* lo, int base_check);
+#define HL_COORD_FIXED INT32_MIN
+int hl_b200_tables_eq_point(hl_tables* t, size_t i, uint32_t start, uint32_t p, const uint64_t* point, int base_check);
+int hl_b200_tables_plane_coords(hl_tables* t, size_t i, const hl_store* store, const uint64_t* d_rows, size_t n_words, const int32_t* coords,
+                                uint32_t n_coords, const uint64_t* fixed, const uint64_t* slices, uint32_t ns, int base_check);
 int hl_b200_tables_plane(hl_tables* t, size_t i, const hl_store* store, const uint64_t* d_rows, size_t n_words, uint64_t used,
                          uint32_t xlo, const uint32_t* inv_lo, const uint32_t* inv_hi, const uint32_t* zbits, uint32_t nz,
                          const uint64_t* eqf, const uint64_t* slices, uint32_t ns, int base_check);

@@ -76,6 +76,8 @@ SIGNATURES.update({
     "hl_b200_tables_put": (_int, [_vp, _sz, _vp]),
     "hl_b200_tables_eq": (_int, [_vp, _sz, _u32, _u32, _vp, _vp, _int]),
     "hl_b200_tables_plane": (_int, [_vp, _sz, _vp, _vp, _sz, _u64, _u32, _vp, _vp, _vp, _u32, _vp, _vp, _u32, _int]),
+    "hl_b200_tables_eq_point": (_int, [_vp, _sz, _u32, _u32, _vp, _int]),
+    "hl_b200_tables_plane_coords": (_int, [_vp, _sz, _vp, _vp, _sz, _vp, _u32, _vp, _vp, _u32, _int]),
     "hl_b200_tables_flush": (_int, [_vp]),
     "hl_b200_tables_read": (_int, [_vp, _sz, _vp]),
     "hl_b200_tables_free": (None, [_vp]),

@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import struct
 from typing import List, Optional, Tuple
 
 import numpy as np
@@ -19,15 +20,14 @@ import numpy as np
 from . import _lib, _results
 
 
-def _ptr(a) -> C.c_void_p:
-    if a is None:
-        return C.c_void_p(0)
-    if isinstance(a, (bytes, bytearray)):
-        return C.cast(C.create_string_buffer(bytes(a), len(a)), C.c_void_p)
-    if isinstance(a, int):
-        return C.c_void_p(a)
-    assert a.flags["C_CONTIGUOUS"]
-    return C.c_void_p(a.ctypes.data)
+def _ptr(a):
+    """what ctypes takes for a `void*`: an array's address, a device address or bytes as they are, or None"""
+    if a is None or isinstance(a, (int, bytes)):
+        return a
+    if isinstance(a, bytearray):
+        return bytes(a)
+    assert a.flags.c_contiguous
+    return a.__array_interface__["data"][0]
 
 
 def _u64(a) -> np.ndarray:
@@ -597,10 +597,13 @@ def plane_maps(n_vars: int, coords):
     return used, xlo, inv_lo, inv_hi, zbits, eqf
 
 
+_COORD_FIXED = -(1 << 31)  # HL_COORD_FIXED
+
+
 class B200Tables:
     """A slot's tables built on the device: the mirror of the reference's `MetalTables` (gpu/metal.rs: `new`, `tables_mut`,
-    `plan_eq`, `plan_plane`, `build_planned` / `flush`, `to_vecs`).  The index maps of a plane are made here, on the host,
-    exactly as the host builder makes them (private_block/argument.rs:486-512); the kernels only read them."""
+    `plan_eq`, `plan_plane`, `build_planned` / `flush`, `to_vecs`).  The index maps of a plane (private_block/argument.rs:486-512;
+    `plane_maps` above is the same in numpy) and the eq halves are made by the library."""
 
     def __init__(self, ctx: Context, k: int, n_vars: int):
         self.ctx, self.k, self.n_vars = ctx, k, n_vars
@@ -616,22 +619,27 @@ class B200Tables:
     def plan_eq(self, i: int, point, start: int, base_check: bool = False) -> None:
         """`Tab::Eq { point, start }`: eq(point, x[start .. start + |point|]) (argument.rs:643-660)"""
         point = _u64(point).reshape(-1, 2)
-        p = point.shape[0]
-        p_lo = p // 2
-        hi, lo = eq_table_msb(point[: p - p_lo]), eq_table_msb(point[p - p_lo:])
-        self.ctx.check(self.ctx.lib.hl_b200_tables_eq(self.h, i, start, p, _ptr(hi), _ptr(lo), 1 if base_check else 0))
+        self.ctx.check(self.ctx.lib.hl_b200_tables_eq_point(self.h, i, start, point.shape[0], _ptr(point), 1 if base_check else 0))
 
     def plan_plane(self, i: int, rows, coords, slices, base_check: bool = False) -> None:
         """`Tab::Priv`: a committed plane (argument.rs:386-577).  `rows`: a `B200Commit` (its resident data rows) or a
         (device address, word count) pair; `coords`: the plane's coordinates, first = most significant index bit, each
         ("rho", k) | ("flip", k) | ("fixed", (c0, c1)); `slices`: [(word offset, (c0, c1))]."""
-        used, xlo, inv_lo, inv_hi, zbits, eqf = plane_maps(self.n_vars, coords)
-        nz = zbits.size
-        sl = np.array([[off, cf[0], cf[1]] for off, cf in slices], dtype=np.uint64)
-        store, d_rows, n_words = (rows.h, None, 0) if isinstance(rows, B200Commit) else (None, C.c_void_p(rows[0]), rows[1])
-        self.ctx.check(self.ctx.lib.hl_b200_tables_plane(self.h, i, store, d_rows, n_words, used, xlo, _ptr(inv_lo), _ptr(inv_hi),
-                                                         _ptr(zbits) if nz else None, nz, _ptr(eqf) if nz else None, _ptr(sl), sl.shape[0],
-                                                         1 if base_check else 0))
+        codes, fixed, read = [], [], []
+        for c in coords:
+            if c[0] == "fixed":
+                codes.append(_COORD_FIXED)
+                fixed += c[1]
+            else:
+                read.append(c[1])
+                codes.append(-1 - c[1] if c[0] == "flip" else c[1])
+        if len(set(read)) != len(read):
+            raise ValueError("plane_maps: a cube variable read by two coordinates (the host builder accumulates; not planned)")
+        sl = [int(v) for off, cf in slices for v in (off, cf[0], cf[1])]
+        store, d_rows, n_words = (rows.h, None, 0) if isinstance(rows, B200Commit) else (None, rows[0], rows[1])
+        self.ctx.check(self.ctx.lib.hl_b200_tables_plane_coords(self.h, i, store, d_rows, n_words, struct.pack(f"{len(codes)}i", *codes), len(codes),
+                                                                struct.pack(f"{len(fixed)}Q", *map(int, fixed)) if fixed else None,
+                                                                struct.pack(f"{len(sl)}Q", *sl), len(sl) // 3, 1 if base_check else 0))
 
     def flush(self) -> None:
         self.ctx.check(self.ctx.lib.hl_b200_tables_flush(self.h))
@@ -664,6 +672,7 @@ class SlotProgram:
         self._words: List[int] = []
         self.n_nodes = 0
         self.n_terms = 0
+        self._flat = None
 
     @staticmethod
     def node(node_id: int) -> int:
@@ -712,11 +721,18 @@ class SlotProgram:
         self._product(coef, list(wrapper) + list(inner))
         self.n_terms += 1
 
+    def _arrays(self):
+        """(words, coefficients) as the C ABI takes them; a program only grows, so its sizes tell whether they still hold"""
+        now = (len(self._words), len(self.coefs))
+        if self._flat is None or self._flat[0] != now:
+            self._flat = now, np.array(self._words, dtype=np.uint32), np.array(self.coefs, dtype=np.uint64).reshape(-1, 2)
+        return self._flat[1:]
+
     def words(self) -> np.ndarray:
-        return np.array(self._words, dtype=np.uint32)
+        return self._arrays()[0].copy()
 
     def coef_array(self) -> np.ndarray:
-        return np.array(self.coefs, dtype=np.uint64).reshape(-1, 2)
+        return self._arrays()[1].copy()
 
 
 class B200Rounds:
@@ -731,8 +747,8 @@ class B200Rounds:
         if isinstance(tables, B200Tables):
             self.ctx, self.k, self._n_vars = ctx, tables.k, tables.n_vars
             if isinstance(poly, SlotProgram):
-                w, cf = poly.words(), poly.coef_array()
-                ctx.check(ctx.lib.hl_b200_rounds_from_tables_ir(ctx.h, degree, tables.h, w.ctypes.data_as(C.c_void_p), w.size, poly.n_nodes,
+                w, cf = poly._arrays()
+                ctx.check(ctx.lib.hl_b200_rounds_from_tables_ir(ctx.h, degree, tables.h, _ptr(w), w.size, poly.n_nodes,
                                                                 poly.n_terms, _ptr(cf) if cf.size else None, cf.shape[0], C.byref(h)))
             else:
                 cf = _u64(coefs).reshape(-1, 2) if coefs is not None else None
@@ -747,8 +763,8 @@ class B200Rounds:
         assert tables.shape[1] == 1 << self._n_vars
         if isinstance(poly, SlotProgram):
             assert poly.n_tables == self.k
-            w, cf = poly.words(), poly.coef_array()
-            ctx.check(ctx.lib.hl_b200_rounds_new_ir(ctx.h, self.k, self._n_vars, degree, _ptr(tables), w.ctypes.data_as(C.c_void_p), w.size,
+            w, cf = poly._arrays()
+            ctx.check(ctx.lib.hl_b200_rounds_new_ir(ctx.h, self.k, self._n_vars, degree, _ptr(tables), _ptr(w), w.size,
                                                     poly.n_nodes, poly.n_terms, _ptr(cf) if cf.size else None, cf.shape[0], C.byref(h)))
         else:
             cf = _u64(coefs).reshape(-1, 2) if coefs is not None else None

@@ -23,11 +23,18 @@ struct hl_rounds {
     size_t stride = 0, len = 0, ncoefs = 0;
     u32 max_blocks = 0;
     u64* d_tables = nullptr;
+    // one device block of everything else: [inverse denominators, extrapolation weights, coefficients, plan] as uploaded at the start,
+    // then [mask rows and table | state] as uploaded by a batch (the mask ends where the state begins), then [rows of the output,
+    // finals], which a batch reads back together with the state, then the CTA partials
+    char* blk = nullptr;
+    size_t blk_bytes = 0, mask_cap = 0;
     u64* d_coefs = nullptr;
     u64* d_partials = nullptr;
     u64* d_out = nullptr;      // n_vars rows of (2 (degree+1) + 1) Fp2
+    u64* d_finals = nullptr;   // k Fp2 behind them
     u64* d_inv_den = nullptr;
     u64* d_extrap = nullptr;   // weights of the points above the evaluated degree (data-form polynomials only)
+    std::vector<u64> finals;   // the finals, once a batch has brought them along with its last round
     u32 eval_degree = 0;
     hlk::ScState* d_state = nullptr;
     hlk::IrDev ir{};           // poly == POLY_IR: the polynomial as data
@@ -44,16 +51,9 @@ namespace {
 void free_rounds(hl_rounds* r) {
     hl_ctx* c = r->ctx;
     if (r->d_tables) dev_free(c, r->d_tables, r->k * r->stride * 16);
-    dev_free(c, r->d_coefs, (r->ncoefs ? r->ncoefs : 1) * 16);
-    dev_free(c, r->d_partials, (size_t)r->max_blocks * (r->degree + 1) * 16);
-    dev_free(c, r->d_out, (r->n_vars ? r->n_vars : 1) * r->out_row() * 8);
-    dev_free(c, r->d_inv_den, ((size_t)r->degree + 1) * 8);
-    if (r->d_extrap) dev_free(c, r->d_extrap, (size_t)hlk::SC_MAX_POINTS * hlk::SC_MAX_POINTS * 8);
-    dev_free(c, r->d_state, sizeof(hlk::ScState));
+    dev_free(c, r->blk, r->blk_bytes);
     if (r->d_cfo) dev_free(c, r->d_cfo, (size_t)(r->gen ? r->gen->n_cfo : 1) * 16);
     if (r->d_nonbase) dev_free(c, r->d_nonbase, 8);
-    if (r->ir.plan) dev_free(c, (void*)r->ir.plan, (size_t)r->ir.plan_words * 4);
-    if (r->ir.coefs) dev_free(c, (void*)r->ir.coefs, (size_t)(r->ir.n_coefs ? r->ir.n_coefs : 1) * 16);
     delete r;
 }
 
@@ -150,25 +150,28 @@ int rounds_build(hl_ctx* c, int poly, size_t k, uint32_t n_vars, uint32_t degree
         r->max_blocks = hlk::sc_ir_max_blocks((u32)(r->len / 2), c->sm_count);
         r->tail_len = hlk::sc_ir_tail_len(r->ir, (int)degree);
     }
-    u64 inv_den[hlk::SC_MAX_POINTS];
-    for (u32 i = 0; i <= degree; i++) {
-        u64 den = 1;
-        for (u32 j = 0; j <= degree; j++)
-            if (j != i) den = gl_mul(den, gl_from_i64((long long)i - (long long)j));
-        inv_den[i] = gl_inv(den);
+    // what the kernels read and no challenge changes, in one upload
+    std::vector<char> head;
+    auto put = [&](size_t bytes) {
+        const size_t at = head.size();
+        head.resize((at + bytes + 15) & ~(size_t)15, 0);
+        return at;
+    };
+    const size_t at_den = put(((size_t)degree + 1) * 8);
+    {
+        u64* inv_den = reinterpret_cast<u64*>(head.data() + at_den);
+        for (u32 i = 0; i <= degree; i++) {
+            u64 den = 1;
+            for (u32 j = 0; j <= degree; j++)
+                if (j != i) den = gl_mul(den, gl_from_i64((long long)i - (long long)j));
+            inv_den[i] = gl_inv(den);
+        }
     }
-    int rc = built ? HL_B200_OK : dev_alloc(c, (void**)&r->d_tables, k * r->stride * 16);
-    if (!rc) rc = dev_alloc(c, (void**)&r->d_coefs, (ncoefs ? ncoefs : 1) * 16);
-    if (!rc) rc = dev_alloc(c, (void**)&r->d_partials, (size_t)r->max_blocks * (degree + 1) * 16);
-    if (!rc) rc = dev_alloc(c, (void**)&r->d_out, (n_vars ? n_vars : 1) * r->out_row() * 8);
-    if (!rc) rc = dev_alloc(c, (void**)&r->d_inv_den, ((size_t)degree + 1) * 8);
-    if (!rc) rc = dev_alloc(c, (void**)&r->d_state, sizeof(hlk::ScState));
-    if (!rc && !built) rc = h2d(c, r->d_tables, tables, k * r->stride * 16);
-    if (!rc && ncoefs) rc = h2d(c, r->d_coefs, coefs, ncoefs * 16);
-    if (!rc) rc = h2d(c, r->d_inv_den, inv_den, ((size_t)degree + 1) * 8);
-    if (!rc && r->eval_degree < degree) {
+    const bool extrapolates = r->eval_degree < degree;
+    const size_t at_ex = extrapolates ? put((size_t)hlk::SC_MAX_POINTS * hlk::SC_MAX_POINTS * 8) : 0;
+    if (extrapolates) {
         // s(p) = sum_i s(i) prod_{j != i} (p - j) / (i - j) over i, j <= eval_degree, for p above it
-        u64 wts[hlk::SC_MAX_POINTS * hlk::SC_MAX_POINTS] = {0};
+        u64* wts = reinterpret_cast<u64*>(head.data() + at_ex);
         const u32 de = r->eval_degree;
         for (u32 pnt = de + 1; pnt <= degree; pnt++)
             for (u32 i = 0; i <= de; i++) {
@@ -180,15 +183,30 @@ int rounds_build(hl_ctx* c, int poly, size_t k, uint32_t n_vars, uint32_t degree
                     }
                 wts[(pnt - de - 1) * (de + 1) + i] = gl_mul(num, gl_inv(den));
             }
-        rc = dev_alloc(c, (void**)&r->d_extrap, sizeof wts);
-        if (!rc) rc = h2d(c, r->d_extrap, wts, sizeof wts);
     }
-    if (!rc && poly == hlk::POLY_IR) {
-        rc = dev_alloc(c, (void**)&r->ir.plan, (size_t)r->ir.plan_words * 4);
-        if (!rc) rc = dev_alloc(c, (void**)&r->ir.coefs, (size_t)(ncoefs ? ncoefs : 1) * 16);
-        if (!rc) rc = h2d(c, (void*)r->ir.plan, plan->data(), (size_t)r->ir.plan_words * 4);
-        if (!rc && ncoefs) rc = h2d(c, (void*)r->ir.coefs, coefs, ncoefs * 16);
+    const size_t at_cf = put((ncoefs ? ncoefs : 1) * 16);
+    if (ncoefs) memcpy(head.data() + at_cf, coefs, ncoefs * 16);
+    const bool is_ir = poly == hlk::POLY_IR;
+    const size_t at_plan = is_ir ? put((size_t)r->ir.plan_words * 4) : 0;
+    if (is_ir) memcpy(head.data() + at_plan, plan->data(), (size_t)r->ir.plan_words * 4);
+    r->mask_cap = ((size_t)63 * degree + 2) * 16 + (size_t)63 * (degree + 1) * 16;
+    const size_t at_state = head.size() + r->mask_cap, state_bytes = (sizeof(hlk::ScState) + 15) & ~(size_t)15;
+    const size_t at_out = at_state + state_bytes, at_fin = at_out + (n_vars ? n_vars : 1) * r->out_row() * 8, at_part = at_fin + k * 16;
+    r->blk_bytes = at_part + (size_t)r->max_blocks * (degree + 1) * 16;
+    int rc = built ? HL_B200_OK : dev_alloc(c, (void**)&r->d_tables, k * r->stride * 16);
+    if (!rc) rc = dev_alloc(c, (void**)&r->blk, r->blk_bytes);
+    if (!rc) {
+        r->d_inv_den = (u64*)(r->blk + at_den);
+        r->d_extrap = extrapolates ? (u64*)(r->blk + at_ex) : nullptr;
+        r->d_coefs = (u64*)(r->blk + at_cf);
+        if (is_ir) { r->ir.plan = (const u32*)(r->blk + at_plan); r->ir.coefs = (const u64*)(r->blk + at_cf); }
+        r->d_state = (hlk::ScState*)(r->blk + at_state);
+        r->d_out = (u64*)(r->blk + at_out);
+        r->d_finals = (u64*)(r->blk + at_fin);
+        r->d_partials = (u64*)(r->blk + at_part);
     }
+    if (!rc && !built) rc = h2d_owned(c, r->d_tables, tables, k * r->stride * 16);
+    if (!rc) rc = h2d_owned(c, r->blk, head.data(), head.size());
     if (!rc) {
         cudaError_t e = cudaMemsetAsync(r->d_state, 0, sizeof(hlk::ScState), c->stream);
         if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "state clear", e);
@@ -208,8 +226,8 @@ int rounds_build(hl_ctx* c, int poly, size_t k, uint32_t n_vars, uint32_t degree
             if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "table typing launch", e);
         }
         if (!rc) rc = d2h(c, &r->nonbase, r->d_nonbase, 8);
+        if (!rc) rc = sync(c, "rounds_new");
     }
-    if (!rc) rc = sync(c, "rounds_new");
     if (rc) { cudaStreamSynchronize(c->stream); free_rounds(r); return rc; }
     if (built) r->d_tables = hl_tables_adopt(built);  // only now: a failed build leaves the set with its owner
     *out = r;
@@ -326,10 +344,17 @@ int hl_b200_rounds_finals(hl_rounds* r, uint64_t* out) {
     hl_ctx* c = r->ctx;
     if (r->next != r->n_vars) return fail(c, HL_B200_ERR_ARG, "rounds_finals: finals need all folds");
     Call g(c);
-    int rc = HL_B200_OK;
-    for (u32 t = 0; t < r->k && !rc; t++) rc = d2h(c, out + 2 * t, r->d_tables + 2 * (size_t)t * r->stride, 16);
-    if (!rc) rc = sync(c, "rounds_finals");
-    return rc;
+    if (r->finals.empty()) {
+        std::vector<u64> got(2 * (size_t)r->k);
+        cudaError_t e = hlk::sc_finals(r->d_tables, r->stride, r->k, r->d_finals, c->stream);
+        c->stats.kernel_launches++;
+        int rc = e == cudaSuccess ? d2h(c, got.data(), r->d_finals, got.size() * 8) : fail(c, HL_B200_ERR_DEVICE, "finals launch", e);
+        if (!rc) rc = sync(c, "rounds_finals");
+        if (rc) return rc;
+        r->finals.swap(got);
+    }
+    memcpy(out, r->finals.data(), r->finals.size() * 8);
+    return HL_B200_OK;
 }
 
 int hl_b200_set_dependent_launch(int on) {
@@ -356,8 +381,8 @@ int hl_b200_rounds_batched(hl_rounds* r, uint32_t nd, hl_fs_state* fs, const uin
     st.claim = f2(fs->claim[0], fs->claim[1]);
     u64 *d_mask = nullptr, *d_mtab = nullptr;
     const size_t mlen = mask_coeffs ? (size_t)mask_vars * r->degree + 2 : 0;
-    const size_t tab_words = (size_t)mask_vars * (r->degree + 1) * 2;
-    std::vector<u64> mtab;
+    const size_t tab_words = mask_coeffs ? (size_t)mask_vars * (r->degree + 1) * 2 : 0;
+    std::vector<u64> up(mlen * 2 + tab_words + (sizeof st + 7) / 8);  // mask, its table, state: one upload that ends with the state
     int rc = HL_B200_OK;
     if (mask_coeffs) {
         st.mask_c = f2(mask_c[0], mask_c[1]);
@@ -365,7 +390,7 @@ int hl_b200_rounds_batched(hl_rounds* r, uint32_t nd, hl_fs_state* fs, const uin
         st.ap = co[1];  // a' times the empty product
         // per round j and point x: 2^(N-1-j) (a0 + sum_{i>j} u_i(1)/2 + u_j(x)) (sumcheck.rs:260-295): the part of g_j(x) no challenge enters
         const u64 half = gl_inv(2);
-        mtab.assign(tab_words, 0);
+        u64* const mtab = up.data() + mlen * 2;
         fp2 run = f2(0, 0);
         for (int i = (int)mask_vars - 1; i >= 0; i--) {
             const fp2* ai = co + 2 + (size_t)i * r->degree;
@@ -381,12 +406,12 @@ int hl_b200_rounds_batched(hl_rounds* r, uint32_t nd, hl_fs_state* fs, const uin
             for (u32 e = 0; e < r->degree; e++) u1 = f2_add(u1, ai[e]);
             run = f2_add(run, f2_mul_base(u1, half));
         }
-        rc = dev_alloc(c, (void**)&d_mask, mlen * 16);
-        if (!rc) rc = dev_alloc(c, (void**)&d_mtab, tab_words * 8);
-        if (!rc) rc = h2d(c, d_mask, mask_coeffs, mlen * 16);
-        if (!rc) rc = h2d(c, d_mtab, mtab.data(), tab_words * 8);
+        memcpy(up.data(), mask_coeffs, mlen * 16);
+        d_mask = (u64*)r->d_state - mlen * 2 - tab_words;
+        d_mtab = (u64*)r->d_state - tab_words;
     }
-    if (!rc) rc = h2d(c, r->d_state, &st, sizeof st);
+    memcpy(up.data() + mlen * 2 + tab_words, &st, sizeof st);
+    rc = h2d(c, (u64*)r->d_state - mlen * 2 - tab_words, up.data(), (mlen * 2 + tab_words) * 8 + sizeof st);
     const u32 first = r->next;
     bool have_claim = fs->recover_one && fs->have_claim;
     {
@@ -452,12 +477,23 @@ int hl_b200_rounds_batched(hl_rounds* r, uint32_t nd, hl_fs_state* fs, const uin
             r->next += left;
         }
     }
-    if (!rc) rc = d2h(c, out, r->d_out + (size_t)first * r->out_row(), (size_t)nd * r->out_row() * 8);
-    if (!rc) rc = d2h(c, &st, r->d_state, sizeof st);
+    const bool last = r->next == r->n_vars;
+    if (!rc && last) {  // the finals come along
+        cudaError_t e = hlk::sc_finals(r->d_tables, r->stride, r->k, r->d_finals, c->stream);
+        c->stats.kernel_launches++;
+        if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "finals launch", e);
+    }
+    const size_t o_out = (size_t)((char*)r->d_out - (char*)r->d_state), o_fin = (size_t)((char*)r->d_finals - (char*)r->d_state);
+    std::vector<char> got(o_fin + r->k * 16);
+    if (!rc) rc = d2h(c, got.data(), r->d_state, last ? got.size() : o_fin);
     if (!rc) rc = sync(c, "rounds_batched");
-    if (d_mask) dev_free(c, d_mask, mlen * 16);
-    if (d_mtab) dev_free(c, d_mtab, tab_words * 8);
     if (rc) return rc;
+    memcpy(out, got.data() + o_out + first * r->out_row() * 8, (size_t)nd * r->out_row() * 8);
+    memcpy(&st, got.data(), sizeof st);
+    if (last) {
+        r->finals.resize(2 * (size_t)r->k);
+        memcpy(r->finals.data(), got.data() + o_fin, r->k * 16);
+    }
     memcpy(fs->state, st.state, 32);
     fs->counter = st.counter;
     fs->claim[0] = st.claim.c0; fs->claim[1] = st.claim.c1;

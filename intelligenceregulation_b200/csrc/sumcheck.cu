@@ -453,6 +453,12 @@ __global__ void __launch_bounds__(TAIL_T) k_sc_tail(u64* __restrict__ tables, si
     }
 }
 
+// the first entry of every table, in a row: one read-back for all of them
+__global__ void __launch_bounds__(64) k_sc_finals(const u64* __restrict__ tables, size_t stride, u32 k, u64* __restrict__ out) {
+    chain_enter();
+    if (threadIdx.x < k) st2(out + 2 * threadIdx.x, ld2(tables + 2 * (size_t)threadIdx.x * stride));
+}
+
 // which tables are extension-valued: one CTA row per table, the second words OR-ed
 __global__ void __launch_bounds__(256) k_sc_nonbase(const u64* __restrict__ tables, size_t stride, size_t len, u64* __restrict__ mask) {
     const u32 t = blockIdx.y;
@@ -1095,6 +1101,10 @@ cudaError_t sc_nonbase_mask(const u64* tables, size_t stride, size_t len, u32 k,
     if (bx > cap) bx = cap;
     k_sc_nonbase<<<dim3((unsigned)bx, k), 256, 0, s>>>(tables, stride, len, d_mask);
     return cudaGetLastError();
+}
+
+cudaError_t sc_finals(const u64* d_tables, size_t stride, u32 k, u64* d_out, cudaStream_t st) {  // k <= 64
+    return chain_launch(k_sc_finals, dim3(1), dim3(64), 0, st, d_tables, stride, k, d_out);
 }
 
 cudaError_t sc_fold(u64* tables, size_t stride, u32 half, u32 k, const ScState* st, cudaStream_t s) {

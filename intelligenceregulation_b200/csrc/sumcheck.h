@@ -77,6 +77,8 @@ cudaError_t sc_tail(int poly, int k, u64* tables, size_t stride, u32 len, const 
                     int first_has_claim, u64* scratch, cudaStream_t s);
 // bit t of *d_mask is set when table t holds a non-zero second word anywhere in its first `len` entries (*d_mask zeroed by the caller)
 cudaError_t sc_nonbase_mask(const u64* tables, size_t stride, size_t len, u32 k, u64* d_mask, int sm_count, cudaStream_t s);
+// the first entry of every table, k Fp2 in a row
+cudaError_t sc_finals(const u64* d_tables, size_t stride, u32 k, u64* d_out, cudaStream_t st);
 cudaError_t sc_fold(u64* tables, size_t stride, u32 half, u32 k, const ScState* st, cudaStream_t s);
 
 }  // namespace hlk

@@ -29,6 +29,8 @@ struct TabDesc {
     u32 xlo, nz, ns;           // plane
     int one_slice, base_check;
     u64 used;
+    u32 ident, split2;         // plane: its index is x itself (under `used`); two slices with coefficients 1 and u, the two words of the entry
+    u64 off_pt;                // eq planned from its point: the point's place in the 64-bit pool (hi / lo are then computed on the device)
     u64 off_a, off_b;          // 64-bit pool: eq hi / lo, or plane eqf / slices
     u64 off_lo, off_hi, off_zb;  // 32-bit pool: plane inv_lo / inv_hi / zbits
     const u64* rows;           // plane: the committed data, flat
@@ -47,6 +49,10 @@ struct hl_tables {
     std::vector<TabDesc> plan;
     std::vector<u64> pool64;
     std::vector<u32> pool32;
+    u64 eq_words = 0;          // words of device-made eq halves, behind the 64-bit pool
+    u64 eq_most = 0;           // entries of the largest pair of them
+    u32 eq_points = 0;         // planned tables that have them
+    bool checked = false;      // a table was declared base-valued: the flush has to ask
     size_t len() const { return (size_t)1 << n_vars; }
     size_t bytes() const { return (size_t)k * len() * 16; }
 };
@@ -65,9 +71,8 @@ struct PlaneArgs {
     const u64* eqf;        // nz Fp2 (unused when nz == 0)
     const u64* slices;     // ns x (offset, c0, c1)
     u64 used;
-    u32 xlo, nz, ns;
+    u32 xlo, nz, ns, ident;
     int one_slice;         // one slice with coefficient 1
-    int base_check;
 };
 
 __device__ __forceinline__ fp2 plane_value(const PlaneArgs& a, size_t idx) {
@@ -82,7 +87,7 @@ __device__ __forceinline__ fp2 plane_value(const PlaneArgs& a, size_t idx) {
 
 __device__ __forceinline__ fp2 plane_entry(const PlaneArgs& a, size_t x) {
     const u64 xu = x & a.used;
-    const size_t im = (size_t)a.inv_hi[xu >> a.xlo] | a.inv_lo[xu & (((u64)1 << a.xlo) - 1)];
+    const size_t im = a.ident ? xu : (size_t)a.inv_hi[xu >> a.xlo] | a.inv_lo[xu & (((u64)1 << a.xlo) - 1)];
     if (a.nz == 0) return plane_value(a, im);
     if (a.one_slice) {
         // sum_z eqf[z] * word: the products are summed as integers and reduced once per component
@@ -105,36 +110,80 @@ __device__ __forceinline__ fp2 plane_entry(const PlaneArgs& a, size_t x) {
     return v;
 }
 
-// every planned table of a set in one launch: blockIdx.y = the plan entry, blockIdx.x over the table's entries
-__global__ void __launch_bounds__(256) k_tab_batch(u64* __restrict__ tables, size_t len, const TabDesc* __restrict__ descs, const u64* __restrict__ p64,
-                                                   const u32* __restrict__ p32, u32* __restrict__ flag) {
+// The two half tables of every eq cube planned from its point: entry e of a half over m coordinates is prod_j (bit ? r_j : 1 - r_j),
+// first coordinate = most significant bit.  A few thousand entries of some ten products each: 4 us on the device, where the host took
+// 80 us for a 2^21 cube and then had them to upload.
+__global__ void __launch_bounds__(128) k_tab_eq_halves(const TabDesc* __restrict__ descs, u32 n_desc, u64* __restrict__ p64) {
+    u32 seen = 0, t = 0;  // the blockIdx.y-th eq entry planned from a point
+    for (; t < n_desc; t++)
+        if (descs[t].kind == 0 && descs[t].off_pt != ~0ull && seen++ == blockIdx.y) break;
+    if (t == n_desc) return;
+    const TabDesc& d = descs[t];
+    const u32 p_hi = d.p - d.p_lo, n_hi = 1u << p_hi, e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= n_hi + (1u << d.p_lo)) return;
+    const bool hi = e < n_hi;
+    const u32 m = hi ? p_hi : d.p_lo, at = hi ? e : e - n_hi;
+    const u64* pt = p64 + d.off_pt + (hi ? 0 : 2 * (size_t)p_hi);
+    fp2 v = f2(1, 0);
+    for (u32 j = 0; j < m; j++) {
+        fp2 r = ld2(pt + 2 * j);
+        if (!((at >> (m - 1 - j)) & 1)) r = f2_sub(f2(1, 0), r);
+        v = f2_mul(v, r);
+    }
+    st2(p64 + (hi ? d.off_a : d.off_b) + 2 * (size_t)at, v);
+}
+
+// Every planned table of a set in one launch: blockIdx.y = the plan entry, blockIdx.x over spans of TAB_SPAN entries.  HBM is what it
+// has to wait for (16 bytes written per entry, 8 or 16 read), so a thread has its TAB_PER loads under way before its first store.
+constexpr u32 TAB_T = 256, TAB_PER = 4, TAB_SPAN = TAB_T * TAB_PER;
+__global__ void __launch_bounds__(TAB_T) k_tab_batch(u64* __restrict__ tables, size_t len, const TabDesc* __restrict__ descs, const u64* __restrict__ p64,
+                                                     const u32* __restrict__ p32, u32* __restrict__ flag) {
     __shared__ TabDesc d;
-    if (threadIdx.x == 0) d = descs[blockIdx.y];
+    if (threadIdx.x < sizeof(TabDesc) / 4) reinterpret_cast<u32*>(&d)[threadIdx.x] = reinterpret_cast<const u32*>(descs + blockIdx.y)[threadIdx.x];
     __syncthreads();
-    const size_t x = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= len) return;
-    fp2 v;
+    const size_t x0 = (size_t)blockIdx.x * TAB_SPAN + threadIdx.x;
+    u64* out = tables + 2 * (size_t)d.table * len;
+    u64 odd = 0;  // any second word, for a table declared base-valued
     if (d.kind == 0) {
-        const size_t y = (x >> d.shift) & (((size_t)1 << d.p) - 1);
-        v = f2_mul(ld2(p64 + d.off_a + 2 * (y >> d.p_lo)), ld2(p64 + d.off_b + 2 * (y & (((size_t)1 << d.p_lo) - 1))));
+        const u64 *hi = p64 + d.off_a, *lo = p64 + d.off_b;
+#pragma unroll
+        for (u32 k = 0; k < TAB_PER; k++) {
+            const size_t x = x0 + k * TAB_T;
+            if (x >= len) break;
+            const size_t y = (x >> d.shift) & (((size_t)1 << d.p) - 1);
+            const fp2 v = f2_mul(ld2(hi + 2 * (y >> d.p_lo)), ld2(lo + 2 * (y & (((size_t)1 << d.p_lo) - 1))));
+            st2(out + 2 * x, v);
+            odd |= v.c1;
+        }
+    } else if (d.ident && d.nz == 0 && (d.one_slice || d.split2)) {
+        const u64 *re = d.rows + p64[d.off_b], *im = d.split2 ? d.rows + p64[d.off_b + 3] : nullptr;
+        u64 a[TAB_PER], b[TAB_PER];
+#pragma unroll
+        for (u32 k = 0; k < TAB_PER; k++) {
+            const size_t x = x0 + k * TAB_T, at = x & d.used;
+            a[k] = x < len ? re[at] : 0;
+            b[k] = im && x < len ? im[at] : 0;
+        }
+#pragma unroll
+        for (u32 k = 0; k < TAB_PER; k++) {
+            const size_t x = x0 + k * TAB_T;
+            if (x >= len) break;
+            st2(out + 2 * x, f2(a[k], b[k]));
+            odd |= b[k];
+        }
     } else {
         PlaneArgs a;
         a.rows = d.rows; a.inv_lo = p32 + d.off_lo; a.inv_hi = p32 + d.off_hi; a.zbits = p32 + d.off_zb; a.eqf = p64 + d.off_a; a.slices = p64 + d.off_b;
-        a.used = d.used; a.xlo = d.xlo; a.nz = d.nz; a.ns = d.ns; a.one_slice = d.one_slice; a.base_check = d.base_check;
-        v = plane_entry(a, x);
+        a.used = d.used; a.xlo = d.xlo; a.nz = d.nz; a.ns = d.ns; a.one_slice = d.one_slice; a.ident = d.ident;
+        for (u32 k = 0; k < TAB_PER; k++) {
+            const size_t x = x0 + k * TAB_T;
+            if (x >= len) break;
+            const fp2 v = plane_entry(a, x);
+            st2(out + 2 * x, v);
+            odd |= v.c1;
+        }
     }
-    st2(tables + 2 * ((size_t)d.table * len + x), v);
-    if (d.base_check && v.c1 != 0) atomicOr(flag, 1u);
-}
-
-// uploads a small host array into a pool allocation; the caller frees it after the launch (stream-ordered)
-template <class T>
-int upload(hl_ctx* c, const void* h, size_t count, T** d) {
-    *d = nullptr;
-    if (count == 0) return HL_B200_OK;
-    int rc = dev_alloc(c, (void**)d, count * sizeof(T));
-    if (!rc) rc = h2d_owned(c, *d, h, count * sizeof(T));
-    return rc;
+    if (d.base_check && odd) atomicOr(flag, 1u);
 }
 
 }  // namespace
@@ -153,39 +202,56 @@ void hl_tables_shape(hl_tables* t, hl_ctx** c, size_t* k, uint32_t* n_vars) {
     *n_vars = t->n_vars;
 }
 
+static void drop_plan(hl_tables* t) {
+    t->plan.clear();
+    t->pool64.clear();
+    t->pool32.clear();
+    t->eq_words = t->eq_most = 0;
+    t->eq_points = 0;
+}
+
 // writes every planned table: one upload of the descriptors and the two pools, one launch; the caller holds the context's lock
 static int launch_planned(hl_tables* t) {
     if (t->plan.empty()) return HL_B200_OK;
     hl_ctx* c = t->ctx;
     for (const TabDesc& d : t->plan)
         if (d.kind == 1 && d.store && !c->stores.count(d.store)) {  // the rows are gone: nothing is launched over them
-            t->plan.clear(); t->pool64.clear(); t->pool32.clear();
+            drop_plan(t);
             return fail(c, HL_B200_ERR_ARG, "tables: a planned plane's commitment was freed before the set was built");
         }
-    TabDesc* d_desc = nullptr;
-    u64* d_p64 = nullptr;
-    u32* d_p32 = nullptr;
-    const size_t nd = t->plan.size(), n64 = t->pool64.size(), n32 = t->pool32.size();
+    if (t->pool64.size() & 1) t->pool64.push_back(0);
+    for (TabDesc& d : t->plan)
+        if (d.kind == 0 && d.off_pt != ~0ull) { d.off_a += t->pool64.size(); d.off_b += t->pool64.size(); }  // the halves lie behind the pool
+    // one block: descriptors, the 32-bit pool, the 64-bit pool, then the eq halves; the first three in one upload
+    const size_t nd = t->plan.size(), b_desc = (nd * sizeof(TabDesc) + 15) & ~(size_t)15, b32 = (t->pool32.size() * 4 + 15) & ~(size_t)15,
+                 b64 = t->pool64.size() * 8, up = b_desc + b32 + b64, total = up + t->eq_words * 8;
+    std::vector<char> h(up);
+    memcpy(h.data(), t->plan.data(), nd * sizeof(TabDesc));
+    if (b32) memcpy(h.data() + b_desc, t->pool32.data(), t->pool32.size() * 4);
+    if (b64) memcpy(h.data() + b_desc + b32, t->pool64.data(), b64);
+    char* blk = nullptr;
     int rc;
     {
         Timed tm(c, HL_T_TABLES);  // the span takes the maps' upload with it: it is part of what building the tables costs
-        rc = upload(c, t->plan.data(), nd, &d_desc);
-        if (!rc) rc = upload(c, t->pool64.data(), n64, &d_p64);
-        if (!rc) rc = upload(c, t->pool32.data(), n32, &d_p32);
+        rc = dev_alloc(c, (void**)&blk, total);
+        if (!rc) rc = h2d_owned(c, blk, h.data(), up);
         if (!rc) {
+            const TabDesc* d_desc = (const TabDesc*)blk;
+            const u32* d_p32 = (const u32*)(blk + b_desc);
+            u64* d_p64 = (u64*)(blk + b_desc + b32);
             const size_t len = t->len();
-            k_tab_batch<<<dim3((unsigned)((len + 255) / 256), (unsigned)nd), 256, 0, c->stream>>>(t->d_tables, len, d_desc, d_p64, d_p32, t->d_flag);
+            if (t->eq_points) {
+                k_tab_eq_halves<<<dim3((unsigned)((t->eq_most + 127) / 128), t->eq_points), 128, 0, c->stream>>>(d_desc, (u32)nd, d_p64);
+                c->stats.kernel_launches++;
+            }
+            k_tab_batch<<<dim3((unsigned)((len + TAB_SPAN - 1) / TAB_SPAN), (unsigned)nd), TAB_T, 0, c->stream>>>(t->d_tables, len, d_desc, d_p64, d_p32, t->d_flag);
             c->stats.kernel_launches++;
             cudaError_t e = cudaGetLastError();
             if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "planned tables launch", e);
         }
     }
-    if (d_desc) dev_free(c, d_desc, nd * sizeof(TabDesc));
-    if (d_p64) dev_free(c, d_p64, n64 * 8);
-    if (d_p32) dev_free(c, d_p32, n32 * 4);
-    t->plan.clear();
-    t->pool64.clear();
-    t->pool32.clear();
+    if (blk) dev_free(c, blk, total);
+    drop_plan(t);
     return rc;
 }
 
@@ -193,10 +259,55 @@ int hl_tables_flush_locked(hl_tables* t) {
     hl_ctx* c = t->ctx;
     u32 flag = 0;
     int rc = launch_planned(t);
+    if (!t->checked) return rc;
     if (!rc) rc = d2h(c, &flag, t->d_flag, 4);
     if (!rc) rc = sync(c, "tables_flush");
     if (!rc && flag) rc = fail(c, HL_B200_ERR_MISMATCH, "tables: a table declared base-valued holds an extension word");
     return rc;
+}
+
+static TabDesc eq_desc(hl_tables* t, size_t i, u32 start, u32 p, int base_check) {
+    TabDesc d;
+    memset(&d, 0, sizeof d);
+    d.kind = 0; d.table = (u32)i; d.shift = t->n_vars - start - p; d.p = p; d.p_lo = p / 2; d.base_check = base_check; d.off_pt = ~0ull;
+    t->checked |= base_check != 0;
+    return d;
+}
+
+// A plane's descriptor without its maps; `all`: the OR of everything its index can be.  Every address the kernel can form stays inside
+// the rows: the index is an OR of map entries.
+static int plane_desc(hl_tables* t, size_t i, const hl_store* store, const uint64_t* d_rows, size_t n_words, u64 all, const uint64_t* slices, u32 ns, int base_check,
+                      TabDesc* d) {
+    hl_ctx* c = t->ctx;
+    if (store) {
+        if (store->ctx != c) return fail(c, HL_B200_ERR_ARG, "tables_plane: the commitment belongs to another context");
+        d_rows = reinterpret_cast<const uint64_t*>(store->d_data);
+        n_words = (size_t)store->rows * store->n();
+    }
+    if (!d_rows) return fail(c, HL_B200_ERR_ARG, "tables_plane: no rows");
+    u64 max_off = 0;
+    for (u32 s = 0; s < ns; s++) max_off = slices[3 * (size_t)s] > max_off ? slices[3 * (size_t)s] : max_off;
+    if (max_off >= n_words || all >= n_words - max_off) return fail(c, HL_B200_ERR_ARG, "tables_plane: a slice reaches past the committed rows");
+    memset(d, 0, sizeof *d);
+    d->kind = 1; d->table = (u32)i; d->ns = ns; d->base_check = base_check; d->off_pt = ~0ull;
+    d->one_slice = ns == 1 && slices[1] == 1 && slices[2] == 0;
+    d->split2 = ns == 2 && slices[1] == 1 && slices[2] == 0 && slices[4] == 0 && slices[5] == 1;
+    d->rows = reinterpret_cast<const u64*>(d_rows);
+    d->store = store;
+    t->checked |= base_check != 0;
+    return HL_B200_OK;
+}
+
+static void plane_pools(hl_tables* t, TabDesc* d, const uint32_t* zbits, const uint64_t* eqf, const uint64_t* slices) {
+    d->off_zb = t->pool32.size();
+    if (d->nz) t->pool32.insert(t->pool32.end(), zbits, zbits + d->nz);
+    if (t->pool64.size() & 1) t->pool64.push_back(0);  // every 64-bit array read as Fp2 starts on a 16-byte boundary
+    d->off_a = t->pool64.size();
+    if (d->nz) t->pool64.insert(t->pool64.end(), eqf, eqf + (size_t)d->nz * 2);
+    d->off_b = t->pool64.size();
+    t->pool64.insert(t->pool64.end(), slices, slices + (size_t)d->ns * 3);
+    if (t->pool64.size() & 1) t->pool64.push_back(0);
+    t->plan.push_back(*d);
 }
 
 extern "C" {
@@ -244,16 +355,31 @@ int hl_b200_tables_eq(hl_tables* t, size_t i, uint32_t start, uint32_t p, const 
     if (!t || !t->d_tables || i >= t->k || !hi || !lo) return HL_B200_ERR_ARG;
     hl_ctx* c = t->ctx;
     if (start + p > t->n_vars) return fail(c, HL_B200_ERR_ARG, "tables_eq: start + |point| exceeds the cube");  // argument.rs:604-607
-    const u32 p_lo = p / 2, shift = t->n_vars - start - p;
     std::lock_guard<std::mutex> g(c->mu);
-    const size_t nhi = (size_t)2 << (p - p_lo), nlo = (size_t)2 << p_lo;
-    TabDesc d;
-    memset(&d, 0, sizeof d);
-    d.kind = 0; d.table = (u32)i; d.shift = shift; d.p = p; d.p_lo = p_lo; d.base_check = base_check;
+    TabDesc d = eq_desc(t, i, start, p, base_check);
     d.off_a = t->pool64.size();
-    t->pool64.insert(t->pool64.end(), hi, hi + nhi);
+    t->pool64.insert(t->pool64.end(), hi, hi + ((size_t)2 << (p - d.p_lo)));
     d.off_b = t->pool64.size();
-    t->pool64.insert(t->pool64.end(), lo, lo + nlo);
+    t->pool64.insert(t->pool64.end(), lo, lo + ((size_t)2 << d.p_lo));
+    t->plan.push_back(d);
+    return HL_B200_OK;
+}
+
+int hl_b200_tables_eq_point(hl_tables* t, size_t i, uint32_t start, uint32_t p, const uint64_t* point, int base_check) {
+    if (!t || !t->d_tables || i >= t->k || (p && !point)) return HL_B200_ERR_ARG;
+    hl_ctx* c = t->ctx;
+    if (start + p > t->n_vars) return fail(c, HL_B200_ERR_ARG, "tables_eq_point: start + |point| exceeds the cube");
+    std::lock_guard<std::mutex> g(c->mu);
+    TabDesc d = eq_desc(t, i, start, p, base_check);
+    if (t->pool64.size() & 1) t->pool64.push_back(0);
+    d.off_pt = t->pool64.size();
+    if (p) t->pool64.insert(t->pool64.end(), point, point + 2 * (size_t)p);
+    const u64 n_hi = (u64)1 << (p - d.p_lo), n_lo = (u64)1 << d.p_lo;
+    d.off_a = t->eq_words;  // from the end of the pool, whose size is known at the launch
+    d.off_b = t->eq_words + 2 * n_hi;
+    t->eq_words += 2 * (n_hi + n_lo);
+    if (n_hi + n_lo > t->eq_most) t->eq_most = n_hi + n_lo;
+    t->eq_points++;
     t->plan.push_back(d);
     return HL_B200_OK;
 }
@@ -263,41 +389,91 @@ int hl_b200_tables_plane(hl_tables* t, size_t i, const hl_store* store, const ui
                          const uint64_t* slices, uint32_t ns, int base_check) {
     if (!t || !t->d_tables || i >= t->k || !inv_lo || !inv_hi || !slices || ns == 0) return HL_B200_ERR_ARG;
     hl_ctx* c = t->ctx;
-    if (store) {
-        if (store->ctx != c) return fail(c, HL_B200_ERR_ARG, "tables_plane: the commitment belongs to another context");
-        d_rows = reinterpret_cast<const uint64_t*>(store->d_data);
-        n_words = (size_t)store->rows * store->n();
-    }
-    if (!d_rows) return fail(c, HL_B200_ERR_ARG, "tables_plane: no rows");
     if (nz && (!zbits || !eqf)) return fail(c, HL_B200_ERR_ARG, "tables_plane: fixed coordinates without their maps");
     if (xlo > t->n_vars || t->n_vars - xlo > 24 || xlo > 24 || nz > (1u << 16)) return fail(c, HL_B200_ERR_UNSUPPORTED, "tables_plane: map sizes");
-    // every address the kernel can form stays inside the rows: the index is an OR of map entries
     const size_t nlo = (size_t)1 << xlo, nhi = (size_t)1 << (t->n_vars - xlo);
-    u64 all = 0, max_off = 0;
-    for (size_t j = 0; j < nlo; j++) all |= inv_lo[j];
-    for (size_t j = 0; j < nhi; j++) all |= inv_hi[j];
+    u64 all = 0;
+    bool ident = true;  // on the entries that `used` lets through, the map is the index itself: the kernel then needs no map
+    for (size_t j = 0; j < nlo; j++) { all |= inv_lo[j]; ident &= (j & ~used) || inv_lo[j] == j; }
+    for (size_t j = 0; j < nhi; j++) { all |= inv_hi[j]; ident &= ((j << xlo) & ~used) || inv_hi[j] == j << xlo; }
     for (u32 z = 0; z < nz; z++) all |= zbits[z];
-    for (u32 s = 0; s < ns; s++) max_off = slices[3 * (size_t)s] > max_off ? slices[3 * (size_t)s] : max_off;
-    if (max_off >= n_words || all >= n_words - max_off) return fail(c, HL_B200_ERR_ARG, "tables_plane: a slice reaches past the committed rows");
     std::lock_guard<std::mutex> g(c->mu);
     TabDesc d;
-    memset(&d, 0, sizeof d);
-    d.kind = 1; d.table = (u32)i; d.xlo = xlo; d.nz = nz; d.ns = ns; d.used = used; d.base_check = base_check;
-    d.one_slice = ns == 1 && slices[1] == 1 && slices[2] == 0;
-    d.rows = reinterpret_cast<const u64*>(d_rows);
-    d.store = store;
-    d.off_lo = t->pool32.size();
-    t->pool32.insert(t->pool32.end(), inv_lo, inv_lo + nlo);
-    d.off_hi = t->pool32.size();
-    t->pool32.insert(t->pool32.end(), inv_hi, inv_hi + nhi);
-    d.off_zb = t->pool32.size();
-    if (nz) t->pool32.insert(t->pool32.end(), zbits, zbits + nz);
-    d.off_a = t->pool64.size();  // even: every 64-bit array read as Fp2 starts on a 16-byte boundary
-    if (nz) t->pool64.insert(t->pool64.end(), eqf, eqf + (size_t)nz * 2);
-    d.off_b = t->pool64.size();
-    t->pool64.insert(t->pool64.end(), slices, slices + (size_t)ns * 3);
-    if (t->pool64.size() & 1) t->pool64.push_back(0);
-    t->plan.push_back(d);
+    if (int rc = plane_desc(t, i, store, d_rows, n_words, all, slices, ns, base_check, &d)) return rc;
+    d.xlo = xlo; d.nz = nz; d.used = used; d.ident = ident;
+    if (!ident) {
+        d.off_lo = t->pool32.size();
+        t->pool32.insert(t->pool32.end(), inv_lo, inv_lo + nlo);
+        d.off_hi = t->pool32.size();
+        t->pool32.insert(t->pool32.end(), inv_hi, inv_hi + nhi);
+    }
+    plane_pools(t, &d, zbits, eqf, slices);
+    return HL_B200_OK;
+}
+
+int hl_b200_tables_plane_coords(hl_tables* t, size_t i, const hl_store* store, const uint64_t* d_rows, size_t n_words, const int32_t* coords, uint32_t n_coords,
+                                const uint64_t* fixed, const uint64_t* slices, uint32_t ns, int base_check) {
+    if (!t || !t->d_tables || i >= t->k || (n_coords && !coords) || !slices || ns == 0) return HL_B200_ERR_ARG;
+    hl_ctx* c = t->ctx;
+    const u32 n = t->n_vars, xlo = n / 2;
+    if (n_coords > 32 || n - xlo > 24) return fail(c, HL_B200_ERR_UNSUPPORTED, "tables_plane_coords: map sizes");
+    // argument.rs:486-512: coordinate j reads bit n_coords - 1 - j of the plane's index, from a cube variable or (fixed) from the point
+    u64 used = 0, zall = 0;
+    u32 to[32] = {0}, fpos[32], nf = 0;
+    bool flip[32] = {false}, ident = true;
+    for (u32 j = 0; j < n_coords; j++) {
+        const u32 ib = n_coords - 1 - j;
+        if (coords[j] == HL_COORD_FIXED) { fpos[nf++] = ib; zall |= (u64)1 << ib; continue; }
+        const u32 k = (u32)(coords[j] < 0 ? -1 - coords[j] : coords[j]);
+        if (k >= n || ((used >> (n - 1 - k)) & 1)) return fail(c, HL_B200_ERR_ARG, "tables_plane_coords: a cube variable outside the cube or read twice");
+        const u32 b = n - 1 - k;
+        used |= (u64)1 << b;
+        to[b] = ib; flip[b] = coords[j] < 0;
+        ident &= ib == b && coords[j] >= 0;
+    }
+    if (nf > 16) return fail(c, HL_B200_ERR_UNSUPPORTED, "tables_plane_coords: more than 16 fixed coordinates");
+    if (nf && !fixed) return HL_B200_ERR_ARG;
+    u64 all = zall;
+    for (u32 b = 0; b < n; b++)
+        if ((used >> b) & 1) all |= (u64)1 << to[b];
+    std::lock_guard<std::mutex> g(c->mu);
+    TabDesc d;
+    if (int rc = plane_desc(t, i, store, d_rows, n_words, all, slices, ns, base_check, &d)) return rc;
+    d.xlo = xlo; d.nz = nf ? 1u << nf : 0; d.used = used; d.ident = ident;
+    if (!ident) {
+        // each half by doubling: an entry is the one without its top bit, with that bit's image toggled
+        auto half = [&](u32 first, u32 bits) {
+            const size_t at = t->pool32.size();
+            t->pool32.resize(at + ((size_t)1 << bits));
+            u32* o = t->pool32.data() + at;
+            o[0] = 0;
+            for (u32 b = 0; b < bits; b++)
+                if (flip[first + b]) o[0] |= 1u << to[first + b];
+            for (u32 b = 0; b < bits; b++) {
+                const u32 img = ((used >> (first + b)) & 1) ? 1u << to[first + b] : 0u;
+                for (size_t v = 0; v < ((size_t)1 << b); v++) o[((size_t)1 << b) + v] = o[v] ^ img;
+            }
+            return (u64)at;
+        };
+        d.off_lo = half(0, xlo);
+        d.off_hi = half(xlo, n - xlo);
+    }
+    std::vector<u32> zbits(d.nz);
+    std::vector<fp2> eqf(d.nz);
+    if (nf) {  // first fixed coordinate = most significant bit of z, and of the eq table
+        for (u32 z = 0; z < d.nz; z++)
+            for (u32 f = 0; f < nf; f++) zbits[z] |= ((z >> (nf - 1 - f)) & 1) << fpos[f];
+        eqf[0] = f2(1, 0);
+        for (u32 f = 0; f < nf; f++) {
+            const fp2 r = f2(fixed[2 * f], fixed[2 * f + 1]);
+            for (size_t e = (size_t)1 << f; e-- > 0;) {
+                const fp2 hi = f2_mul(eqf[e], r);
+                eqf[2 * e + 1] = hi;
+                eqf[2 * e] = f2_sub(eqf[e], hi);
+            }
+        }
+    }
+    plane_pools(t, &d, zbits.data(), reinterpret_cast<const uint64_t*>(eqf.data()), slices);
     return HL_B200_OK;
 }
 
