@@ -71,6 +71,8 @@ int h2d(hl_ctx* c, void* d, const void* h, size_t bytes);
 int h2d_on(hl_ctx* c, void* d, const void* h, size_t bytes, cudaStream_t s);
 int h2d_owned(hl_ctx* c, void* d, const void* h, size_t bytes);
 int d2h(hl_ctx* c, void* h, const void* d, size_t bytes);
+// the same on a second stream; the context's stream waits for it
+int d2h_on(hl_ctx* c, void* h, const void* d, size_t bytes, cudaStream_t s);
 int sync(hl_ctx* c, const char* what);
 void host_copy_retain();
 void host_copy_release(hl_ctx* c);
@@ -88,9 +90,33 @@ int root_powers(hl_ctx* c, u32 lognn, const u64** out);
 int upload_key(hl_ctx* c, const uint8_t* key32, uint32_t** d_key);
 int log2_exact(size_t v);
 void store_release(hl_store* st);  // frees a store; the caller holds the context's lock
-// a hiding commitment of rows that are on the device already (hl_b200_commit_zk_dev); the caller holds the context's lock
+// a hiding commitment of rows that are on the device already (hl_b200_commit_zk_dev); the caller holds the context's lock.
+// leaves false: the encoding alone is wanted, its columns are not hashed
 int commit_resident(hl_ctx* c, u32 log_cols, u32 inv_rate, const u64* d_data, size_t rows, const u64* d_pads, size_t q, const u64* d_pows,
-                    const uint8_t* key32, hl_store** store, uint8_t* d_leaves32);
+                    const uint8_t* key32, hl_store** store, uint8_t* d_leaves32, bool leaves = true);
+
+// rho^T [M | pads] for k host vectors over a device matrix, each by the kernel for its support
+struct FoldSource {
+    const u64* d = nullptr;   // element (i, j) at d[i ld + j ir]
+    const u64* pads = nullptr;
+    size_t ld = 0;
+    u32 rows = 0, n = 0, q = 0, ir = 1;
+};
+struct FoldPlan {
+    hl_ctx* c = nullptr;
+    FoldSource src;
+    u32 kd = 0, ks = 0, few = 0, splits = 1;
+    std::vector<u32> sparse_map;
+    char* blk = nullptr;
+    size_t blk_bytes = 0, part_bytes = 0;
+    u64 *d_rhos = nullptr, *d_sw = nullptr, *d_part = nullptr;
+    u32 *d_soff = nullptr, *d_srows = nullptr, *d_dmap = nullptr, *d_smap = nullptr;
+    int make(hl_ctx* c, const FoldSource& src, const uint64_t* rhos, size_t k);
+    bool sparse_span(u32* first) const;  // whether the sparse vectors are neighbours, and where they start
+    int launch_sparse(u64* d_out);
+    int launch_dense(u64* d_out);
+    void release();
+};
 
 // Brackets the launches of one kernel family with two events when the context's timing is on.
 struct Timed {

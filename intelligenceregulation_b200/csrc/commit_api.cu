@@ -5,6 +5,98 @@
 
 using namespace hlapi;
 
+namespace hlapi {
+
+// An opening's group vectors are zero outside their claims' rows (pcs.rs:851-891), its proximity vector is dense.  Vectors with few
+// non-zero rows go to the list kernel, the others to the dense ones; all write the caller's order.
+int FoldPlan::make(hl_ctx* ctx, const FoldSource& source, const uint64_t* rhos, size_t k) {
+    c = ctx;
+    src = source;
+    const u32 rows = src.rows;
+    std::vector<u32> dense, s_off{0}, s_rows;
+    std::vector<u64> s_w;
+    for (size_t g = 0; g < k; g++) {
+        const uint64_t* r = rhos + g * (size_t)rows * 2;
+        const size_t from = s_rows.size();
+        bool is_sparse = true;
+        for (u32 i0 = 0; i0 < rows && is_sparse; i0 += 8) {
+            const u32 i1 = i0 + 8 < rows ? i0 + 8 : rows;
+            u64 any = 0;
+            for (u32 i = 2 * i0; i < 2 * i1; i++) any |= r[i];
+            if (!any) continue;
+            for (u32 i = i0; i < i1; i++)
+                if (r[2 * i] | r[2 * i + 1]) { s_rows.push_back(i); s_w.push_back(r[2 * i]); s_w.push_back(r[2 * i + 1]); }
+            is_sparse = (s_rows.size() - from) * 8u <= rows;
+        }
+        if (is_sparse) {
+            s_off.push_back((u32)s_rows.size());
+            sparse_map.push_back((u32)g);
+        } else {
+            s_rows.resize(from);
+            s_w.resize(2 * from);
+            dense.push_back((u32)g);
+        }
+    }
+    kd = (u32)dense.size();
+    ks = (u32)sparse_map.size();
+    // one upload: 64-bit words first
+    const size_t wd = (size_t)kd * rows * 2, words = wd + s_w.size(), ints = s_rows.size() + s_off.size() + kd + ks;
+    std::vector<u64> up(words + (ints + 1) / 2);
+    for (u32 i = 0; i < kd; i++) memcpy(up.data() + (size_t)i * rows * 2, rhos + dense[i] * (size_t)rows * 2, (size_t)rows * 16);
+    if (s_w.size()) memcpy(up.data() + wd, s_w.data(), s_w.size() * 8);
+    u32* ip = reinterpret_cast<u32*>(up.data() + words);
+    const size_t o_rows = s_off.size(), o_dmap = o_rows + s_rows.size(), o_smap = o_dmap + kd;
+    memcpy(ip, s_off.data(), s_off.size() * 4);
+    if (s_rows.size()) memcpy(ip + o_rows, s_rows.data(), s_rows.size() * 4);
+    if (kd) memcpy(ip + o_dmap, dense.data(), kd * 4);
+    if (ks) memcpy(ip + o_smap, sparse_map.data(), ks * 4);
+    few = kd ? hlk::fold_few_ranges(rows, src.n, src.q, kd, src.ir, c->sm_count) : 0;
+    splits = kd && !few ? hlk::fold_row_splits(rows, src.n, src.q, kd, c->sm_count) : 1;
+    const size_t w = (size_t)src.n + src.q;
+    part_bytes = few ? (size_t)few * kd * w * 16 : splits > 1 ? (size_t)splits * kd * w * 16 : 0;
+    blk_bytes = ((up.size() * 8 + 15) & ~(size_t)15) + part_bytes;
+    int rc = dev_alloc(c, (void**)&blk, blk_bytes);
+    if (!rc) rc = h2d(c, blk, up.data(), up.size() * 8);
+    if (rc) return rc;
+    d_rhos = (u64*)blk;
+    d_sw = d_rhos + wd;
+    d_soff = (u32*)(d_rhos + words);
+    d_srows = d_soff + o_rows;
+    d_dmap = d_soff + o_dmap;
+    d_smap = d_soff + o_smap;
+    d_part = part_bytes ? (u64*)(blk + blk_bytes - part_bytes) : nullptr;
+    return HL_B200_OK;
+}
+
+bool FoldPlan::sparse_span(u32* first) const {
+    if (!ks || sparse_map.back() - sparse_map.front() + 1 != ks) return false;  // the map is increasing
+    *first = sparse_map.front();
+    return true;
+}
+
+int FoldPlan::launch_sparse(u64* d_out) {
+    if (!ks) return HL_B200_OK;
+    cudaError_t e = hlk::fold_rows_sparse(src.d, src.n, src.ld, src.ir, src.pads, src.q, src.q, d_soff, d_srows, d_sw, ks, d_smap, d_out, src.n + src.q, c->stream);
+    c->stats.kernel_launches++;
+    return e == cudaSuccess ? HL_B200_OK : fail(c, HL_B200_ERR_DEVICE, "fold launch", e);
+}
+
+int FoldPlan::launch_dense(u64* d_out) {
+    if (!kd) return HL_B200_OK;
+    const u32 w = src.n + src.q;
+    cudaError_t e = few ? hlk::fold_rows_few(src.d, src.rows, src.n, src.ld, src.pads, src.q, src.q, d_rhos, kd, d_dmap, d_out, w, few, d_part, c->stream)
+                        : hlk::fold_rows(src.d, src.rows, src.n, src.ld, src.ir, src.pads, src.q, src.q, d_rhos, kd, d_dmap, d_out, w, c->stream, splits, d_part);
+    c->stats.kernel_launches += few || splits > 1 ? 2 : 1;
+    return e == cudaSuccess ? HL_B200_OK : fail(c, HL_B200_ERR_DEVICE, "fold launch", e);
+}
+
+void FoldPlan::release() {
+    if (blk) dev_free(c, blk, blk_bytes);
+    blk = nullptr;
+}
+
+}  // namespace hlapi
+
 static int merkle_on_device(hl_ctx* c, const uint32_t* d_leaves, const uint32_t* d_salts, size_t nn, const uint8_t* leaf_key32,
                             const uint8_t* node_key32, uint32_t* d_levels) {
     uint32_t *d_lk = nullptr, *d_nk = nullptr;
@@ -48,7 +140,7 @@ struct HostRows {
 // uploaded here in row chunks on the context's copy stream while the encoder works on the chunks that
 // have arrived (the upload of a block-sized matrix takes longer than its encoding).  Packed rows travel as
 // their narrow bytes and are widened into st->d_data by the encoder's first pass.  Leaves stay in st->d_leaves.
-int commit_on_device(hl_ctx* c, hl_store* st, const u64* d_pows, const uint8_t* key32, const HostRows& hr) {
+int commit_on_device(hl_ctx* c, hl_store* st, const u64* d_pows, const uint8_t* key32, const HostRows& hr, bool leaves = true) {
     const u32 logn = st->logn, lognn = st->logn + st->logr;
     const size_t n = st->n(), nn = st->nn();
     // rows above 2^14 words run as 2 or 4 shared-memory transforms of 2^14 (encode_core.cuh)
@@ -68,7 +160,7 @@ int commit_on_device(hl_ctx* c, hl_store* st, const u64* d_pows, const uint8_t* 
     u64* d_row_off = nullptr;
     const size_t scratch_words = hlk::encode_scratch_words(logb, T, c->sm_count, st->rows);
     const u32 nchunks = hlk::hash_chunks(st->rows);
-    const size_t cvs_bytes = nchunks > 1 ? (size_t)nchunks * nn * 32 : 0;
+    const size_t cvs_bytes = nchunks > 1 && leaves ? (size_t)nchunks * nn * 32 : 0;
     const size_t total_bytes = packed ? (size_t)hr.off[st->rows] : (size_t)st->rows * n * 8;
     rc = upload_key(c, key32, &d_key);
     if (!rc) rc = dev_alloc(c, (void**)&scratch, scratch_words * 8);
@@ -187,7 +279,7 @@ int commit_on_device(hl_ctx* c, hl_store* st, const u64* d_pows, const uint8_t* 
         c->stats.kernel_launches += 1;
         if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "column hash merge launch", e);
     }
-    if (!rc && !pieces) {
+    if (!rc && !pieces && leaves) {
         Timed t(c, HL_T_HASH);
         cudaError_t e = hlk::hash_columns(st->d_enc, st->rows, (u32)nn, d_key, cvs, st->d_leaves, c->stream);
         c->stats.kernel_launches += nchunks > 1 ? 2 : 1;
@@ -273,7 +365,7 @@ void hlapi::store_release(hl_store* st) { free_store(st); }
 
 // hl_b200_commit_zk_dev without the lock: for entry points that hold it already
 int hlapi::commit_resident(hl_ctx* c, u32 log_cols, u32 inv_rate, const u64* d_data, size_t rows, const u64* d_pads, size_t q, const u64* d_pows,
-                           const uint8_t* key32, hl_store** store, uint8_t* d_leaves32) {
+                           const uint8_t* key32, hl_store** store, uint8_t* d_leaves32, bool leaves) {
     Shape s;
     int rc = check_shape(c, log_cols, inv_rate, rows, q, true, 0, &s);
     if (rc) return rc;
@@ -285,7 +377,7 @@ int hlapi::commit_resident(hl_ctx* c, u32 log_cols, u32 inv_rate, const u64* d_d
     const size_t nn = st->nn();
     rc = dev_alloc(c, (void**)&st->d_enc, (size_t)s.rows * nn * 8);
     if (!rc) rc = dev_alloc(c, (void**)&st->d_leaves, nn * 32);
-    if (!rc) rc = commit_on_device(c, st, d_pows, key32, HostRows());
+    if (!rc) rc = commit_on_device(c, st, d_pows, key32, HostRows(), leaves);
     if (!rc && d_leaves32) {
         cudaError_t e = cudaMemcpyAsync(d_leaves32, st->d_leaves, nn * 32, cudaMemcpyDeviceToDevice, c->stream);
         if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "leaf copy", e);
@@ -402,83 +494,40 @@ int hl_b200_store_fold(hl_store* st, const uint64_t* rhos, size_t k, int with_pa
     if (k > 0xFFFFu * 8u) return fail(c, HL_B200_ERR_ARG, "store_fold: too many vectors");
     Call g(c);
     const u32 n = (u32)st->n(), q = with_pads ? st->q : 0, w = n + q, rows = st->rows;
-    // An opening's group vectors are zero outside their claims' rows (pcs.rs:851-891), its proximity vector is dense.
-    // Vectors with few non-zero rows go to the list kernel, the others to the dense one; both write the caller's order.
-    std::vector<u32> dense_map, sparse_map, s_off{0}, s_rows;
-    std::vector<u64> dense_rhos, s_w;
-    for (size_t g = 0; g < k; g++) {
-        const uint64_t* r = rhos + g * (size_t)rows * 2;
-        u32 support = 0;
-        for (u32 i = 0; i < rows; i++) support += (r[2 * i] | r[2 * i + 1]) != 0;
-        if (support * 8u <= rows) {
-            for (u32 i = 0; i < rows; i++)
-                if (r[2 * i] | r[2 * i + 1]) { s_rows.push_back(i); s_w.push_back(r[2 * i]); s_w.push_back(r[2 * i + 1]); }
-            s_off.push_back((u32)s_rows.size());
-            sparse_map.push_back((u32)g);
-        } else {
-            dense_rhos.insert(dense_rhos.end(), r, r + (size_t)rows * 2);
-            dense_map.push_back((u32)g);
-        }
-    }
-    const u32 kd = (u32)dense_map.size(), ks = (u32)sparse_map.size();
-    u64 *d_rhos = nullptr, *d_out = nullptr, *d_sw = nullptr;
-    u32 *d_dmap = nullptr, *d_smap = nullptr, *d_soff = nullptr, *d_srows = nullptr;
-    const size_t rb = (size_t)(kd ? kd : 1) * rows * 16, ob = k * (size_t)w * 16, ne = s_rows.size() ? s_rows.size() : 1;
+    const size_t row_bytes = (size_t)w * 16, ob = k * row_bytes;
+    // hiding form: the message is the resident data (the encoding is not systematic, pcs.rs:985-987);
+    // plain form: the systematic positions of the encoding (pcs.rs:332-340)
+    FoldSource src;
+    const bool from_data = st->zk || st->fold_data;
+    src.rows = rows; src.n = n; src.q = q;
+    src.d = from_data ? st->d_data : st->d_enc;
+    src.ld = from_data ? n : st->nn();
+    src.ir = from_data ? 1u : 1u << st->logr;
+    src.pads = st->zk && q ? st->d_pads : nullptr;
+    u64* d_out = nullptr;
+    FoldPlan plan;
     int rc = dev_alloc(c, (void**)&d_out, ob);
-    if (!rc && kd) {
-        rc = dev_alloc(c, (void**)&d_rhos, rb);
-        if (!rc) rc = dev_alloc(c, (void**)&d_dmap, kd * 4);
-        if (!rc) rc = h2d(c, d_rhos, dense_rhos.data(), (size_t)kd * rows * 16);
-        if (!rc) rc = h2d(c, d_dmap, dense_map.data(), kd * 4);
-    }
-    if (!rc && ks) {
-        rc = dev_alloc(c, (void**)&d_smap, ks * 4);
-        if (!rc) rc = dev_alloc(c, (void**)&d_soff, (ks + 1) * 4);
-        if (!rc) rc = dev_alloc(c, (void**)&d_srows, ne * 4);
-        if (!rc) rc = dev_alloc(c, (void**)&d_sw, ne * 16);
-        if (!rc) rc = h2d(c, d_smap, sparse_map.data(), ks * 4);
-        if (!rc) rc = h2d(c, d_soff, s_off.data(), (ks + 1) * 4);
-        if (!rc && s_rows.size()) rc = h2d(c, d_srows, s_rows.data(), s_rows.size() * 4);
-        if (!rc && s_rows.size()) rc = h2d(c, d_sw, s_w.data(), s_w.size() * 8);
-    }
-    const bool contiguous = st->zk || st->fold_data;
-    const u32 few = kd ? hlk::fold_few_ranges(rows, n, q, kd, contiguous ? 1u : 2u, c->sm_count) : 0;
-    const u32 fsplits = kd && !few ? hlk::fold_row_splits(rows, n, q, kd, c->sm_count) : 1;
-    u64* d_part = nullptr;
-    const size_t part_bytes = few ? (size_t)few * kd * w * 16 : fsplits > 1 ? (size_t)fsplits * kd * w * 16 : 0;
-    if (!rc && part_bytes) rc = dev_alloc(c, (void**)&d_part, part_bytes);
+    if (!rc) rc = plan.make(c, src, rhos, k);
+    u32 first = 0, sparse_done = 0;  // the sparse vectors' results, when they lie together, go back while the dense ones are computed
     if (!rc) {
         Timed t(c, HL_T_FOLD);
-        // hiding form: the message is the resident data (the encoding is not systematic, pcs.rs:985-987);
-        // plain form: the systematic positions of the encoding (pcs.rs:332-340)
-        const bool from_data = st->zk || st->fold_data;
-        const u64* src = from_data ? st->d_data : st->d_enc;
-        const size_t ld = from_data ? n : st->nn();
-        const u32 ir = from_data ? 1u : 1u << st->logr;
-        const u64* src2 = st->zk && q ? st->d_pads : nullptr;
-        cudaError_t e = cudaSuccess;
-        if (kd && few) {
-            e = hlk::fold_rows_few(src, rows, n, ld, src2, q, q, d_rhos, kd, d_dmap, d_out, w, few, d_part, c->stream);
-            c->stats.kernel_launches += 2;
-        } else if (kd) {
-            e = hlk::fold_rows(src, rows, n, ld, ir, src2, q, q, d_rhos, kd, d_dmap, d_out, w, c->stream, fsplits, d_part);
-            c->stats.kernel_launches += fsplits > 1 ? 2 : 1;
+        rc = plan.launch_sparse(d_out);
+        if (!rc && plan.kd && plan.sparse_span(&first)) {
+            cudaError_t e = cudaEventRecord(c->ev_main, c->stream);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(c->copy_stream, c->ev_main, 0);
+            if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "stream ordering", e);
+            sparse_done = plan.ks;
         }
-        if (e == cudaSuccess && ks) {
-            e = hlk::fold_rows_sparse(src, n, ld, ir, src2, q, q, d_soff, d_srows, d_sw, ks, d_smap, d_out, w, c->stream);
-            c->stats.kernel_launches++;
-        }
-        if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "fold launch", e);
+        if (!rc) rc = plan.launch_dense(d_out);
     }
-    if (!rc) rc = d2h(c, out, d_out, ob);
+    auto back = [&](u32 g0, u32 g1, cudaStream_t s) {
+        return g1 > g0 ? d2h_on(c, (char*)out + g0 * row_bytes, (char*)d_out + g0 * row_bytes, (g1 - g0) * row_bytes, s) : HL_B200_OK;
+    };
+    if (!rc) rc = back(first, first + sparse_done, c->copy_stream);
+    if (!rc) rc = back(0, first, c->stream);
+    if (!rc) rc = back(first + sparse_done, (u32)k, c->stream);
     if (!rc) rc = sync(c, "store_fold");
-    if (d_part) dev_free(c, d_part, part_bytes);
-    if (d_rhos) dev_free(c, d_rhos, rb);
-    if (d_dmap) dev_free(c, d_dmap, kd * 4);
-    if (d_smap) dev_free(c, d_smap, ks * 4);
-    if (d_soff) dev_free(c, d_soff, (ks + 1) * 4);
-    if (d_srows) dev_free(c, d_srows, ne * 4);
-    if (d_sw) dev_free(c, d_sw, ne * 16);
+    plan.release();
     if (d_out) dev_free(c, d_out, ob);
     if (!rc) c->stats.folds++;
     return rc;

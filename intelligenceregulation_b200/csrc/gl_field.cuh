@@ -41,51 +41,101 @@ GL_HD u64 gl_canon(u64 v) { return v >= GL_P ? v - GL_P : v; }
 // On the device they are PTX carry chains over 32-bit limbs (the 64-bit C forms cost ~1.5x the ALU-pipe
 // instructions); the multiply builds the 128-bit product with four 32x32 multiply-adds.
 #ifdef __CUDA_ARCH__
-__device__ __forceinline__ u64 gl_mul_lazy(u64 a, u64 b) {
-    const u32 a0 = (u32)a, a1 = (u32)(a >> 32), b0 = (u32)b, b1 = (u32)(b >> 32);
-    const u64 x = (u64)a0 * b0;
-    const u64 y = (u64)a0 * b1 + (x >> 32);
-    const u64 z = (u64)a1 * b0 + (u32)y;
-    const u64 w = (u64)a1 * b1 + (y >> 32) + (z >> 32);
-    const u32 p0 = (u32)x, p1 = (u32)z, p2 = (u32)w, p3 = (u32)(w >> 32);
-    u32 r0, r1;
-    // (p1:p0) - p3 [borrow: - EPS]  + p2 * EPS [carry: + EPS]
+// the 128-bit product in four words: two 32 x 32 products and two multiply-add chains whose carries stay in the carry flag
+__device__ __forceinline__ void gl_product(u64 a, u64 b, u32& p0, u32& p1, u32& p2, u32& p3) {
     asm("{\n\t"
-        ".reg .u32 t0,t1,m,q0,q1;\n\t"
-        ".reg .u64 q;\n\t"
-        "sub.cc.u32 t0, %2, %5;\n\t"
-        "subc.cc.u32 t1, %3, 0;\n\t"
-        "subc.u32 m, 0, 0;\n\t"
-        "sub.cc.u32 t0, t0, m;\n\t"
-        "subc.u32 t1, t1, 0;\n\t"
-        "mul.wide.u32 q, %4, 0xFFFFFFFF;\n\t"
-        "mov.b64 {q0,q1}, q;\n\t"
-        "add.cc.u32 t0, t0, q0;\n\t"
-        "addc.cc.u32 t1, t1, q1;\n\t"
-        "addc.u32 m, 0, 0;\n\t"
-        "mov.b64 q, {t0,t1};\n\t"
-        "mad.wide.u32 q, m, 0xFFFFFFFF, q;\n\t"
-        "mov.b64 {%0,%1}, q;\n\t"
+        "mul.lo.u32 %0, %4, %6;\n\t"
+        "mul.hi.u32 %1, %4, %6;\n\t"
+        "mul.lo.u32 %2, %5, %7;\n\t"
+        "mul.hi.u32 %3, %5, %7;\n\t"
+        "mad.lo.cc.u32 %1, %4, %7, %1;\n\t"
+        "madc.hi.cc.u32 %2, %4, %7, %2;\n\t"
+        "addc.u32 %3, %3, 0;\n\t"
+        "mad.lo.cc.u32 %1, %5, %6, %1;\n\t"
+        "madc.hi.cc.u32 %2, %5, %6, %2;\n\t"
+        "addc.u32 %3, %3, 0;\n\t"
         "}"
-        : "=r"(r0), "=r"(r1)
-        : "r"(p0), "r"(p1), "r"(p2), "r"(p3));
+        : "=&r"(p0), "=&r"(p1), "=&r"(p2), "=&r"(p3)
+        : "r"((u32)a), "r"((u32)(a >> 32)), "r"((u32)b), "r"((u32)(b >> 32)));
+}
+// (c:p3:p2:p1:p0) += a b
+__device__ __forceinline__ void gl_product_acc(u64 a, u64 b, u32& p0, u32& p1, u32& p2, u32& p3, u32& c) {
+    asm("{\n\t"
+        "mad.lo.cc.u32 %0, %5, %7, %0;\n\t"
+        "madc.hi.cc.u32 %1, %5, %7, %1;\n\t"
+        "madc.lo.cc.u32 %2, %6, %8, %2;\n\t"
+        "madc.hi.cc.u32 %3, %6, %8, %3;\n\t"
+        "addc.u32 %4, %4, 0;\n\t"
+        "mad.lo.cc.u32 %1, %5, %8, %1;\n\t"
+        "madc.hi.cc.u32 %2, %5, %8, %2;\n\t"
+        "addc.cc.u32 %3, %3, 0;\n\t"
+        "addc.u32 %4, %4, 0;\n\t"
+        "mad.lo.cc.u32 %1, %6, %7, %1;\n\t"
+        "madc.hi.cc.u32 %2, %6, %7, %2;\n\t"
+        "addc.cc.u32 %3, %3, 0;\n\t"
+        "addc.u32 %4, %4, 0;\n\t"
+        "}"
+        : "+r"(p0), "+r"(p1), "+r"(p2), "+r"(p3), "+r"(c)
+        : "r"((u32)a), "r"((u32)(a >> 32)), "r"((u32)b), "r"((u32)(b >> 32)));
+}
+// (c:p3:p2) += h b for a small h: the part of a product above its first factor's 64 bits
+__device__ __forceinline__ void gl_product_top(u32 h, u64 b, u32& p2, u32& p3, u32& c) {
+    asm("mad.lo.cc.u32 %0, %3, %4, %0;\n\t"
+        "madc.hi.cc.u32 %1, %3, %4, %1;\n\t"
+        "addc.u32 %2, %2, 0;\n\t"
+        "mad.lo.cc.u32 %1, %3, %5, %1;\n\t"
+        "madc.hi.u32 %2, %3, %5, %2;\n\t"
+        : "+r"(p2), "+r"(p3), "+r"(c)
+        : "r"(h), "r"((u32)b), "r"((u32)(b >> 32)));
+}
+// (s3:s2:s1:s0) + c 2^128 as a lazy word: V = (s1:s0) + s2 2^32 - (s2 + s3) - c 2^32   (2^96 = -1, 2^128 = -2^32 mod p).  V lies in
+// (-2^34, 2^65), so one correction by k = floor(V / 2^64) in {-1, 0, 1} is enough: V - k 2^64 + k (2^32 - 1) is a word again.
+__device__ __forceinline__ u64 gl_red129_lazy(u32 s0, u32 s1, u32 s2, u32 s3, u32 c) {
+    u32 r0, r1;
+    asm("{\n\t"
+        ".reg .u32 t0,t1,m,k,g;\n\t"
+        "add.cc.u32 t0, %4, %5;\n\t"
+        "addc.u32 t1, %6, 0;\n\t"
+        "add.cc.u32 %1, %3, %4;\n\t"
+        "addc.u32 m, 0, 0;\n\t"
+        "sub.cc.u32 %0, %2, t0;\n\t"
+        "subc.cc.u32 %1, %1, t1;\n\t"
+        "subc.u32 k, m, 0;\n\t"
+        "shr.s32 g, k, 31;\n\t"
+        "sub.u32 g, g, k;\n\t"
+        "sub.cc.u32 %0, %0, k;\n\t"
+        "subc.u32 %1, %1, g;\n\t"
+        "}"
+        : "=&r"(r0), "=&r"(r1)
+        : "r"(s0), "r"(s1), "r"(s2), "r"(s3), "r"(c));
     return ((u64)r1 << 32) | r0;
+}
+__device__ __forceinline__ u64 gl_mul_lazy(u64 a, u64 b) {
+    u32 p0, p1, p2, p3;
+    gl_product(a, b, p0, p1, p2, p3);
+    return gl_red129_lazy(p0, p1, p2, p3, 0u);
 }
 // r >= p  <=>  high limb all ones and low limb non-zero; then r - p = low limb - 1
 __device__ __forceinline__ u64 gl_canon_fast(u64 r) {
-    const u32 r0 = (u32)r, r1 = (u32)(r >> 32);
-    return (r1 == 0xFFFFFFFFu && r0 != 0) ? (u64)(r0 - 1) : r;
+    u32 r0 = (u32)r, r1 = (u32)(r >> 32);
+    asm("{\n\t.reg .pred p;\n\t"
+        "setp.eq.u32 p, %1, 0xFFFFFFFF;\n\t"
+        "setp.ne.and.u32 p, %0, 0, p;\n\t"
+        "@p add.u32 %0, %0, -1;\n\t"
+        "@p mov.u32 %1, 0;\n\t}"
+        : "+r"(r0), "+r"(r1));
+    return ((u64)r1 << 32) | r0;
 }
 __device__ __forceinline__ u64 gl_add_lazy(u64 u, u64 v) {
     const u32 u0 = (u32)u, u1 = (u32)(u >> 32), v0 = (u32)v, v1 = (u32)(v >> 32);
     u32 r0, r1;
-    asm("{\n\t.reg .u32 m;\n\t.reg .u64 q;\n\t"
+    asm("{\n\t.reg .u32 m;\n\t"
         "add.cc.u32 %0, %2, %4;\n\t"
         "addc.cc.u32 %1, %3, %5;\n\t"
         "addc.u32 m, 0, 0;\n\t"
-        "mov.b64 q, {%0,%1};\n\t"
-        "mad.wide.u32 q, m, 0xFFFFFFFF, q;\n\t"
-        "mov.b64 {%0,%1}, q;\n\t}"
+        "neg.s32 m, m;\n\t"
+        "add.cc.u32 %0, %0, m;\n\t"
+        "addc.u32 %1, %1, 0;\n\t}"
         : "=&r"(r0), "=&r"(r1) : "r"(u0), "r"(u1), "r"(v0), "r"(v1));
     return ((u64)r1 << 32) | r0;
 }
@@ -157,33 +207,6 @@ GL_HD u64 gl_sub(u64 a, u64 b) {
 
 GL_HD u64 gl_neg(u64 a) { return a ? GL_P - a : 0; }
 
-#ifdef __CUDA_ARCH__
-// (s3:s2:s1:s0) + c 2^128 as a lazy word: (s1:s0) - s3 - c 2^32 + s2 (2^32 - 1)   (2^96 = -1, 2^128 = -2^32 mod p)
-__device__ __forceinline__ u64 gl_red129_lazy(u32 s0, u32 s1, u32 s2, u32 s3, u32 c) {
-    u32 r0, r1;
-    asm("{\n\t"
-        ".reg .u32 t0,t1,m,q0,q1;\n\t"
-        ".reg .u64 q;\n\t"
-        "sub.cc.u32 t0, %2, %5;\n\t"
-        "subc.cc.u32 t1, %3, %6;\n\t"
-        "subc.u32 m, 0, 0;\n\t"
-        "sub.cc.u32 t0, t0, m;\n\t"
-        "subc.u32 t1, t1, 0;\n\t"
-        "mul.wide.u32 q, %4, 0xFFFFFFFF;\n\t"
-        "mov.b64 {q0,q1}, q;\n\t"
-        "add.cc.u32 t0, t0, q0;\n\t"
-        "addc.cc.u32 t1, t1, q1;\n\t"
-        "addc.u32 m, 0, 0;\n\t"
-        "mov.b64 q, {t0,t1};\n\t"
-        "mad.wide.u32 q, m, 0xFFFFFFFF, q;\n\t"
-        "mov.b64 {%0,%1}, q;\n\t"
-        "}"
-        : "=r"(r0), "=r"(r1)
-        : "r"(s0), "r"(s1), "r"(s2), "r"(s3), "r"(c));
-    return ((u64)r1 << 32) | r0;
-}
-#endif
-
 GL_HD u64 gl_reduce128(u64 lo, u64 hi) {
 #ifdef GL_DEVICE_CHAINS
     return gl_canon_fast(gl_red129_lazy((u32)lo, (u32)(lo >> 32), (u32)hi, (u32)(hi >> 32), 0u));
@@ -205,13 +228,10 @@ struct gl_wide {
 GL_HD gl_wide gl_mulw(u64 a, u64 b) {
     gl_wide r;
 #ifdef __CUDA_ARCH__
-    const u32 a0 = (u32)a, a1 = (u32)(a >> 32), b0 = (u32)b, b1 = (u32)(b >> 32);
-    const u64 x = (u64)a0 * b0;
-    const u64 y = (u64)a0 * b1 + (x >> 32);
-    const u64 z = (u64)a1 * b0 + (u32)y;
-    const u64 w = (u64)a1 * b1 + (y >> 32) + (z >> 32);
-    r.lo = (z << 32) | (u32)x;
-    r.hi = w;
+    u32 p0, p1, p2, p3;
+    gl_product(a, b, p0, p1, p2, p3);
+    r.lo = ((u64)p1 << 32) | p0;
+    r.hi = ((u64)p3 << 32) | p2;
 #else
     unsigned __int128 x = (unsigned __int128)a * b;
     r.lo = (u64)x;
@@ -232,15 +252,13 @@ GL_HD u64 gl_mul(u64 a, u64 b) {
 
 // a b + c d with ONE reduction: the 129-bit sum's top bit weighs 2^128 = -2^32 (mod p).  Device: any a, b, c, d (lazy operands too).
 GL_HD u64 gl_mul_add2(u64 a, u64 b, u64 c, u64 d) {
-    const gl_wide p = gl_mulw(a, b), q = gl_mulw(c, d);
 #ifdef GL_DEVICE_CHAINS
-    u32 s0, s1, s2, s3, cy;
-    asm("add.cc.u32 %0, %5, %9;\n\taddc.cc.u32 %1, %6, %10;\n\taddc.cc.u32 %2, %7, %11;\n\taddc.cc.u32 %3, %8, %12;\n\taddc.u32 %4, 0, 0;"
-        : "=r"(s0), "=r"(s1), "=r"(s2), "=r"(s3), "=r"(cy)
-        : "r"((u32)p.lo), "r"((u32)(p.lo >> 32)), "r"((u32)p.hi), "r"((u32)(p.hi >> 32)), "r"((u32)q.lo), "r"((u32)(q.lo >> 32)), "r"((u32)q.hi),
-          "r"((u32)(q.hi >> 32)));
-    return gl_canon_fast(gl_red129_lazy(s0, s1, s2, s3, cy));
+    u32 p0, p1, p2, p3, cy = 0;
+    gl_product(a, b, p0, p1, p2, p3);
+    gl_product_acc(c, d, p0, p1, p2, p3, cy);
+    return gl_canon_fast(gl_red129_lazy(p0, p1, p2, p3, cy));
 #else
+    const gl_wide p = gl_mulw(a, b), q = gl_mulw(c, d);
     const u64 lo = p.lo + q.lo, cy = lo < p.lo ? 1u : 0u;
     const u64 h0 = p.hi + q.hi, c2 = h0 < p.hi ? 1u : 0u;
     const u64 hi = h0 + cy, c3 = hi < h0 ? 1u : 0u;
@@ -301,11 +319,17 @@ GL_HD fp2 f2_mul_base(fp2 a, u64 b) { return f2(gl_mul(a.c0, b), gl_mul(a.c1, b)
 // (a0 + a1 u)(b0 + b1 u) with u^2 = 7 (field.rs:163-169)
 GL_HD fp2 f2_mul(fp2 a, fp2 b) {
 #ifdef GL_DEVICE_CHAINS
-    const u64 a17 = gl_sub_lazy(gl_add_lazy(a.c1 << 3, (a.c1 >> 61) * GL_EPS), a.c1);  // 7 a1 = 8 a1 - a1, a lazy word (the products take any word)
+    // 7 a1 in three words, the top one below 7: its product with b1 goes straight into the upper words
+    const u64 q = (u64)(u32)a.c1 * 7u, t = (a.c1 >> 32) * 7u + (q >> 32);
+    u32 p0, p1, p2, p3, cy = 0;
+    gl_product(a.c0, b.c0, p0, p1, p2, p3);
+    gl_product_acc((t << 32) | (u32)q, b.c1, p0, p1, p2, p3, cy);
+    gl_product_top((u32)(t >> 32), b.c1, p2, p3, cy);
+    return f2(gl_canon_fast(gl_red129_lazy(p0, p1, p2, p3, cy)), gl_mul_add2(a.c0, b.c1, a.c1, b.c0));
 #else
     const u64 a17 = gl_sub(gl_reduce128(a.c1 << 3, a.c1 >> 61), a.c1);  // 7 a1 = 8 a1 - a1
-#endif
     return f2(gl_mul_add2(a.c0, b.c0, a17, b.c1), gl_mul_add2(a.c0, b.c1, a.c1, b.c0));
+#endif
 }
 GL_HD bool f2_is_zero(fp2 a) { return (a.c0 | a.c1) == 0; }
 // conj(a) / (a0^2 - 7 a1^2) (field.rs:180-185)

@@ -333,23 +333,29 @@ int h2d_owned(hl_ctx* c, void* d, const void* h, size_t bytes) {
 }
 
 // The bytes are in the caller's memory after the next `sync`.
-int d2h(hl_ctx* c, void* h, const void* d, size_t bytes) {
+int d2h_on(hl_ctx* c, void* h, const void* d, size_t bytes, cudaStream_t s) {
     if (!bytes) return HL_B200_OK;
     cudaError_t e;
     CopyRing* r;
     char* slot;
     if (bytes <= SMALL && (slot = arena_slot(c, bytes)) != nullptr) {
-        e = cudaMemcpyAsync(slot, d, bytes, cudaMemcpyDeviceToHost, c->stream);
+        e = cudaMemcpyAsync(slot, d, bytes, cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) c->pending.push_back({h, slot, bytes});
     } else if (pageable(h) && (r = ring_of(c)) != nullptr) {
-        e = ring_down(r, (char*)h, (const char*)d, bytes, c->stream);
+        e = ring_down(r, (char*)h, (const char*)d, bytes, s);
     } else {
-        e = cudaMemcpyAsync(h, d, bytes, cudaMemcpyDeviceToHost, c->stream);
+        e = cudaMemcpyAsync(h, d, bytes, cudaMemcpyDeviceToHost, s);
+    }
+    if (e == cudaSuccess && s != c->stream) {
+        e = cudaEventRecord(c->ev_main, s);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(c->stream, c->ev_main, 0);
     }
     if (e != cudaSuccess) return fail(c, HL_B200_ERR_DEVICE, "copy from device", e);
     c->stats.bytes_d2h += bytes;
     return HL_B200_OK;
 }
+
+int d2h(hl_ctx* c, void* h, const void* d, size_t bytes) { return d2h_on(c, h, d, bytes, c->stream); }
 
 int sync(hl_ctx* c, const char* what) {
     cudaError_t e = cudaStreamSynchronize(c->stream);

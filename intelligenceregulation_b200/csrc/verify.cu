@@ -7,7 +7,7 @@
 //
 // Layout: the caller's columns are ncols runs of `rows` words.  They are transposed once into a rows x ncols matrix, which is
 // the layout the commitment's own column hash and row fold read (32 neighbouring columns per warp and row), so the two heavy
-// parts run through the same kernels as the prover's.  One thread per column then salts the leaf, walks the path and compares
+// parts run through the same kernels as the prover's.  One warp per column then salts the leaf, walks the path and compares
 // the combinations; it writes one verdict word per column.
 #include <vector>
 
@@ -37,21 +37,39 @@ __global__ void __launch_bounds__(256) k_cols_to_rows(const u64* __restrict__ in
 // verdict[c]: 0 all checks hold; 1 the Merkle path fails; 2 + g the column disagrees with clear vector g (the first such g).
 // The order is the reference's: the path is checked before the combinations.
 // wants: k x ncols Fp2 from the caller, or (wants == NULL) rows 2g / 2g + 1 of `enc` (row length nn) at position idx[c].
-__global__ void __launch_bounds__(128) k_verify_columns(const uint32_t* __restrict__ leaves, const uint32_t* __restrict__ salts,
+// A warp per column: the path is a serial chain of depth + 1 hashes (0.55 us each), which every lane walks over siblings staged in
+// shared memory, and the lanes share the comparisons.  (A thread per column loaded each sibling and each expected value at the latency
+// of its own miss: 280 columns, 39 vectors 50 us; now 12 us.)
+constexpr int VC_WARPS = 4;
+constexpr u32 VC_DEPTH = 40;
+__global__ void __launch_bounds__(32 * VC_WARPS) k_verify_columns(const uint32_t* __restrict__ leaves, const uint32_t* __restrict__ salts,
                                                         const uint32_t* __restrict__ paths, u32 depth, const u64* __restrict__ idx,
                                                         const uint32_t* __restrict__ root, const uint32_t* __restrict__ leaf_key,
                                                         const uint32_t* __restrict__ node_key, const u64* __restrict__ acc, u32 k,
                                                         const u64* __restrict__ wants, const u64* __restrict__ enc, size_t nn, u32 ncols,
                                                         int32_t* __restrict__ verdict) {
-    const u32 c = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ uint32_t path_s[VC_WARPS][VC_DEPTH * 8];
+    const u32 warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = blockIdx.x * VC_WARPS + warp;
     if (c >= ncols) return;
+    for (u32 i = lane; i < depth * 8; i += 32) path_s[warp][i] = paths[(size_t)c * depth * 8 + i];
     uint32_t m[16], cur[8];
 #pragma unroll
     for (int i = 0; i < 8; i++) { m[i] = leaves[(size_t)c * 8 + i]; m[8 + i] = salts[(size_t)c * 8 + i]; }
+    const u64 j = idx[c];
+    u32 bad = 0xffffffffu;  // the first vector that this lane found wrong
+    for (u32 g = lane; g < k && bad == 0xffffffffu; g += 32) {
+        const u64 a0 = acc[((size_t)g * ncols + c) * 2], a1 = acc[((size_t)g * ncols + c) * 2 + 1];
+        u64 w0, w1;
+        if (wants) { w0 = wants[((size_t)g * ncols + c) * 2]; w1 = wants[((size_t)g * ncols + c) * 2 + 1]; }
+        else { w0 = enc[(size_t)(2 * g) * nn + j]; w1 = enc[(size_t)(2 * g + 1) * nn + j]; }
+        if (a0 != w0 || a1 != w1) bad = g;
+    }
+    bad = __reduce_min_sync(0xffffffffu, bad);
+    __syncwarp();
     b3::hash64(cur, m, leaf_key);
-    u64 pos = idx[c];
+    u64 pos = j;
     for (u32 l = 0; l < depth; l++) {
-        const uint32_t* sib = paths + ((size_t)c * depth + l) * 8;
+        const uint32_t* sib = path_s[warp] + 8 * l;
         const bool right = pos & 1ull;  // this node is the right child: the sibling goes first
 #pragma unroll
         for (int i = 0; i < 8; i++) { m[i] = right ? sib[i] : cur[i]; m[8 + i] = right ? cur[i] : sib[i]; }
@@ -61,18 +79,7 @@ __global__ void __launch_bounds__(128) k_verify_columns(const uint32_t* __restri
     bool ok = true;
 #pragma unroll
     for (int i = 0; i < 8; i++) ok = ok && cur[i] == root[i];
-    int32_t v = ok ? 0 : 1;
-    if (ok) {
-        const u64 j = idx[c];
-        for (u32 g = 0; g < k; g++) {
-            const u64 a0 = acc[((size_t)g * ncols + c) * 2], a1 = acc[((size_t)g * ncols + c) * 2 + 1];
-            u64 w0, w1;
-            if (wants) { w0 = wants[((size_t)g * ncols + c) * 2]; w1 = wants[((size_t)g * ncols + c) * 2 + 1]; }
-            else { w0 = enc[(size_t)(2 * g) * nn + j]; w1 = enc[(size_t)(2 * g + 1) * nn + j]; }
-            if (a0 != w0 || a1 != w1) { v = 2 + (int32_t)g; break; }
-        }
-    }
-    verdict[c] = v;
+    if (lane == 0) verdict[c] = !ok ? 1 : bad == 0xffffffffu ? 0 : 2 + (int32_t)bad;
 }
 
 // vecs: k vectors of n + q Fp2 -> 2k base rows (re of vector 0, im of vector 0, re of vector 1, ..): the first n words of each into
@@ -115,7 +122,8 @@ static int verify_columns_locked(hl_ctx* c, const uint64_t* cols, size_t rows, s
     const size_t cb = rows * ncols * 8, pb = (size_t)(depth ? depth : 1) * ncols * 32, ab = (k ? k : 1) * ncols * 16;
     const u32 nchunks = hlk::hash_chunks((u32)rows);
     const size_t cvs_bytes = nchunks > 1 ? (size_t)nchunks * ncols * 32 : 0;
-    u64 *d_cols = nullptr, *d_mat = nullptr, *d_idx = nullptr, *d_rhos = nullptr, *d_acc = nullptr, *d_wants = nullptr;
+    u64 *d_cols = nullptr, *d_mat = nullptr, *d_idx = nullptr, *d_acc = nullptr, *d_wants = nullptr;
+    FoldPlan plan;
     uint32_t *d_salts = nullptr, *d_paths = nullptr, *d_root = nullptr, *d_ck = nullptr, *d_lk = nullptr, *d_nk = nullptr, *d_leaves = nullptr, *d_cvs = nullptr;
     int32_t* d_verdict = nullptr;
     int rc = dev_alloc(c, (void**)&d_cols, cb);
@@ -128,14 +136,19 @@ static int verify_columns_locked(hl_ctx* c, const uint64_t* cols, size_t rows, s
     if (!rc && cvs_bytes) rc = dev_alloc(c, (void**)&d_cvs, cvs_bytes);
     if (!rc) rc = dev_alloc(c, (void**)&d_acc, ab);
     if (!rc) rc = dev_alloc(c, (void**)&d_verdict, ncols * 4);
-    if (!rc && k) rc = dev_alloc(c, (void**)&d_rhos, k * rows * 16);
     if (!rc && k && wants) rc = dev_alloc(c, (void**)&d_wants, ab);
     if (!rc) rc = h2d(c, d_cols, cols, cb);
     if (!rc) rc = h2d(c, d_idx, idx, ncols * 8);
     if (!rc) rc = h2d(c, d_salts, salts32, ncols * 32);
     if (!rc && depth) rc = h2d(c, d_paths, paths32, (size_t)depth * ncols * 32);
     if (!rc) rc = h2d(c, d_root, root32, 32);
-    if (!rc && k) rc = h2d(c, d_rhos, rhos, k * rows * 16);
+    if (!rc && k) {
+        // the opened columns as a matrix of `ncols` columns: the commitment's own row folds, each weight vector by the kernel for its
+        // support (39 vectors of an opening, 37 of them living on 34 rows: all through the dense kernel took 640 us)
+        FoldSource src;
+        src.d = d_mat; src.ld = ncols; src.rows = (u32)rows; src.n = (u32)ncols;
+        rc = plan.make(c, src, rhos, k);
+    }
     if (!rc && d_wants) rc = h2d(c, d_wants, wants, ab);
     if (!rc) rc = upload_key(c, column_key32, &d_ck);
     if (!rc) rc = upload_key(c, leaf_key32, &d_lk);
@@ -150,15 +163,16 @@ static int verify_columns_locked(hl_ctx* c, const uint64_t* cols, size_t rows, s
         }
         if (e == cudaSuccess && k) {
             Timed t(c, HL_T_FOLD);
-            e = hlk::fold_rows(d_mat, (u32)rows, (u32)ncols, ncols, 1u, nullptr, 0u, 0, d_rhos, (u32)k, nullptr, d_acc, (u32)ncols, c->stream);
+            rc = plan.launch_sparse(d_acc);
+            if (!rc) rc = plan.launch_dense(d_acc);
         }
-        if (e == cudaSuccess) {
-            k_verify_columns<<<(unsigned)((ncols + 127) / 128), 128, 0, c->stream>>>(
+        if (e == cudaSuccess && !rc) {
+            k_verify_columns<<<(unsigned)((ncols + VC_WARPS - 1) / VC_WARPS), 32 * VC_WARPS, 0, c->stream>>>(
                 d_leaves, d_salts, d_paths, depth, d_idx, d_root, d_lk, d_nk, d_acc, (u32)k, d_wants, vec_store ? vec_store->d_enc : nullptr,
                 vec_store ? vec_store->nn() : 0, (u32)ncols, d_verdict);
             e = cudaGetLastError();
         }
-        c->stats.kernel_launches += 2 + (nchunks > 1 ? 2 : 1) + (k ? 1 : 0);
+        c->stats.kernel_launches += 2 + (nchunks > 1 ? 2 : 1);
         if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "verify_columns launch", e);
     }
     if (!rc) rc = d2h(c, verdict, d_verdict, ncols * 4);
@@ -173,7 +187,7 @@ static int verify_columns_locked(hl_ctx* c, const uint64_t* cols, size_t rows, s
     dev_free(c, d_paths, pb); dev_free(c, d_root, 32); dev_free(c, d_leaves, ncols * 32);
     if (d_cvs) dev_free(c, d_cvs, cvs_bytes);
     dev_free(c, d_acc, ab); dev_free(c, d_verdict, ncols * 4);
-    if (d_rhos) dev_free(c, d_rhos, k * rows * 16);
+    plan.release();
     if (d_wants) dev_free(c, d_wants, ab);
     if (d_ck) dev_free(c, d_ck, 32);
     if (d_lk) dev_free(c, d_lk, 32);
@@ -216,7 +230,7 @@ extern "C" int hl_b200_verify_opening(hl_ctx* c, uint32_t log_cols, uint32_t inv
         if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "verify_opening launch", e);
     }
     // the commitment's own encoder on the 2k rows; the shape checks (inv_rate a power of two, n + q <= nn) are its
-    if (!rc) rc = commit_resident(c, log_cols, inv_rate, d_data, 2 * k, d_pads, q, d_pows, nullptr, &st, nullptr);
+    if (!rc) rc = commit_resident(c, log_cols, inv_rate, d_data, 2 * k, d_pads, q, d_pows, nullptr, &st, nullptr, false);
     if (!rc)
         rc = verify_columns_locked(c, cols, rows, ncols, idx, salts32, paths32, depth, root32, column_key32, leaf_key32, node_key32, rhos, k, nullptr, st,
                                    verdict, first_bad);
