@@ -6,9 +6,8 @@ a block goes back when the last array over it is gone, at most ``KEEP`` bytes wa
 """
 from __future__ import annotations
 
-import ctypes as C
+import math
 import threading
-import weakref
 from typing import List
 
 import numpy as np
@@ -18,34 +17,50 @@ KEEP = 192 << 20   # a block's logup columns twice over (the caller holds one re
 
 _lock = threading.RLock()  # a block may come back from a garbage collection inside `empty`
 _idle: List[np.ndarray] = []
+_bytes = 0
 
 
-def _back(block: np.ndarray) -> None:
-    with _lock:
-        _idle.append(block)
-        while sum(b.nbytes for b in _idle) > KEEP:
-            _idle.pop(0)
+class _Hold:
+    """What the arrays over a block have for a base: when the last of them is gone, so is this, and the block goes back."""
+
+    __slots__ = ("block", "__array_interface__")
+
+    def __init__(self, block: np.ndarray, shape, dtype: np.dtype):
+        self.block = block
+        self.__array_interface__ = {"shape": shape, "typestr": dtype.str, "data": (block.__array_interface__["data"][0], False), "version": 3}
+
+    def __del__(self):
+        global _bytes
+        with _lock:
+            _idle.append(self.block)
+            _bytes += self.block.nbytes
+            while _bytes > KEEP:
+                _bytes -= _idle.pop(0).nbytes
 
 
 def empty(shape, dtype) -> np.ndarray:
     """``np.empty(shape, dtype)``, over reused memory where it is large"""
-    dtype = np.dtype(dtype)
-    nbytes = int(np.prod(shape, dtype=np.int64)) * dtype.itemsize
+    global _bytes
+    dtype, shape = np.dtype(dtype), tuple(shape) if isinstance(shape, (tuple, list)) else (int(shape),)
+    nbytes = math.prod(shape) * dtype.itemsize
     if nbytes < SMALL:
         return np.empty(shape, dtype)
     block = None
     with _lock:
-        fits = [b for b in _idle if nbytes <= b.nbytes <= nbytes + (nbytes >> 2)]
-        if fits:
-            best = min(fits, key=lambda b: b.nbytes)
-            block = _idle.pop(next(i for i, b in enumerate(_idle) if b is best))
+        best = -1
+        for i, b in enumerate(_idle):
+            if nbytes <= b.nbytes <= nbytes + (nbytes >> 2) and (best < 0 or b.nbytes < _idle[best].nbytes):
+                best = i
+        if best >= 0:
+            block = _idle.pop(best)
+            _bytes -= block.nbytes
     if block is None:
         block = np.empty(nbytes, np.uint8)
-    hold = (C.c_ubyte * nbytes).from_buffer(block)
-    weakref.finalize(hold, _back, block).atexit = False
-    return np.frombuffer(hold, dtype=dtype).reshape(shape)
+    return np.asarray(_Hold(block, shape, dtype))
 
 
 def release() -> None:
+    global _bytes
     with _lock:
         _idle.clear()
+        _bytes = 0
