@@ -6,6 +6,7 @@
 #include "api_internal.h"
 #include "../../include/hl_b200_bench.h"
 #include "slot_gen.cuh"
+#include "slot_vm.cuh"
 #include "sumcheck.h"
 
 using namespace hlapi;
@@ -24,12 +25,15 @@ struct hl_rounds {
     u32 max_blocks = 0;
     u64* d_tables = nullptr;
     // one device block of everything else: [inverse denominators, extrapolation weights, coefficients, plan] as uploaded at the start,
-    // then [mask rows and table | state] as uploaded by a batch (the mask ends where the state begins), then [rows of the output,
+    // then [mask rows and table | state | what the resident CTAs share] as uploaded by a batch (the mask ends where the state begins), then [rows of the output,
     // finals], which a batch reads back together with the state, then the CTA partials
     char* blk = nullptr;
     size_t blk_bytes = 0, mask_cap = 0;
     u64* d_coefs = nullptr;
     u64* d_partials = nullptr;
+    u64* d_slots = nullptr;    // slots of a slot program that shared memory does not hold
+    size_t slot_bytes = 0;
+    hlk::ScSync* d_sync = nullptr;
     u64* d_out = nullptr;      // n_vars rows of (2 (degree+1) + 1) Fp2
     u64* d_finals = nullptr;   // k Fp2 behind them
     u64* d_inv_den = nullptr;
@@ -42,7 +46,6 @@ struct hl_rounds {
     u64* d_cfo = nullptr;      // its coefficients by occurrence
     u64* d_nonbase = nullptr;  // one word: bit t set when table t is extension-valued before the first fold
     u64 nonbase = ~0ull;
-    u32 tail_len = hlk::SC_TAIL_LEN;
     size_t out_row() const { return (2 * ((size_t)degree + 1) + 1) * 2; }
 };
 
@@ -76,7 +79,7 @@ int launch_round(hl_rounds* r, int eval_one, int fs, int use_claim, int recover,
     hl_ctx* c = r->ctx;
     const u32 half = (u32)(r->len / 2);
     const bool is_ir = r->poly == hlk::POLY_IR;
-    u32 nb = is_ir ? hlk::sc_ir_blocks(r->ir, half, (int)r->degree, c->sm_count) : hlk::sc_round_blocks(half, c->sm_count);
+    u32 nb = is_ir ? hlk::sc_ir_blocks(half, c->sm_count) : hlk::sc_round_blocks(half, c->sm_count);
     if (nb > r->max_blocks) return fail(c, HL_B200_ERR_DEVICE, "round launch: more partial rows than the buffer holds");  // the two grid rules agree by construction
     cudaError_t e;
     if (is_ir && r->gen && c->slot_kernels) {
@@ -92,7 +95,7 @@ int launch_round(hl_rounds* r, int eval_one, int fs, int use_claim, int recover,
         c->stats.generated_rounds++;
         e = r->gen->launch(r0, per_point, bx, r->d_tables, r->stride, half, r->d_cfo, (int)r->degree, npe, skip, r->d_partials, c->stream);
     } else {
-        e = is_ir ? hlk::sc_round_ir(r->ir, (int)r->k, r->d_tables, r->stride, half, (int)r->degree, eval_one, r->d_partials, nb, c->stream)
+        e = is_ir ? hlk::sc_round_ir(r->ir, r->d_tables, r->stride, half, (int)r->degree, eval_one, r->d_slots, r->d_partials, nb, c->stream)
                   : hlk::sc_round(r->poly, (int)r->k, r->d_tables, r->stride, half, r->d_coefs, eval_one, r->d_partials, nb, c->stream);
     }
     c->stats.kernel_launches++;
@@ -127,7 +130,7 @@ struct GenAsk {  // a slot program's generated kernel, looked up by the caller
 };
 
 int rounds_build(hl_ctx* c, int poly, size_t k, uint32_t n_vars, uint32_t degree, const uint64_t* tables, const uint64_t* coefs,
-                 size_t ncoefs, const std::vector<u32>* plan, hl_rounds** out, hl_tables* built = nullptr, const GenAsk* gen = nullptr) {
+                 size_t ncoefs, const vm::Program* program, hl_rounds** out, hl_tables* built = nullptr, const GenAsk* gen = nullptr) {
     Call g(c);
     if (built) {
         if (int rc = hl_tables_flush_locked(built)) return rc;
@@ -138,18 +141,16 @@ int rounds_build(hl_ctx* c, int poly, size_t k, uint32_t n_vars, uint32_t degree
     r->max_blocks = hlk::sc_round_blocks((u32)(r->len / 2), c->sm_count);
     r->eval_degree = degree;
     if (poly == hlk::POLY_IR) {
-        const std::vector<u32>& pw = *plan;
-        r->eval_degree = r->ir.eval_degree = pw[16];
-        r->ir.all_points = ir::tpair_all_fits(pw.data()) ? 1 : 0;
-        r->ir.plan_words = (u32)pw.size(); r->ir.n_coefs = (u32)ncoefs; r->ir.n_tables = (u32)k;
-        r->ir.n_nodes = pw[1]; r->ir.n_units = pw[2];
-        if (!hlk::sc_ir_fits(r->ir, (int)degree)) {
-            delete r;
-            return fail(c, HL_B200_ERR_UNSUPPORTED, "slot program: tables x nodes x points beyond one CTA's shared memory");
-        }
-        r->max_blocks = hlk::sc_ir_max_blocks((u32)(r->len / 2), c->sm_count);
-        r->tail_len = hlk::sc_ir_tail_len(r->ir, (int)degree);
+        const vm::Program& pg = *program;
+        r->eval_degree = r->ir.eval_degree = pg.degree < degree ? pg.degree : degree;
+        r->ir.n_code = (u32)pg.code.size(); r->ir.n_coefs = (u32)pg.coefs.size(); r->ir.n_tables = (u32)k;
+        r->ir.p_slots = pg.p_slots; r->ir.a_slots = pg.a_slots;
+        r->max_blocks = (u32)c->sm_count * 4;
+        const size_t long_slots = hlk::sc_ir_slot_bytes(r->ir, hlk::sc_ir_blocks((u32)(r->len / 2), c->sm_count)),
+                     run_slots = hlk::sc_run_slot_bytes(poly, r->ir, (int)k, (int)r->eval_degree, c->sm_count);
+        r->slot_bytes = long_slots > run_slots ? long_slots : run_slots;
     }
+    if (r->max_blocks < (u32)c->sm_count) r->max_blocks = (u32)c->sm_count;  // the one-launch rounds have a partial row per SM
     // what the kernels read and no challenge changes, in one upload
     std::vector<char> head;
     auto put = [&](size_t bytes) {
@@ -184,26 +185,30 @@ int rounds_build(hl_ctx* c, int poly, size_t k, uint32_t n_vars, uint32_t degree
                 wts[(pnt - de - 1) * (de + 1) + i] = gl_mul(num, gl_inv(den));
             }
     }
-    const size_t at_cf = put((ncoefs ? ncoefs : 1) * 16);
-    if (ncoefs) memcpy(head.data() + at_cf, coefs, ncoefs * 16);
     const bool is_ir = poly == hlk::POLY_IR;
-    const size_t at_plan = is_ir ? put((size_t)r->ir.plan_words * 4) : 0;
-    if (is_ir) memcpy(head.data() + at_plan, plan->data(), (size_t)r->ir.plan_words * 4);
+    const size_t n_cf = is_ir ? program->coefs.size() : ncoefs;
+    const size_t at_cf = put((n_cf ? n_cf : 1) * 16);
+    if (n_cf) memcpy(head.data() + at_cf, is_ir ? (const void*)program->coefs.data() : (const void*)coefs, n_cf * 16);
+    const size_t at_code = is_ir ? put(program->code.size() * 8) : 0;
+    if (is_ir) memcpy(head.data() + at_code, program->code.data(), program->code.size() * 8);
     r->mask_cap = ((size_t)63 * degree + 2) * 16 + (size_t)63 * (degree + 1) * 16;
     const size_t at_state = head.size() + r->mask_cap, state_bytes = (sizeof(hlk::ScState) + 15) & ~(size_t)15;
-    const size_t at_out = at_state + state_bytes, at_fin = at_out + (n_vars ? n_vars : 1) * r->out_row() * 8, at_part = at_fin + k * 16;
-    r->blk_bytes = at_part + (size_t)r->max_blocks * (degree + 1) * 16;
+    const size_t at_sync = at_state + state_bytes, at_out = at_sync + ((sizeof(hlk::ScSync) + 15) & ~(size_t)15), at_fin = at_out + (n_vars ? n_vars : 1) * r->out_row() * 8, at_part = at_fin + k * 16;
+    const size_t at_slots = at_part + (size_t)r->max_blocks * (degree + 1) * 16;
+    r->blk_bytes = at_slots + r->slot_bytes;
     int rc = built ? HL_B200_OK : dev_alloc(c, (void**)&r->d_tables, k * r->stride * 16);
     if (!rc) rc = dev_alloc(c, (void**)&r->blk, r->blk_bytes);
     if (!rc) {
         r->d_inv_den = (u64*)(r->blk + at_den);
         r->d_extrap = extrapolates ? (u64*)(r->blk + at_ex) : nullptr;
         r->d_coefs = (u64*)(r->blk + at_cf);
-        if (is_ir) { r->ir.plan = (const u32*)(r->blk + at_plan); r->ir.coefs = (const u64*)(r->blk + at_cf); }
+        if (is_ir) { r->ir.code = (const u64*)(r->blk + at_code); r->ir.coefs = (const u64*)(r->blk + at_cf); }
         r->d_state = (hlk::ScState*)(r->blk + at_state);
         r->d_out = (u64*)(r->blk + at_out);
         r->d_finals = (u64*)(r->blk + at_fin);
         r->d_partials = (u64*)(r->blk + at_part);
+        r->d_slots = r->slot_bytes ? (u64*)(r->blk + at_slots) : nullptr;
+        r->d_sync = (hlk::ScSync*)(r->blk + at_sync);
     }
     if (!rc && !built) rc = h2d_owned(c, r->d_tables, tables, k * r->stride * 16);
     if (!rc) rc = h2d_owned(c, r->blk, head.data(), head.size());
@@ -260,15 +265,11 @@ int hl_b200_rounds_new_ir(hl_ctx* c, size_t k, uint32_t n_vars, uint32_t degree,
         snprintf(buf, sizeof buf, "rounds_new_ir: malformed program (check %d)", why);
         return fail(c, HL_B200_ERR_ARG, buf);
     }
-    std::vector<u32> plan;
-    if (int why = ir::build_plan(sh, words, degree, plan)) {
-        char buf[96];
-        snprintf(buf, sizeof buf, "rounds_new_ir: the program does not fit the evaluator's plan (reason %d)", why);
-        return fail(c, HL_B200_ERR_UNSUPPORTED, buf);
-    }
+    vm::Compiler prog;
+    prog.run(sh, words, reinterpret_cast<const fp2*>(coefs));
     GenAsk gen;
     gen.entry = sg::find(ir::signature(sh, words, reinterpret_cast<const fp2*>(coefs), &gen.cfo));
-    return rounds_build(c, hlk::POLY_IR, k, n_vars, degree, tables, coefs, ncoefs, &plan, out, nullptr, &gen);
+    return rounds_build(c, hlk::POLY_IR, k, n_vars, degree, tables, coefs, ncoefs, &prog.out, out, nullptr, &gen);
 }
 
 int hl_b200_rounds_from_tables(hl_ctx* c, int poly, uint32_t degree, hl_tables* t, const uint64_t* coefs, size_t ncoefs, hl_rounds** out) {
@@ -296,11 +297,11 @@ int hl_b200_rounds_from_tables_ir(hl_ctx* c, uint32_t degree, hl_tables* t, cons
         return fail(c, HL_B200_ERR_UNSUPPORTED, "rounds_from_tables_ir: table count, degree or program size beyond the evaluator's limits");
     ir::Shape sh{(u32)k, n_nodes, n_terms, (u32)ncoefs, (u32)n_words};
     if (ir::validate(sh, words)) return fail(c, HL_B200_ERR_ARG, "rounds_from_tables_ir: malformed program");
-    std::vector<u32> plan;
-    if (ir::build_plan(sh, words, degree, plan)) return fail(c, HL_B200_ERR_UNSUPPORTED, "rounds_from_tables_ir: the program does not fit the evaluator's plan");
+    vm::Compiler prog;
+    prog.run(sh, words, reinterpret_cast<const fp2*>(coefs));
     GenAsk gen;
     gen.entry = sg::find(ir::signature(sh, words, reinterpret_cast<const fp2*>(coefs), &gen.cfo));
-    return rounds_build(c, hlk::POLY_IR, k, n_vars, degree, nullptr, coefs, ncoefs, &plan, out, t, &gen);
+    return rounds_build(c, hlk::POLY_IR, k, n_vars, degree, nullptr, coefs, ncoefs, &prog.out, out, t, &gen);
 }
 
 void hl_b200_rounds_free(hl_rounds* r) {
@@ -380,17 +381,20 @@ int hl_b200_rounds_batched(hl_rounds* r, uint32_t nd, hl_fs_state* fs, const uin
     st.keyed = fs->keyed;
     st.claim = f2(fs->claim[0], fs->claim[1]);
     u64 *d_mask = nullptr, *d_mtab = nullptr;
-    const size_t mlen = mask_coeffs ? (size_t)mask_vars * r->degree + 2 : 0;
-    const size_t tab_words = mask_coeffs ? (size_t)mask_vars * (r->degree + 1) * 2 : 0;
-    std::vector<u64> up(mlen * 2 + tab_words + (sizeof st + 7) / 8);  // mask, its table, state: one upload that ends with the state
+    const size_t row_words = mask_coeffs ? (size_t)mask_vars * r->degree * 2 : 0, tab_words = mask_coeffs ? (size_t)mask_vars * (r->degree + 1) * 2 : 0;
+    const size_t st_words = (size_t)((char*)r->d_out - (char*)r->d_state) / 8;  // the state and, zeroed, what the resident CTAs share
+    std::vector<u64> up(row_words + tab_words + st_words);
     int rc = HL_B200_OK;
     if (mask_coeffs) {
-        st.mask_c = f2(mask_c[0], mask_c[1]);
-        const fp2* co = reinterpret_cast<const fp2*>(mask_coeffs);
-        st.ap = co[1];  // a' times the empty product
+        // the mask scaled by its challenge: the device then adds c g_j without a product
+        const fp2 mc = f2(mask_c[0], mask_c[1]);
+        std::vector<fp2> scaled((size_t)mask_vars * r->degree + 2);
+        for (size_t i = 0; i < scaled.size(); i++) scaled[i] = f2_mul(mc, reinterpret_cast<const fp2*>(mask_coeffs)[i]);
+        const fp2* co = scaled.data();
+        st.ap = co[1];  // c a' times the empty product
         // per round j and point x: 2^(N-1-j) (a0 + sum_{i>j} u_i(1)/2 + u_j(x)) (sumcheck.rs:260-295): the part of g_j(x) no challenge enters
         const u64 half = gl_inv(2);
-        u64* const mtab = up.data() + mlen * 2;
+        u64* const mtab = up.data() + row_words;
         fp2 run = f2(0, 0);
         for (int i = (int)mask_vars - 1; i >= 0; i--) {
             const fp2* ai = co + 2 + (size_t)i * r->degree;
@@ -406,19 +410,20 @@ int hl_b200_rounds_batched(hl_rounds* r, uint32_t nd, hl_fs_state* fs, const uin
             for (u32 e = 0; e < r->degree; e++) u1 = f2_add(u1, ai[e]);
             run = f2_add(run, f2_mul_base(u1, half));
         }
-        memcpy(up.data(), mask_coeffs, mlen * 16);
-        d_mask = (u64*)r->d_state - mlen * 2 - tab_words;
+        memcpy(up.data(), co + 2, row_words * 8);
+        d_mask = (u64*)r->d_state - row_words - tab_words;
         d_mtab = (u64*)r->d_state - tab_words;
     }
-    memcpy(up.data() + mlen * 2 + tab_words, &st, sizeof st);
-    rc = h2d(c, (u64*)r->d_state - mlen * 2 - tab_words, up.data(), (mlen * 2 + tab_words) * 8 + sizeof st);
-    const u32 first = r->next;
+    memcpy(up.data() + row_words + tab_words, &st, sizeof st);
+    rc = h2d(c, (u64*)r->d_state - row_words - tab_words, up.data(), up.size() * 8);
+    // with the generated kernels switched on they take the rounds down to 2^11 pairs: the switch is there to compare them
+    const u32 first = r->next, run_len = r->gen && c->slot_kernels ? 1u << 12 : hlk::sc_run_len(r->poly);
     bool have_claim = fs->recover_one && fs->have_claim;
     {
         Timed t(c, HL_T_ROUNDS);
         u32 i = 0;
         if (r->poly == hlk::POLY_IR) {
-            for (; i < nd && !rc && r->len > r->tail_len; i++) {
+            for (; i < nd && !rc && r->len > run_len; i++) {
                 rc = launch_round(r, have_claim ? 0 : 1, 1, have_claim ? 1 : 0, fs->recover_one ? 1 : 0, d_mask, d_mtab, (int)mask_vars);
                 if (!rc) rc = launch_fold(r);
                 have_claim = fs->recover_one != 0;
@@ -428,7 +433,7 @@ int hl_b200_rounds_batched(hl_rounds* r, uint32_t nd, hl_fs_state* fs, const uin
             // (two launches per round, every table word read once and written once); `pending`: the tables are still stored at
             // twice r->len
             bool pending = false;
-            for (; i < nd && !rc && r->len > r->tail_len; i++) {
+            for (; i < nd && !rc && r->len > run_len; i++) {
                 const int eval_one = have_claim ? 0 : 1;
                 // While a round's arithmetic fills the machine (the first rounds of a large cube) the fused pass is the slower
                 // one (it folds both halves before it can evaluate: measured 79 us against 40 + 15 at 2^19 pairs); once a round
@@ -460,19 +465,17 @@ int hl_b200_rounds_batched(hl_rounds* r, uint32_t nd, hl_fs_state* fs, const uin
                 if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "fold launch", e);
             }
         }
-        if (!rc && i < nd) {  // the short rounds: one CTA, no launches in between
+        if (!rc && i < nd) {  // the short rounds: one launch (sumcheck_run.cu)
             hlk::ScStep a;
             a.partials = r->d_partials; a.nblocks = 1; a.degree = (int)r->degree; a.round = (int)r->next;
             a.use_claim = 0; a.recover = fs->recover_one ? 1 : 0; a.fs = 1; a.mask = d_mask; a.mask_tab = d_mtab; a.mask_vars = (int)mask_vars;
             a.inv_den = r->d_inv_den; a.state = r->d_state; a.out = r->d_out;
             a.eval_degree = (int)r->eval_degree; a.extrap = r->d_extrap;
             const u32 left = nd - i;
-            cudaError_t e = r->poly == hlk::POLY_IR
-                                ? hlk::sc_tail_ir(r->ir, (int)r->k, r->d_tables, r->stride, (u32)r->len, (int)r->degree, a, (int)left, have_claim ? 1 : 0, c->stream)
-                                : hlk::sc_tail(r->poly, (int)r->k, r->d_tables, r->stride, (u32)r->len, r->d_coefs, a, (int)left, have_claim ? 1 : 0,
-                                               r->d_partials, c->stream);
+            cudaError_t e = hlk::sc_run(r->poly, r->ir, (int)r->k, r->d_tables, r->stride, (u32)r->len, r->d_coefs, a, (int)left, have_claim ? 1 : 0, r->d_sync,
+                                        r->d_partials, r->d_slots, c->sm_count, c->stream);
             c->stats.kernel_launches++;
-            if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "tail rounds launch", e);
+            if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "short rounds launch", e);
             r->len >>= left;
             r->next += left;
         }
@@ -488,6 +491,9 @@ int hl_b200_rounds_batched(hl_rounds* r, uint32_t nd, hl_fs_state* fs, const uin
     if (!rc) rc = d2h(c, got.data(), r->d_state, last ? got.size() : o_fin);
     if (!rc) rc = sync(c, "rounds_batched");
     if (rc) return rc;
+    hlk::ScSync sync_got;
+    memcpy(&sync_got, got.data() + ((char*)r->d_sync - (char*)r->d_state), sizeof sync_got);
+    if (sync_got.failed) return fail(c, HL_B200_ERR_TIMEOUT, "rounds_batched: a device wait ran out");
     memcpy(out, got.data() + o_out + first * r->out_row() * 8, (size_t)nd * r->out_row() * 8);
     memcpy(&st, got.data(), sizeof st);
     if (last) {

@@ -1,0 +1,187 @@
+// The Fiat-Shamir step of a sumcheck round, by one warp (sumcheck/rounds.rs:94-160, transcript.rs:67-148, sumcheck.rs:194-299).
+//
+// A serial chain runs through every round: sums -> masked message -> two hashes -> challenge -> next round's tables.  So what does not
+// lie on it is done beside it: the three parts are called apart, and only `step_challenge` is waited for.
+//
+//   step_ahead      before the sums are there: the mask's round polynomial, one evaluation point per lane, and the message's head.
+//                   The host scales the mask by its challenge c, so that no product is left for later:
+//                   c g_j(x) = c 2^(N-1-j) (a0 + sum_{i>j} u_i(1)/2 + u_j(x))  [table]  + 2^(N-1-j) acc + x ap,
+//                   acc = c sum_{i<j} u_i(r_i), ap = c a' prod_{i<j} r_i.
+//   step_challenge  s(1) from the claim, the points above the attained degree, the message (one addition per point), absorb, squeeze.
+//                   Every lane computes the hashes; lane 0 writes.
+//   step_after      the next claim and the mask's running terms, which the NEXT round's message needs: while the other warps fold.
+#pragma once
+#include "b3.cuh"
+#include "gl_field.cuh"
+#include "sumcheck.h"
+
+namespace {
+
+__device__ __forceinline__ fp2 ld2(const u64* p) {
+    ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
+    return f2(v.x, v.y);
+}
+__device__ __forceinline__ void st2(u64* p, fp2 v) { *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(v.c0, v.c1); }
+
+// one chunk, at most 1024 bytes
+__device__ __forceinline__ void hash_small(const uint32_t* key, const uint32_t* words, u32 len, uint32_t (&out)[8]) {
+    b3::init_cv(out, key);
+    const u32 nb = len ? (len + 63) / 64 : 1;
+#pragma unroll 1
+    for (u32 b = 0; b < nb; b++) {
+        uint32_t m[16];
+#pragma unroll
+        for (int i = 0; i < 16; i++) m[i] = words[16 * b + i];
+        uint32_t flags = (key ? b3::KEYED : 0u) | (b == 0 ? b3::CHUNK_START : 0u) | (b == nb - 1 ? (b3::CHUNK_END | b3::ROOT) : 0u);
+        b3::compress(out, m, 0, b == nb - 1 ? len - 64 * b : 64, flags);
+    }
+}
+
+__device__ __forceinline__ u64 reduce_le16(const uint32_t* w) {  // 128-bit little-endian draw mod p (transcript.rs:133-148)
+    return gl_reduce128(((u64)w[1] << 32) | w[0], ((u64)w[3] << 32) | w[2]);
+}
+
+struct StepSmem {
+    __align__(16) u64 sums[2 * hlk::SC_MAX_POINTS];
+    __align__(16) uint32_t msg[64];  // 256 bytes
+};
+
+// v 2^k mod p, 0 <= k <= 62
+__device__ __forceinline__ u64 gl_mul_pow2(u64 v, int k) { return gl_reduce128(v << k, k ? v >> (64 - k) : 0ull); }
+
+__device__ __forceinline__ fp2 shfl_down8_f2(fp2 v, int d) {  // within groups of eight lanes
+    u32 a0 = __shfl_down_sync(0xffffffffu, (u32)v.c0, d, 8), a1 = __shfl_down_sync(0xffffffffu, (u32)(v.c0 >> 32), d, 8);
+    u32 b0 = __shfl_down_sync(0xffffffffu, (u32)v.c1, d, 8), b1 = __shfl_down_sync(0xffffffffu, (u32)(v.c1 >> 32), d, 8);
+    return f2(((u64)a1 << 32) | a0, ((u64)b1 << 32) | b0);
+}
+
+// What the steps of a batch read, resolved once: operands that sit in registers or shared memory.
+struct StepArgs {
+    int degree, recover, fs, mask_vars, eval_degree;
+    const fp2* rows;    // c a_{j,e}: `degree` per round, from round `row0` on; NULL: no mask
+    const fp2* tab;     // degree + 1 per round, likewise
+    int row0;
+    const u64* inv_den;
+    const u64* extrap;  // or NULL
+    hlk::ScState* state;
+    u64* out;
+};
+
+__device__ __forceinline__ fp2 step_ahead(const StepArgs& a, StepSmem& sm, int j, int lane) {
+    const int np = a.degree + 1;
+    const hlk::ScState* st = a.state;
+    if (!a.fs) return f2(0, 0);
+    // state' = H(state || LE64(8) || "sc-round" || LE64(16 np) || bytes) (transcript.rs:67-74); the values go to word 14 on
+    const int nw = 14 + 4 * np;
+    for (int i = lane; i < 64; i += 32)
+        if (i < 14 || i >= nw)
+            sm.msg[i] = i < 8 ? st->state[i] : i == 8 ? 8u : i == 10 ? 0x722d6373u : i == 11 ? 0x646e756fu : i == 12 ? 16u * np : 0u;  // "sc-r" "ound"
+    fp2 g = f2(0, 0);
+    if (a.rows && lane < np) {
+        const int sh = a.mask_vars - 1 - j;  // mask_vars <= 63
+        g = f2_add(a.tab[(size_t)(j - a.row0) * np + lane], f2(gl_mul_pow2(st->acc.c0, sh), gl_mul_pow2(st->acc.c1, sh)));
+        g = f2_add(g, f2_mul_base(st->ap, (u64)lane));
+    }
+    __syncwarp();
+    return g;
+}
+
+// sm.sums holds the round's sums at the points 0 .. eval_degree (the point 1 left open when use_claim); returns the challenge in every lane
+__device__ __forceinline__ fp2 step_challenge(const StepArgs& a, StepSmem& sm, int j, bool use_claim, fp2 g, int lane) {
+    const int np = a.degree + 1;
+    hlk::ScState* st = a.state;
+    fp2* s = reinterpret_cast<fp2*>(sm.sums);
+    if (lane == 0 && use_claim) s[1] = f2_sub(st->claim, s[0]);  // s(1) = claim - s(0) (rounds.rs:137-140)
+    __syncwarp();
+    if (a.extrap && a.eval_degree < a.degree) {
+        // a polynomial of degree eval_degree is fixed by its values at 0..eval_degree: the points above, exactly
+        fp2 v = f2(0, 0);
+        if (lane > a.eval_degree && lane < np) {
+            const u64* wrow = a.extrap + (size_t)(lane - a.eval_degree - 1) * (a.eval_degree + 1);
+            for (int i = 0; i <= a.eval_degree; i++) v = f2_add(v, f2_mul_base(s[i], wrow[i]));
+        }
+        __syncwarp();
+        if (lane > a.eval_degree && lane < np) s[lane] = v;
+        __syncwarp();
+    }
+    u64* orow = a.out + (size_t)j * (2 * (size_t)np + 1) * 2;
+    if (lane < np) st2(orow + 2 * lane, s[lane]);
+    if (!a.fs) return f2(0, 0);  // plain round(): the host drives the transcript
+    if (lane < np) {
+        const fp2 m = f2_add(s[lane], g);
+        st2(orow + 2 * (np + lane), m);
+        uint2* mw = reinterpret_cast<uint2*>(sm.msg + 14 + 4 * lane);
+        mw[0] = make_uint2((u32)m.c0, (u32)(m.c0 >> 32));
+        mw[1] = make_uint2((u32)m.c1, (u32)(m.c1 >> 32));
+    }
+    __syncwarp();
+    const uint32_t* key = st->keyed ? st->key : nullptr;
+    uint32_t h[8];
+    hash_small(key, sm.msg, 56 + 16 * np, h);
+    // squeeze: out = H(state || "squeeze" || LE64(counter)); counter++; state = out (transcript.rs:120-130)
+    const u64 ctr = st->counter;
+    uint32_t m[16] = {h[0], h[1], h[2], h[3], h[4], h[5], h[6], h[7],
+                      0x65757173u,                                   // "sque"
+                      0x00657a65u | ((uint32_t)(ctr & 0xff) << 24),  // "eze" then counter byte 0
+                      (uint32_t)(ctr >> 8), (uint32_t)(ctr >> 40),   // counter bytes 5..7; the message ends there
+                      0u, 0u, 0u, 0u};
+    b3::init_cv(h, key);
+    b3::compress(h, m, 0, 47, b3::CHUNK_START | b3::CHUNK_END | b3::ROOT | (key ? b3::KEYED : 0u));
+    const fp2 r = f2(reduce_le16(h), reduce_le16(h + 4));
+    __syncwarp();
+    if (lane == 0) {
+        st->counter = ctr + 1;
+#pragma unroll
+        for (int i = 0; i < 8; i++) st->state[i] = h[i];
+        st->r = r;
+        st2(orow + 4 * np, r);
+    }
+    return r;
+}
+
+// Every lane runs the SAME product tree over eight (or four) factors and one multiplier: lanes 0..7 a Lagrange numerator
+// prod_{j != i} (r - j) times s_i / den_i, lanes 8..15 a power r^e times the mask coefficient, lane 16 the product r ap; sums over groups
+// of eight lanes give the next claim (rounds.rs:145-147, mle.rs:338-351) and c u_j(r_j).
+__device__ __forceinline__ void step_after(const StepArgs& a, StepSmem& sm, int j, fp2 r, int lane) {
+    const int np = a.degree + 1;
+    const bool masked = a.rows != nullptr;
+    hlk::ScState* st = a.state;
+    if (!a.fs || (!a.recover && !masked)) return;
+    const int grp = lane >> 3, li = lane & 7;
+    fp2 f[8], mult = f2(0, 0);
+#pragma unroll
+    for (int t = 0; t < 8; t++) f[t] = f2(1, 0);
+    if (grp == 0) {
+        if (a.recover && li < np) {
+#pragma unroll
+            for (int t = 0; t < 7; t++) {  // the points other than li, in order
+                const int jj = t < li ? t : t + 1;
+                if (jj < np) f[t] = f2(gl_sub(r.c0, (u64)jj), r.c1);
+            }
+            mult = f2_mul_base(reinterpret_cast<const fp2*>(sm.sums)[li], a.inv_den[li]);
+        }
+    } else if (grp == 1) {
+        if (masked && li < a.degree) {  // r^(li + 1) c a_{j, li + 1}
+#pragma unroll
+            for (int t = 0; t < 7; t++)
+                if (t <= li) f[t] = r;
+            mult = a.rows[(size_t)(j - a.row0) * a.degree + li];
+        }
+    } else if (lane == 16 && masked) {
+        f[0] = r;
+        f[1] = st->ap;
+        mult = f2(1, 0);
+    }
+    fp2 prod = f2_mul(f2_mul(f[0], f[1]), f2_mul(f[2], f[3]));
+    if (a.degree > 4) prod = f2_mul(prod, f2_mul(f2_mul(f[4], f[5]), f2_mul(f[6], f[7])));
+    fp2 term = f2_mul(prod, mult);
+    const fp2 own = term;
+#pragma unroll
+    for (int off = 4; off >= 1; off >>= 1) term = f2_add(term, shfl_down8_f2(term, off));
+    if (lane == 0 && a.recover) st->claim = term;
+    if (lane == 8 && masked) st->acc = f2_add(st->acc, term);
+    if (lane == 16 && masked) st->ap = own;
+    __syncwarp();
+}
+
+}  // namespace
