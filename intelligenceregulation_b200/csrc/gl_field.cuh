@@ -331,6 +331,25 @@ GL_HD fp2 f2_mul(fp2 a, fp2 b) {
     return f2(gl_mul_add2(a.c0, b.c0, a17, b.c1), gl_mul_add2(a.c0, b.c1, a.c1, b.c0));
 #endif
 }
+// Lazy forms (any words congruent to the value) for chains that end in one `f2_canon`:
+//   f2_mul_lazy, f2_mul_base_lazy    any operands       f2_add_lazy(u, v)    v canonical
+GL_HD fp2 f2_canon(fp2 a) { return f2(gl_canon_fast(a.c0), gl_canon_fast(a.c1)); }
+GL_HD fp2 f2_add_lazy(fp2 u, fp2 v) { return f2(gl_add_lazy(u.c0, v.c0), gl_add_lazy(u.c1, v.c1)); }
+GL_HD fp2 f2_mul_base_lazy(fp2 a, u64 b) { return f2(gl_mul_lazy(a.c0, b), gl_mul_lazy(a.c1, b)); }
+GL_HD fp2 f2_mul_lazy(fp2 a, fp2 b) {
+#ifdef GL_DEVICE_CHAINS
+    const u64 q = (u64)(u32)a.c1 * 7u, t = (a.c1 >> 32) * 7u + (q >> 32);
+    u32 p0, p1, p2, p3, cp = 0, s0, s1, s2, s3, cs = 0;
+    gl_product(a.c0, b.c0, p0, p1, p2, p3);
+    gl_product(a.c0, b.c1, s0, s1, s2, s3);
+    gl_product_acc((t << 32) | (u32)q, b.c1, p0, p1, p2, p3, cp);
+    gl_product_acc(a.c1, b.c0, s0, s1, s2, s3, cs);
+    gl_product_top((u32)(t >> 32), b.c1, p2, p3, cp);
+    return f2(gl_red129_lazy(p0, p1, p2, p3, cp), gl_red129_lazy(s0, s1, s2, s3, cs));
+#else
+    return f2_mul(f2_canon(a), f2_canon(b));
+#endif
+}
 GL_HD bool f2_is_zero(fp2 a) { return (a.c0 | a.c1) == 0; }
 // conj(a) / (a0^2 - 7 a1^2) (field.rs:180-185)
 GL_HD fp2 f2_inv(fp2 a) {

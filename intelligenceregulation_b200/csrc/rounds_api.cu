@@ -79,7 +79,7 @@ int launch_round(hl_rounds* r, int eval_one, int fs, int use_claim, int recover,
     hl_ctx* c = r->ctx;
     const u32 half = (u32)(r->len / 2);
     const bool is_ir = r->poly == hlk::POLY_IR;
-    u32 nb = is_ir ? hlk::sc_ir_blocks(half, c->sm_count) : hlk::sc_round_blocks(half, c->sm_count);
+    u32 nb = is_ir ? hlk::sc_ir_rows(r->ir, half, c->sm_count) : hlk::sc_round_blocks(half, c->sm_count);
     if (nb > r->max_blocks) return fail(c, HL_B200_ERR_DEVICE, "round launch: more partial rows than the buffer holds");  // the two grid rules agree by construction
     cudaError_t e;
     if (is_ir && r->gen && c->slot_kernels) {
@@ -95,7 +95,7 @@ int launch_round(hl_rounds* r, int eval_one, int fs, int use_claim, int recover,
         c->stats.generated_rounds++;
         e = r->gen->launch(r0, per_point, bx, r->d_tables, r->stride, half, r->d_cfo, (int)r->degree, npe, skip, r->d_partials, c->stream);
     } else {
-        e = is_ir ? hlk::sc_round_ir(r->ir, r->d_tables, r->stride, half, (int)r->degree, eval_one, r->d_slots, r->d_partials, nb, c->stream)
+        e = is_ir ? hlk::sc_round_ir(r->ir, r->d_tables, r->stride, half, (int)r->degree, eval_one, r->d_slots, r->d_partials, c->sm_count, c->stream)
                   : hlk::sc_round(r->poly, (int)r->k, r->d_tables, r->stride, half, r->d_coefs, eval_one, r->d_partials, nb, c->stream);
     }
     c->stats.kernel_launches++;
@@ -124,6 +124,14 @@ namespace {
 // the evaluator of either kind; `words` is the data form of the polynomial when poly == POLY_IR
 constexpr size_t FUSED_FOLD_MAX_PAIRS = (size_t)1 << 15;
 
+// A program of more than some twenty instructions is also cut into parts of about that many, for the rounds with few pairs.
+void compile(vm::Compiler& prog, const ir::Shape& sh, const uint32_t* words, const uint64_t* coefs) {
+    const fp2* cf = reinterpret_cast<const fp2*>(coefs);
+    prog.run(sh, words, cf);
+    const u32 parts = ((u32)prog.out.code.size() + 19) / 20;
+    if (parts > 1) prog.split(sh, words, cf, parts < vm::MAX_PARTS ? parts : vm::MAX_PARTS);
+}
+
 struct GenAsk {  // a slot program's generated kernel, looked up by the caller
     const sg::Entry* entry = nullptr;
     std::vector<fp2> cfo;
@@ -144,9 +152,10 @@ int rounds_build(hl_ctx* c, int poly, size_t k, uint32_t n_vars, uint32_t degree
         const vm::Program& pg = *program;
         r->eval_degree = r->ir.eval_degree = pg.degree < degree ? pg.degree : degree;
         r->ir.n_code = (u32)pg.code.size(); r->ir.n_coefs = (u32)pg.coefs.size(); r->ir.n_tables = (u32)k;
-        r->ir.p_slots = pg.p_slots; r->ir.a_slots = pg.a_slots;
+        r->ir.p_slots = pg.p_slots; r->ir.a_slots = pg.a_slots; r->ir.parts = pg.parts;
+        for (u32 w = 0; w < pg.parts; w++) r->ir.start[w] = pg.start[w];
         r->max_blocks = (u32)c->sm_count * 4;
-        const size_t long_slots = hlk::sc_ir_slot_bytes(r->ir, hlk::sc_ir_blocks((u32)(r->len / 2), c->sm_count)),
+        const size_t long_slots = hlk::sc_ir_slot_bytes(r->ir, c->sm_count),
                      run_slots = hlk::sc_run_slot_bytes(poly, r->ir, (int)k, (int)r->eval_degree, c->sm_count);
         r->slot_bytes = long_slots > run_slots ? long_slots : run_slots;
     }
@@ -266,7 +275,7 @@ int hl_b200_rounds_new_ir(hl_ctx* c, size_t k, uint32_t n_vars, uint32_t degree,
         return fail(c, HL_B200_ERR_ARG, buf);
     }
     vm::Compiler prog;
-    prog.run(sh, words, reinterpret_cast<const fp2*>(coefs));
+    compile(prog, sh, words, coefs);
     GenAsk gen;
     gen.entry = sg::find(ir::signature(sh, words, reinterpret_cast<const fp2*>(coefs), &gen.cfo));
     return rounds_build(c, hlk::POLY_IR, k, n_vars, degree, tables, coefs, ncoefs, &prog.out, out, nullptr, &gen);
@@ -298,7 +307,7 @@ int hl_b200_rounds_from_tables_ir(hl_ctx* c, uint32_t degree, hl_tables* t, cons
     ir::Shape sh{(u32)k, n_nodes, n_terms, (u32)ncoefs, (u32)n_words};
     if (ir::validate(sh, words)) return fail(c, HL_B200_ERR_ARG, "rounds_from_tables_ir: malformed program");
     vm::Compiler prog;
-    prog.run(sh, words, reinterpret_cast<const fp2*>(coefs));
+    compile(prog, sh, words, coefs);
     GenAsk gen;
     gen.entry = sg::find(ir::signature(sh, words, reinterpret_cast<const fp2*>(coefs), &gen.cfo));
     return rounds_build(c, hlk::POLY_IR, k, n_vars, degree, nullptr, coefs, ncoefs, &prog.out, out, t, &gen);

@@ -13,6 +13,8 @@
 // An instruction is one 64-bit word (op, source, class and index of a coefficient, slot or table), the same for all threads of a CTA.
 // Exact arithmetic on canonical words: any order of the sums and products gives the graph's value.
 #pragma once
+#include <algorithm>
+#include <utility>
 #include <vector>
 
 #include "slot_ir.cuh"
@@ -32,9 +34,14 @@ GL_HD u32 cls_of(u64 w) { return ((u32)w >> 6) & 3u; }
 GL_HD u32 idx_of(u64 w) { return (u32)w >> 16; }
 GL_HD u32 coef_of(u64 w) { return (u32)(w >> 32); }
 
+// `parts` programs whose values sum to the polynomial's: part w starts at code[start[w]].  One part is the whole; where a round has fewer
+// pairs than the device has threads, several threads take a pair's parts.
+constexpr u32 MAX_PARTS = 4;
 struct Program {
     std::vector<u64> code;
     std::vector<fp2> coefs;   // the general ones, in the order of their first use
+    u32 parts = 1;
+    u32 start[MAX_PARTS + 1] = {0};  // [parts]: the end
     u32 p_slots = 0, a_slots = 0;
     u32 degree = 0;           // attained along one variable
 };
@@ -42,11 +49,65 @@ struct Program {
 class Compiler {
   public:
     Program out;
+    // the whole, at code[0]
     void run(const ir::Shape& s, const u32* w, const fp2* cf) {
         parse(s, w, cf);
         out.degree = ir::attained_degree(s, w);
-        sum(nodes_[s.n_nodes].units);
-        out.code.push_back(ins(END, 0, 0, 0, 0));
+        const std::vector<Node> graph = nodes_;
+        part(graph.back().units);
+        out.start[1] = (u32)out.code.size();
+    }
+    // behind it, the same in `parts` parts of about equal cost (fewer where there is less to share out)
+    void split(const ir::Shape& s, const u32* w, const fp2* cf, u32 parts) {
+        parse(s, w, cf);
+        const std::vector<Node> graph = nodes_;
+        // a term whose one non-linear factor is a sum that only it uses: the sum's units, each under the term's other factors
+        struct Item { size_t prefix; Unit u; u32 cost; };
+        std::vector<Unit> prefixes;
+        std::vector<Item> items;
+        count_uses();
+        for (auto& u : nodes_.back().units) {
+            Unit pre{u.c, {}};
+            u32 non = 0, inner = 0;
+            for (u32 f : u.f) {
+                if (is_linear(f)) pre.f.push_back(f);
+                else { non++; inner = f & ~ir::IR_NODE; }
+            }
+            prefixes.push_back(non == 1 && nodes_[inner].uses == 1 ? pre : Unit{f2(1, 0), {}});
+            if (non == 1 && nodes_[inner].uses == 1)
+                for (auto& v : nodes_[inner].units) items.push_back({prefixes.size() - 1, v, unit_cost(v)});
+            else items.push_back({prefixes.size() - 1, u, unit_cost(u)});
+        }
+        std::sort(items.begin(), items.end(), [](const Item& x, const Item& y) { return x.cost > y.cost; });
+        if (parts > items.size()) parts = (u32)items.size();
+        if (parts < 2) return;
+        std::vector<std::vector<const Item*>> bins(parts);
+        std::vector<u32> load(parts, 0);
+        for (auto& it : items) {  // the largest first, each to the lightest part
+            const size_t w0 = std::min_element(load.begin(), load.end()) - load.begin();
+            bins[w0].push_back(&it);
+            load[w0] += it.cost + 1;
+        }
+        out.parts = parts;
+        for (u32 k = 0; k < parts; k++) {
+            nodes_ = graph;
+            std::vector<Unit> top;
+            for (size_t p = 0; p < prefixes.size(); p++) {
+                Node sum;
+                for (auto* it : bins[k])
+                    if (it->prefix == p) sum.units.push_back(it->u);
+                if (sum.units.empty()) continue;
+                const Unit& pre = prefixes[p];
+                if (pre.f.empty() && pre.c.c0 == 1 && pre.c.c1 == 0) { top.insert(top.end(), sum.units.begin(), sum.units.end()); continue; }
+                Unit u = pre;
+                u.f.push_back(ir::IR_NODE | (u32)nodes_.size());
+                nodes_.push_back(sum);
+                top.push_back(u);
+            }
+            out.start[k] = (u32)out.code.size();
+            part(top);
+        }
+        out.start[parts] = (u32)out.code.size();
     }
 
   private:
@@ -80,19 +141,52 @@ class Compiler {
             }
         }
         for (u32 t = 0; t < s.n_terms; t++) product(nodes_[s.n_nodes]);
+        mark_linear();
+    }
+    void mark_linear() {  // nodes refer to earlier ones only
         for (auto& nd : nodes_)
-            for (auto& u : nd.units) {
-                if (u.f.size() > 1 || (u.f.size() == 1 && (u.f[0] & ir::IR_NODE) && !nodes_[u.f[0] & ~ir::IR_NODE].linear)) nd.linear = false;
-            }
-        // what the last node needs, and how often
+            for (auto& u : nd.units)
+                if (u.f.size() > 1 || (u.f.size() == 1 && !is_linear(u.f[0]))) nd.linear = false;
+    }
+    void count_uses() {  // what the last node needs, and how often
         std::vector<bool> live(nodes_.size(), false);
         live.back() = true;
+        for (auto& nd : nodes_) nd.uses = 0;
         for (size_t n = nodes_.size(); n-- > 0;) {
             if (!live[n]) continue;
             for (auto& u : nodes_[n].units)
                 for (u32 f : u.f)
                     if (f & ir::IR_NODE) { live[f & ~ir::IR_NODE] = true; nodes_[f & ~ir::IR_NODE].uses++; }
         }
+    }
+    // instructions, about; a shared node counts with everyone who uses it, since it may end up in several parts
+    u32 unit_cost(const Unit& u) const {
+        u32 c = 2;
+        for (u32 f : u.f) c += factor_cost(f);
+        return c;
+    }
+    u32 factor_cost(u32 f) const {
+        if (!(f & ir::IR_NODE)) return 1;
+        u32 c = 1;
+        for (auto& u : nodes_[f & ~ir::IR_NODE].units) { c += unit_cost(u); if (c > 4096) return 4096; }
+        return c;
+    }
+    void part(const std::vector<Unit>& top) {
+        Node root;
+        root.units = top;
+        nodes_.push_back(root);
+        mark_linear();
+        count_uses();
+        p_free_.clear();
+        a_free_.clear();
+        // slot numbers start over in every part; the counts are the largest
+        const u32 p_most = out.p_slots, a_most = out.a_slots;
+        out.p_slots = out.a_slots = 0;
+        const std::vector<Unit> units = nodes_.back().units;
+        sum(units);
+        out.code.push_back(ins(END, 0, 0, 0, 0));
+        out.p_slots = std::max(out.p_slots, p_most);
+        out.a_slots = std::max(out.a_slots, a_most);
     }
     static u32 take(std::vector<u32>& free_list, u32& high) {
         if (!free_list.empty()) { const u32 q = free_list.back(); free_list.pop_back(); return q; }
@@ -254,20 +348,21 @@ class Compiler {
 // Fp2 entries of one thread's slots; with one point per thread R and A are values at that point
 GL_HD u32 slot_entries(u32 p_slots, u32 a_slots, int npt) { return p_slots * (u32)npt + a_slots * (npt == 1 ? 1u : 2u); }
 
+// a coefficient times any word; the result is lazy
 GL_HD fp2 apply(u32 cls, const fp2* cf, u32 ci, fp2 x) {
     if (cls == ONE) return x;
-    if (cls == NEG) return f2_neg(x);
-    if (cls == BASE) return f2_mul_base(x, cf[ci].c0);
-    return x.c1 == 0 ? f2_mul_base(cf[ci], x.c0) : f2_mul(cf[ci], x);
+    if (cls == NEG) return f2_neg(f2_canon(x));
+    if (cls == BASE) return f2_mul_base_lazy(x, cf[ci].c0);
+    return x.c1 == 0 ? f2_mul_base_lazy(cf[ci], x.c0) : f2_mul_lazy(cf[ci], x);
 }
 GL_HD fp2 constant(u32 cls, const fp2* cf, u32 ci) { return cls == ONE ? f2(1, 0) : cls == NEG ? f2(GL_P - 1, 0) : cf[ci]; }
 
-// The program at NPT evaluation points p_first, p_first + 1, .. (after the point 0 comes the point 2 when `skip` is set: the point 1 is
+// The program at NPT >= 2 evaluation points p_first, p_first + 1, .. (after the point 0 comes the point 2 when `skip` is set: the point 1 is
 // known from the claim).  table(t, lo, hi): the two ends of a table's pair; slots: this thread's entries, entry e at slots[e * stride].
-// The ends of the next instruction's table are fetched before this one's arithmetic.
+// The ends of the next instruction's table are fetched before this one's arithmetic.  X is lazy throughout (so is the result), R and the
+// slots are canonical: a sum then has one canonical operand, and a product takes anything.
 template <int NPT, class Table>
 GL_HD void eval(const u64* code, const fp2* cf, Table table, fp2* slots, u32 stride, u32 a_base, u32 p_first, bool skip, fp2 (&X)[NPT]) {
-    constexpr bool ONE_POINT = NPT == 1;
     fp2 rv = f2(0, 0), rd = f2(0, 0), lo = f2(0, 0), hi = f2(0, 0);
     u64 w = code[0];
     if (src_of(w) == TABLE && op_of(w) <= R_ADD) table(idx_of(w), lo, hi);
@@ -282,40 +377,34 @@ GL_HD void eval(const u64* code, const fp2* cf, Table table, fp2* slots, u32 str
             if (src == TABLE) {
                 v = lo;
                 d = f2_sub(hi, lo);
-                if constexpr (ONE_POINT) {
-                    for (u32 p = 0; p < p_first; p++) v = f2_add(v, d);
-                }
             } else if (src == ASLOT) {
-                v = slots[(a_base + (ONE_POINT ? idx : 2 * idx)) * stride];
-                if constexpr (!ONE_POINT) d = slots[(a_base + 2 * idx + 1) * stride];
+                v = slots[(a_base + 2 * idx) * stride];
+                d = slots[(a_base + 2 * idx + 1) * stride];
             } else {
                 v = rv;
                 d = rd;
             }
             if (src != PSLOT && cls != ONE) {
                 v = apply(cls, cf, ci, v);
-                if constexpr (!ONE_POINT) d = apply(cls, cf, ci, d);
+                d = f2_canon(apply(cls, cf, ci, d));
             }
             if (op >= R_SET) {
-                if (op == R_SET) { rv = v; rd = d; }
-                else { rv = f2_add(rv, v); if constexpr (!ONE_POINT) rd = f2_add(rd, d); }
+                if (op == R_SET) { rv = f2_canon(v); rd = d; }
+                else { rv = f2_canon(f2_add_lazy(v, rv)); rd = f2_add(rd, d); }
             } else {
                 fp2 y[NPT];
                 bool base = false;
                 if (src == PSLOT) {
 #pragma unroll
                     for (int j = 0; j < NPT; j++) y[j] = slots[(idx * NPT + j) * stride];
-                } else if constexpr (ONE_POINT) {
-                    y[0] = v;
-                    base = v.c1 == 0;
                 } else {
                     base = (v.c1 | d.c1) == 0;
-                    for (u32 p = 0; p < p_first; p++) v = f2_add(v, d);
+                    for (u32 p = 0; p < p_first; p++) v = f2_add_lazy(v, d);
                     y[0] = v;
 #pragma unroll
                     for (int j = 1; j < NPT; j++) {
-                        v = f2_add(v, d);
-                        if (j == 1 && skip && p_first == 0) v = f2_add(v, d);
+                        v = f2_add_lazy(v, d);
+                        if (j == 1 && skip && p_first == 0) v = f2_add_lazy(v, d);
                         y[j] = v;
                     }
                 }
@@ -324,30 +413,30 @@ GL_HD void eval(const u64* code, const fp2* cf, Table table, fp2* slots, u32 str
                     for (int j = 0; j < NPT; j++) X[j] = y[j];
                 } else if (base) {
 #pragma unroll
-                    for (int j = 0; j < NPT; j++) X[j] = f2_mul_base(X[j], y[j].c0);
+                    for (int j = 0; j < NPT; j++) X[j] = f2_mul_base_lazy(X[j], y[j].c0);
                 } else {
 #pragma unroll
-                    for (int j = 0; j < NPT; j++) X[j] = f2_mul(X[j], y[j]);
+                    for (int j = 0; j < NPT; j++) X[j] = f2_mul_lazy(X[j], y[j]);
                 }
             }
         } else {
             switch (op) {
                 case R_CONST: rv = constant(cls, cf, ci); rd = f2(0, 0); break;
                 case A_SET:
-                    slots[(a_base + (ONE_POINT ? idx : 2 * idx)) * stride] = rv;
-                    if constexpr (!ONE_POINT) slots[(a_base + 2 * idx + 1) * stride] = rd;
+                    slots[(a_base + 2 * idx) * stride] = rv;
+                    slots[(a_base + 2 * idx + 1) * stride] = rd;
                     break;
                 case P_SET:
 #pragma unroll
-                    for (int j = 0; j < NPT; j++) slots[(idx * NPT + j) * stride] = X[j];
+                    for (int j = 0; j < NPT; j++) slots[(idx * NPT + j) * stride] = f2_canon(X[j]);
                     break;
                 case P_ACC:
 #pragma unroll
-                    for (int j = 0; j < NPT; j++) slots[(idx * NPT + j) * stride] = f2_add(slots[(idx * NPT + j) * stride], X[j]);
+                    for (int j = 0; j < NPT; j++) slots[(idx * NPT + j) * stride] = f2_canon(f2_add_lazy(X[j], slots[(idx * NPT + j) * stride]));
                     break;
                 case X_ADDP:
 #pragma unroll
-                    for (int j = 0; j < NPT; j++) X[j] = f2_add(X[j], slots[(idx * NPT + j) * stride]);
+                    for (int j = 0; j < NPT; j++) X[j] = f2_add_lazy(X[j], slots[(idx * NPT + j) * stride]);
                     break;
                 case X_MULC:
 #pragma unroll
@@ -363,6 +452,42 @@ GL_HD void eval(const u64* code, const fp2* cf, Table table, fp2* slots, u32 str
         w = nw;
         lo = nlo;
         hi = nhi;
+    }
+}
+
+// The program at ONE point, where a round waits for its chain and not for its instructions: table(t) is the table's value at the point.
+template <class Table>
+GL_HD fp2 eval_one(const u64* code, const fp2* cf, Table table, fp2* slots, u32 stride, u32 a_base) {
+    fp2 X = f2(0, 0), R = f2(0, 0), next = f2(0, 0);
+    u64 w = code[0];
+    if (src_of(w) == TABLE && op_of(w) <= R_ADD) next = table(idx_of(w));
+    for (u32 pc = 0;; pc++) {
+        const u32 op = op_of(w), src = src_of(w), cls = cls_of(w), idx = idx_of(w), ci = coef_of(w);
+        if (op == END) return X;
+        const u64 nw = code[pc + 1];
+        fp2 y = next;
+        if (src_of(nw) == TABLE && op_of(nw) <= R_ADD) next = table(idx_of(nw));
+        if (op <= R_ADD) {
+            if (src == ASLOT) y = slots[(a_base + idx) * stride];
+            else if (src == PSLOT) y = slots[idx * stride];
+            else if (src == REG) y = R;
+            if (src != PSLOT) y = apply(cls, cf, ci, y);
+            if (op == MUL) X = y.c1 == 0 ? f2_mul_base_lazy(X, y.c0) : f2_mul_lazy(X, y);
+            else if (op == R_ADD) R = f2_canon(f2_add_lazy(y, R));
+            else if (op == INIT) X = y;
+            else R = f2_canon(y);
+        } else {
+            switch (op) {
+                case R_CONST: R = constant(cls, cf, ci); break;
+                case A_SET: slots[(a_base + idx) * stride] = R; break;
+                case P_SET: slots[idx * stride] = f2_canon(X); break;
+                case P_ACC: slots[idx * stride] = f2_canon(f2_add_lazy(X, slots[idx * stride])); break;
+                case X_ADDP: X = f2_add_lazy(X, slots[idx * stride]); break;
+                case X_MULC: X = apply(cls, cf, ci, X); break;
+                default: X = constant(cls, cf, ci);
+            }
+        }
+        w = nw;
     }
 }
 

@@ -267,8 +267,9 @@ __global__ void __launch_bounds__(VMT) k_sc_round_vm(const u64* __restrict__ tab
     fp2* cf = reinterpret_cast<fp2*>(vm_smem + (((size_t)p.n_code * 8 + 15) & ~(size_t)15));
     for (u32 x = threadIdx.x; x < p.n_code; x += VMT) code[x] = p.code[x];
     for (u32 x = threadIdx.x; x < p.n_coefs; x += VMT) cf[x] = ld2(p.coefs + 2 * (size_t)x);
-    const u32 entries = vm::slot_entries(p.p_slots, p.a_slots, NPT);
-    fp2* slots = (slots_g ? slots_g + (size_t)(blockIdx.y * gridDim.x + blockIdx.x) * entries * VMT : cf + p.n_coefs) + threadIdx.x;
+    const u32 entries = vm::slot_entries(p.p_slots, p.a_slots, NPT), row = blockIdx.z * gridDim.x + blockIdx.x;
+    fp2* slots = (slots_g ? slots_g + (size_t)(blockIdx.y * gridDim.x * gridDim.z + row) * entries * VMT : cf + p.n_coefs) + threadIdx.x;
+    const u64* prog = gridDim.z > 1 ? code + p.start[blockIdx.z] : code;
     __syncthreads();
     const u32 e0 = blockIdx.y * NPT;  // this thread's first evaluated point, by its position among them
     const u32 first = skip && e0 ? e0 + 1 : e0;
@@ -277,16 +278,29 @@ __global__ void __launch_bounds__(VMT) k_sc_round_vm(const u64* __restrict__ tab
     for (int j = 0; j < NPT; j++) acc[j] = f2(0, 0);
     for (u32 i = blockIdx.x * VMT + threadIdx.x; i < half; i += gridDim.x * VMT) {
         fp2 x[NPT];
-        vm::eval<NPT>(
-            code, cf,
-            [&](u32 t, fp2& lo, fp2& hi) {
-                const u64* tb = tables + 2 * ((size_t)t * stride + i);
-                lo = ld2(tb);
-                hi = ld2(tb + 2 * (size_t)half);
-            },
-            slots, VMT, p.p_slots * NPT, first, skip, x);
+        if constexpr (NPT == 1) {
+            x[0] = vm::eval_one(
+                prog, cf,
+                [&](u32 t) {
+                    const u64* tb = tables + 2 * ((size_t)t * stride + i);
+                    const fp2 lo = ld2(tb), d = f2_sub(ld2(tb + 2 * (size_t)half), lo);
+                    fp2 v = lo;
+                    for (u32 q = 0; q < first; q++) v = f2_add(v, d);
+                    return v;
+                },
+                slots, VMT, p.p_slots);
+        } else {
+            vm::eval<NPT>(
+                prog, cf,
+                [&](u32 t, fp2& lo, fp2& hi) {
+                    const u64* tb = tables + 2 * ((size_t)t * stride + i);
+                    lo = ld2(tb);
+                    hi = ld2(tb + 2 * (size_t)half);
+                },
+                slots, VMT, p.p_slots * NPT, first, skip, x);
+        }
 #pragma unroll
-        for (int j = 0; j < NPT; j++) acc[j] = f2_add(acc[j], x[j]);
+        for (int j = 0; j < NPT; j++) acc[j] = f2_canon(f2_add_lazy(x[j], acc[j]));
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
@@ -303,7 +317,7 @@ __global__ void __launch_bounds__(VMT) k_sc_round_vm(const u64* __restrict__ tab
     const u32 w = threadIdx.x, np = (u32)degree + 1;
     if (w < 2 * np) {
         const u32 pt = w >> 1, e = skip && pt ? pt - 1 : pt;
-        u64* dst = partials + (size_t)blockIdx.x * 2 * np + w;
+        u64* dst = partials + (size_t)row * 2 * np + w;
         if ((skip && pt == 1) || e >= npe) {
             if (blockIdx.y == 0) *dst = 0;
         } else if (e >= e0 && e < e0 + NPT) {
@@ -317,10 +331,19 @@ __global__ void __launch_bounds__(VMT) k_sc_round_vm(const u64* __restrict__ tab
 // points per thread and threads per pair for `npe` evaluated points
 u32 vm_npt(u32 npe) { return npe <= (u32)vm::MAX_NPT ? npe : (npe + 1) / 2; }
 size_t vm_fixed_bytes(const hlk::IrDev& p) { return (((size_t)p.n_code * 8 + 15) & ~(size_t)15) + (size_t)p.n_coefs * 16; }
+// A thread per pair, at most four CTAs of them per SM (that many fit); where the pairs fill less than that, a pair's parts go to threads
+// of their own.
+struct VmGrid { u32 blocks, parts; };
+VmGrid vm_grid(const hlk::IrDev& p, u32 half, int sm_count) {
+    const u32 cap = (u32)sm_count * 4, b = (half + VMT - 1) / VMT;
+    VmGrid g{b < 1 ? 1u : b > cap ? cap : b, 1u};
+    if (g.blocks * p.parts <= cap) g.parts = p.parts;
+    return g;
+}
 constexpr size_t VM_SLOT_SMEM = 40 * 1024;  // above this the slots of a CTA go to global memory
 
 template <int NPT>
-cudaError_t launch_vm(const hlk::IrDev& p, const u64* tables, size_t stride, u32 half, int degree, u32 npe, bool skip, u64* slots, u64* partials, u32 nblocks,
+cudaError_t launch_vm(const hlk::IrDev& p, const u64* tables, size_t stride, u32 half, int degree, u32 npe, bool skip, u64* slots, u64* partials, VmGrid g,
                       cudaStream_t s) {
     const size_t slot_bytes = (size_t)vm::slot_entries(p.p_slots, p.a_slots, NPT) * VMT * 16;
     const size_t smem = vm_fixed_bytes(p) + (slots ? 0 : slot_bytes);
@@ -328,7 +351,7 @@ cudaError_t launch_vm(const hlk::IrDev& p, const u64* tables, size_t stride, u32
         cudaError_t e = cudaFuncSetAttribute(k_sc_round_vm<NPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    return chain_launch(k_sc_round_vm<NPT>, dim3(nblocks, (npe + NPT - 1) / NPT), dim3(VMT), smem, s, tables, stride, half, p, degree, npe, skip,
+    return chain_launch(k_sc_round_vm<NPT>, dim3(g.blocks, (npe + NPT - 1) / NPT, g.parts), dim3(VMT), smem, s, tables, stride, half, p, degree, npe, skip,
                         reinterpret_cast<fp2*>(slots), partials);
 }
 
@@ -348,36 +371,36 @@ u32 sc_round_blocks(u32 half, int sm_count) {
     return b > cap ? cap : b;
 }
 
-u32 sc_ir_blocks(u32 half, int sm_count) {
-    u32 b = (half + VMT - 1) / VMT, cap = (u32)sm_count * 4;
-    if (b < 1) b = 1;
-    return b > cap ? cap : b;
+u32 sc_ir_rows(const IrDev& p, u32 half, int sm_count) {
+    const VmGrid g = vm_grid(p, half, sm_count);
+    return g.blocks * g.parts;
 }
 
-// bytes of global memory for the slots of a grid of that size, 0 where they fit shared memory
-size_t sc_ir_slot_bytes(const IrDev& p, u32 nblocks) {
+// bytes of global memory for the slots of any round's grid, 0 where they fit shared memory
+size_t sc_ir_slot_bytes(const IrDev& p, int sm_count) {
     size_t most = 0;
     for (u32 npe = p.eval_degree; npe <= p.eval_degree + 1; npe++) {
         if (npe == 0) continue;
         const u32 npt = vm_npt(npe);
-        const size_t cta = (size_t)vm::slot_entries(p.p_slots, p.a_slots, (int)npt) * VMT * 16;
-        if (cta > VM_SLOT_SMEM && cta * nblocks * ((npe + npt - 1) / npt) > most) most = cta * nblocks * ((npe + npt - 1) / npt);
+        const size_t cta = (size_t)vm::slot_entries(p.p_slots, p.a_slots, (int)npt) * VMT * 16, all = cta * sm_count * 4 * ((npe + npt - 1) / npt);
+        if (cta > VM_SLOT_SMEM && all > most) most = all;
     }
     return most;
 }
 
-cudaError_t sc_round_ir(const IrDev& p, const u64* tables, size_t stride, u32 half, int degree, int eval_one, u64* slots, u64* partials, u32 nblocks,
+cudaError_t sc_round_ir(const IrDev& p, const u64* tables, size_t stride, u32 half, int degree, int eval_one, u64* slots, u64* partials, int sm_count,
                         cudaStream_t s) {
     const bool skip = !eval_one && p.eval_degree >= 1;
     const u32 npe = p.eval_degree + (skip ? 0u : 1u), npt = vm_npt(npe);
     const size_t cta = (size_t)vm::slot_entries(p.p_slots, p.a_slots, (int)npt) * VMT * 16;
     u64* sl = cta > VM_SLOT_SMEM ? slots : nullptr;
+    const VmGrid g = vm_grid(p, half, sm_count);
     switch (npt) {
-        case 1: return launch_vm<1>(p, tables, stride, half, degree, npe, skip, sl, partials, nblocks, s);
-        case 2: return launch_vm<2>(p, tables, stride, half, degree, npe, skip, sl, partials, nblocks, s);
-        case 3: return launch_vm<3>(p, tables, stride, half, degree, npe, skip, sl, partials, nblocks, s);
-        case 4: return launch_vm<4>(p, tables, stride, half, degree, npe, skip, sl, partials, nblocks, s);
-        case 5: return launch_vm<5>(p, tables, stride, half, degree, npe, skip, sl, partials, nblocks, s);
+        case 1: return launch_vm<1>(p, tables, stride, half, degree, npe, skip, sl, partials, g, s);
+        case 2: return launch_vm<2>(p, tables, stride, half, degree, npe, skip, sl, partials, g, s);
+        case 3: return launch_vm<3>(p, tables, stride, half, degree, npe, skip, sl, partials, g, s);
+        case 4: return launch_vm<4>(p, tables, stride, half, degree, npe, skip, sl, partials, g, s);
+        case 5: return launch_vm<5>(p, tables, stride, half, degree, npe, skip, sl, partials, g, s);
     }
     return cudaErrorInvalidValue;
 }

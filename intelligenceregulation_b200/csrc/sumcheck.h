@@ -47,6 +47,7 @@ struct IrDev {
     const u64* code;
     const u64* coefs;  // n_coefs Fp2
     u32 n_code, n_coefs, n_tables, p_slots, a_slots;
+    u32 parts, start[4];   // the program in parts (slot_vm.cuh); code[0] starts the whole
     u32 eval_degree;   // min(declared, attained): the points the kernels evaluate are 0 .. eval_degree
 };
 
@@ -62,10 +63,11 @@ struct ScSync {
 void sc_set_dependent_launch(bool on);
 bool sc_dependent_launch();
 u32 sc_round_blocks(u32 half, int sm_count);
-// the long rounds of a slot program; slots: sc_ir_slot_bytes of scratch (NULL when that is 0)
-u32 sc_ir_blocks(u32 half, int sm_count);
-size_t sc_ir_slot_bytes(const IrDev& p, u32 nblocks);
-cudaError_t sc_round_ir(const IrDev& p, const u64* tables, size_t stride, u32 half, int degree, int eval_one, u64* slots, u64* partials, u32 nblocks,
+// the long rounds of a slot program; sc_ir_rows: the partial rows that a round writes; slots: sc_ir_slot_bytes of scratch (NULL when
+// that is 0)
+u32 sc_ir_rows(const IrDev& p, u32 half, int sm_count);
+size_t sc_ir_slot_bytes(const IrDev& p, int sm_count);
+cudaError_t sc_round_ir(const IrDev& p, const u64* tables, size_t stride, u32 half, int degree, int eval_one, u64* slots, u64* partials, int sm_count,
                         cudaStream_t s);
 // all remaining rounds in one launch, from a table length of at most sc_run_len (sumcheck_run.cu).  partials: sc_run_partial_bytes;
 // slots: sc_run_slot_bytes of scratch (NULL when that is 0); sync: zeroed

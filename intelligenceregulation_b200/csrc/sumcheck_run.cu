@@ -31,7 +31,7 @@ struct RunArgs {
     u64* tables;
     size_t stride;
     u32 len;             // live entries per table at the first round
-    u32 k, nrounds, chunk, npe_max;
+    u32 k, nrounds, chunk, planes, parts, npe_max;
     int have_claim;      // the first round's claim is known
     hlk::ScStep step;    // step.round: the first round's number
     hlk::ScSync* sync;   // zero at the launch
@@ -39,10 +39,19 @@ struct RunArgs {
 };
 
 // Shared memory: [evaluator's own][table chunk][its successor, half as long], the two swapping roles once one CTA is left.
-// A chunk holds entry i of table t at [(t * 2 + side) * chunk + i], side 0 the low half of a pair, side 1 the high half.
+// A chunk holds table t of pair i at point p at [(t * planes + p) * chunk + i]: the ends of the pair (the points 0 and 1) and, where
+// they all fit, the points above.  An evaluator then reads a value where it would step to it, and every evaluator of the pair would.
 struct TabSmem {
     const fp2* base;
-    u32 chunk;
+    u32 chunk, planes;
+    __device__ __forceinline__ fp2 at(u32 t, u32 i, u32 point) const {
+        const fp2* b = base + (size_t)t * planes * chunk + i;
+        if (point < planes) return b[point * chunk];
+        fp2 v = b[chunk];
+        const fp2 d = f2_sub(v, b[0]);
+        for (u32 p = 1; p < point; p++) v = f2_add(v, d);
+        return v;
+    }
 };
 
 // The closed-form families (sumcheck.h), one evaluation point
@@ -50,16 +59,10 @@ template <int POLY, int K>
 struct ClosedEval {
     const u64* coefs;
     __device__ u32 stage(char*, u32) { return 0; }
-    __device__ fp2 at(const TabSmem& tab, u32 i, u32 point, u32) const {
+    __device__ fp2 at(const TabSmem& tab, u32 i, u32 point, u32, u32) const {
         fp2 v[K];
 #pragma unroll
-        for (int t = 0; t < K; t++) {
-            v[t] = tab.base[(2 * t) * tab.chunk + i];
-            if (point) {
-                const fp2 d = f2_sub(tab.base[(2 * t + 1) * tab.chunk + i], v[t]);
-                for (u32 p = 0; p < point; p++) v[t] = f2_add(v[t], d);
-            }
-        }
+        for (int t = 0; t < K; t++) v[t] = tab.at(t, i, point);
         const fp2* cf = reinterpret_cast<const fp2*>(coefs);
         return hlk::poly_eval<POLY, K>(v, cf);
     }
@@ -91,21 +94,25 @@ struct ProgramEval {
         slots = (slots_g ? slots_g + (size_t)blockIdx.x * entries : reinterpret_cast<fp2*>(mem + used)) + threadIdx.x;
         return slots_g ? used : used + entries * 16;
     }
-    __device__ fp2 at(const TabSmem& tab, u32 i, u32 point, u32 threads) const {
-        fp2 x[1];
-        vm::eval<1>(
-            code, cf,
-            [&](u32 t, fp2& lo, fp2& hi) {
-                lo = tab.base[(2 * t) * tab.chunk + i];
-                hi = tab.base[(2 * t + 1) * tab.chunk + i];
-            },
-            slots, threads, p.p_slots, point, false, x);
-        return x[0];
+    __device__ fp2 at(const TabSmem& tab, u32 i, u32 point, u32 part, u32 threads) const {
+        return f2_canon(vm::eval_one(p.parts > 1 ? code + p.start[part] : code, cf, [&](u32 t) { return tab.at(t, i, point); }, slots, threads, p.p_slots));
     }
 };
 
+__device__ __forceinline__ fp2 warp_sum(fp2 v) {
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1) {
+        const u32 a0 = __shfl_down_sync(0xffffffffu, (u32)v.c0, off), a1 = __shfl_down_sync(0xffffffffu, (u32)(v.c0 >> 32), off);
+        const u32 b0 = __shfl_down_sync(0xffffffffu, (u32)v.c1, off), b1 = __shfl_down_sync(0xffffffffu, (u32)(v.c1 >> 32), off);
+        v = f2_add(v, f2(((u64)a1 << 32) | a0, ((u64)b1 << 32) | b0));
+    }
+    return v;
+}
+
+constexpr u32 RUN_MAX_T = 512, RUN_PASSES = 4;
+
 template <class Eval>
-__global__ void __launch_bounds__(512) k_sc_run(RunArgs a, Eval ev) {
+__global__ void __launch_bounds__(RUN_MAX_T) k_sc_run(RunArgs a, Eval ev) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     extern __shared__ __align__(16) char smem[];
@@ -114,7 +121,7 @@ __global__ void __launch_bounds__(512) k_sc_run(RunArgs a, Eval ev) {
     __shared__ __align__(16) u64 rows_s[2 * 63 * (hlk::SC_MAX_POINTS - 1)];
     __shared__ __align__(16) u64 tab_s[2 * 63 * hlk::SC_MAX_POINTS];
     __shared__ u64 invden_s[hlk::SC_MAX_POINTS], extrap_s[hlk::SC_MAX_POINTS * hlk::SC_MAX_POINTS];
-    __shared__ fp2 warp_s[16];          // one sum per warp
+    __shared__ fp2 task_s[RUN_PASSES * RUN_MAX_T / 32];  // one sum per warp and pass: [task][warp of the chunk]
     __shared__ fp2 cta_s[hlk::SC_MAX_POINTS];
     __shared__ fp2 r_s;
     __shared__ u32 failed_s;
@@ -122,7 +129,7 @@ __global__ void __launch_bounds__(512) k_sc_run(RunArgs a, Eval ev) {
     const int degree = a.step.degree, np = degree + 1;
     const u32 own = ev.stage(smem, T);
     fp2* const buf0 = reinterpret_cast<fp2*>(smem + own);
-    fp2* const buf1 = buf0 + (size_t)a.k * 2 * C;  // with half the stride: it only ever holds the rounds after the first one
+    fp2* const buf1 = buf0 + (size_t)a.k * a.planes * C;  // with half the stride: it only ever holds the rounds after the first one
     if (tid == 0) failed_s = 0;
     if (cta == 0) {
         const u32* src = reinterpret_cast<const u32*>(a.step.state);
@@ -174,7 +181,11 @@ __global__ void __launch_bounds__(512) k_sc_run(RunArgs a, Eval ev) {
         const u32 npe = a.step.eval_degree + (skip ? 0 : 1);
         // CTA 0's first warp is behind: it still has to bring the claim and the mask up to the challenge just published
         const u32 ft = cta == 0 && rd > 0 ? T - 32 : T, f0 = cta == 0 && rd > 0 ? tid - 32 : tid;
-        fp2 acc = f2(0, 0);
+        // a task is one point and one part of the polynomial, for all pairs of a chunk; a warp lies within one task
+        const u32 tasks = npe * a.parts, tslots = T / C, my = tid / C, ti = tid - my * C;
+        fp2 acc[RUN_PASSES];
+#pragma unroll
+        for (u32 q = 0; q < RUN_PASSES; q++) acc[q] = f2(0, 0);
         for (u32 c0 = cta * C; c0 < half; c0 += ncta * C) {
             const u32 cn = min(C, half - c0), lcn = __ffs((int)cn) - 1;  // powers of two, all of them
             if (c0 != cta * C) __syncthreads();  // the chunk before has been evaluated
@@ -185,44 +196,60 @@ __global__ void __launch_bounds__(512) k_sc_run(RunArgs a, Eval ev) {
                 step_after(sa, sm, j - 1, r, lane);
                 g = step_ahead(sa, sm, j, lane);
             } else if (cta != 0 || rd == 0 || warp > 0) {
-                const u32 items = a.k * 2 * cn;
-                for (u32 x = f0; x < items; x += ft) {
-                    const u32 ts = x >> lcn, i = x & (cn - 1), t = ts >> 1, side = ts & 1, e = c0 + i + side * half;  // entry e of table t
-                    fp2 v;
+                for (u32 x = f0; x < a.k * cn; x += ft) {
+                    const u32 t = x >> lcn, i = x & (cn - 1);
+                    fp2 v[2];  // the pair's two entries, c0 + i and c0 + i + half of the table
                     if (resident) {
-                        const fp2* from = (second ? buf1 : buf0) + (size_t)t * 2 * ts_from;
-                        const fp2 lo = from[e];
-                        v = f2_add(lo, f2_mul(r, f2_sub(from[ts_from + e], lo)));
+                        const fp2* from = (second ? buf1 : buf0) + (size_t)t * a.planes * ts_from + i;
+#pragma unroll
+                        for (u32 e = 0; e < 2; e++) {
+                            const fp2 lo = from[e * half];
+                            v[e] = f2_add(lo, f2_mul(r, f2_sub(from[ts_from + e * half], lo)));
+                        }
                     } else {
-                        u64* p = a.tables + 2 * ((size_t)t * a.stride + e);
-                        v = ld2(p);
+                        u64* p = a.tables + 2 * ((size_t)t * a.stride + c0 + i);
+#pragma unroll
+                        for (u32 e = 0; e < 2; e++) v[e] = ld2(p + 2 * (size_t)e * half);
                         if (rd > 0) {
-                            v = f2_add(v, f2_mul(r, f2_sub(ld2(p + 2 * (size_t)len), v)));
-                            if (ncta > 1 || half > C) st2(p, v);
+#pragma unroll
+                            for (u32 e = 0; e < 2; e++) v[e] = f2_add(v[e], f2_mul(r, f2_sub(ld2(p + 2 * ((size_t)e * half + len)), v[e])));
+                            if (half > C) {
+#pragma unroll
+                                for (u32 e = 0; e < 2; e++) st2(p + 2 * (size_t)e * half, v[e]);
+                            }
                         }
                     }
-                    to[(size_t)ts * ts_to + i] = v;
+                    fp2* o = to + (size_t)t * a.planes * ts_to + i;
+                    o[0] = v[0];
+                    o[ts_to] = v[1];
+                    if (a.planes > 2) {
+                        const fp2 d = f2_sub(v[1], v[0]);
+                        fp2 y = v[1];
+                        for (u32 p = 2; p < a.planes; p++) { y = f2_add(y, d); o[p * ts_to] = y; }
+                    }
                 }
             }
             __syncthreads();
-            const TabSmem tab{to, ts_to};
-            const u32 pi = tid / C, i = tid - pi * C;
-            if (pi < npe && i < cn) acc = f2_add(acc, ev.at(tab, i, skip && pi ? pi + 1 : pi, T));
+            const TabSmem tab{to, ts_to, a.planes};
+#pragma unroll
+            for (u32 q = 0; q < RUN_PASSES; q++) {
+                const u32 task = my + q * tslots, part = task / npe, pi = task - part * npe;
+                if (task < tasks && ti < cn) acc[q] = f2_add(acc[q], ev.at(tab, ti, skip && pi ? pi + 1 : pi, part, T));
+            }
         }
         if (resident) second = !second;
         else if (half <= C) resident = true;
-        // sums over the pairs: a warp lies within one point
 #pragma unroll
-        for (int off = 16; off >= 1; off >>= 1) {
-            const u32 a0 = __shfl_down_sync(0xffffffffu, (u32)acc.c0, off), a1 = __shfl_down_sync(0xffffffffu, (u32)(acc.c0 >> 32), off);
-            const u32 b0 = __shfl_down_sync(0xffffffffu, (u32)acc.c1, off), b1 = __shfl_down_sync(0xffffffffu, (u32)(acc.c1 >> 32), off);
-            acc = f2_add(acc, f2(((u64)a1 << 32) | a0, ((u64)b1 << 32) | b0));
+        for (u32 q = 0; q < RUN_PASSES; q++) {
+            if (q * tslots >= tasks) break;
+            acc[q] = warp_sum(acc[q]);
+            if (lane == 0) task_s[q * (T / 32) + warp] = acc[q];
         }
-        if (lane == 0) warp_s[warp] = acc;
         __syncthreads();
         if (tid < npe) {
             fp2 s = f2(0, 0);
-            for (u32 w = tid * (C / 32); w < (tid + 1) * (C / 32); w++) s = f2_add(s, warp_s[w]);
+            for (u32 part = 0; part < a.parts; part++)
+                for (u32 w = 0; w < C / 32; w++) s = f2_add(s, task_s[(part * npe + tid) * (C / 32) + w]);
             cta_s[tid] = s;
             if (cta != 0) st2(a.partials + 2 * ((size_t)cta * a.npe_max + tid), s);
         }
@@ -252,12 +279,7 @@ __global__ void __launch_bounds__(512) k_sc_run(RunArgs a, Eval ev) {
                         const ulonglong2 v = __ldcg(reinterpret_cast<const ulonglong2*>(a.partials + 2 * ((size_t)b * a.npe_max + pi)));
                         s = f2_add(s, f2(v.x, v.y));
                     }
-#pragma unroll
-                    for (int off = 16; off >= 1; off >>= 1) {
-                        const u32 a0 = __shfl_down_sync(0xffffffffu, (u32)s.c0, off), a1 = __shfl_down_sync(0xffffffffu, (u32)(s.c0 >> 32), off);
-                        const u32 b0 = __shfl_down_sync(0xffffffffu, (u32)s.c1, off), b1 = __shfl_down_sync(0xffffffffu, (u32)(s.c1 >> 32), off);
-                        s = f2_add(s, f2(((u64)a1 << 32) | a0, ((u64)b1 << 32) | b0));
-                    }
+                    s = warp_sum(s);
                     if (lane == 0) cta_s[pi] = f2_add(cta_s[pi], s);
                 }
                 __syncthreads();
@@ -305,7 +327,7 @@ __global__ void __launch_bounds__(512) k_sc_run(RunArgs a, Eval ev) {
             const u32 t = x >> lcn, i = x & (cn - 1);
             u64* p = a.tables + 2 * ((size_t)t * a.stride + c0 + i);
             fp2 lo, hi;
-            if (resident) { lo = b[(size_t)(2 * t) * st + i]; hi = b[(size_t)(2 * t + 1) * st + i]; }
+            if (resident) { lo = b[(size_t)t * a.planes * st + i]; hi = b[((size_t)t * a.planes + 1) * st + i]; }
             else { lo = ld2(p); hi = ld2(p + 2 * (size_t)len); }
             st2(p, f2_add(lo, f2_mul(r, f2_sub(hi, lo))));
         }
@@ -321,22 +343,32 @@ __global__ void __launch_bounds__(512) k_sc_run(RunArgs a, Eval ev) {
 constexpr size_t RUN_SMEM = 200 * 1024;
 constexpr size_t RUN_CODE = 64 * 1024;
 
+// How much of a round fits one CTA: the larger chunk with every point's values, then less of both; a task per thread group where the
+// threads suffice, several passes otherwise.
 struct RunShape {
-    u32 chunk, threads;
+    u32 chunk, planes, parts, threads;
     bool slots_global, code_fits;
     size_t smem;
 };
 RunShape run_shape(int poly, const hlk::IrDev& p, int k, int eval_degree) {
     RunShape s;
-    s.slots_global = false;
-    const size_t fixed = poly == hlk::POLY_IR ? (((size_t)p.n_code * 8 + 15) & ~(size_t)15) + (size_t)p.n_coefs * 16 : 0;
+    const u32 points = (u32)eval_degree + 1, usual = eval_degree > 0 ? (u32)eval_degree : 1u;  // the point 1 comes from the claim
+    const bool is_ir = poly == hlk::POLY_IR;
+    s.parts = is_ir ? p.parts : 1u;
+    const size_t fixed = is_ir ? (((size_t)p.n_code * 8 + 15) & ~(size_t)15) + (size_t)p.n_coefs * 16 : 0;
     s.code_fits = fixed <= RUN_CODE;
-    for (int pass = 0; pass < 3; pass++) {
+    for (int pass = 0; pass < 4; pass++) {
         s.chunk = pass == 0 ? 64 : 32;
-        s.threads = s.chunk * (u32)(eval_degree + 1);
-        s.slots_global = pass == 2;
-        const size_t slots = poly == hlk::POLY_IR && !s.slots_global ? (size_t)vm::slot_entries(p.p_slots, p.a_slots, 1) * s.threads * 16 : 0;
-        s.smem = (s.code_fits ? fixed : 0) + slots + (size_t)k * s.chunk * 48;
+        s.planes = pass < 2 && points > 2 ? points : 2;
+        s.slots_global = pass == 3;
+        u32 groups = usual * s.parts, most = RUN_MAX_T / s.chunk;
+        if (groups > most) groups = most;
+        while (groups * RUN_PASSES < points * s.parts) groups++;
+        s.threads = s.chunk * groups;
+        if (s.threads < 64) s.threads = 64;  // CTA 0 folds with all warps but one
+        const size_t slots = is_ir && !s.slots_global ? (size_t)vm::slot_entries(p.p_slots, p.a_slots, 1) * s.threads * 16 : 0;
+        s.smem = (s.code_fits ? fixed : 0) + slots + (size_t)k * s.planes * s.chunk * 24;
+        if (pass == 0 && groups < usual * s.parts) continue;  // the smaller chunk has a thread group for every task
         if (s.smem <= RUN_SMEM) break;
     }
     return s;
@@ -390,7 +422,7 @@ cudaError_t sc_run(int poly, const IrDev& p, int k, u64* tables, size_t stride, 
     a.tables = tables; a.stride = stride; a.len = len; a.k = (u32)k; a.nrounds = (u32)nrounds; a.npe_max = (u32)step.eval_degree + 1;
     a.have_claim = have_claim; a.step = step; a.sync = sync; a.partials = partials;
     const RunShape sh = run_shape(poly, p, k, step.eval_degree);
-    a.chunk = sh.chunk;
+    a.chunk = sh.chunk; a.planes = sh.planes; a.parts = sh.parts;
     if (poly == POLY_IR) {
         ProgramEval ev;
         ev.p = p; ev.slots_g = sh.slots_global ? reinterpret_cast<fp2*>(slots) : nullptr; ev.code_fits = sh.code_fits;

@@ -31,13 +31,13 @@ def _check(emul, prog, desc, n_tables, seed):
         v = [tuple((int(lo[t][c]) + d * (int(hi[t][c]) - int(lo[t][c]))) % U.P for c in (0, 1)) for t in range(n_tables)]
         return U.py_eval(desc, v)
 
-    for npt, first, skip in ((1, 0, 0), (1, 3, 0), (2, 0, 1), (3, 0, 0), (4, 0, 1), (5, 0, 0), (2, 4, 1)):
+    for npt, first, skip, parts in ((1, 0, 0, 1), (1, 3, 0, 2), (1, 2, 0, 4), (2, 0, 1, 1), (3, 0, 0, 1), (4, 0, 1, 1), (5, 0, 0, 1), (2, 4, 1, 1)):
         out = np.zeros((npt, 2), dtype=np.uint64)
         emul.emul_vm(w.ctypes.data_as(C.c_void_p), w.size, n_tables, prog.n_nodes, prog.n_terms, cf.ctypes.data_as(C.c_void_p), cf.shape[0],
-                     lo.ctypes.data_as(C.c_void_p), hi.ctypes.data_as(C.c_void_p), npt, first, skip, out.ctypes.data_as(C.c_void_p), info.ctypes.data_as(C.c_void_p))
+                     lo.ctypes.data_as(C.c_void_p), hi.ctypes.data_as(C.c_void_p), npt, first, skip, parts, out.ctypes.data_as(C.c_void_p), info.ctypes.data_as(C.c_void_p))
         for j in range(npt):
             d = first + j + (1 if skip and first == 0 and j > 0 else 0)
-            assert tuple(int(x) for x in out[j]) == at(d), (npt, first, skip, j)
+            assert tuple(int(x) for x in out[j]) == at(d), (npt, first, skip, parts, j)
     return info
 
 
