@@ -34,6 +34,7 @@ struct hl_rounds {
     u64* d_slots = nullptr;    // slots of a slot program that shared memory does not hold
     size_t slot_bytes = 0;
     hlk::ScSync* d_sync = nullptr;
+    u64* d_other = nullptr;    // the one-launch rounds' second table buffer
     u64* d_out = nullptr;      // n_vars rows of (2 (degree+1) + 1) Fp2
     u64* d_finals = nullptr;   // k Fp2 behind them
     u64* d_inv_den = nullptr;
@@ -60,27 +61,28 @@ void free_rounds(hl_rounds* r) {
     delete r;
 }
 
-// the reduce + Fiat-Shamir step of round r->next over `nb` partial rows
-int launch_step(hl_rounds* r, u32 nb, int fs, int use_claim, int recover, const u64* d_mask, const u64* d_mtab, int mask_vars) {
-    hl_ctx* c = r->ctx;
+// What every round of a batch takes its step with; a plain round() leaves it as it is made.
+struct StepPlan {
+    int fs = 0, recover = 0, mask_vars = 0, between = 0;
+    const u64 *mask = nullptr, *mask_tab = nullptr;
+};
+
+hlk::ScStep step_of(const hl_rounds* r, u32 round, u32 nb, int use_claim, const StepPlan& p) {
     hlk::ScStep a;
-    a.partials = r->d_partials; a.nblocks = nb; a.degree = (int)r->degree; a.round = (int)r->next;
-    a.use_claim = use_claim; a.recover = recover; a.fs = fs; a.mask = d_mask; a.mask_tab = d_mtab; a.mask_vars = mask_vars;
+    a.partials = r->d_partials; a.nblocks = nb; a.degree = (int)r->degree; a.round = (int)round;
+    a.use_claim = use_claim; a.recover = p.recover; a.fs = p.fs; a.mask = p.mask; a.mask_tab = p.mask_tab; a.mask_vars = p.mask_vars;
     a.inv_den = r->d_inv_den; a.state = r->d_state; a.out = r->d_out;
-    a.eval_degree = (int)r->eval_degree; a.extrap = r->d_extrap;
-    cudaError_t e = hlk::sc_step(a, c->stream);
-    c->stats.kernel_launches++;
-    if (e != cudaSuccess) return fail(c, HL_B200_ERR_DEVICE, "round step launch", e);
-    return HL_B200_OK;
+    a.eval_degree = (int)r->eval_degree; a.extrap = r->d_extrap; a.between = p.between;
+    return a;
 }
 
-// launches round j's kernels; the caller holds the context lock
-int launch_round(hl_rounds* r, int eval_one, int fs, int use_claim, int recover, const u64* d_mask, const u64* d_mtab, int mask_vars) {
+// launches round r->next, its sums and its step; the caller holds the context lock
+int launch_round(hl_rounds* r, int eval_one, int use_claim, const StepPlan& plan) {
     hl_ctx* c = r->ctx;
     const u32 half = (u32)(r->len / 2);
     const bool is_ir = r->poly == hlk::POLY_IR;
-    u32 nb = is_ir ? hlk::sc_ir_rows(r->ir, half, c->sm_count) : hlk::sc_round_blocks(half, c->sm_count);
-    if (nb > r->max_blocks) return fail(c, HL_B200_ERR_DEVICE, "round launch: more partial rows than the buffer holds");  // the two grid rules agree by construction
+    const u32 nb = hlk::sc_round_blocks(half, c->sm_count);
+    const hlk::ScStep step = step_of(r, r->next, nb, use_claim, plan);
     cudaError_t e;
     if (is_ir && r->gen && c->slot_kernels) {
         // the generated kernel of this graph: the first-round typing while the tables it reads as base words are base-valued
@@ -91,16 +93,17 @@ int launch_round(hl_rounds* r, int eval_one, int fs, int use_claim, int recover,
         if (bx > cap) bx = cap;
         if (bx > r->max_blocks) bx = r->max_blocks;
         if (bx < 1) bx = 1;
-        nb = bx;
         c->stats.generated_rounds++;
         e = r->gen->launch(r0, per_point, bx, r->d_tables, r->stride, half, r->d_cfo, (int)r->degree, npe, skip, r->d_partials, c->stream);
+        c->stats.kernel_launches++;
+        if (e == cudaSuccess) e = hlk::sc_step(step_of(r, r->next, bx, use_claim, plan), c->stream);
     } else {
-        e = is_ir ? hlk::sc_round_ir(r->ir, r->d_tables, r->stride, half, (int)r->degree, eval_one, r->d_slots, r->d_partials, c->sm_count, c->stream)
-                  : hlk::sc_round(r->poly, (int)r->k, r->d_tables, r->stride, half, r->d_coefs, eval_one, r->d_partials, nb, c->stream);
+        e = is_ir ? hlk::sc_round_ir(r->ir, r->d_tables, r->stride, half, (int)r->degree, eval_one, r->d_slots, c->sm_count, step, r->d_sync, c->stream)
+                  : hlk::sc_round(r->poly, (int)r->k, r->d_tables, r->stride, half, r->d_coefs, eval_one, step, r->d_sync, c->stream);
     }
     c->stats.kernel_launches++;
     if (e != cudaSuccess) return fail(c, HL_B200_ERR_DEVICE, "round launch", e);
-    return launch_step(r, nb, fs, use_claim, recover, d_mask, d_mtab, mask_vars);
+    return HL_B200_OK;
 }
 
 int launch_fold(hl_rounds* r) {
@@ -122,13 +125,11 @@ extern "C" {
 namespace {
 
 // the evaluator of either kind; `words` is the data form of the polynomial when poly == POLY_IR
-constexpr size_t FUSED_FOLD_MAX_PAIRS = (size_t)1 << 15;
-
-// A program of more than some twenty instructions is also cut into parts of about that many, for the rounds with few pairs.
+// A program of more than a dozen instructions is also cut into parts of about that many, for the rounds with few pairs.
 void compile(vm::Compiler& prog, const ir::Shape& sh, const uint32_t* words, const uint64_t* coefs) {
     const fp2* cf = reinterpret_cast<const fp2*>(coefs);
     prog.run(sh, words, cf);
-    const u32 parts = ((u32)prog.out.code.size() + 19) / 20;
+    const u32 parts = ((u32)prog.out.code.size() + 11) / 12;
     if (parts > 1) prog.split(sh, words, cf, parts < vm::MAX_PARTS ? parts : vm::MAX_PARTS);
 }
 
@@ -159,7 +160,7 @@ int rounds_build(hl_ctx* c, int poly, size_t k, uint32_t n_vars, uint32_t degree
                      run_slots = hlk::sc_run_slot_bytes(poly, r->ir, (int)k, (int)r->eval_degree, c->sm_count);
         r->slot_bytes = long_slots > run_slots ? long_slots : run_slots;
     }
-    if (r->max_blocks < (u32)c->sm_count) r->max_blocks = (u32)c->sm_count;  // the one-launch rounds have a partial row per SM
+    const u32 run_len = hlk::sc_run_len(poly, r->ir) < r->len ? hlk::sc_run_len(poly, r->ir) : (u32)r->len;
     // what the kernels read and no challenge changes, in one upload
     std::vector<char> head;
     auto put = [&](size_t bytes) {
@@ -204,7 +205,8 @@ int rounds_build(hl_ctx* c, int poly, size_t k, uint32_t n_vars, uint32_t degree
     const size_t at_state = head.size() + r->mask_cap, state_bytes = (sizeof(hlk::ScState) + 15) & ~(size_t)15;
     const size_t at_sync = at_state + state_bytes, at_out = at_sync + ((sizeof(hlk::ScSync) + 15) & ~(size_t)15), at_fin = at_out + (n_vars ? n_vars : 1) * r->out_row() * 8, at_part = at_fin + k * 16;
     const size_t at_slots = at_part + (size_t)r->max_blocks * (degree + 1) * 16;
-    r->blk_bytes = at_slots + r->slot_bytes;
+    const size_t at_other = (at_slots + r->slot_bytes + 15) & ~(size_t)15;
+    r->blk_bytes = at_other + hlk::sc_run_other_bytes((int)k, run_len);
     int rc = built ? HL_B200_OK : dev_alloc(c, (void**)&r->d_tables, k * r->stride * 16);
     if (!rc) rc = dev_alloc(c, (void**)&r->blk, r->blk_bytes);
     if (!rc) {
@@ -218,11 +220,12 @@ int rounds_build(hl_ctx* c, int poly, size_t k, uint32_t n_vars, uint32_t degree
         r->d_partials = (u64*)(r->blk + at_part);
         r->d_slots = r->slot_bytes ? (u64*)(r->blk + at_slots) : nullptr;
         r->d_sync = (hlk::ScSync*)(r->blk + at_sync);
+        r->d_other = (u64*)(r->blk + at_other);
     }
     if (!rc && !built) rc = h2d_owned(c, r->d_tables, tables, k * r->stride * 16);
     if (!rc) rc = h2d_owned(c, r->blk, head.data(), head.size());
     if (!rc) {
-        cudaError_t e = cudaMemsetAsync(r->d_state, 0, sizeof(hlk::ScState), c->stream);
+        cudaError_t e = cudaMemsetAsync(r->d_state, 0, (char*)r->d_out - (char*)r->d_state, c->stream);
         if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "state clear", e);
     }
     if (!rc && c->slot_kernels && gen && gen->entry && gen->entry->n_tables == k && gen->entry->n_cfo == gen->cfo.size()) {
@@ -328,7 +331,7 @@ int hl_b200_rounds_round(hl_rounds* r, uint32_t j, int eval_one, uint64_t* sums)
     int rc;
     {
         Timed t(c, HL_T_ROUNDS);
-        rc = launch_round(r, eval_one, 0, 0, 0, nullptr, nullptr, 0);
+        rc = launch_round(r, eval_one, 0, StepPlan());
     }
     if (!rc) rc = d2h(c, sums, r->d_out + (size_t)j * r->out_row(), ((size_t)r->degree + 1) * 16);
     if (!rc) rc = sync(c, "rounds_round");
@@ -426,63 +429,28 @@ int hl_b200_rounds_batched(hl_rounds* r, uint32_t nd, hl_fs_state* fs, const uin
     memcpy(up.data() + row_words + tab_words, &st, sizeof st);
     rc = h2d(c, (u64*)r->d_state - row_words - tab_words, up.data(), up.size() * 8);
     // with the generated kernels switched on they take the rounds down to 2^11 pairs: the switch is there to compare them
-    const u32 first = r->next, run_len = r->gen && c->slot_kernels ? 1u << 12 : hlk::sc_run_len(r->poly);
+    const u32 first = r->next, run_len = r->gen && c->slot_kernels ? 1u << 12 : hlk::sc_run_len(r->poly, r->ir);
     bool have_claim = fs->recover_one && fs->have_claim;
     {
         Timed t(c, HL_T_ROUNDS);
+        StepPlan plan;
+        plan.fs = 1; plan.recover = fs->recover_one ? 1 : 0; plan.mask = d_mask; plan.mask_tab = d_mtab; plan.mask_vars = (int)mask_vars;
         u32 i = 0;
-        if (r->poly == hlk::POLY_IR) {
-            for (; i < nd && !rc && r->len > run_len; i++) {
-                rc = launch_round(r, have_claim ? 0 : 1, 1, have_claim ? 1 : 0, fs->recover_one ? 1 : 0, d_mask, d_mtab, (int)mask_vars);
-                if (!rc) rc = launch_fold(r);
-                have_claim = fs->recover_one != 0;
-            }
-        } else {
-            // closed-form families: after the first long round the fold with the last challenge rides on the next round's pass
-            // (two launches per round, every table word read once and written once); `pending`: the tables are still stored at
-            // twice r->len
-            bool pending = false;
-            for (; i < nd && !rc && r->len > run_len; i++) {
-                const int eval_one = have_claim ? 0 : 1;
-                // While a round's arithmetic fills the machine (the first rounds of a large cube) the fused pass is the slower
-                // one (it folds both halves before it can evaluate: measured 79 us against 40 + 15 at 2^19 pairs); once a round
-                // is down at the launch floor it saves one launch of three.
-                if (pending && r->len / 2 > FUSED_FOLD_MAX_PAIRS) {
-                    cudaError_t e = hlk::sc_fold(r->d_tables, r->stride, (u32)r->len, r->k, r->d_state, c->stream);
-                    c->stats.kernel_launches++;
-                    if (e != cudaSuccess) { rc = fail(c, HL_B200_ERR_DEVICE, "fold launch", e); break; }
-                    pending = false;
-                }
-                if (!pending) {
-                    rc = launch_round(r, eval_one, 1, have_claim ? 1 : 0, fs->recover_one ? 1 : 0, d_mask, d_mtab, (int)mask_vars);
-                } else {
-                    const u32 nb = hlk::sc_round_blocks((u32)(r->len / 2), c->sm_count);
-                    cudaError_t e = hlk::sc_fold_round(r->poly, (int)r->k, r->d_tables, r->stride, (u32)r->len, r->d_coefs, r->d_state, eval_one, r->d_partials,
-                                                       nb, c->stream);
-                    c->stats.kernel_launches++;
-                    if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "fold + round launch", e);
-                    if (!rc) rc = launch_step(r, nb, 1, have_claim ? 1 : 0, fs->recover_one ? 1 : 0, d_mask, d_mtab, (int)mask_vars);
-                }
-                r->len /= 2;
-                r->next++;
-                pending = true;
-                have_claim = fs->recover_one != 0;
-            }
-            if (!rc && pending) {  // the last challenge's fold
-                cudaError_t e = hlk::sc_fold(r->d_tables, r->stride, (u32)r->len, r->k, r->d_state, c->stream);
-                c->stats.kernel_launches++;
-                if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "fold launch", e);
-            }
+        for (; i < nd && !rc && r->len > run_len; i++) {
+            rc = launch_round(r, have_claim ? 0 : 1, have_claim ? 1 : 0, plan);
+            if (!rc) rc = launch_fold(r);
+            have_claim = fs->recover_one != 0;
+            plan.between = 1;
+        }
+        if (!rc && i == nd) {  // the batch ends here: the last challenge's claim
+            cudaError_t e = hlk::sc_between(step_of(r, r->next, 0, 0, plan), c->stream);
+            c->stats.kernel_launches++;
+            if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "step launch", e);
         }
         if (!rc && i < nd) {  // the short rounds: one launch (sumcheck_run.cu)
-            hlk::ScStep a;
-            a.partials = r->d_partials; a.nblocks = 1; a.degree = (int)r->degree; a.round = (int)r->next;
-            a.use_claim = 0; a.recover = fs->recover_one ? 1 : 0; a.fs = 1; a.mask = d_mask; a.mask_tab = d_mtab; a.mask_vars = (int)mask_vars;
-            a.inv_den = r->d_inv_den; a.state = r->d_state; a.out = r->d_out;
-            a.eval_degree = (int)r->eval_degree; a.extrap = r->d_extrap;
             const u32 left = nd - i;
-            cudaError_t e = hlk::sc_run(r->poly, r->ir, (int)r->k, r->d_tables, r->stride, (u32)r->len, r->d_coefs, a, (int)left, have_claim ? 1 : 0, r->d_sync,
-                                        r->d_partials, r->d_slots, c->sm_count, c->stream);
+            cudaError_t e = hlk::sc_run(r->poly, r->ir, (int)r->k, r->d_tables, r->stride, (u32)r->len, r->d_coefs, step_of(r, r->next, 1, 0, plan), (int)left,
+                                        have_claim ? 1 : 0, r->d_sync, r->d_slots, r->d_other, c->sm_count, c->stream);
             c->stats.kernel_launches++;
             if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "short rounds launch", e);
             r->len >>= left;

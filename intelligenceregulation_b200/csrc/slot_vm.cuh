@@ -14,6 +14,7 @@
 // Exact arithmetic on canonical words: any order of the sums and products gives the graph's value.
 #pragma once
 #include <algorithm>
+#include <functional>
 #include <utility>
 #include <vector>
 
@@ -36,7 +37,7 @@ GL_HD u32 coef_of(u64 w) { return (u32)(w >> 32); }
 
 // `parts` programs whose values sum to the polynomial's: part w starts at code[start[w]].  One part is the whole; where a round has fewer
 // pairs than the device has threads, several threads take a pair's parts.
-constexpr u32 MAX_PARTS = 4;
+constexpr u32 MAX_PARTS = 8;
 struct Program {
     std::vector<u64> code;
     std::vector<fp2> coefs;   // the general ones, in the order of their first use
@@ -61,23 +62,26 @@ class Compiler {
     void split(const ir::Shape& s, const u32* w, const fp2* cf, u32 parts) {
         parse(s, w, cf);
         const std::vector<Node> graph = nodes_;
-        // a term whose one non-linear factor is a sum that only it uses: the sum's units, each under the term's other factors
+        // a unit whose one non-linear factor is a sum that only it uses: the sum's units, each under the unit's other factors
         struct Item { size_t prefix; Unit u; u32 cost; };
         std::vector<Unit> prefixes;
         std::vector<Item> items;
         count_uses();
-        for (auto& u : nodes_.back().units) {
-            Unit pre{u.c, {}};
-            u32 non = 0, inner = 0;
-            for (u32 f : u.f) {
-                if (is_linear(f)) pre.f.push_back(f);
-                else { non++; inner = f & ~ir::IR_NODE; }
+        std::function<void(const Unit&, const std::vector<Unit>&)> flatten = [&](const Unit& pre, const std::vector<Unit>& units) {
+            prefixes.push_back(pre);
+            const size_t here = prefixes.size() - 1;
+            for (auto& u : units) {
+                Unit deeper{f2_mul(pre.c, u.c), pre.f};
+                u32 non = 0, inner = 0;
+                for (u32 f : u.f) {
+                    if (is_linear(f)) deeper.f.push_back(f);
+                    else { non++; inner = f & ~ir::IR_NODE; }
+                }
+                if (non == 1 && nodes_[inner].uses == 1 && nodes_[inner].units.size() > 1 && deeper.f.size() <= 2) flatten(deeper, nodes_[inner].units);
+                else items.push_back({here, u, unit_cost(u)});
             }
-            prefixes.push_back(non == 1 && nodes_[inner].uses == 1 ? pre : Unit{f2(1, 0), {}});
-            if (non == 1 && nodes_[inner].uses == 1)
-                for (auto& v : nodes_[inner].units) items.push_back({prefixes.size() - 1, v, unit_cost(v)});
-            else items.push_back({prefixes.size() - 1, u, unit_cost(u)});
-        }
+        };
+        flatten(Unit{f2(1, 0), {}}, nodes_.back().units);
         std::sort(items.begin(), items.end(), [](const Item& x, const Item& y) { return x.cost > y.cost; });
         if (parts > items.size()) parts = (u32)items.size();
         if (parts < 2) return;

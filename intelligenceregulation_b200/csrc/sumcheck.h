@@ -16,16 +16,19 @@ struct ScState {
     uint32_t key[8];
     u64 counter;
     int keyed;
-    int pad_;
+    int pending;    // 1 + the round whose claim and mask terms are still to be taken from `sums` and `r` (0: none)
     fp2 claim;
     fp2 r;
     fp2 acc;        // c sum_{i<j} u_i(r_i), c the mask's challenge
     fp2 ap;         // c a' prod_{i<j} r_i (the mask's linear term, sumcheck.rs:260-295)
+    fp2 sums[SC_MAX_POINTS];  // of the pending round
+    fp2 g[SC_MAX_POINTS];     // the mask's values for round ahead - 1
+    int ahead, pad_;
 };
 
 struct ScStep {
-    const u64* partials;        // nblocks x (degree+1) Fp2
-    u32 nblocks;
+    const u64* partials;        // nblocks x (degree+1) Fp2 (the generated kernels' rounds; the others add to ScSync)
+    u32 nblocks;                // rows, or the grid of a closed form's round
     int degree, round;
     int use_claim;              // s(1) := claim - s(0)
     int recover;                // keep the running claim (rounds.rs recover_one)
@@ -40,6 +43,7 @@ struct ScStep {
     const u64* extrap;          // (degree - eval_degree) rows of eval_degree + 1 base-field weights, or NULL
     ScState* state;
     u64* out;                   // per round: (degree+1) sums, (degree+1) masked, r  (Fp2 each)
+    int between = 0;            // a CTA beside the round's takes what the round before left pending
 };
 
 // a slot polynomial as a program (slot_vm.cuh), resident on the device
@@ -47,7 +51,7 @@ struct IrDev {
     const u64* code;
     const u64* coefs;  // n_coefs Fp2
     u32 n_code, n_coefs, n_tables, p_slots, a_slots;
-    u32 parts, start[4];   // the program in parts (slot_vm.cuh); code[0] starts the whole
+    u32 parts, start[8];   // the program in parts (slot_vm.cuh); code[0] starts the whole
     u32 eval_degree;   // min(declared, attained): the points the kernels evaluate are 0 .. eval_degree
 };
 
@@ -57,36 +61,37 @@ struct ScSync {
     u32 flag;         // rounds whose challenge is published
     u32 arrived;      // sums handed in so far
     u32 failed;       // a wait ran out
-    u32 pad_;
+    u32 done;         // CTAs of a round's own launch that have handed in their sums (back at zero with the last one)
+    // A round's sums, added up by all CTAs: per point the low and high halves of the two words, as plain integers (below 2^32 CTAs they
+    // do not wrap).  Two sets: the one that has been read is cleared for the round after the next.
+    u64 sums[2][SC_MAX_POINTS][4];
 };
 
 void sc_set_dependent_launch(bool on);
 bool sc_dependent_launch();
 u32 sc_round_blocks(u32 half, int sm_count);
-// the long rounds of a slot program; sc_ir_rows: the partial rows that a round writes; slots: sc_ir_slot_bytes of scratch (NULL when
-// that is 0)
-u32 sc_ir_rows(const IrDev& p, u32 half, int sm_count);
+// the long rounds of a slot program; slots: sc_ir_slot_bytes of scratch (NULL when that is 0)
 size_t sc_ir_slot_bytes(const IrDev& p, int sm_count);
-cudaError_t sc_round_ir(const IrDev& p, const u64* tables, size_t stride, u32 half, int degree, int eval_one, u64* slots, u64* partials, int sm_count,
+cudaError_t sc_round_ir(const IrDev& p, const u64* tables, size_t stride, u32 half, int degree, int eval_one, u64* slots, int sm_count, const ScStep& step, ScSync* sync,
                         cudaStream_t s);
-// all remaining rounds in one launch, from a table length of at most sc_run_len (sumcheck_run.cu).  partials: sc_run_partial_bytes;
-// slots: sc_run_slot_bytes of scratch (NULL when that is 0); sync: zeroed
-u32 sc_run_len(int poly);
-size_t sc_run_partial_bytes(int eval_degree, int sm_count);
+// all remaining rounds in one launch, from a table length of at most sc_run_len (sumcheck_run.cu).  slots: sc_run_slot_bytes of scratch (NULL when that is 0); other: sc_run_other_bytes; sync: zeroed
+constexpr int SC_RUN_CTAS = 4;  // per SM, at most
+u32 sc_run_len(int poly, const IrDev& p);
+size_t sc_run_other_bytes(int k, u32 len);
 size_t sc_run_slot_bytes(int poly, const IrDev& p, int k, int eval_degree, int sm_count);
 cudaError_t sc_run(int poly, const IrDev& p, int k, u64* tables, size_t stride, u32 len, const u64* coefs, const ScStep& a, int nrounds, int have_claim,
-                   ScSync* sync, u64* partials, u64* slots, int sm_count, cudaStream_t s);
+                   ScSync* sync, u64* slots, u64* other, int sm_count, cudaStream_t s);
 bool sc_supported(int poly, int k, int degree);
-cudaError_t sc_round(int poly, int k, const u64* tables, size_t stride, u32 half, const u64* coefs, int eval_one, u64* partials,
-                     u32 nblocks, cudaStream_t s);
-cudaError_t sc_step(const ScStep& a, cudaStream_t s);
-// closed-form families: fold with the challenge in `st` and sum the next round (length n after the fold) in one pass
-cudaError_t sc_fold_round(int poly, int k, u64* tables, size_t stride, u32 n, const u64* coefs, const ScState* st, int eval_one, u64* partials,
-                          u32 nblocks, cudaStream_t s);
+// A round's sums and, by the CTA that finishes last, its step (sync: zero, and left ready for the next round)
+cudaError_t sc_round(int poly, int k, const u64* tables, size_t stride, u32 half, const u64* coefs, int eval_one, const ScStep& step, ScSync* sync,
+                     cudaStream_t s);
+cudaError_t sc_step(const ScStep& a, cudaStream_t s);  // the step alone
 // bit t of *d_mask is set when table t holds a non-zero second word anywhere in its first `len` entries (*d_mask zeroed by the caller)
 cudaError_t sc_nonbase_mask(const u64* tables, size_t stride, size_t len, u32 k, u64* d_mask, int sm_count, cudaStream_t s);
 // the first entry of every table, k Fp2 in a row
 cudaError_t sc_finals(const u64* d_tables, size_t stride, u32 k, u64* d_out, cudaStream_t st);
 cudaError_t sc_fold(u64* tables, size_t stride, u32 half, u32 k, const ScState* st, cudaStream_t s);
+// takes what the round before a.round left pending
+cudaError_t sc_between(const ScStep& a, cudaStream_t s);
 
 }  // namespace hlk
