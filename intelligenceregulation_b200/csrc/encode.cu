@@ -36,8 +36,8 @@ __global__ void k_encode_generic(enc::RowArgs a, u32 logn) {
     }
 }
 
-template <int LOGN, int THREADS, int FORM = enc::FORM_PCS, bool NARROW = false>
-__global__ void __launch_bounds__(THREADS) k_encode_fast(enc::RowArgs a) {
+template <int LOGN, int THREADS, int MINB, int FORM, bool NARROW, bool LONG, bool SPLIT>
+__global__ void __launch_bounds__(THREADS, MINB) k_encode_fast(enc::RowArgs a) {
     using F = enc::Fast<LOGN>;
     extern __shared__ u64 smem[];
     u64* S = smem;
@@ -46,22 +46,20 @@ __global__ void __launch_bounds__(THREADS) k_encode_fast(enc::RowArgs a) {
     u64* X = a.scratch + (size_t)blockIdx.x * a.T * F::N;
     F::load_twiddles(a, TW, tid, THREADS);
     __syncthreads();
-    if (a.split) {
-        for (u32 unit = blockIdx.x; unit < (a.rows << a.logr); unit += gridDim.x) {
-            const u32 row = unit >> a.logr, s = unit & ((1u << a.logr) - 1u);
-            F::template row_coeffs<CtaSync, FORM, NARROW>(a, row, S, TW, X, tid, THREADS, CtaSync());
-            __syncthreads();
-            F::row_residue(a, row, s, S, TW, X, tid, THREADS, CtaSync());
+    // a unit of work: a whole row, or (split) one output residue of a row with the row's inverse transform before it
+    const u32 A = LONG ? 1u << a.loga : 1u, R = 1u << a.logr;
+    const u32 units = SPLIT ? a.rows << a.logr : a.rows;
+    for (u32 unit = blockIdx.x; unit < units; unit += gridDim.x) {
+        const u32 row = SPLIT ? unit >> a.logr : unit;
+        if constexpr (FORM == enc::FORM_COEF) {
+            F::row_given(a, row, X, tid, THREADS);
             __syncthreads();
         }
-        return;
-    }
-    for (u32 row = blockIdx.x; row < a.rows; row += gridDim.x) {
-        F::template row_coeffs<CtaSync, FORM, NARROW>(a, row, S, TW, X, tid, THREADS, CtaSync());
-        __syncthreads();  // the scratch slot is complete and shared memory is free again
-        for (u32 s = 0; s < (1u << a.logr); s++) {
-            F::row_residue(a, row, s, S, TW, X, tid, THREADS, CtaSync());
-            __syncthreads();
+        const u32 first = SPLIT ? unit & (R - 1u) : 0u, end = A + (SPLIT ? 1u : R);
+        for (u32 k = FORM == enc::FORM_COEF ? A : 0u; k < end; k++) {
+            const u32 step = k < A ? k : k + first;
+            F::template row_step<FORM, NARROW, LONG>(a, row, step, S, TW, X, tid, THREADS, CtaSync());
+            __syncthreads();  // the scratch slot is complete and shared memory is free again
         }
     }
 }
@@ -82,11 +80,20 @@ constexpr int fast_threads() {
     return g < 32 ? 32 : (g > 1024 ? 1024 : g);
 }
 
-template <int LOGN, int FORM = enc::FORM_PCS, bool NARROW = false>
-cudaError_t launch_fast(const enc::RowArgs& a, int sm_count, size_t scratch_words, cudaStream_t st, int* grid_out) {
+// Registers for 1,024 threads an SM, which is also what the rows' shared memory allows (12 n bytes a CTA of n / 16 threads): 64 a
+// thread.  With the 113 to 170 that the compiler takes otherwise only half as many fit, and rows wait on their passes' latencies:
+// 1,480 rows of 2^13 574 -> 474 us, 2,600 of 2^11 261 -> 201, 300 of 2^12 79 -> 69 (38 rows of 2^12, a CTA for each residue:
+// 32 -> 36, so split rows keep up to 128).
+template <int LOGN>
+constexpr int fast_min_ctas() {
+    return 1024 / fast_threads<LOGN>();
+}
+
+template <int LOGN, int FORM, bool NARROW, bool LONG, bool SPLIT>
+cudaError_t launch_fast_as(const enc::RowArgs& a, int sm_count, size_t scratch_words, cudaStream_t st, int* grid_out) {
     using F = enc::Fast<LOGN>;
     constexpr int T = fast_threads<LOGN>();
-    auto kern = k_encode_fast<LOGN, T, FORM, NARROW>;
+    auto kern = k_encode_fast<LOGN, T, SPLIT ? (T > 256 ? 1 : 512 / T) : fast_min_ctas<LOGN>(), FORM, NARROW, LONG, SPLIT>;
     size_t smem = (size_t)(F::N + F::TW_WORDS) * 8;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -95,7 +102,7 @@ cudaError_t launch_fast(const enc::RowArgs& a, int sm_count, size_t scratch_word
     if (e != cudaSuccess) return e;
     if (per_sm < 1) per_sm = 1;
     size_t grid = (size_t)sm_count * per_sm;
-    const size_t units = a.split ? (size_t)a.rows << a.logr : (size_t)a.rows;
+    const size_t units = SPLIT ? (size_t)a.rows << a.logr : (size_t)a.rows;
     if (grid > units) grid = units;
     size_t max_by_scratch = scratch_words / ((size_t)a.T * F::N);
     if (grid > max_by_scratch) grid = max_by_scratch;
@@ -103,6 +110,14 @@ cudaError_t launch_fast(const enc::RowArgs& a, int sm_count, size_t scratch_word
     *grid_out = (int)grid;
     kern<<<(unsigned)grid, T, smem, st>>>(a);
     return cudaGetLastError();
+}
+
+// split rows are few (a CTA per SM or fewer in a commitment): they get the registers that a row's latency wants
+template <int LOGN, int FORM = enc::FORM_PCS, bool NARROW = false, bool LONG = false>
+cudaError_t launch_fast(const enc::RowArgs& a, int sm_count, size_t scratch_words, cudaStream_t st, int* grid_out) {
+    if constexpr (!LONG)
+        if (a.split) return launch_fast_as<LOGN, FORM, NARROW, LONG, true>(a, sm_count, scratch_words, st, grid_out);
+    return launch_fast_as<LOGN, FORM, NARROW, LONG, false>(a, sm_count, scratch_words, st, grid_out);
 }
 
 }  // namespace
@@ -143,7 +158,9 @@ cudaError_t encode_rows(const enc::RowArgs& a, u32 logn, bool allow_fast, int sm
             case 11: return launch_fast<11>(a, sm_count, scratch_words, st, &grid);
             case 12: return launch_fast<12>(a, sm_count, scratch_words, st, &grid);
             case 13: return launch_fast<13>(a, sm_count, scratch_words, st, &grid);
-            case 14: return launch_fast<14>(a, sm_count, scratch_words, st, &grid);
+            case 14:
+                if (a.loga) return launch_fast<14, enc::FORM_PCS, false, true>(a, sm_count, scratch_words, st, &grid);
+                return launch_fast<14>(a, sm_count, scratch_words, st, &grid);
         }
     }
     if (logn < 1 || logn > 14) return cudaErrorInvalidValue;

@@ -76,7 +76,7 @@ struct RowArgs {
                        // for a handful of rows (fewer than SMs / residues) the latency of a row falls from 1 + R transforms to 2
 };
 
-// What a row is and how its coefficients are twisted (template argument of Fast::row_coeffs).
+// What a row is and how its coefficients are twisted (template argument of Fast::row_step).
 //   FORM_PCS    the commitment forms above: plain (no twist) or hiding (pads folded in, coset powers)
 //   FORM_COSET  n evaluations -> n coefficients c, x[i] = c[i] h^i, c kept in coef_out (a masking commitment's message rows,
 //               hashline/src/zk.rs:463-476: pads sit inside the message, the coset is applied to every row)
@@ -209,13 +209,13 @@ struct Fast {
         }
     }
 
-    // first pass: element i of the transform's input comes from source(i); lanes take neighbouring i
-    template <class Source>
-    GL_HD static void first_pass(u64* S, const u64* TW, u32 tid, u32 nt, Source source) {
+    // first pass: fill(t, e) brings the thread's 16 inputs, e[j] = element t + brev4(j) n/16 (position 16 brev(t) + j holds index
+    // brev(16 brev(t) + j)); lanes take neighbouring t
+    template <class Fill>
+    GL_HD static void first_pass(u64* S, const u64* TW, u32 tid, u32 nt, Fill fill) {
         for (u32 t = tid; t < GROUPS; t += nt) {
             u64 e[16];
-#pragma unroll
-            for (int j = 0; j < 16; j++) e[j] = source(t + brev4((u32)j) * GROUPS);  // position 16 g + j holds index brev(16 g + j)
+            fill(t, e);
             stages<0, 0, 4>(e, TW, 0);
             const u32 sb = swz(gl_brev(t, LOGN - 4) << 4);
 #pragma unroll
@@ -236,104 +236,159 @@ struct Fast {
         }
     }
 
-    // last pass: output k = g + j n/16 goes to sink(k, lazy value)
-    template <class Sink>
-    GL_HD static void last_pass(const u64* S, const u64* TW, u32 tid, u32 nt, Sink sink) {
+    // last pass: drain(g, e) takes the outputs k = g + j n/16, lazy words
+    template <class Drain>
+    GL_HD static void last_pass(const u64* S, const u64* TW, u32 tid, u32 nt, Drain drain) {
         for (u32 g = tid; g < GROUPS; g += nt) {
             const u32 sb = swz(g);
             u64 e[16];
 #pragma unroll
             for (int j = 0; j < 16; j++) e[j] = S[sb ^ swzc((u32)j << LASTW)];
             stages<LASTW, LASTLO, LOGN>(e, TW, g);
-#pragma unroll
-            for (int j = 0; j < 16; j++) sink(g + ((u32)j << LASTW), e[j]);
+            drain(g, e);
         }
     }
 
-    template <class Source, class Sink, class Sync>
-    GL_HD static void transform(u64* S, const u64* TW, u32 tid, u32 nt, Source source, Sink sink, Sync sync) {
-        first_pass(S, TW, tid, nt, source);
+    template <class Fill, class Drain, class Sync>
+    GL_HD static void transform(u64* S, const u64* TW, u32 tid, u32 nt, Fill fill, Drain drain, Sync sync) {
+        first_pass(S, TW, tid, nt, fill);
         sync();
         // full 4-stage windows below the last pass's first stage: [4,8) when LASTLO >= 8, [8,12) when LASTLO >= 12
         if constexpr (LASTLO >= 8) { mid_pass<4>(S, TW, tid, nt); sync(); }
         if constexpr (LASTLO >= 12) { mid_pass<8>(S, TW, tid, nt); sync(); }
-        last_pass(S, TW, tid, nt, sink);
+        last_pass(S, TW, tid, nt, drain);
     }
 
-    // ---- the row pipeline ----
-    // inverse transform of the message row, then the coefficient blocks x[idx] into the scratch slot.
-    // c[i] = F[(n - i) mod n] / n with F the forward transform of the message, one residue a of F per pass set.
-    template <class Sync, int FORM = FORM_PCS, bool NARROW = false>
-    GL_HD static void row_coeffs(const RowArgs& a, u32 row, u64* S, const u64* TW, u64* X, u32 tid, u32 nt, Sync sync) {
-        const u32 A = 1u << a.loga, n = N << a.loga, nn = N << a.logr, lognn = LOGN + a.logr;
-        if constexpr (FORM == FORM_COEF) {
-            const u64* cs = a.data + (size_t)row * (n + a.q);
-            for (u32 i = tid; i < n + a.q; i += nt) X[i] = gl_mul(cs[i], a.pows[i]);
-            return;
-        }
+    // ---- the row pipeline: A = n / N inverse transforms, then A transforms per output residue s < R = nn / n ----
+    // Step r < A belongs to the message's inverse transform: c[i] = F[(n - i) mod n] / n with F the forward transform of the message,
+    // and the coefficients x[idx] go into the scratch slot.  Step A + A s + r belongs to output residue s: the size-n transform of the
+    // twisted coefficients, stored at out[R k + s].  Both kinds run through ONE copy of the passes, and what differs (where a
+    // thread's 16 words come from and go to) is a branch of the whole grid: two unrolled transforms in one kernel did not fit the
+    // instruction cache (2,606 rows of 2^14: 2,090 us with two, 1,920 with one; 38 rows of 2^12: 42 and 32).
+    //
+    // LONG, rows of A = 2 or 4 times N words: step r transforms the words A m + r, and with p_r[k] = w_n^(r k) Y_r[k] the size-n
+    // outputs are Z[k + N b] = sum_r w_A^(r b) p_r[k].  The p_r of r < A - 1 wait in the row's own output, at the places that the
+    // same thread fills when it has p_(A-1): every output word is then written R words from the last, not A R (a 2^16-word row at
+    // rate 1/2 wrote 8 bytes to each 64 and went to memory for the rest of every sector: 400 rows 2,825 -> 1,930 us).
+    template <int FORM, bool NARROW, bool LONG, class Sync>
+    GL_HD static void row_step(const RowArgs& a, u32 row, u32 step, u64* S, const u64* TW, u64* X, u32 tid, u32 nt, Sync sync) {
+        const u32 loga = LONG ? a.loga : 0u, A = 1u << loga, n = N << loga, nn = N << a.logr, logr = a.logr - loga;
+        bool inverse = false;
+        if constexpr (FORM != FORM_COEF) inverse = step < A;
+        const u32 s = inverse ? 0u : (step - A) >> loga, r = step & (A - 1u);
         const u64* src = a.data + (size_t)row * n;
-        const u64* pad = a.pads + (size_t)row * a.q;
-        const u32 Tn = a.zk ? (n + a.q + n - 1) / n : 1u;
-        const unsigned char* nsrc = nullptr;
-        u32 nw = 8;
-        if constexpr (NARROW) { nsrc = a.narrow + a.row_off[row]; nw = a.row_w[row]; }
-        for (u32 ra = 0; ra < A; ra++) {
-            transform(S, TW, tid, nt,
-                      [&](u32 i) {
-                          u64 y;
-                          if constexpr (NARROW) {  // loga == 0 on this path: every word of the row passes here exactly once
-                              y = widen_word(nsrc, i, nw);
-                              const_cast<u64*>(src)[i] = y;
-                          } else {
-                              y = src[i];
+        u64* dst = a.enc + (size_t)row * nn;
+        transform(S, TW, tid, nt,
+                  [&](u32 t0, u64 (&e)[16]) {
+                      if (!inverse) {
+                          const u32 live = n + a.q;  // x is zero from n + q on (plain form: q = 0); those words are never written or read
+#pragma unroll
+                          for (int j = 0; j < 16; j++) {
+                              const u32 m = t0 + brev4((u32)j) * GROUPS, i = (m << loga) + r;
+                              u64 y = ENC_LDCG(X + r * N + m);
+#pragma unroll 1
+                              for (u32 k = i + n; k < live; k += n)  // the pads' copies above the message
+                                  y = gl_add(y, gl_mul_fast(ENC_LDCG(X + k), a.tw_nn[((k - i) * s) & (nn - 1)]));
+                              if (s) y = gl_mul_lazy(y, a.tw_nn[(i * s) & (nn - 1)]);  // a pass takes lazy words
+                              e[j] = y;
                           }
-                          if (a.loga) {
-                              for (u32 t = 1; t < A; t++)
-                                  y = gl_add(y, gl_mul_fast(src[i + t * N], a.tw_nn[((t * ra) << (lognn - a.loga)) & (nn - 1)]));  // w_A^(t a)
-                              if (ra) y = gl_mul_lazy(y, a.tw_nn[((i * ra) << (a.logr - a.loga)) & (nn - 1)]);                // w_n^(i a); a pass takes lazy words
+                      } else if constexpr (NARROW) {  // never LONG: every word of the row passes here exactly once
+                          const unsigned char* nsrc = a.narrow + a.row_off[row];
+                          const u32 nw = a.row_w[row];
+#pragma unroll
+                          for (int j = 0; j < 16; j++) {
+                              const u32 i = t0 + brev4((u32)j) * GROUPS;
+                              e[j] = widen_word(nsrc, i, nw);
+                              const_cast<u64*>(src)[i] = e[j];
                           }
-                          return y;
-                      },
-                      [&](u32 k, u64 v) {
-                          const u32 i = (n - ((k << a.loga) + ra)) & (n - 1);
-                          const u64 c = gl_mul_fast(v, a.ninv);
-                          if constexpr (FORM == FORM_COSET) {
-                              X[i] = gl_mul(c, a.pows[i]);
-                              if (a.coef_out) a.coef_out[(size_t)row * 2 * n + i] = c;
-                          } else {
-                              for (u32 t = 0; t < Tn; t++) {
-                                  const u32 idx = i + t * n;
-                                  u64 x = t == 0 ? c : 0;
-                                  if (a.zk) {
-                                      if (idx >= n + a.q) break;
-                                      if (idx < a.q) x = gl_sub(x, pad[idx]);
-                                      if (idx >= n && idx - n < a.q) x = gl_add(x, pad[idx - n]);
-                                      x = gl_mul_fast(x, a.pows[idx]);
-                                  }
-                                  X[idx] = x;
+                      } else {
+#pragma unroll
+                          for (int j = 0; j < 16; j++) e[j] = src[((t0 + brev4((u32)j) * GROUPS) << loga) + r];
+                      }
+                  },
+                  [&](u32 g, u64 (&e)[16]) {
+                      if constexpr (LONG) {
+                          for (int j = 0; j < 16; j++) {  // rolled: 16 copies were 15 % slower (instruction cache)
+                              const u32 k = g + ((u32)j << LASTW);
+                              u64 p = e[j];
+                              if (r) p = gl_mul_fast(p, a.tw_nn[((r * k) << logr) & (nn - 1)]);  // w_n^(r k)
+                              u64* at = dst + ((size_t)k << logr) + s;  // b words of N << logr further on: output k + N b
+                              const size_t step_b = (size_t)N << logr;
+                              if (r + 1 < A) {
+                                  at[r * step_b] = p;
+                                  continue;
+                              }
+                              u64 z[4] = {gl_canon_fast(at[0]), 0, 0, 0};
+                              if (loga == 1) {
+                                  z[1] = gl_sub(z[0], p);
+                                  z[0] = gl_add(z[0], p);
+                              } else {
+                                  const u64 p1 = at[step_b], p2 = at[2 * step_b];
+                                  const u64 c = gl_add(z[0], p2), d = gl_sub(z[0], p2), f = gl_add(p1, p), h = gl_mul_fast(gl_sub(p1, p), a.tw_nn[nn / 4]);
+                                  z[0] = gl_add(c, f);
+                                  z[1] = gl_add(d, h);
+                                  z[2] = gl_sub(c, f);
+                                  z[3] = gl_sub(d, h);
+                              }
+                              for (u32 b = 0; b < A; b++) {
+                                  if (inverse) store_coeff<FORM>(a, row, (n - (k + N * b)) & (n - 1), n, loga, z[b], X);
+                                  else at[b * step_b] = z[b];
                               }
                           }
-                      },
-                      sync);
-            if (ra + 1 < A) sync();  // the next residue's first pass overwrites the shared-memory row
-        }
+                      } else if (!inverse) {
+#pragma unroll
+                          for (int j = 0; j < 16; j++) dst[((size_t)(g + ((u32)j << LASTW)) << logr) + s] = gl_canon_fast(e[j]);
+                      } else {
+#pragma unroll
+                          for (int j = 0; j < 16; j++) store_coeff<FORM>(a, row, (n - (g + ((u32)j << LASTW))) & (n - 1), n, 0, e[j], X);
+                      }
+                  },
+                  sync);
     }
 
-    // output residue s: the size-N transform of the twisted coefficients, stored at out[(nn/N) k + s]
+    // coefficient i of a row from the inverse transform's word v = n c[i] (lazy) into the scratch slot, where words i < n stand by
+    // i mod A first (the order the transforms read them in)
+    template <int FORM>
+    GL_HD static void store_coeff(const RowArgs& a, u32 row, u32 i, u32 n, u32 loga, u64 v, u64* X) {
+        u64 c = gl_mul_fast(v, a.ninv);
+        if constexpr (FORM == FORM_COSET) {
+            if (a.coef_out) a.coef_out[(size_t)row * 2 * n + i] = c;
+            c = gl_mul(c, a.pows[i]);
+        } else if (a.zk) {
+            const u64* pad = a.pads + (size_t)row * a.q;
+            if (i < a.q) {
+                c = gl_sub(c, pad[i]);
+#pragma unroll 1
+                for (u32 k = i; k < a.q; k += n) {  // the pads' copies above the message: x[n + k] = pad[k] - pad[n + k]
+                    u64 u = pad[k];
+                    if (k + n < a.q) u = gl_sub(u, pad[k + n]);
+                    X[n + k] = gl_mul_fast(u, a.pows[n + k]);
+                }
+            }
+            c = gl_mul_fast(c, a.pows[i]);
+        }
+        X[(i & ((1u << loga) - 1u)) * N + (i >> loga)] = c;
+    }
+
+    // rows given as coefficients: straight into the scratch slot
+    GL_HD static void row_given(const RowArgs& a, u32 row, u64* X, u32 tid, u32 nt) {
+        const u64* cs = a.data + (size_t)row * (N + a.q);
+        for (u32 i = tid; i < N + a.q; i += nt) X[i] = gl_mul(cs[i], a.pows[i]);
+    }
+
+    // the pipeline a half at a time: the message's coefficients, then the transform of step A + s (s < A R)
     template <class Sync>
-    GL_HD static void row_residue(const RowArgs& a, u32 row, u32 s, u64* S, const u64* TW, const u64* X, u32 tid, u32 nt, Sync sync) {
-        const u32 nn = N << a.logr, live = (N << a.loga) + a.q;  // x is zero from n + q on (plain form: q = 0)
-        u64* dst = a.enc + ((size_t)row * N << a.logr) + s;
-        transform(S, TW, tid, nt,
-                  [&](u32 i) {
-                      u64 y = ENC_LDCG(X + i);
-                      // the scratch words from n + q on are never written and never read
-                      for (u32 t = 1; t < a.T && i + t * N < live; t++)
-                          y = gl_add(y, gl_mul_fast(ENC_LDCG(X + (size_t)t * N + i), a.tw_nn[(t * s * N) & (nn - 1)]));
-                      if (s) y = gl_mul_lazy(y, a.tw_nn[(i * s) & (nn - 1)]);  // a pass takes lazy words
-                      return y;
-                  },
-                  [&](u32 k, u64 v) { dst[(size_t)k << a.logr] = gl_canon_fast(v); }, sync);
+    GL_HD static void row_coeffs(const RowArgs& a, u32 row, u64* S, const u64* TW, u64* X, u32 tid, u32 nt, Sync sync) {
+        for (u32 r = 0; r < (1u << a.loga); r++) {
+            if (r) sync();  // the next residue's first pass overwrites the shared-memory row
+            if (a.loga) row_step<FORM_PCS, false, LOGN == 14>(a, row, r, S, TW, X, tid, nt, sync);
+            else row_step<FORM_PCS, false, false>(a, row, r, S, TW, X, tid, nt, sync);
+        }
+    }
+    template <class Sync>
+    GL_HD static void row_residue(const RowArgs& a, u32 row, u32 s, u64* S, const u64* TW, u64* X, u32 tid, u32 nt, Sync sync) {
+        if (a.loga) row_step<FORM_PCS, false, LOGN == 14>(a, row, (1u << a.loga) + s, S, TW, X, tid, nt, sync);
+        else row_step<FORM_PCS, false, false>(a, row, 1u + s, S, TW, X, tid, nt, sync);
     }
 };
 

@@ -1,0 +1,36 @@
+"""Encoded rows at the edges of the row encoder's forms: one CTA per (row, residue) against one per row on both sides of a CTA an SM,
+every transform size, and rows of two and four transforms (one output residue, pads above twice the row)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+P = 0xFFFFFFFF00000001
+
+
+@pytest.fixture(scope="module")
+def dev():
+    from intelligenceregulation_b200 import backend
+
+    d = backend.B200Backend(device=0)
+    yield d
+    d.ctx.close()
+
+
+CASES = [(n, 2, rows, 33) for n in range(8, 15) for rows in (1, 74, 75)]
+CASES += [(9, 4, 38, 600), (14, 1, 2, 0), (15, 1, 2, 0), (16, 1, 1, 0), (15, 2, 3, 1), (16, 4, 1, 150000)]
+
+
+@pytest.mark.parametrize("log_cols,inv_rate,rows,q", CASES)
+def test_encoded_rows_match_the_oracle(dev, oracle, log_cols, inv_rate, rows, q):
+    n, nn = 1 << log_cols, inv_rate << log_cols
+    rng = np.random.default_rng(log_cols * 1000 + rows)
+    data = rng.integers(0, P, size=rows * n, dtype=np.uint64)
+    if q:
+        pads, pows = rng.integers(0, P, size=rows * q, dtype=np.uint64), oracle.coset_powers(7, nn)
+        want = oracle.encode_rows_zk(data, rows, n, pads, q, pows, 18)
+        store, leaves = dev.try_commit_zk_keyed(log_cols, inv_rate, data, pads, pows, 18, None)
+    else:
+        want = oracle.encode_rows_plain(data, rows, n, nn, 18)
+        store, leaves = dev.try_commit(log_cols, inv_rate, data, 18)
+    assert (leaves == oracle.hash_columns(want, rows, nn)).all()
+    store.free()
