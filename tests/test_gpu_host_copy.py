@@ -54,3 +54,12 @@ def test_two_contexts_at_once():
     for t in threads:
         t.join()
     assert not bad, bad
+
+
+@pytest.mark.parametrize("extra", [16384 - 1, 16384, 16384 + 1, 3 * 16384 + 1])
+def test_last_piece_of_whole_and_short_shares(extra):
+    from intelligenceregulation_b200 import backend
+
+    ctx = backend.Context(0)
+    _same_back(ctx, _words(2 * 65536 + extra, extra))  # pieces of 64 Ki words, each filled and emptied in four shares
+    ctx.close()
