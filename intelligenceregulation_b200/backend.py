@@ -625,14 +625,9 @@ class B200Tables:
         """`Tab::Priv`: a committed plane (argument.rs:386-577).  `rows`: a `B200Commit` (its resident data rows) or a
         (device address, word count) pair; `coords`: the plane's coordinates, first = most significant index bit, each
         ("rho", k) | ("flip", k) | ("fixed", (c0, c1)); `slices`: [(word offset, (c0, c1))]."""
-        codes, fixed, read = [], [], []
-        for c in coords:
-            if c[0] == "fixed":
-                codes.append(_COORD_FIXED)
-                fixed += c[1]
-            else:
-                read.append(c[1])
-                codes.append(-1 - c[1] if c[0] == "flip" else c[1])
+        fixed = [w for c in coords if c[0] == "fixed" for w in c[1]]
+        codes = [c[1] if c[0] == "rho" else -1 - c[1] if c[0] == "flip" else _COORD_FIXED for c in coords]
+        read = [c[1] for c in coords if c[0] != "fixed"] if fixed else [c[1] for c in coords]
         if len(set(read)) != len(read):
             raise ValueError("plane_maps: a cube variable read by two coordinates (the host builder accumulates; not planned)")
         sl = [int(v) for off, cf in slices for v in (off, cf[0], cf[1])]

@@ -309,6 +309,12 @@ int hl_b200_rounds_from_tables_ir(hl_ctx* c, uint32_t degree, hl_tables* t, cons
         return fail(c, HL_B200_ERR_UNSUPPORTED, "rounds_from_tables_ir: table count, degree or program size beyond the evaluator's limits");
     ir::Shape sh{(u32)k, n_nodes, n_terms, (u32)ncoefs, (u32)n_words};
     if (ir::validate(sh, words)) return fail(c, HL_B200_ERR_ARG, "rounds_from_tables_ir: malformed program");
+    {
+        // the tables' kernels go first: the device builds them (the width check's 37 of 2^19 entries: 90 us) while this thread compiles
+        // the program (its 250 instructions and their parts: 90 us)
+        Call g(c);
+        if (int rc = hl_tables_flush_locked(t)) return rc;
+    }
     vm::Compiler prog;
     compile(prog, sh, words, coefs);
     GenAsk gen;

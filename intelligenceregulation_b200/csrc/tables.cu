@@ -263,6 +263,7 @@ int hl_tables_flush_locked(hl_tables* t) {
     if (!rc) rc = d2h(c, &flag, t->d_flag, 4);
     if (!rc) rc = sync(c, "tables_flush");
     if (!rc && flag) rc = fail(c, HL_B200_ERR_MISMATCH, "tables: a table declared base-valued holds an extension word");
+    if (!rc) t->checked = false;  // asked and answered: the next plan asks again
     return rc;
 }
 
