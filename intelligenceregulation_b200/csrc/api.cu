@@ -161,7 +161,7 @@ void hl_b200_shutdown(hl_ctx* c) {
     cudaSetDevice(c->device);
     cudaStreamSynchronize(c->stream);
     for (auto& kv : c->tw) cudaFree(kv.second);
-    if (c->d_wp_flag) cudaFree(c->d_wp_flag);
+    if (c->wp_flag) cudaFreeHost(c->wp_flag);
     host_copy_release(c);
     if (c->arena) cudaFreeHost(c->arena);
     for (auto& s : c->spans) { cudaEventDestroy(s.a); cudaEventDestroy(s.b); }

@@ -38,7 +38,7 @@ struct hl_ctx {
     size_t arena_off = 0;
     struct Pending { void* to; const char* from; size_t bytes; };
     std::vector<Pending> pending;  // small results in the bounce area, handed out by the next `sync`
-    int* d_wp_flag = nullptr;  // the witness products' status word: zero between calls
+    int* wp_flag = nullptr;  // page-locked: the witness products' status word: zero between calls
     bool wp_attr = false;      // the product kernel's shared-memory size has been raised on this device
     std::set<const struct hl_store*> stores;  // the live commitment stores (a planned slot table that reads one checks it is still there when it is built)
     size_t alloc_live = 0;   // bytes handed out and not yet returned

@@ -4,9 +4,11 @@
 //   k_wp_pack      x (int64, row stride xs) -> two byte planes per 128-token tile: hi = x >> 8 (signed), lo = x & 255
 //                  (unsigned), K padded with zeros to a multiple of 128; an activation outside int16 raises the flag
 //   k_wp_repack    weights the product kernel cannot read in place (in_out layout, or K not a multiple of 128) -> rows of Kp bytes
+//                  in whole boxes, zeros included
 //   k_wp_umma      out[128 x 256 tile] = 256 (A_hi B) + (A_lo B): tcgen05.mma kind::i8 (signed x signed for the high bytes,
 //                  unsigned x signed for the low bytes), int32 accumulators in TMEM, int64 result written by the epilogue;
-//                  split over K with integer atomics (integer addition: any order gives the same words)
+//                  split over K inside a cluster (partial sums through distributed shared memory), and beyond four CTAs of a
+//                  cluster with integer atomics (integer addition: any order gives the same words)
 // |sum lo w| <= K * 255 * 128 < 2^31 for K <= 65,536 (metal.rs:4234 states the same bound), so int32 never wraps.
 #include <cuda.h>
 
@@ -28,6 +30,7 @@ __global__ void __launch_bounds__(256) k_wp_pack(const long long* __restrict__ x
     for (size_t i = ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x; i < clear_words;
          i += (size_t)gridDim.x * gridDim.y * blockDim.x)
         clear[i] = 0;
+    asm volatile("griddepcontrol.launch_dependents;\n" ::);  // the product kernel may set itself up and fetch weights meanwhile
     const u32 t = blockIdx.y;  // padded token index
     const u32 mt = t / WP_MT, r = t % WP_MT;
     uint8_t* hi = A + ((size_t)mt * 2 * WP_MT + r) * Kp;
@@ -46,32 +49,70 @@ __global__ void __launch_bounds__(256) k_wp_pack(const long long* __restrict__ x
             h |= (u32)((v >> 8) & 255) << (8 * j);
             l |= (u32)(v & 255) << (8 * j);
         }
-        if (bad) atomicExch(flag, 1);
+        if (bad) *reinterpret_cast<volatile int*>(flag) = 1;
         *reinterpret_cast<u32*>(hi + k) = h;
         *reinterpret_cast<u32*>(lo + k) = l;
     }
 }
 
-// in_out: src[i * N + j] -> dst[j * Kp + i]; else src[j * K + i] -> dst[j * Kp + i]; dst is zero beyond K (memset before)
-__global__ void __launch_bounds__(256) k_wp_repack(const int8_t* __restrict__ src, u32 K, u32 N, u32 Kp, int in_out, int8_t* __restrict__ dst) {
-    __shared__ int8_t tile[64][65];
-    const u32 k0 = blockIdx.x * 64, n0 = blockIdx.y * 64;
+// four bytes from p on, of which the first `valid` belong to the row (the others read as zero); `lo` and `hi` bound the readable bytes
+__device__ __forceinline__ u32 wp_load4(const int8_t* p, int valid, const int8_t* lo, const int8_t* hi) {
+    const uintptr_t at = (uintptr_t)p & ~(uintptr_t)3;
+    if (valid >= 4 && at >= (uintptr_t)lo && at + 8 <= (uintptr_t)hi) {
+        const u32* w = reinterpret_cast<const u32*>(at);
+        return __funnelshift_r(w[0], w[1], 8 * (u32)((uintptr_t)p & 3));
+    }
+    u32 v = 0;
+    for (int j = 0; j < 4 && j < valid; j++) v |= (u32)(uint8_t)p[j] << (8 * j);
+    return v;
+}
+
+// in_out: src[i * N + j] -> dst[j * Kp + i]; else src[j * K + i] -> dst[j * Kp + i]; zero beyond K and N.  A CTA fills 128 rows of 128
+// bytes in 16-byte stores.  The transposing form turns 16 words (16 k, 4 n each) into 4 rows of 16 bytes per thread; the tile's words
+// stand rotated by their row block, so that both its accesses take 32 banks.  Bound by memory: 16.8 MB transposed 26 us by single
+// bytes, 12 now.  It reads nothing of the packing kernel's and may run beside it; it ends after it, so that whoever waits for this kernel has both.
+__global__ void __launch_bounds__(256) k_wp_repack(const int8_t* __restrict__ src, size_t src_len, u32 K, u32 N, u32 Kp, int in_out, int8_t* __restrict__ dst) {
+    __shared__ u32 tile[128][32];
+    asm volatile("griddepcontrol.launch_dependents;\n" ::);
+    const u32 k0 = blockIdx.x * 128, n0 = blockIdx.y * 128;
+    const int8_t* end = src + src_len;
+    const u32 seg = threadIdx.x & 7, grp = threadIdx.x >> 3;  // 16 bytes of a row; a group of four rows
     if (in_out) {
-        for (u32 e = threadIdx.x; e < 64 * 64; e += blockDim.x) {
-            const u32 kk = e / 64, nn = e % 64;  // consecutive threads along n: contiguous in the source
-            tile[kk][nn] = (k0 + kk < K && n0 + nn < N) ? src[(size_t)(k0 + kk) * N + n0 + nn] : (int8_t)0;
+#pragma unroll 4
+        for (u32 e = threadIdx.x; e < 128 * 32; e += 256) {
+            const u32 kk = e >> 5, n4 = e & 31, n = n0 + 4 * n4;
+            tile[kk][(n4 + 4 * (kk >> 4)) & 31] = k0 + kk < K && n < N ? wp_load4(src + (size_t)(k0 + kk) * N + n, (int)min(N - n, 4u), src, end) : 0u;
         }
         __syncthreads();
-        for (u32 e = threadIdx.x; e < 64 * 64; e += blockDim.x) {
-            const u32 nn = e / 64, kk = e % 64;
-            if (n0 + nn < N && k0 + kk < K) dst[(size_t)(n0 + nn) * Kp + k0 + kk] = tile[kk][nn];
+        u32 o[4][4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            u32 w[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) w[j] = tile[seg * 16 + 4 * q + j][(grp + 4 * seg) & 31];
+            const u32 a = __byte_perm(w[0], w[1], 0x5140), b = __byte_perm(w[2], w[3], 0x5140), c = __byte_perm(w[0], w[1], 0x7362),
+                      d = __byte_perm(w[2], w[3], 0x7362);
+            o[0][q] = __byte_perm(a, b, 0x5410);
+            o[1][q] = __byte_perm(a, b, 0x7632);
+            o[2][q] = __byte_perm(c, d, 0x5410);
+            o[3][q] = __byte_perm(c, d, 0x7632);
         }
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+            *reinterpret_cast<uint4*>(dst + (size_t)(n0 + 4 * grp + r) * Kp + k0 + 16 * seg) = make_uint4(o[r][0], o[r][1], o[r][2], o[r][3]);
     } else {
-        for (u32 e = threadIdx.x; e < 64 * 64; e += blockDim.x) {
-            const u32 nn = e / 64, kk = e % 64;
-            if (n0 + nn < N && k0 + kk < K) dst[(size_t)(n0 + nn) * Kp + k0 + kk] = src[(size_t)(n0 + nn) * K + k0 + kk];
+        const u32 k = k0 + 16 * seg;
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            const u32 n = n0 + grp + 32 * r;
+            u32 o[4] = {0, 0, 0, 0};
+#pragma unroll
+            for (u32 q = 0; q < 4; q++)
+                if (n < N && k + 4 * q < K) o[q] = wp_load4(src + (size_t)n * K + k + 4 * q, (int)min(K - k - 4 * q, 4u), src, end);
+            *reinterpret_cast<uint4*>(dst + (size_t)n * Kp + k) = make_uint4(o[0], o[1], o[2], o[3]);
         }
     }
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -137,11 +178,44 @@ __device__ __forceinline__ void um_ld32(u32 taddr, u32 (&r)[32]) {
         : "r"(taddr));
 }
 
+__device__ __forceinline__ void um_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+// 32 result words of one row; a lane's words are consecutive, so a vector store of 32 bytes fills a sector (8-byte stores alone took
+// longer than the tile's arithmetic at 128 tokens)
+__device__ __forceinline__ void um_store32(long long* o, const u32 (&hi)[32], const u32 (&lo)[32], u32 live, bool add, u32 align) {
+    if (add || live < 32 || (align & 15)) {
+#pragma unroll
+        for (int j = 0; j < 32; j++) {
+            if ((u32)j >= live) continue;
+            const long long v = 256ll * (int)hi[j] + (int)lo[j];
+            if (add) atomicAdd(reinterpret_cast<unsigned long long*>(o + j), (unsigned long long)v);
+            else o[j] = v;
+        }
+    } else if (align & 31) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 2)
+            *reinterpret_cast<longlong2*>(o + j) = make_longlong2(256ll * (int)hi[j] + (int)lo[j], 256ll * (int)hi[j + 1] + (int)lo[j + 1]);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 32; j += 4)
+            asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};\n" ::"l"(o + j), "l"(256ll * (int)hi[j] + (int)lo[j]),
+                         "l"(256ll * (int)hi[j + 1] + (int)lo[j + 1]), "l"(256ll * (int)hi[j + 2] + (int)lo[j + 2]), "l"(256ll * (int)hi[j + 3] + (int)lo[j + 3])
+                         : "memory");
+    }
+}
+
 // grid (N tiles of 256, K splits, token tiles).  map_a: the packed activations, (tiles * 256) rows of Kp bytes; map_b: the weights,
 // N rows of K bytes (rows past N read as zero).  Barriers: full[s] (the stage's two boxes have landed), empty[s] (the instructions
 // that read the stage have completed), done.
+// Clusters of S = 1, 2 or 4 CTAs along the K splits: CTA d of a cluster finishes the tile's columns [256 d / S, 256 (d + 1) / S).  The
+// others hand it their partial sums (32-bit pairs: |sums| stay below 2^31 over all of K) into its stage memory, which is idle by then:
+// (S - 1) x 128 x 256 / S pairs, at most the 192 KB there are.
+// What bounds it: the operands' latency, two stages in flight a CTA (tensor pipe 31 % busy).  128 x 4096 x 14336, 56 tiles on 148
+// SMs: 40 us unsplit, 27 in clusters of two, part of it beside the packing.  Tiles that start K at places of their own: the same.
 __global__ void __launch_bounds__(UM_THREADS, 1) k_wp_umma(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, u32 N,
-                                                          u32 Kp, u32 t_rows, size_t os, long long* __restrict__ out, int* __restrict__ err) {
+                                                          u32 Kp, u32 t_rows, size_t os, long long* __restrict__ out, int* __restrict__ err,
+                                                          u32 S, u32 weights_first) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
     __shared__ __align__(8) u64 bars[2 * UM_STAGES + 1];
     __shared__ u32 tmem_slot;
@@ -172,13 +246,22 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_wp_umma(const __grid_constant
 
     bool ok = true;
     if (tid == 0) {
-        auto load_stage = [&](u32 kt, u32 st) {
-            const u32 sa = smem_base + st * UM_STAGE_BYTES;
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(full0 + 8 * st), "r"(UM_STAGE_BYTES) : "memory");
-            um_tma_2d(sa, &map_a, full0 + 8 * st, (int)(kt * UM_KT), (int)(mt * 2 * WP_MT));
-            um_tma_2d(sa + 2 * UM_A_BYTES, &map_b, full0 + 8 * st, (int)(kt * UM_KT), (int)n0);
+        auto load_a = [&](u32 kt, u32 st) {
+            um_tma_2d(smem_base + st * UM_STAGE_BYTES, &map_a, full0 + 8 * st, (int)(kt * UM_KT), (int)(mt * 2 * WP_MT));
         };
-        for (u32 s = 0; s < UM_STAGES && s < nkt; s++) load_stage(kt0 + s, s);
+        auto load_b = [&](u32 kt, u32 st) {
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(full0 + 8 * st), "r"(UM_STAGE_BYTES) : "memory");
+            um_tma_2d(smem_base + st * UM_STAGE_BYTES + 2 * UM_A_BYTES, &map_b, full0 + 8 * st, (int)(kt * UM_KT), (int)n0);
+        };
+        auto load_stage = [&](u32 kt, u32 st) {
+            load_b(kt, st);
+            load_a(kt, st);
+        };
+        // the activations wait for the packing kernel, the caller's weights do not
+        if (!weights_first) asm volatile("griddepcontrol.wait;\n" ::: "memory");
+        for (u32 s = 0; s < UM_STAGES && s < nkt; s++) load_b(kt0 + s, s);
+        if (weights_first) asm volatile("griddepcontrol.wait;\n" ::: "memory");
+        for (u32 s = 0; s < UM_STAGES && s < nkt; s++) load_a(kt0 + s, s);
         for (u32 it = 0; it < nkt && ok; it++) {
             const u32 st = it % UM_STAGES;
             ok = um_wait(full0 + 8 * st, (it / UM_STAGES) & 1);
@@ -217,32 +300,57 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_wp_umma(const __grid_constant
     }
     const bool failed = __syncthreads_or(!ready);
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
-    if (!failed) {
-        // warp w reads TMEM lanes 32 (w % 4) .. +31 (the rows of the token tile), columns 128 (w / 4) .. +127
-        const u32 q = warp & 3, half = warp >> 2;
-        const u32 row = q * 32 + lane, t = mt * WP_MT + row;
-        const bool split = gridDim.y > 1;
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");  // what the packing kernel cleared
+    // warp w reads TMEM lanes 32 (w % 4) .. +31 (the rows of the token tile) and every other 32 columns
+    const u32 q = warp & 3, half = warp >> 2, row = q * 32 + lane, t = mt * WP_MT + row;
+    const u32 rank = S > 1 ? blockIdx.y % S : 0u, W = UM_NT / S;
+    auto fetch = [&](u32 col, u32 (&hi)[32], u32 (&lo)[32]) {
+        um_ld32(tmem + ((q * 32) << 16) + col, hi);
+        um_ld32(tmem + ((q * 32) << 16) + 256 + col, lo);
+        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+    };
+    if (S > 1) {
+        um_cluster_sync();  // every CTA's instructions have read their stages (or it gave up: it comes here all the same)
+        if (!failed) {
 #pragma unroll 1
-        for (u32 cc = 0; cc < 4; cc++) {
-            const u32 col = half * 128 + cc * 32;
-            u32 hi[32], lo[32];
-            um_ld32(tmem + ((q * 32) << 16) + col, hi);
-            um_ld32(tmem + ((q * 32) << 16) + 256 + col, lo);
-            asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-            if (t < t_rows) {
-                long long* o = out + (size_t)t * os + n0 + col;
+            for (u32 cc = half * 32; cc < UM_NT; cc += 64) {
+                const u32 d = cc / W;
+                if (d == rank) continue;
+                u32 hi[32], lo[32], remote;
+                fetch(cc, hi, lo);
+                const u32 slot = rank < d ? rank : rank - 1;  // [slot][column][row], a pair each: lanes side by side
+                const u32 at = smem_base + ((slot * W + cc % W) * WP_MT + row) * 8;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(remote) : "r"(at), "r"(d));
 #pragma unroll
-                for (int j = 0; j < 32; j++) {
-                    if (n0 + col + j < N) {
-                        const long long v = 256ll * (int)hi[j] + (int)lo[j];
-                        if (split) atomicAdd(reinterpret_cast<unsigned long long*>(o + j), (unsigned long long)v);
-                        else o[j] = v;
-                    }
-                }
+                for (int j = 0; j < 32; j++)
+                    asm volatile("st.shared::cluster.v2.b32 [%0], {%1, %2};\n" ::"r"(remote + (u32)j * WP_MT * 8), "r"(hi[j]), "r"(lo[j]) : "memory");
             }
         }
+        um_cluster_sync();
     }
-    if (failed && tid == 0) atomicExch(err, 2);
+    if (!failed) {
+        const bool add = gridDim.y > S;
+        const u32 align = (u32)((uintptr_t)out | (os * 8));
+#pragma unroll 1
+        for (u32 cc = rank * W + half * 32; cc < (rank + 1) * W; cc += 64) {
+            u32 hi[32], lo[32];
+            fetch(cc, hi, lo);
+#pragma unroll 1
+            for (u32 slot = 0; slot + 1 < S; slot++) {
+                const u32 at = smem_base + ((slot * W + cc % W) * WP_MT + row) * 8;
+#pragma unroll
+                for (int j = 0; j < 32; j++) {
+                    u32 h, l;
+                    asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];\n" : "=r"(h), "=r"(l) : "r"(at + (u32)j * WP_MT * 8) : "memory");
+                    hi[j] += h;
+                    lo[j] += l;
+                }
+            }
+            const u32 left = n0 + cc < N ? N - n0 - cc : 0;
+            if (t < t_rows && left) um_store32(out + (size_t)t * os + n0 + cc, hi, lo, left, add, align);
+        }
+    }
+    if (failed && tid == 0) *reinterpret_cast<volatile int*>(err) = 2;
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(512u));
@@ -281,46 +389,56 @@ int product_on_device(hl_ctx* c, size_t t_rows, const int64_t* d_x, size_t xs, c
     uint8_t* d_a = nullptr;
     int8_t* d_b = nullptr;
     int rc = dev_alloc(c, (void**)&d_a, a_bytes);
-    if (!rc && !c->d_wp_flag) {  // the status word lives with the context and is zero between calls: no clear on the launch path
-        if (cudaMalloc((void**)&c->d_wp_flag, 4) != cudaSuccess || cudaMemsetAsync(c->d_wp_flag, 0, 4, c->stream) != cudaSuccess) {
-            c->d_wp_flag = nullptr;
+    if (!rc && !c->wp_flag) {  // the status word: page-locked host memory that the kernels write to when something is wrong, zero between calls
+        if (cudaHostAlloc((void**)&c->wp_flag, 4, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+            c->wp_flag = nullptr;
             rc = fail(c, HL_B200_ERR_OOM, "witness product: status word");
+        } else {
+            *c->wp_flag = 0;
         }
     }
-    int* d_flag = c->d_wp_flag;
+    int* d_flag = c->wp_flag;
     if (!rc && b_bytes) rc = dev_alloc(c, (void**)&d_b, b_bytes);
     CUtensorMap map_a, map_b;
     if (!rc) rc = byte_matrix_map(c, d_a, Kp, (size_t)tiles * 2 * WP_MT, Kp, &map_a);
     if (!rc) rc = byte_matrix_map(c, in_place ? (const void*)d_w : (const void*)d_b, Kp, in_place ? N : n_pad, Kp, &map_b);
-    // The split over K by a cost model fitted to measurements on B200: a CTA streams one K stage (64 KB of operands) in about
-    // 1.3 us, CTAs run in waves of one per SM, and every split beyond the first adds a pass of 64-bit integer atomics over the
-    // result plane at about 195 G atomics per second.
+    // The split over K, S CTAs of a cluster times sp clusters, by a cost model fitted to measurements on B200: a CTA streams one K stage
+    // (64 KB of operands) in about 1.3 us, CTAs run in waves of one per SM (clusters of four leave some SMs out), handing partial sums
+    // over inside a cluster takes about 3 us, and every cluster beyond the first adds a pass of 64-bit integer atomics over the result
+    // plane at about 195 G atomics per second.
     const u32 n_tiles = (u32)((N + UM_NT - 1) / UM_NT), kt_all = Kp / UM_KT;
-    const u32 slots = (u32)c->sm_count, base = n_tiles * tiles;
-    u32 splits = 1;
+    const u32 base = n_tiles * tiles;
+    u32 splits = 1, S = 1;
     double best = 1e30;
-    for (u32 sp = 1; sp <= 64 && sp <= kt_all; sp++) {
-        const u64 ctas = (u64)base * sp;
-        const double waves = (double)((ctas + slots - 1) / slots), stages = (double)((kt_all + sp - 1) / sp);
-        const double cost = waves * stages * 1.3e-6 + (sp > 1 ? (double)sp * (double)tiles * WP_MT * (double)N / 195e9 : 0.0);
-        if (cost < best * 0.98) { best = cost; splits = sp; }
+    for (u32 cl = 1; cl <= 4; cl *= 2) {
+        const u32 slots = cl == 4 ? (u32)c->sm_count * 7 / 8 : (u32)c->sm_count;
+        for (u32 sp = 1; sp * cl <= 64 && sp * cl <= kt_all; sp++) {
+            const u64 ctas = (u64)base * sp * cl;
+            const double waves = (double)((ctas + slots - 1) / slots), stages = (double)((kt_all + sp * cl - 1) / (sp * cl));
+            const double cost = waves * (stages * 1.3e-6 + (cl > 1 ? 3e-6 : 0.0)) + (sp > 1 ? (double)sp * (double)t_rows * (double)N / 195e9 : 0.0);
+            if (cost < best * 0.98) { best = cost; splits = sp * cl; S = cl; }
+        }
     }
     int flag = 0;
     if (!rc) {
         Timed t(c, HL_T_WITNESS);
         // the plane is cleared unless the product kernel writes every word of it exactly once
-        const bool dense = splits == 1 && os == N && out_len == t_rows * N;
-        cudaError_t e = cudaSuccess;
-        if (e == cudaSuccess && b_bytes) e = cudaMemsetAsync(d_b, 0, b_bytes, c->stream);
-        if (e == cudaSuccess) {
-            k_wp_pack<<<dim3((Kp + 1023) / 1024, tiles * WP_MT), 256, 0, c->stream>>>((const long long*)d_x, xs, (u32)t_rows, (u32)K, Kp, d_a, d_flag,
-                                                                                       (long long*)d_out, dense ? 0 : out_len);
-            e = cudaGetLastError();
-            c->stats.kernel_launches++;
-        }
+        const bool dense = splits == S && os == N && out_len == t_rows * N;
+        // the kernels after the packing may start beside the one before them and wait inside for what they read
+        cudaLaunchAttribute at[2];
+        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[0].val.programmaticStreamSerializationAllowed = 1;
+        at[1].id = cudaLaunchAttributeClusterDimension;
+        at[1].val.clusterDim.x = 1; at[1].val.clusterDim.y = S; at[1].val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.stream = c->stream; cfg.attrs = at;
+        k_wp_pack<<<dim3((Kp + 1023) / 1024, tiles * WP_MT), 256, 0, c->stream>>>((const long long*)d_x, xs, (u32)t_rows, (u32)K, Kp, d_a, d_flag,
+                                                                                   (long long*)d_out, dense ? 0 : out_len);
+        cudaError_t e = cudaGetLastError();
+        c->stats.kernel_launches++;
         if (e == cudaSuccess && b_bytes) {
-            k_wp_repack<<<dim3(Kp / 64, (unsigned)((N + 63) / 64)), 256, 0, c->stream>>>(d_w, (u32)K, (u32)N, Kp, in_out, d_b);
-            e = cudaGetLastError();
+            cfg.gridDim = dim3(Kp / 128, (unsigned)(n_pad / 128)); cfg.blockDim = dim3(256); cfg.dynamicSmemBytes = 0; cfg.numAttrs = 1;
+            e = cudaLaunchKernelEx(&cfg, k_wp_repack, d_w, K * N, (u32)K, (u32)N, Kp, in_out, d_b);
             c->stats.kernel_launches++;
         }
         const size_t smem = (size_t)UM_STAGES * UM_STAGE_BYTES + 1024;
@@ -329,16 +447,18 @@ int product_on_device(hl_ctx* c, size_t t_rows, const int64_t* d_x, size_t xs, c
             c->wp_attr = e == cudaSuccess;
         }
         if (e == cudaSuccess) {
-            k_wp_umma<<<dim3(n_tiles, splits, tiles), UM_THREADS, smem, c->stream>>>(map_a, map_b, (u32)N, Kp, (u32)t_rows, os, (long long*)d_out, d_flag);
-            e = cudaGetLastError();
+            cfg.gridDim = dim3(n_tiles, splits, tiles); cfg.blockDim = dim3(UM_THREADS); cfg.dynamicSmemBytes = smem; cfg.numAttrs = 2;
+            e = cudaLaunchKernelEx(&cfg, k_wp_umma, map_a, map_b, (u32)N, Kp, (u32)t_rows, os, (long long*)d_out, d_flag, S, (u32)(in_place ? 1 : 0));
             c->stats.kernel_launches++;
         }
         if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "witness product launch", e);
     }
-    if (!rc) rc = d2h(c, &flag, d_flag, 4);
     if (!rc) rc = sync(c, "witness_product");
     else cudaStreamSynchronize(c->stream);
-    if (flag && d_flag) cudaMemsetAsync(d_flag, 0, 4, c->stream);  // back to zero for the next call
+    if (d_flag) {
+        flag = *reinterpret_cast<volatile int*>(d_flag);
+        *d_flag = 0;  // for the next call
+    }
     if (d_a) dev_free(c, d_a, a_bytes);
     if (d_b) dev_free(c, d_b, b_bytes);
     if (!rc && flag == 2) rc = fail(c, HL_B200_ERR_TIMEOUT, "witness product: a bounded wait on the tensor-core pipeline ran out");
