@@ -1,0 +1,64 @@
+"""The launch that takes a sumcheck's short rounds together, where its forms part: one chunk of pairs and one pair past it, tables at and
+above the length it takes over at, batches that end inside it, and programs whose live values do not fit its shared memory."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from intelligenceregulation_b200 import backend
+
+    c = backend.Context(0)
+    yield c
+    c.close()
+
+
+def _check(ctx, o, poly, tables, deg, n, batches, what=None, coefs=None):
+    from intelligenceregulation_b200 import backend
+
+    tr = o.Transcript(b"sc-run")
+    t_cpu = tr.clone()
+    want = o.sc_prove(poly, tables, deg, t_cpu, coefs=coefs)
+    ev = backend.B200Rounds(ctx, what if what is not None else poly, tables, deg)
+    got, st, ctr = [], tr.state, tr.counter
+    for b in batches:
+        r = ev.batched(b, st, ctr, None)
+        got.append(r[0])
+        st, ctr = r[3], r[4]
+    assert sum(batches) == n and (np.concatenate(got) == want.rounds).all() and st == t_cpu.state
+    assert (ev.finals() == want.finals).all()
+    ev.free()
+
+
+@pytest.mark.parametrize("n,batches", [(1, [1]), (6, [6]), (7, [6, 1]), (8, [1] * 8), (18, [18]), (18, [3, 15]), (19, [1, 17, 1]), (20, [2, 18])])
+@pytest.mark.parametrize("k,deg", [(2, 2), (3, 3)])
+def test_closed_forms(ctx, oracle, n, batches, k, deg):
+    tables = oracle.ZkRng(n, b"sc-run").fp2_vec(k << n).reshape(k, 1 << n, 2)
+    _check(ctx, oracle, 0, tables, deg, n, batches)
+
+
+def _program(o, nodes):
+    """every node is used twice, at the end: all of them live at once"""
+    from intelligenceregulation_b200 import backend
+
+    SP = backend.SlotProgram
+    cf = [tuple(map(int, c)) for c in o.ZkRng(nodes, b"sc-run-ir").fp2_vec(3 * nodes)]
+    p = SP(4)
+    ids = [p.sum([(cf[3 * i], [1 + i % 3, 1 + i // 3 % 3]), (cf[3 * i + 1], [1 + i % 3])]) for i in range(nodes)]
+    a = p.sum([(cf[3 * i + 2], [SP.node(d)]) for i, d in enumerate(ids)])
+    b = p.sum([(SP.NEG_ONE if i % 2 else SP.ONE, [SP.node(d)]) for i, d in enumerate(ids)])
+    p.term(SP.ONE, [0], [SP.node(a)])
+    p.term(cf[0], [], [SP.node(b)])
+    return p
+
+
+@pytest.mark.parametrize("nodes,n,batches", [(1, 5, [5]), (1, 6, [5, 1]), (2, 14, [14]), (2, 15, [15]), (30, 11, [11]), (30, 12, [1, 10, 1]), (120, 9, [9]),
+                                             (120, 12, [12])])
+def test_programs(ctx, oracle, nodes, n, batches):
+    p = _program(oracle, nodes)
+    tables = oracle.ZkRng(n, b"sc-run-tabs").fp2_vec(4 << n).reshape(4, 1 << n, 2)
+    c = p.coef_array()
+    oracle.ir_set(p.words(), p.n_nodes, p.n_terms)
+    _check(ctx, oracle, oracle.POLY_IR, tables, 3, n, batches, what=p, coefs=c if c.size else None)
