@@ -101,11 +101,12 @@ __global__ void __launch_bounds__(256) k_split_vectors(const u64* __restrict__ v
 
 }  // namespace
 
-// the body of hl_b200_verify_columns; the caller holds the context's lock
+// the body of hl_b200_verify_columns; the caller holds the context's lock.  `early`: room for the columns that the copy stream may
+// write already (the caller made it, ordered the copy stream behind that and frees it); NULL: made here, copied in the stream's order
 static int verify_columns_locked(hl_ctx* c, const uint64_t* cols, size_t rows, size_t ncols, const uint64_t* idx, const uint8_t* salts32,
                                  const uint8_t* paths32, uint32_t depth, const uint8_t* root32, const uint8_t* column_key32,
                                  const uint8_t* leaf_key32, const uint8_t* node_key32, const uint64_t* rhos, size_t k, const uint64_t* wants,
-                                 const hl_store* vec_store, int32_t* verdict, int64_t* first_bad) {
+                                 const hl_store* vec_store, int32_t* verdict, int64_t* first_bad, u64* early = nullptr) {
     if (!cols || !idx || !salts32 || !root32 || !verdict || rows == 0 || ncols == 0) return fail(c, HL_B200_ERR_ARG, "verify_columns: null or empty argument");
     if (depth && !paths32) return fail(c, HL_B200_ERR_ARG, "verify_columns: paths missing");
     if (depth > 40) return fail(c, HL_B200_ERR_ARG, "verify_columns: a path of more than 40 entries");
@@ -126,7 +127,8 @@ static int verify_columns_locked(hl_ctx* c, const uint64_t* cols, size_t rows, s
     FoldPlan plan;
     uint32_t *d_salts = nullptr, *d_paths = nullptr, *d_root = nullptr, *d_ck = nullptr, *d_lk = nullptr, *d_nk = nullptr, *d_leaves = nullptr, *d_cvs = nullptr;
     int32_t* d_verdict = nullptr;
-    int rc = dev_alloc(c, (void**)&d_cols, cb);
+    int rc = early ? HL_B200_OK : dev_alloc(c, (void**)&d_cols, cb);
+    if (early) d_cols = early;
     if (!rc) rc = dev_alloc(c, (void**)&d_mat, cb);
     if (!rc) rc = dev_alloc(c, (void**)&d_idx, ncols * 8);
     if (!rc) rc = dev_alloc(c, (void**)&d_salts, ncols * 32);
@@ -137,7 +139,6 @@ static int verify_columns_locked(hl_ctx* c, const uint64_t* cols, size_t rows, s
     if (!rc) rc = dev_alloc(c, (void**)&d_acc, ab);
     if (!rc) rc = dev_alloc(c, (void**)&d_verdict, ncols * 4);
     if (!rc && k && wants) rc = dev_alloc(c, (void**)&d_wants, ab);
-    if (!rc) rc = h2d(c, d_cols, cols, cb);
     if (!rc) rc = h2d(c, d_idx, idx, ncols * 8);
     if (!rc) rc = h2d(c, d_salts, salts32, ncols * 32);
     if (!rc && depth) rc = h2d(c, d_paths, paths32, (size_t)depth * ncols * 32);
@@ -153,6 +154,12 @@ static int verify_columns_locked(hl_ctx* c, const uint64_t* cols, size_t rows, s
     if (!rc) rc = upload_key(c, column_key32, &d_ck);
     if (!rc) rc = upload_key(c, leaf_key32, &d_lk);
     if (!rc) rc = upload_key(c, node_key32, &d_nk);
+    if (!rc) rc = h2d_on(c, d_cols, cols, cb, early ? c->copy_stream : c->stream);
+    if (!rc && early) {
+        cudaError_t e = cudaEventRecord(c->ev_main, c->copy_stream);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(c->stream, c->ev_main, 0);
+        if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "verify_columns: stream ordering", e);
+    }
     if (!rc) {
         const dim3 grid((unsigned)((rows + 31) / 32), (unsigned)((ncols + 31) / 32));
         k_cols_to_rows<<<grid, dim3(32, 8), 0, c->stream>>>(d_cols, (u32)ncols, (u32)rows, d_mat);
@@ -183,7 +190,9 @@ static int verify_columns_locked(hl_ctx* c, const uint64_t* cols, size_t rows, s
             if (verdict[i]) { *first_bad = (int64_t)i; break; }
     }
     if (rc) cudaStreamSynchronize(c->stream);  // copies already queued read the caller's memory: none outlives the call
-    dev_free(c, d_cols, cb); dev_free(c, d_mat, cb); dev_free(c, d_idx, ncols * 8); dev_free(c, d_salts, ncols * 32);
+    if (early) { if (rc) cudaStreamSynchronize(c->copy_stream); }
+    else dev_free(c, d_cols, cb);
+    dev_free(c, d_mat, cb); dev_free(c, d_idx, ncols * 8); dev_free(c, d_salts, ncols * 32);
     dev_free(c, d_paths, pb); dev_free(c, d_root, 32); dev_free(c, d_leaves, ncols * 32);
     if (d_cvs) dev_free(c, d_cvs, cvs_bytes);
     dev_free(c, d_acc, ab); dev_free(c, d_verdict, ncols * 4);
@@ -214,9 +223,19 @@ extern "C" int hl_b200_verify_opening(hl_ctx* c, uint32_t log_cols, uint32_t inv
     if (log_cols < 1 || log_cols > 16 || k > 0x7FFFu) return fail(c, HL_B200_ERR_ARG, "verify_opening: shape");
     Call g(c);
     const size_t n = (size_t)1 << log_cols, nn = n * inv_rate, w = n + q;
-    u64 *d_vecs = nullptr, *d_data = nullptr, *d_pads = nullptr, *d_pows = nullptr;
+    u64 *d_vecs = nullptr, *d_data = nullptr, *d_pads = nullptr, *d_pows = nullptr, *d_cols = nullptr;
     hl_store* st = nullptr;
+    // The opened columns come on the copy stream, beside the encoding of the clear vectors (37 of 2^14 and 280 columns of 2,504 rows: 100
+    // of 730 us).  Below half a megabyte a copy takes less than the ordering of two streams.
+    const size_t cb = rows && ncols <= (size_t)-1 / 8 / rows ? rows * ncols * 8 : 0;
     int rc = dev_alloc(c, (void**)&d_vecs, k * w * 16);
+    if (!rc && cols && cb > ((size_t)512 << 10)) {
+        rc = dev_alloc(c, (void**)&d_cols, cb);
+        cudaError_t e = cudaSuccess;
+        if (!rc) e = cudaEventRecord(c->ev_main, c->stream);
+        if (!rc && e == cudaSuccess) e = cudaStreamWaitEvent(c->copy_stream, c->ev_main, 0);
+        if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "verify_opening: stream ordering", e);
+    }
     if (!rc) rc = dev_alloc(c, (void**)&d_data, 2 * k * n * 8);
     if (!rc) rc = dev_alloc(c, (void**)&d_pads, 2 * k * q * 8);
     if (!rc) rc = dev_alloc(c, (void**)&d_pows, nn * 8);
@@ -233,9 +252,10 @@ extern "C" int hl_b200_verify_opening(hl_ctx* c, uint32_t log_cols, uint32_t inv
     if (!rc) rc = commit_resident(c, log_cols, inv_rate, d_data, 2 * k, d_pads, q, d_pows, nullptr, &st, nullptr, false);
     if (!rc)
         rc = verify_columns_locked(c, cols, rows, ncols, idx, salts32, paths32, depth, root32, column_key32, leaf_key32, node_key32, rhos, k, nullptr, st,
-                                   verdict, first_bad);
+                                   verdict, first_bad, d_cols);
     if (rc) cudaStreamSynchronize(c->stream);  // a refusal on the way: the copies above may still be reading the caller's memory
     if (st) store_release(st);
+    if (d_cols) dev_free(c, d_cols, cb);
     dev_free(c, d_vecs, k * w * 16);
     dev_free(c, d_data, 2 * k * n * 8);
     dev_free(c, d_pads, 2 * k * q * 8);
