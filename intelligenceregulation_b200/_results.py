@@ -17,7 +17,17 @@ KEEP = 192 << 20   # a block's logup columns twice over (the caller holds one re
 
 _lock = threading.RLock()  # a block may come back from a garbage collection inside `empty`
 _idle: List[np.ndarray] = []
+_late: List[np.ndarray] = []  # came back while `empty` was looking through `_idle`
+_looking = False
 _bytes = 0
+
+
+def _back(block: np.ndarray) -> None:
+    global _bytes
+    _idle.append(block)
+    _bytes += block.nbytes
+    while _bytes > KEEP:
+        _bytes -= _idle.pop(0).nbytes
 
 
 class _Hold:
@@ -30,30 +40,32 @@ class _Hold:
         self.__array_interface__ = {"shape": shape, "typestr": dtype.str, "data": (block.__array_interface__["data"][0], False), "version": 3}
 
     def __del__(self):
-        global _bytes
         with _lock:
-            _idle.append(self.block)
-            _bytes += self.block.nbytes
-            while _bytes > KEEP:
-                _bytes -= _idle.pop(0).nbytes
+            if _looking:
+                _late.append(self.block)
+            else:
+                _back(self.block)
 
 
 def empty(shape, dtype) -> np.ndarray:
     """``np.empty(shape, dtype)``, over reused memory where it is large"""
-    global _bytes
+    global _bytes, _looking
     dtype, shape = np.dtype(dtype), tuple(shape) if isinstance(shape, (tuple, list)) else (int(shape),)
     nbytes = math.prod(shape) * dtype.itemsize
     if nbytes < SMALL:
         return np.empty(shape, dtype)
     block = None
     with _lock:
-        best = -1
+        _looking, best = True, -1
         for i, b in enumerate(_idle):
             if nbytes <= b.nbytes <= nbytes + (nbytes >> 2) and (best < 0 or b.nbytes < _idle[best].nbytes):
                 best = i
         if best >= 0:
             block = _idle.pop(best)
             _bytes -= block.nbytes
+        _looking = False
+        while _late:
+            _back(_late.pop())
     if block is None:
         block = np.empty(nbytes, np.uint8)
     return np.asarray(_Hold(block, shape, dtype))

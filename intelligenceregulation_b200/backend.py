@@ -326,9 +326,9 @@ class B200Commit:
         return int(self.ctx.lib.hl_b200_store_leaves_dev(self.h) or 0)
 
     def free(self) -> None:
-        if self.h:
+        if self.h and self.ctx.h:  # a handle that outlived its context went with it
             self.ctx.lib.hl_b200_store_free(self.h)
-            self.h = None
+        self.h = None
 
     def __del__(self):
         try:
@@ -809,9 +809,9 @@ class B200Rounds:
         return out[:, :np_], out[:, np_:2 * np_], out[:, 2 * np_], bytes(fs.state), int(fs.counter), (int(fs.claim[0]), int(fs.claim[1]))
 
     def free(self) -> None:
-        if self.h:
+        if self.h and self.ctx.h:  # a handle that outlived its context went with it
             self.ctx.lib.hl_b200_rounds_free(self.h)
-            self.h = None
+        self.h = None
 
     def __del__(self):
         try:

@@ -236,21 +236,32 @@ __global__ void __launch_bounds__(FEW_THREADS) k_fold_rows_few(FoldSeg seg0, Fol
     }
 }
 
-// out[map[g]][j] = sum_z part[z][g][j]
+// out[map[g]][j] = sum_z part[z][g][j]: 32 words a CTA, its eight warps share their ranges (one thread a word walked 156 ranges of a
+// narrow fold in 22 us)
 __global__ void __launch_bounds__(256) k_fold_sum(const u64* __restrict__ part, u32 splits, u32 k, u32 out_ld, const u32* __restrict__ out_map,
                                                   u64* __restrict__ out) {
-    const size_t words = (size_t)out_ld * 2, i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const u32 g = blockIdx.y;
-    if (i >= words) return;
+    __shared__ u64 sums[8][32];
+    const u32 x = threadIdx.x & 31, y = threadIdx.x >> 5, g = blockIdx.y;
+    const size_t words = (size_t)out_ld * 2, i = (size_t)blockIdx.x * 32 + x;
     u64 s = 0;
-    for (u32 z = 0; z < splits; z++) s = gl_add(s, part[((size_t)z * k + g) * words + i]);
+    if (i < words)
+#pragma unroll 4
+        for (u32 z = y; z < splits; z += 8) s = gl_add(s, part[((size_t)z * k + g) * words + i]);
+    sums[y][x] = s;
+    __syncthreads();
+    if (y || i >= words) return;
+#pragma unroll
+    for (u32 w = 1; w < 8; w++) s = gl_add(s, sums[w][x]);
     out[(size_t)(out_map ? out_map[g] : g) * words + i] = s;
 }
 
 // The same combination for a vector that is zero outside a few rows (an opening's group weights live on their claims'
 // rows only, pcs.rs:851-891): the rows and weights arrive as a list, one thread per column walks it.  Products are
 // summed as 128-bit integers with a wrap count and reduced once per component (2^128 = -2^32 mod p).
+// Bound by the latency of the rows' words: eight entries' words are asked for before the first is used (37 vectors on 34 rows each,
+// 16,664 columns: 81 us one at a time, 60 now).
 constexpr int SPARSE_COLS = 256;
+constexpr u32 SPARSE_AHEAD = 8;
 __global__ void __launch_bounds__(SPARSE_COLS) k_fold_sparse(FoldSeg seg0, FoldSeg seg1, const u32* __restrict__ off /* vectors + 1 */,
                                                             const u32* __restrict__ srow, const u64* __restrict__ sw /* 2 per entry */,
                                                             const u32* __restrict__ out_map, u64* __restrict__ out, u32 out_ld) {
@@ -260,19 +271,27 @@ __global__ void __launch_bounds__(SPARSE_COLS) k_fold_sparse(FoldSeg seg0, FoldS
     if (col >= sg.ncols) return;
     const u32 v = blockIdx.y;
     const u64* p = sg.src + (size_t)col * sg.ir;
-    u64 lo0 = 0, hi0 = 0, w0 = 0, lo1 = 0, hi1 = 0, w1 = 0;
-    for (u32 e = off[v]; e < off[v + 1]; e++) {
-        const u64 d = p[(size_t)srow[e] * sg.ld];
-        const gl_wide p0 = gl_mulw(sw[2 * (size_t)e], d), p1 = gl_mulw(sw[2 * (size_t)e + 1], d);
-        u64 t = lo0 + p0.lo, c = t < lo0; lo0 = t;
-        t = hi0 + p0.hi; u64 c2 = t < hi0; hi0 = t + c; c2 += hi0 < t; w0 += c2;
-        t = lo1 + p1.lo; c = t < lo1; lo1 = t;
-        t = hi1 + p1.hi; c2 = t < hi1; hi1 = t + c; c2 += hi1 < t; w1 += c2;
+#ifdef __CUDA_ARCH__  // the accumulating product is device code
+    u32 s0[5] = {0, 0, 0, 0, 0}, s1[5] = {0, 0, 0, 0, 0};
+    const u32 end = off[v + 1];
+    u32 e = off[v];
+    auto take = [&](u32 at, u64 d) {
+        gl_product_acc(sw[2 * (size_t)at], d, s0[0], s0[1], s0[2], s0[3], s0[4]);
+        gl_product_acc(sw[2 * (size_t)at + 1], d, s1[0], s1[1], s1[2], s1[3], s1[4]);
+    };
+    for (; e + SPARSE_AHEAD <= end; e += SPARSE_AHEAD) {
+        u64 d[SPARSE_AHEAD];
+#pragma unroll
+        for (u32 j = 0; j < SPARSE_AHEAD; j++) d[j] = p[(size_t)srow[e + j] * sg.ld];
+#pragma unroll
+        for (u32 j = 0; j < SPARSE_AHEAD; j++) take(e + j, d[j]);
     }
+    for (; e < end; e++) take(e, p[(size_t)srow[e] * sg.ld]);
     const u64 two128 = 0xFFFFFFFE00000001ull;  // 2^128 mod p
     u64* o = out + ((size_t)out_map[v] * out_ld + sg.out_off + col) * 2;
-    o[0] = gl_add(gl_reduce128(lo0, hi0), gl_mul(w0, two128));
-    o[1] = gl_add(gl_reduce128(lo1, hi1), gl_mul(w1, two128));
+    auto word = [&](const u32 (&s)[5]) { return gl_add(gl_reduce128(((u64)s[1] << 32) | s[0], ((u64)s[3] << 32) | s[2]), gl_mul(s[4], two128)); };
+    *reinterpret_cast<ulonglong2*>(o) = make_ulonglong2(word(s0), word(s1));
+#endif
 }
 
 // out[c * rows + i] = enc[i * nn + idx[c]]   (pcs.rs:1055-1067; order of idx, duplicates repeated)
@@ -309,7 +328,7 @@ cudaError_t fold_rows_few(const u64* src, u32 rows, u32 ncols, size_t ld, const 
     else k_fold_rows_few<2><<<grid, FEW_THREADS, 0, st>>>(a, b, rows, per_z, d_rhos, k, d_part, out_ld);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_fold_sum<<<dim3((out_ld * 2 + 255) / 256, k), 256, 0, st>>>(d_part, ranges, k, out_ld, d_out_map, d_out);
+    k_fold_sum<<<dim3((out_ld * 2 + 31) / 32, k), 256, 0, st>>>(d_part, ranges, k, out_ld, d_out_map, d_out);
     return cudaGetLastError();
 }
 
@@ -336,7 +355,7 @@ cudaError_t fold_rows(const u64* src, u32 rows, u32 ncols, size_t ld, u32 ir, co
     k_fold_rows<<<grid, FOLD_THREADS, 0, st>>>(a, b, rows, d_rhos, k, nullptr, d_part, out_ld);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_fold_sum<<<dim3((out_ld * 2 + 255) / 256, k), 256, 0, st>>>(d_part, splits, k, out_ld, d_out_map, d_out);
+    k_fold_sum<<<dim3((out_ld * 2 + 31) / 32, k), 256, 0, st>>>(d_part, splits, k, out_ld, d_out_map, d_out);
     return cudaGetLastError();
 }
 
