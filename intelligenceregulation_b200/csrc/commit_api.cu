@@ -255,7 +255,7 @@ int commit_on_device(hl_ctx* c, hl_store* st, const u64* d_pows, const uint8_t* 
             a.ninv = gl_inv((u64)n); a.coef_out = nullptr;
             if (fused_widen) { a.narrow = d_narrow; a.row_off = d_row_off + r0; a.row_w = d_row_w + r0; }
             // a handful of rows (a boundary commitment, the last piece of an upload): one CTA per (row, residue)
-            a.split = (loga == 0 && st->logr >= 1 && ((u64)nr << st->logr) <= (u64)c->sm_count) ? 1 : 0;
+            a.split = hlk::encode_split_pays(logb, st->logr, nr, c->sm_count) ? 1 : 0;
             cudaError_t e = hlk::encode_rows(a, logb, c->fast_encoder || loga, c->sm_count, scratch_words, c->stream, &st->encoder_path);
             c->stats.kernel_launches += 1;
             if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "row encoder launch", e);

@@ -47,18 +47,18 @@ __global__ void __launch_bounds__(THREADS, MINB) k_encode_fast(enc::RowArgs a) {
     F::load_twiddles(a, TW, tid, THREADS);
     __syncthreads();
     // a unit of work: a whole row, or (split) one output residue of a row with the row's inverse transform before it
-    const u32 A = LONG ? 1u << a.loga : 1u, R = 1u << a.logr;
-    const u32 units = SPLIT ? a.rows << a.logr : a.rows;
+    const u32 A = LONG ? 1u << a.loga : 1u, logR = LONG ? a.logr - a.loga : a.logr, R = 1u << logR;
+    const u32 units = SPLIT ? a.rows << logR : a.rows;
     for (u32 unit = blockIdx.x; unit < units; unit += gridDim.x) {
-        const u32 row = SPLIT ? unit >> a.logr : unit;
+        const u32 row = SPLIT ? unit >> logR : unit;
         if constexpr (FORM == enc::FORM_COEF) {
             F::row_given(a, row, X, tid, THREADS);
             __syncthreads();
         }
-        const u32 first = SPLIT ? unit & (R - 1u) : 0u, end = A + (SPLIT ? 1u : R);
+        const u32 first = SPLIT ? unit & (R - 1u) : 0u, end = A + A * (SPLIT ? 1u : R);
         for (u32 k = FORM == enc::FORM_COEF ? A : 0u; k < end; k++) {
-            const u32 step = k < A ? k : k + first;
-            F::template row_step<FORM, NARROW, LONG>(a, row, step, S, TW, X, tid, THREADS, CtaSync());
+            const u32 step = k < A ? k : k + A * first;
+            F::template row_step<FORM, NARROW, LONG>(a, row, step, S, TW, X, tid, THREADS, CtaSync(), first);
             __syncthreads();  // the scratch slot is complete and shared memory is free again
         }
     }
@@ -102,7 +102,7 @@ cudaError_t launch_fast_as(const enc::RowArgs& a, int sm_count, size_t scratch_w
     if (e != cudaSuccess) return e;
     if (per_sm < 1) per_sm = 1;
     size_t grid = (size_t)sm_count * per_sm;
-    const size_t units = SPLIT ? (size_t)a.rows << a.logr : (size_t)a.rows;
+    const size_t units = SPLIT ? (size_t)a.rows << (a.logr - a.loga) : (size_t)a.rows;
     if (grid > units) grid = units;
     size_t max_by_scratch = scratch_words / ((size_t)a.T * F::N);
     if (grid > max_by_scratch) grid = max_by_scratch;
@@ -112,11 +112,10 @@ cudaError_t launch_fast_as(const enc::RowArgs& a, int sm_count, size_t scratch_w
     return cudaGetLastError();
 }
 
-// split rows are few (a CTA per SM or fewer in a commitment): they get the registers that a row's latency wants
+// split rows are few: they get the registers that a row's latency wants
 template <int LOGN, int FORM = enc::FORM_PCS, bool NARROW = false, bool LONG = false>
 cudaError_t launch_fast(const enc::RowArgs& a, int sm_count, size_t scratch_words, cudaStream_t st, int* grid_out) {
-    if constexpr (!LONG)
-        if (a.split) return launch_fast_as<LOGN, FORM, NARROW, LONG, true>(a, sm_count, scratch_words, st, grid_out);
+    if (a.split) return launch_fast_as<LOGN, FORM, NARROW, LONG, true>(a, sm_count, scratch_words, st, grid_out);
     return launch_fast_as<LOGN, FORM, NARROW, LONG, false>(a, sm_count, scratch_words, st, grid_out);
 }
 
@@ -125,12 +124,25 @@ cudaError_t launch_fast(const enc::RowArgs& a, int sm_count, size_t scratch_word
 namespace hlk {
 
 size_t encode_scratch_words(u32 logn, u32 T, int sm_count, u32 rows) {
-    // enough for the largest grid any path launches: 32 CTAs per SM at most, one per row (or, for a handful of rows, one per
-    // (row, residue): at most one CTA per SM then)
+    // enough for the largest grid any path launches: 32 CTAs per SM at most, one per row or, for a handful of rows, one per
+    // (row, residue)
     size_t ctas = (size_t)sm_count * 32;
-    if (ctas > rows && rows >= (u32)sm_count) ctas = rows;
-    if (rows < (u32)sm_count) ctas = (size_t)sm_count;
+    const size_t units = encode_split_units(logn, sm_count);
+    if (ctas > rows) ctas = rows > units ? rows : units;
     return ctas * T * ((size_t)1 << logn);
+}
+
+// How many (row, residue) CTAs a launch of split rows takes at once: one per SM, or half of those that an SM holds where a CTA is far from
+// filling one (two of 256 threads take 1.2 times the time of one, four of them 2)
+size_t encode_split_units(u32 logn, int sm_count) {
+    const u32 t = logn > 9 ? 1u << (logn - 4) : 32u;
+    return (size_t)sm_count * (t > 512 ? 1 : 512 / t);
+}
+// Splitting rows by residue repeats their inverse transform: 2 transforms a CTA instead of 1 + R, R times the CTAs.  It pays when it
+// takes fewer turns of the machine (40 rows of 2^16 540 -> 386 us, 60 of 2^15 at rate 1/4 494 -> 410, 200 of 2^10 at rate 1/4 51 -> 29).
+bool encode_split_pays(u32 logn, u32 logR, u32 rows, int sm_count) {
+    const u64 at_once = encode_split_units(logn, sm_count), units = (u64)rows << logR;
+    return logR >= 1 && (units + at_once - 1) / at_once * 2 < (rows + at_once - 1) / at_once * (1 + ((u64)1 << logR));
 }
 
 cudaError_t encode_rows(const enc::RowArgs& a, u32 logn, bool allow_fast, int sm_count, size_t scratch_words,

@@ -73,7 +73,7 @@ struct RowArgs {
     const u64* row_off = nullptr;
     const unsigned char* row_w = nullptr;
     int split;         // fast path: a CTA takes one (row, output residue) instead of a whole row, repeating the row's inverse transform:
-                       // for a handful of rows (fewer than SMs / residues) the latency of a row falls from 1 + R transforms to 2
+                       // for a handful of rows the latency of a row falls from 1 + R transforms of its size to 2
 };
 
 // What a row is and how its coefficients are twisted (template argument of Fast::row_step).
@@ -269,9 +269,10 @@ struct Fast {
     // LONG, rows of A = 2 or 4 times N words: step r transforms the words A m + r, and with p_r[k] = w_n^(r k) Y_r[k] the size-n
     // outputs are Z[k + N b] = sum_r w_A^(r b) p_r[k].  The p_r of r < A - 1 wait in the row's own output, at the places that the
     // same thread fills when it has p_(A-1): every output word is then written R words from the last, not A R (a 2^16-word row at
-    // rate 1/2 wrote 8 bytes to each 64 and went to memory for the rest of every sector: 400 rows 2,825 -> 1,930 us).
+    // rate 1/2 wrote 8 bytes to each 64 and went to memory for the rest of every sector: 400 rows 2,825 -> 1,930 us).  Those of the inverse
+    // wait in the places of output residue `wait`: where the residues of a row have a CTA each, its own.
     template <int FORM, bool NARROW, bool LONG, class Sync>
-    GL_HD static void row_step(const RowArgs& a, u32 row, u32 step, u64* S, const u64* TW, u64* X, u32 tid, u32 nt, Sync sync) {
+    GL_HD static void row_step(const RowArgs& a, u32 row, u32 step, u64* S, const u64* TW, u64* X, u32 tid, u32 nt, Sync sync, u32 wait = 0) {
         const u32 loga = LONG ? a.loga : 0u, A = 1u << loga, n = N << loga, nn = N << a.logr, logr = a.logr - loga;
         bool inverse = false;
         if constexpr (FORM != FORM_COEF) inverse = step < A;
@@ -312,7 +313,7 @@ struct Fast {
                               const u32 k = g + ((u32)j << LASTW);
                               u64 p = e[j];
                               if (r) p = gl_mul_fast(p, a.tw_nn[((r * k) << logr) & (nn - 1)]);  // w_n^(r k)
-                              u64* at = dst + ((size_t)k << logr) + s;  // b words of N << logr further on: output k + N b
+                              u64* at = dst + ((size_t)k << logr) + (inverse ? wait : s);  // b words of N << logr further on: output k + N b
                               const size_t step_b = (size_t)N << logr;
                               if (r + 1 < A) {
                                   at[r * step_b] = p;

@@ -8,6 +8,8 @@ namespace hlk {
 
 // encode.cu
 size_t encode_scratch_words(u32 logn, u32 T, int sm_count, u32 rows);
+size_t encode_split_units(u32 logn, int sm_count);
+bool encode_split_pays(u32 logn, u32 logR, u32 rows, int sm_count);
 cudaError_t encode_rows(const enc::RowArgs& a, u32 logn, bool allow_fast, int sm_count, size_t scratch_words,
                         cudaStream_t st, int* path_out);
 cudaError_t widen_rows(const unsigned char* narrow, const u64* row_off, const unsigned char* row_w, u64* out, u32 rows, u32 n, int sm_count, cudaStream_t st);
