@@ -175,7 +175,8 @@ inline u64 signature(const Shape& s, const u32* w, const fp2* cf, std::vector<fp
 }
 
 // ---------------------------------------------------------------------------------------------
-// The evaluation plan: the same graph regrouped for the kernels.  Every node becomes a sum of UNITS
+// The evaluation plan: a second regrouping of the graph with its own evaluators, which the host runs against the oracle as a check on
+// this file's grammar that shares nothing with the sumcheck kernels' programs (slot_vm.cuh).  Every node becomes a sum of UNITS
 // (coef * prod(factors); an affine term is a unit with one table factor, its constant a unit with none),
 // the top-level terms become the units of one more node (id n_nodes) whose value is the polynomial.
 // Node order: the affine nodes first, then the others by LEVEL (one more than the highest level a node
@@ -480,7 +481,7 @@ GL_HD void tpair_sums_all_t(const u32* pw, const fp2* cf, const fp2* V, const fp
         if (!(SKIP && p == 1)) out[p] = acc[p];
 }
 
-// host-side dispatch for the emulation (the kernels are instantiated per point count)
+// dispatch by point count
 inline void tpair_sums_all(const u32* pw, const fp2* cf, const fp2* V, const fp2* D, fp2* W, bool skip_one, fp2* out) {
     const u32 npw = pw[16] + 1;
 #define IR_TP(N) case N: if (skip_one) tpair_sums_all_t<N, true>(pw, cf, V, D, W, out); else tpair_sums_all_t<N, false>(pw, cf, V, D, W, out); break;
