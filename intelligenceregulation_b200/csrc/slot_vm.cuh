@@ -67,6 +67,7 @@ class Compiler {
         std::vector<Unit> prefixes;
         std::vector<Item> items;
         count_uses();
+        count_costs();
         std::function<void(const Unit&, const std::vector<Unit>&)> flatten = [&](const Unit& pre, const std::vector<Unit>& units) {
             prefixes.push_back(pre);
             const size_t here = prefixes.size() - 1;
@@ -116,7 +117,8 @@ class Compiler {
 
   private:
     struct Unit { fp2 c; std::vector<u32> f; };
-    struct Node { std::vector<Unit> units; bool linear = true; u32 uses = 0; int slot = -1; };
+    struct Node { std::vector<Unit> units; bool linear = true; u32 uses = 0, cost = 0; int slot = -1; };
+    static constexpr u32 COST_CAP = 4096;
     std::vector<Node> nodes_;
     std::vector<u32> p_free_, a_free_;
 
@@ -163,17 +165,18 @@ class Compiler {
                     if (f & ir::IR_NODE) { live[f & ~ir::IR_NODE] = true; nodes_[f & ~ir::IR_NODE].uses++; }
         }
     }
-    // instructions, about; a shared node counts with everyone who uses it, since it may end up in several parts
+    // instructions, about; a shared node counts with everyone who uses it, since it may end up in several parts.  Nodes refer to earlier
+    // ones only: each is counted once, in their order (a chain of nodes that use the one before twice would be 2^nodes visits), up to a cap.
     u32 unit_cost(const Unit& u) const {
         u32 c = 2;
-        for (u32 f : u.f) c += factor_cost(f);
+        for (u32 f : u.f) c += f & ir::IR_NODE ? nodes_[f & ~ir::IR_NODE].cost : 1;
         return c;
     }
-    u32 factor_cost(u32 f) const {
-        if (!(f & ir::IR_NODE)) return 1;
-        u32 c = 1;
-        for (auto& u : nodes_[f & ~ir::IR_NODE].units) { c += unit_cost(u); if (c > 4096) return 4096; }
-        return c;
+    void count_costs() {
+        for (auto& nd : nodes_) {
+            nd.cost = 1;
+            for (auto& u : nd.units) nd.cost = std::min(nd.cost + unit_cost(u), COST_CAP);
+        }
     }
     void part(const std::vector<Unit>& top) {
         Node root;

@@ -3,6 +3,7 @@ linear and non-linear nodes, constants, repeated factors, zero coefficients) aga
 import ctypes as C
 import os
 import subprocess
+import threading
 
 import numpy as np
 import pytest
@@ -81,3 +82,37 @@ def test_random_graphs(emul, seed):
         prog.term(c, [], fs)
         desc["terms"].append((c, fs))
     _check(emul, prog, desc, k, seed)
+
+
+def _within(seconds, fn):
+    """fn() on a thread of its own (the compiler runs without the interpreter's lock), which a compilation without end does not hold up"""
+    got = []
+    t = threading.Thread(target=lambda: got.append(fn()), daemon=True)
+    t.start()
+    t.join(seconds)
+    assert not t.is_alive(), "still compiling"
+    assert got
+    return got[0]
+
+
+@pytest.mark.parametrize("nodes", [4, 24, 126])
+def test_every_node_uses_the_one_before_twice(emul, nodes):
+    """2^nodes paths through the graph, `nodes` nodes of work"""
+    from intelligenceregulation_b200 import backend
+
+    SP, r = backend.SlotProgram, U.Rand(nodes)
+    prog, desc = SP(2), {"nodes": [], "terms": []}
+
+    def node(subs):
+        desc["nodes"].append(("sum", subs))
+        return prog.sum(subs)
+
+    prev = node([(r.coef("chal"), []), (r.coef("chal"), [])])
+    for _ in range(nodes):
+        prev = node([(r.coef("chal"), [SP.node(prev), SP.node(prev)]), (r.coef("kbase"), [])])
+    for t in (0, 1):
+        c = r.coef("chal")
+        prog.term(c, [], [t, SP.node(prev)])
+        desc["terms"].append((c, [t, SP.node(prev)]))
+    info = _within(60, lambda: _check(emul, prog, desc, 2, nodes))
+    assert info[3] == 1
