@@ -146,7 +146,6 @@ int hl_b200_act_histogram(hl_ctx* c, const int64_t* gates, const int64_t* output
     if (!rc) rc = d2h(c, counts, d_cnt, nb * 8);
     if (!rc) rc = d2h(c, misses, d_cnt + nb, 8);
     if (!rc) rc = sync(c, "act_histogram");
-    else cudaStreamSynchronize(c->stream);
     return rc;
 }
 
@@ -184,7 +183,6 @@ int hl_b200_act_helpers(hl_ctx* c, const int64_t* gates, const int64_t* outputs,
     int flag = 0;
     if (!rc) rc = d2h(c, &flag, d_err, 4);
     if (!rc) rc = sync(c, "act_helpers");
-    else cudaStreamSynchronize(c->stream);
     if (!rc && flag) return fail(c, HL_B200_ERR_ZERO, "zero LogUp denominator; discard attempt");
     if (!rc) rc = d2h(c, h, d_h, n * 16);
     if (!rc) rc = sync(c, "act_helpers");
@@ -225,7 +223,6 @@ int hl_b200_act_table(hl_ctx* c, const int64_t* tables, size_t groups, size_t le
     int flag = 0;
     if (!rc) rc = d2h(c, &flag, d_err, 4);
     if (!rc) rc = sync(c, "act_table");
-    else cudaStreamSynchronize(c->stream);
     if (!rc && flag) return fail(c, HL_B200_ERR_ZERO, "zero LogUp denominator; discard attempt");
     if (!rc && compressed) rc = d2h(c, compressed, d_v, len * 16);
     if (!rc) rc = d2h(c, ht, d_h, len * 16);

@@ -18,8 +18,15 @@ int fail(hl_ctx* c, int code, const char* what, cudaError_t e) {
         std::lock_guard<std::mutex> g(c->err_mu);
         c->last_error = buf;
         c->stats.declines++;
+        c->failed = true;
     }
     return code;
+}
+
+void settle(hl_ctx* c) {
+    if (!c->failed) return;
+    cudaStreamSynchronize(c->copy_stream);
+    cudaStreamSynchronize(c->stream);
 }
 
 // Stream-ordered allocation from the device's default pool, whose release threshold is
@@ -39,6 +46,7 @@ int dev_alloc(hl_ctx* c, void** p, size_t bytes) {
 
 void dev_free(hl_ctx* c, void* p, size_t bytes) {
     if (!p) return;
+    settle(c);
     cudaFreeAsync(p, c->stream);
     if (bytes == 0) bytes = 16;
     c->alloc_live = c->alloc_live >= bytes ? c->alloc_live - bytes : 0;
@@ -159,6 +167,7 @@ int hl_b200_init(int device, hl_ctx** out) {
 void hl_b200_shutdown(hl_ctx* c) {
     if (!c) return;
     cudaSetDevice(c->device);
+    cudaStreamSynchronize(c->copy_stream);
     cudaStreamSynchronize(c->stream);
     for (auto& kv : c->tw) cudaFree(kv.second);
     if (c->wp_flag) cudaFreeHost(c->wp_flag);
@@ -168,7 +177,6 @@ void hl_b200_shutdown(hl_ctx* c) {
     for (auto e : c->ev_pool) cudaEventDestroy(e);
     for (auto e : c->ev_chunks) cudaEventDestroy(e);
     cudaEventDestroy(c->ev_main);
-    cudaStreamSynchronize(c->copy_stream);
     cudaStreamDestroy(c->copy_stream);
     cudaStreamDestroy(c->own_stream);
     delete c;

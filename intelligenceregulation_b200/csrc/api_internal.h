@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <map>
 #include <set>
 #include <mutex>
@@ -41,6 +42,8 @@ struct hl_ctx {
     int* wp_flag = nullptr;  // page-locked: the witness products' status word: zero between calls
     bool wp_attr = false;      // the product kernel's shared-memory size has been raised on this device
     std::set<const struct hl_store*> stores;  // the live commitment stores (a planned slot table that reads one checks it is still there when it is built)
+    // something of the present call has failed: its copies may still be under way, on either stream (`settle`)
+    std::atomic<bool> failed{false};
     size_t alloc_live = 0;   // bytes handed out and not yet returned
     size_t alloc_cap = 0;    // 0 = none; a host-side failure-injection cap (mod.rs:121 set_alloc_cap_for_test)
 };
@@ -64,6 +67,7 @@ namespace hlapi {
 int fail(hl_ctx* c, int code, const char* what, cudaError_t e = cudaSuccess);
 int dev_alloc(hl_ctx* c, void** p, size_t bytes);
 void dev_free(hl_ctx* c, void* p, size_t bytes);
+void settle(hl_ctx* c);  // waits for both streams if something of the present call has failed
 // host_copy.cu: uploads on the context's stream (h2d_on: on another one that the context's stream waits for before the call ends);
 // h2d_owned: the caller's bytes are no longer needed when it returns, whatever kind of host memory they live in;
 // d2h: the bytes are in place after the next `sync`
@@ -78,13 +82,21 @@ void host_copy_retain();
 void host_copy_release(hl_ctx* c);
 void host_copy_drop();
 
-// What every entry point that works on a context holds: its lock and its device.  Results that a failed call left in the bounce area
-// go with it: nothing may write to that caller's memory later.
+// What every entry point that works on a context holds: its lock and its device.  A call that succeeds has waited for what it queued, or
+// keeps it on the context's stream.  One that fails on the way has not, and `dev_free` orders what it gives back after the context's stream
+// alone: so a failed call settles before it frees anything and before it returns.  Results that it left in the bounce area go with it:
+// nothing may write to that caller's memory later.
 struct Call {
     hl_ctx* c;
     std::lock_guard<std::mutex> g;
-    explicit Call(hl_ctx* ctx) : c(ctx), g(ctx->mu) { cudaSetDevice(c->device); }
-    ~Call() { c->pending.clear(); }
+    explicit Call(hl_ctx* ctx) : c(ctx), g(ctx->mu) {
+        cudaSetDevice(c->device);
+        c->failed = false;
+    }
+    ~Call() {
+        settle(c);
+        c->pending.clear();
+    }
 };
 int root_powers(hl_ctx* c, u32 lognn, const u64** out);
 int upload_key(hl_ctx* c, const uint8_t* key32, uint32_t** d_key);

@@ -352,7 +352,7 @@ int commit_host(hl_ctx* c, const Shape& s, const HostRows& data, const uint64_t*
     if (d_pows) dev_free(c, d_pows, nn * 8);
     if (d_salts) dev_free(c, d_salts, nn * 32);
     if (d_levels) dev_free(c, d_levels, (2 * nn - 1) * 32);
-    if (rc) { cudaStreamSynchronize(c->copy_stream); cudaStreamSynchronize(c->stream); free_store(st); return rc; }
+    if (rc) { free_store(st); return rc; }
     c->stats.commits++;
     c->stores.insert(st);
     *store = st;
@@ -382,7 +382,7 @@ int hlapi::commit_resident(hl_ctx* c, u32 log_cols, u32 inv_rate, const u64* d_d
         cudaError_t e = cudaMemcpyAsync(d_leaves32, st->d_leaves, nn * 32, cudaMemcpyDeviceToDevice, c->stream);
         if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "leaf copy", e);
     }
-    if (rc) { cudaStreamSynchronize(c->stream); free_store(st); return rc; }
+    if (rc) { free_store(st); return rc; }
     c->stats.commits++;
     c->stores.insert(st);
     *store = st;

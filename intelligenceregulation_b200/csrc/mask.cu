@@ -188,7 +188,6 @@ int hl_b200_mask_commit(hl_ctx* c, uint32_t log_msg, uint32_t log_dom, const uin
     }
     if (!rc) rc = d2h(c, leaves32, st->d_leaves, dom * 32);
     if (!rc) rc = sync(c, "mask_commit");
-    else cudaStreamSynchronize(c->stream);
     dev_free(c, d_msgs, n_msg_rows * m * 8);
     dev_free(c, d_pows, dom * 8);
     dev_free(c, scratch, scratch_words * 8);
@@ -236,7 +235,6 @@ int hl_b200_mask_open_q(hl_store* st, size_t n_masks, const uint64_t* ws, uint64
     }
     if (!rc) rc = d2h(c, q, d_q, m2 * 16);
     if (!rc) rc = sync(c, "mask_open_q");
-    else cudaStreamSynchronize(c->stream);
     dev_free(c, d_ws, n_masks * m * 16);
     dev_free(c, d_part, n_masks * 2 * m2 * 8);
     dev_free(c, d_q, m2 * 16);

@@ -245,7 +245,7 @@ int rounds_build(hl_ctx* c, int poly, size_t k, uint32_t n_vars, uint32_t degree
         if (!rc) rc = d2h(c, &r->nonbase, r->d_nonbase, 8);
         if (!rc) rc = sync(c, "rounds_new");
     }
-    if (rc) { cudaStreamSynchronize(c->stream); free_rounds(r); return rc; }
+    if (rc) { free_rounds(r); return rc; }
     if (built) r->d_tables = hl_tables_adopt(built);  // only now: a failed build leaves the set with its owner
     *out = r;
     return HL_B200_OK;

@@ -454,7 +454,6 @@ int product_on_device(hl_ctx* c, size_t t_rows, const int64_t* d_x, size_t xs, c
         if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "witness product launch", e);
     }
     if (!rc) rc = sync(c, "witness_product");
-    else cudaStreamSynchronize(c->stream);
     if (d_flag) {
         flag = *reinterpret_cast<volatile int*>(d_flag);
         *d_flag = 0;  // for the next call
@@ -508,7 +507,6 @@ int hl_b200_witness_product(hl_ctx* c, size_t t_rows, const int64_t* x, size_t x
     if (!rc) rc = product_on_device(c, t_rows, d_x, xs, d_w, inner, outer, os, out_len, in_out, d_out, taken);
     if (!rc && *taken) rc = d2h(c, out, d_out, ob);
     if (!rc) rc = sync(c, "witness_product");
-    else cudaStreamSynchronize(c->stream);
     if (d_x) dev_free(c, d_x, xb);
     if (d_w) dev_free(c, d_w, wb);
     if (d_out) dev_free(c, d_out, ob);

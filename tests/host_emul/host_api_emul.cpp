@@ -1,0 +1,162 @@
+// The library's host code over a runtime without a device (fake_cuda.h).
+//   host_api_emul failures     every entry point below with every fallible call of it failing in turn: whatever happens, no memory goes while
+//                              a copy uses it, no copy uses the caller's memory once the call is over, and nothing is lost
+//   host_api_emul threads N    large copies where the process can make only N threads
+#include "fake_cuda.h"
+
+#include <dlfcn.h>
+#include <pthread.h>
+
+#include <cerrno>
+#include <cstdio>
+#include <functional>
+
+#include "../../intelligenceregulation_b200/csrc/api_internal.h"
+
+static long g_threads = -1;  // how many more threads may be made (-1: any number)
+extern "C" int pthread_create(pthread_t* t, const pthread_attr_t* a, void* (*f)(void*), void* x) noexcept {
+    static auto real = (int (*)(pthread_t*, const pthread_attr_t*, void* (*)(void*), void*))dlsym(RTLD_NEXT, "pthread_create");
+    if (g_threads == 0) return EAGAIN;
+    if (g_threads > 0) g_threads--;
+    return real(t, a, f, x);
+}
+
+namespace hlk {
+static cudaError_t launch() { return fake::fails() ? cudaErrorUnknown : cudaSuccess; }
+size_t encode_scratch_words(u32, u32, int, u32) { return 64; }
+bool encode_split_pays(u32, u32, u32, int) { return false; }
+cudaError_t encode_rows(const enc::RowArgs&, u32, bool, int, size_t, cudaStream_t, int*) { return launch(); }
+cudaError_t widen_rows(const unsigned char*, const u64*, const unsigned char*, u64*, u32, u32, int, cudaStream_t) { return launch(); }
+u32 hash_chunks(u32 rows) { return (rows + 127) / 128; }
+cudaError_t hash_column_chunks(const u64*, u32, u32, const uint32_t*, u32, u32, uint32_t*, uint32_t*, cudaStream_t) { return launch(); }
+cudaError_t hash_column_merge(u32, u32, const uint32_t*, const uint32_t*, uint32_t*, cudaStream_t) { return launch(); }
+cudaError_t hash_columns(const u64*, u32, u32, const uint32_t*, uint32_t*, uint32_t*, cudaStream_t) { return launch(); }
+cudaError_t merkle_tree(const uint32_t*, const uint32_t*, u32, const uint32_t*, const uint32_t*, uint32_t*, cudaStream_t, int* n) { *n = 1; return launch(); }
+u32 fold_row_splits(u32, u32, u32, u32, int) { return 1; }
+u32 fold_few_ranges(u32, u32, u32, u32, u32, int) { return 0; }
+cudaError_t fold_rows_few(const u64*, u32, u32, size_t, const u64*, u32, size_t, const u64*, u32, const u32*, u64*, u32, u32, u64*, cudaStream_t) { return launch(); }
+cudaError_t fold_rows(const u64*, u32, u32, size_t, u32, const u64*, u32, size_t, const u64*, u32, const u32*, u64*, u32, cudaStream_t, u32, u64*) { return launch(); }
+cudaError_t fold_rows_sparse(const u64*, u32, size_t, u32, const u64*, u32, size_t, const u32*, const u32*, const u64*, u32, const u32*, u64*, u32, cudaStream_t) { return launch(); }
+cudaError_t gather_columns(const u64*, u32, size_t, const u64*, u32, u64*, cudaStream_t) { return launch(); }
+// out: a + b, a - b, a b, three words a pair.  Here: a, b, 0, which shows that both arrays arrived and the results came back
+cudaError_t probe_field(const u64* a, const u64* b, size_t n, u64* out, cudaStream_t st) {
+    cudaStreamSynchronize(st);
+    for (size_t i = 0; i < n; i++) { out[3 * i] = a[i]; out[3 * i + 1] = b[i]; out[3 * i + 2] = 0; }
+    return launch();
+}
+cudaError_t butterfly_peak(const u64*, u64*, u32, int, cudaStream_t) { return launch(); }
+cudaError_t compress_peak(const u64*, u64*, u32, int, cudaStream_t) { return launch(); }
+}  // namespace hlk
+
+// memory of the caller, page-locked or not
+struct Host {
+    std::vector<std::vector<uint64_t>> all;
+    bool lock;
+    explicit Host(bool l) : lock(l) {}
+    uint64_t* words(size_t n) {
+        all.emplace_back(n, 1);
+        if (lock) fake::locked[(const char*)all.back().data()] = n * 8;
+        return all.back().data();
+    }
+    uint8_t* bytes(size_t n) { return (uint8_t*)words((n + 7) / 8); }
+    bool busy() const {
+        for (auto& v : all)
+            if (fake::busy(v.data(), v.size() * 8)) return true;
+        return false;
+    }
+    ~Host() {
+        if (lock)
+            for (auto& v : all) fake::locked.erase((const char*)v.data());
+    }
+};
+
+static int g_bad = 0;
+static void bad(const char* what, const std::string& how) {
+    if (g_bad++ < 200) printf("%s: %s\n", what, how.c_str());
+}
+
+static void sweep(const char* what, hl_ctx* c, Host& h, const std::function<int()>& call) {
+    fake::fail_at = -1;
+    if (call()) bad(what, "fails with nothing failing");
+    const size_t blocks = fake::device.size(), live = c->alloc_live;
+    for (long at = 0;; at++) {
+        fake::calls = 0;
+        fake::fail_at = at;
+        const int rc = call();
+        const bool past = fake::calls <= at;
+        fake::fail_at = -1;
+        const std::string where = " (call " + std::to_string(at) + ", rc " + std::to_string(rc) + ")";
+        if (h.busy()) bad(what, "a copy uses the caller's memory after the call" + where);
+        for (auto& f : fake::faults) bad(what, f + where);
+        fake::faults.clear();
+        cudaStreamSynchronize(c->stream);
+        cudaStreamSynchronize(c->copy_stream);
+        for (auto& f : fake::faults) bad(what, f + ", later" + where);
+        fake::faults.clear();
+        if (fake::device.size() != blocks || c->alloc_live != live) bad(what, "device memory lost" + where);
+        if (past) break;
+    }
+    if (call()) bad(what, "does not recover");
+}
+
+static void failures(bool lock) {
+    hl_ctx* c = nullptr;
+    hl_b200_init(0, &c);
+    const uint8_t key[32] = {1};
+    for (const u32 rows : {6u, 300u}) {  // whole, and in pieces (32 MiB and more than four waves of the encoder)
+        const u32 lc = rows == 6 ? 12 : 14, q = 40;
+        const size_t n = (size_t)1 << lc, nn = 2 * n;
+        Host h(lock);
+        uint64_t *data = h.words(rows * n), *pads = h.words(rows * q), *pows = h.words(nn);
+        uint8_t *salts = h.bytes(nn * 32), *levels = h.bytes((2 * nn - 1) * 32), *leaves = h.bytes(nn * 32), *widths = h.bytes(rows);
+        memset(widths, 8, rows);
+        const char* names[2] = {"commit_zk_packed", "commit_zk_tree"};
+        for (int form = 0; form < (rows == 6 ? 2 : 1); form++)
+            sweep(names[form], c, h, [&] {
+                hl_store* st = nullptr;
+                const int rc = form ? hl_b200_commit_zk_tree(c, lc, 2, data, rows, pads, q, pows, lc + 1, key, salts, key, key, &st, leaves, levels)
+                                    : hl_b200_commit_zk_packed(c, lc, 2, data, widths, rows, pads, q, pows, lc + 1, key, salts, key, key, &st, leaves, levels);
+                hl_b200_store_free(st);
+                return rc;
+            });
+        hl_store* st = nullptr;
+        hl_b200_commit_zk(c, lc, 2, data, rows, pads, q, pows, lc + 1, key, &st, leaves);
+        if (rows == 6) sweep("store_merkle", c, h, [&] { return hl_b200_store_merkle(st, salts, key, key, levels); });
+        if (rows == 6) sweep("merkle", c, h, [&] { return hl_b200_merkle(c, leaves, salts, nn, key, key, levels); });
+        const size_t k = 9, cols = 70;  // eight vectors that live on one row, together, and a dense one: their results go back on both streams
+        uint64_t *rhos = h.words(k * rows * 2), *out = h.words(k * (n + q) * 2), *idx = h.words(cols), *got = h.words(cols * rows);
+        for (size_t g = 0; g + 1 < k; g++) memset(rhos + (g * rows + 1) * 2, 0, (rows - 1) * 16);
+        sweep("store_fold", c, h, [&] { return hl_b200_store_fold(st, rhos, k, 1, out); });
+        sweep("store_columns", c, h, [&] { return hl_b200_store_columns(st, idx, cols, got); });
+        hl_b200_store_free(st);
+    }
+    hl_b200_shutdown(c);
+}
+
+static void threads() {
+    hl_ctx* c = nullptr;
+    hl_b200_init(0, &c);
+    for (const size_t n : {(size_t)1000, (size_t)100000, (size_t)3000000}) {
+        std::vector<uint64_t> a(n), b(n), out(3 * n);
+        for (size_t i = 0; i < n; i++) { a[i] = i * 0x9E3779B97F4A7C15ull; b[i] = ~a[i]; }
+        for (int rep = 0; rep < 3; rep++) {
+            std::fill(out.begin(), out.end(), 7);
+            if (hl_b200_probe_field(c, a.data(), b.data(), n, out.data())) bad("probe_field", "refused");
+            for (size_t i = 0; i < n; i++)
+                if (out[3 * i] != a[i] || out[3 * i + 1] != b[i] || out[3 * i + 2]) { bad("probe_field", "wrong bytes"); break; }
+        }
+    }
+    hl_b200_shutdown(c);
+}
+
+int main(int argc, char** argv) {
+    if (argc == 3 && !strcmp(argv[1], "threads")) {
+        g_threads = atol(argv[2]);
+        threads();
+    } else {
+        failures(false);
+        failures(true);
+    }
+    if (!g_bad) printf("ok\n");
+    return g_bad != 0;
+}
