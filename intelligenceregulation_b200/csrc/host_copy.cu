@@ -12,6 +12,7 @@
 #include <atomic>
 #include <condition_variable>
 #include <cstring>
+#include <exception>
 #include <functional>
 #include <thread>
 #if defined(__x86_64__)
@@ -88,7 +89,11 @@ class Helpers {
         const unsigned hw = std::thread::hardware_concurrency();
         // half the cores at most; four threads saturate the bus, two more help where the destination's pages are fresh
         const int n = hw >= 12 ? 5 : hw >= 4 ? (int)hw / 2 - 1 : 0;
-        for (int i = 0; i < n; i++) threads_.emplace_back([this, e = epoch_] { loop(e); });
+        // a process that may not make (all of) them, under a limit on threads or memory, copies with those there are
+        try {
+            for (int i = 0; i < n; i++) threads_.emplace_back([this, e = epoch_] { loop(e); });
+        } catch (const std::exception&) {
+        }
     }
     void loop(u64 seen) {
         std::unique_lock<std::mutex> g(mu_);

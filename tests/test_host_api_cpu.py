@@ -27,3 +27,8 @@ def test_a_failing_call_leaves_no_copy_behind(emul):
     """every fallible runtime call of the commitments and openings fails in turn: no memory is freed while a copy on another stream uses it,
     no copy uses the caller's memory after the call, nothing is lost, and the next call works"""
     _ok(emul, "failures")
+
+
+@pytest.mark.parametrize("threads", [0, 1, 3, 100])
+def test_large_copies_where_few_threads_can_be_made(emul, threads):
+    _ok(emul, "threads", str(threads))
