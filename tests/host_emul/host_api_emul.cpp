@@ -1,7 +1,8 @@
 // The library's host code over a runtime without a device (fake_cuda.h).
 //   host_api_emul failures     every entry point below with every fallible call of it failing in turn: whatever happens, no memory goes while
 //                              a copy uses it, no copy uses the caller's memory once the call is over, and nothing is lost
-//   host_api_emul threads N    large copies where the process can make only N threads
+//   host_api_emul copies       the bytes of copies of all sizes and alignments
+//   host_api_emul threads N    the same where the process can make only N threads
 #include "fake_cuda.h"
 
 #include <dlfcn.h>
@@ -133,17 +134,22 @@ static void failures(bool lock) {
     hl_b200_shutdown(c);
 }
 
-static void threads() {
+// every size class of the copies and both sides of its limits, at every alignment that words have
+static void sizes() {
     hl_ctx* c = nullptr;
     hl_b200_init(0, &c);
-    for (const size_t n : {(size_t)1000, (size_t)100000, (size_t)3000000}) {
-        std::vector<uint64_t> a(n), b(n), out(3 * n);
-        for (size_t i = 0; i < n; i++) { a[i] = i * 0x9E3779B97F4A7C15ull; b[i] = ~a[i]; }
-        for (int rep = 0; rep < 3; rep++) {
+    for (const size_t n : {1, 7, 8191, 8192, 8193, 16384, 16385, 21845, 21846, 32769, 43691, 65536, 65537, 100001, 3000001}) {
+        std::vector<uint64_t> a(n + 8), b(n + 8), out(3 * n + 8);
+        for (size_t i = 0; i < n + 8; i++) { a[i] = i * 0x9E3779B97F4A7C15ull; b[i] = ~a[i]; }
+        for (size_t off = 0; off < (n > 1000000 ? 2u : 8u); off++) {
             std::fill(out.begin(), out.end(), 7);
-            if (hl_b200_probe_field(c, a.data(), b.data(), n, out.data())) bad("probe_field", "refused");
-            for (size_t i = 0; i < n; i++)
-                if (out[3 * i] != a[i] || out[3 * i + 1] != b[i] || out[3 * i + 2]) { bad("probe_field", "wrong bytes"); break; }
+            if (hl_b200_probe_field(c, a.data() + off, b.data() + off, n, out.data() + off)) bad("probe_field", "refused");
+            const uint64_t* o = out.data() + off;
+            bool ok = true;
+            for (size_t i = 0; i < n && ok; i++) ok = o[3 * i] == a[off + i] && o[3 * i + 1] == b[off + i] && !o[3 * i + 2];
+            for (size_t i = 0; i < off; i++) ok = ok && out[i] == 7;
+            for (size_t i = 3 * n + off; i < out.size(); i++) ok = ok && out[i] == 7;
+            if (!ok) bad("probe_field", "wrong bytes at " + std::to_string(n) + " words, offset " + std::to_string(off));
         }
     }
     hl_b200_shutdown(c);
@@ -152,7 +158,9 @@ static void threads() {
 int main(int argc, char** argv) {
     if (argc == 3 && !strcmp(argv[1], "threads")) {
         g_threads = atol(argv[2]);
-        threads();
+        sizes();
+    } else if (argc == 2 && !strcmp(argv[1], "copies")) {
+        sizes();
     } else {
         failures(false);
         failures(true);

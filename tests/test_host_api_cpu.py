@@ -29,6 +29,11 @@ def test_a_failing_call_leaves_no_copy_behind(emul):
     _ok(emul, "failures")
 
 
+def test_copies_of_all_sizes(emul):
+    """the limits between the forms of a copy, unaligned ends, and more small copies in a call than the bounce areas hold"""
+    _ok(emul, "copies")
+
+
 @pytest.mark.parametrize("threads", [0, 1, 3, 100])
-def test_large_copies_where_few_threads_can_be_made(emul, threads):
+def test_copies_where_few_threads_can_be_made(emul, threads):
     _ok(emul, "threads", str(threads))
