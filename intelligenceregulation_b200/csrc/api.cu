@@ -172,7 +172,9 @@ void hl_b200_shutdown(hl_ctx* c) {
     for (auto& kv : c->tw) cudaFree(kv.second);
     if (c->wp_flag) cudaFreeHost(c->wp_flag);
     host_copy_release(c);
-    if (c->arena) cudaFreeHost(c->arena);
+    if (c->up.mem) cudaFreeHost(c->up.mem);
+    if (c->down.mem) cudaFreeHost(c->down.mem);
+    for (auto e : c->ev_spare) cudaEventDestroy(e);
     for (auto& s : c->spans) { cudaEventDestroy(s.a); cudaEventDestroy(s.b); }
     for (auto e : c->ev_pool) cudaEventDestroy(e);
     for (auto e : c->ev_chunks) cudaEventDestroy(e);

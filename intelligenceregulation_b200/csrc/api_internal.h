@@ -35,10 +35,12 @@ struct hl_ctx {
     std::vector<cudaEvent_t> ev_pool;  // events ready for reuse
     hl_timing timing_acc{};
     hlapi::CopyRing* ring = nullptr;  // page-locked slots for large copies of pageable host memory (host_copy.cu, made on first use)
-    char* arena = nullptr;     // page-locked bounce area for small copies in either direction, empty after every synchronisation
-    size_t arena_off = 0;
-    struct Pending { void* to; const char* from; size_t bytes; };
-    std::vector<Pending> pending;  // small results in the bounce area, handed out by the next `sync`
+    // page-locked bounce areas for small copies (host_copy.cu), empty after every synchronisation
+    struct Bounce { char* mem = nullptr; size_t off = 0; } up, down;
+    bool up_elsewhere = false;  // a copy from the upload area went to the copy stream
+    struct Pending { void* to; const char* from; size_t bytes; cudaEvent_t ev; };  // ev: when the piece has arrived (none: with the stream)
+    std::vector<Pending> pending;  // pieces of results on their way through the bounce area, handed out by the next `sync`
+    std::vector<cudaEvent_t> ev_spare;
     int* wp_flag = nullptr;  // page-locked: the witness products' status word: zero between calls
     bool wp_attr = false;      // the product kernel's shared-memory size has been raised on this device
     std::set<const struct hl_store*> stores;  // the live commitment stores (a planned slot table that reads one checks it is still there when it is built)
@@ -78,6 +80,7 @@ int d2h(hl_ctx* c, void* h, const void* d, size_t bytes);
 // the same on a second stream; the context's stream waits for it
 int d2h_on(hl_ctx* c, void* h, const void* d, size_t bytes, cudaStream_t s);
 int sync(hl_ctx* c, const char* what);
+void drop_pending(hl_ctx* c);
 void host_copy_retain();
 void host_copy_release(hl_ctx* c);
 void host_copy_drop();
@@ -95,7 +98,7 @@ struct Call {
     }
     ~Call() {
         settle(c);
-        c->pending.clear();
+        drop_pending(c);
     }
 };
 int root_powers(hl_ctx* c, u32 lognn, const u64** out);

@@ -1,11 +1,11 @@
 // Copies between the caller's host memory and the device.  Every entry point of the C ABI takes plain host pointers, so what a caller
 // waits for is mostly this file: page-locked memory goes to the copy engine as it is, everything else through page-locked memory here.
 //
-//   tiny uploads             (<= TINY bytes) as they are: the driver puts the bytes into its command stream (1.9 us, against 3.6 us of
-//                            a copy from page-locked memory).
-//   small (<= SMALL bytes)   through the context's bounce area: one memcpy and one asynchronous copy.  Results come back at the next
-//                            synchronisation (`sync` hands them out), so a call with several small results waits once.  The driver's
-//                            own path for pageable memory stages and waits inside every single call.
+//   tiny uploads             (<= TINY bytes) as they are: the driver puts the bytes into its command stream, and a kernel that reads them
+//                            need not wait for the copy engine (an int8 fold of 48 KB: 39 us a call, through the bounce area 52).
+//   small (<= SMALL_UP and   through the context's bounce areas: pieces that the host copies while the engine moves the one before.  Results
+//   SMALL_DOWN bytes)        come back at the next synchronisation (`sync` hands them out), so a call with several small results waits
+//                            once.  The driver's own path for pageable memory stages and waits inside every single call.
 //   large, pageable          through a ring of page-locked slots, filled and emptied by a few host threads beside the copy engine.
 //                            One core moves about 18 GB/s (and far less into fresh pages, which it has to fault in), the bus 55 GB/s.
 //   page-locked or managed   one asynchronous copy.
@@ -30,9 +30,15 @@ namespace hlapi {
 
 namespace {
 
-constexpr size_t ARENA_BYTES = (size_t)4 << 20;
-constexpr size_t TINY = (size_t)16 << 10;
-constexpr size_t SMALL = (size_t)512 << 10;  // a memcpy of this size costs about what waking the helper threads does (10 - 20 us)
+constexpr size_t AREA_BYTES = (size_t)4 << 20;
+// Up to here the driver's own copy, of pageable bytes, stays out of the copy engine's queue (its limit is 64 KB)
+constexpr size_t TINY = (size_t)64 << 10;
+// Up to here one thread, from here on it and the helpers, which have to be woken.  Calls of one upload from memory that is not in the
+// caller's caches, and of one result, in us, one thread against the helpers: up 330 KB 73 .. 77 against 73 .. 84, 400 KB 91 .. 97 against
+// 76 .. 83, 500 KB 98 .. 101 against 78 .. 86; down 544 KB 134 .. 143 against 149 .. 155, 768 KB 154 .. 165 against 161 .. 163, 896 KB
+// 171 .. 179 against 163 .. 168 (straight after the call before, and half a millisecond later).
+constexpr size_t SMALL_UP = (size_t)384 << 10, SMALL_DOWN = (size_t)768 << 10;
+constexpr size_t PIECE_UP = (size_t)128 << 10, PIECE_DOWN = (size_t)256 << 10;
 
 inline void relax() {
 #if defined(__x86_64__)
@@ -344,36 +350,65 @@ static cudaError_t ring_down(CopyRing* r, char* h, const char* d, size_t bytes, 
     return err;
 }
 
-static char* arena_slot(hl_ctx* c, size_t bytes) {
-    if (!c->arena && cudaHostAlloc((void**)&c->arena, ARENA_BYTES, cudaHostAllocDefault) != cudaSuccess) {
+// The bounce areas: one for uploads, which the host only writes, past its caches, and one for results, which the host only reads.  (One
+// area for both had the uploads write over lines that the results before had left in the caches: 512 KB 84 us instead of 50.)
+static char* bounce(hl_ctx* c, hl_ctx::Bounce& b, size_t bytes) {
+    if (!b.mem && cudaHostAlloc((void**)&b.mem, AREA_BYTES, cudaHostAllocDefault) != cudaSuccess) {
         cudaGetLastError();
-        c->arena = nullptr;
+        b.mem = nullptr;
         return nullptr;
     }
     const size_t need = (bytes + 63) & ~(size_t)63;
-    if (c->arena_off + need > ARENA_BYTES && sync(c, "bounce area") != HL_B200_OK) return nullptr;  // a synchronisation empties the area
-    char* slot = c->arena + c->arena_off;
-    c->arena_off += need;
+    if (b.off + need > AREA_BYTES && sync(c, "bounce area") != HL_B200_OK) return nullptr;  // a synchronisation empties both
+    char* slot = b.mem + b.off;
+    b.off += need;
     return slot;
+}
+
+static cudaError_t bounce_up(char* slot, char* d, const char* h, size_t bytes, cudaStream_t s) {
+    cudaError_t e = cudaSuccess;
+    for (size_t at = 0; at < bytes && e == cudaSuccess; at += PIECE_UP) {
+        const size_t n = bytes - at < PIECE_UP ? bytes - at : PIECE_UP;
+        copy_past_caches(slot + at, h + at, n);
+        e = cudaMemcpyAsync(d + at, slot + at, n, cudaMemcpyHostToDevice, s);
+    }
+    return e;
+}
+
+// a result's pieces, each but the last with an event (that one comes with the stream)
+static cudaError_t bounce_down(hl_ctx* c, char* slot, char* h, const char* d, size_t bytes, cudaStream_t s) {
+    cudaError_t e = cudaSuccess;
+    for (size_t at = 0; at < bytes && e == cudaSuccess; at += PIECE_DOWN) {
+        const size_t n = bytes - at < PIECE_DOWN ? bytes - at : PIECE_DOWN;
+        cudaEvent_t ev = nullptr;
+        e = cudaMemcpyAsync(slot + at, d + at, n, cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess && at + n < bytes) {
+            if (c->ev_spare.empty()) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+            else { ev = c->ev_spare.back(); c->ev_spare.pop_back(); }
+        }
+        if (e != cudaSuccess) break;
+        c->pending.push_back({h + at, slot + at, n, ev});
+        if (ev) e = cudaEventRecord(ev, s);
+    }
+    return e;
 }
 
 // On return the caller's bytes are no longer needed, unless they are page-locked (then they are read by the end of the call that the
 // copy is part of).
 int h2d_on(hl_ctx* c, void* d, const void* h, size_t bytes, cudaStream_t s) {
     if (!bytes) return HL_B200_OK;
-    const void* from = h;
     cudaError_t e;
+    char* slot;
     CopyRing* r;
     if (bytes <= TINY && pageable(h)) {
         e = cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, s);
-    } else if (bytes <= SMALL) {
-        char* slot = arena_slot(c, bytes);
-        if (slot) { copy_past_caches(slot, (const char*)h, bytes); from = slot; }
-        e = cudaMemcpyAsync(d, from, bytes, cudaMemcpyHostToDevice, s);
+    } else if (bytes <= SMALL_UP && (slot = bounce(c, c->up, bytes)) != nullptr) {
+        c->up_elsewhere |= s != c->stream;
+        e = bounce_up(slot, (char*)d, (const char*)h, bytes, s);
     } else if (pageable(h) && (r = ring_of(c)) != nullptr) {
         e = ring_up(r, (char*)d, (const char*)h, bytes, s);
     } else {
-        e = cudaMemcpyAsync(d, from, bytes, cudaMemcpyHostToDevice, s);
+        e = cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, s);
     }
     if (e != cudaSuccess) return fail(c, HL_B200_ERR_DEVICE, "copy to device", e);
     c->stats.bytes_h2d += bytes;
@@ -385,7 +420,7 @@ int h2d(hl_ctx* c, void* d, const void* h, size_t bytes) { return h2d_on(c, d, h
 // The same for calls that return before the stream has been waited for: page-locked bytes are waited for here.
 int h2d_owned(hl_ctx* c, void* d, const void* h, size_t bytes) {
     int rc = h2d(c, d, h, bytes);
-    if (!rc && bytes > SMALL && !pageable(h)) rc = sync(c, "copy to device");
+    if (!rc && bytes > SMALL_UP && !pageable(h)) rc = sync(c, "copy to device");
     return rc;
 }
 
@@ -395,9 +430,8 @@ int d2h_on(hl_ctx* c, void* h, const void* d, size_t bytes, cudaStream_t s) {
     cudaError_t e;
     CopyRing* r;
     char* slot;
-    if (bytes <= SMALL && (slot = arena_slot(c, bytes)) != nullptr) {
-        e = cudaMemcpyAsync(slot, d, bytes, cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) c->pending.push_back({h, slot, bytes});
+    if (bytes <= SMALL_DOWN && (slot = bounce(c, c->down, bytes)) != nullptr) {
+        e = bounce_down(c, slot, (char*)h, (const char*)d, bytes, s);
     } else if (pageable(h) && (r = ring_of(c)) != nullptr) {
         e = ring_down(r, (char*)h, (const char*)d, bytes, s);
     } else {
@@ -414,14 +448,31 @@ int d2h_on(hl_ctx* c, void* h, const void* d, size_t bytes, cudaStream_t s) {
 
 int d2h(hl_ctx* c, void* h, const void* d, size_t bytes) { return d2h_on(c, h, d, bytes, c->stream); }
 
+// hands the results in the bounce area out, each piece when it has arrived, and waits for the stream
 int sync(hl_ctx* c, const char* what) {
-    cudaError_t e = cudaStreamSynchronize(c->stream);
-    if (e == cudaSuccess)
-        for (const auto& p : c->pending) memcpy(p.to, p.from, p.bytes);
-    c->pending.clear();
-    c->arena_off = 0;
+    cudaError_t e = cudaSuccess;
+    bool through = false;  // the stream has been waited for
+    for (const auto& p : c->pending) {
+        if (!through) {
+            e = p.ev ? cudaEventSynchronize(p.ev) : cudaStreamSynchronize(c->stream);
+            through = !p.ev;
+        }
+        if (e != cudaSuccess) break;
+        memcpy(p.to, p.from, p.bytes);
+    }
+    if (!through && e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    if (c->up_elsewhere && e == cudaSuccess) e = cudaStreamSynchronize(c->copy_stream);  // it reads the upload area too
+    c->up_elsewhere = false;
+    drop_pending(c);
+    c->up.off = c->down.off = 0;
     if (e != cudaSuccess) return fail(c, HL_B200_ERR_DEVICE, what, e);
     return HL_B200_OK;
+}
+
+void drop_pending(hl_ctx* c) {
+    for (const auto& p : c->pending)
+        if (p.ev) c->ev_spare.push_back(p.ev);
+    c->pending.clear();
 }
 
 }  // namespace hlapi

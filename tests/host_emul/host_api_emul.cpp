@@ -138,7 +138,7 @@ static void failures(bool lock) {
 static void sizes() {
     hl_ctx* c = nullptr;
     hl_b200_init(0, &c);
-    for (const size_t n : {1, 7, 8191, 8192, 8193, 16384, 16385, 21845, 21846, 32769, 43691, 65536, 65537, 100001, 3000001}) {
+    for (const size_t n : {1, 7, 8191, 8192, 8193, 16384, 16385, 21845, 32768, 32769, 43691, 49152, 49153, 65537, 100001, 3000001}) {
         std::vector<uint64_t> a(n + 8), b(n + 8), out(3 * n + 8);
         for (size_t i = 0; i < n + 8; i++) { a[i] = i * 0x9E3779B97F4A7C15ull; b[i] = ~a[i]; }
         for (size_t off = 0; off < (n > 1000000 ? 2u : 8u); off++) {
@@ -155,12 +155,35 @@ static void sizes() {
     hl_b200_shutdown(c);
 }
 
+// more small copies in one call than the bounce areas hold, on both streams in turn
+static void areas() {
+    hl_ctx* c = nullptr;
+    hl_b200_init(0, &c);
+    const size_t n = 40000, count = 50;
+    std::vector<uint64_t> a(n * count), out(n * count);
+    for (size_t i = 0; i < a.size(); i++) a[i] = i * 0x9E3779B97F4A7C15ull;
+    {
+        hlapi::Call g(c);
+        u64* d = nullptr;
+        int rc = hlapi::dev_alloc(c, (void**)&d, a.size() * 8);
+        for (size_t i = 0; i < count && !rc; i++) rc = hlapi::h2d_on(c, d + i * n, a.data() + i * n, n * 8, i % 3 ? c->copy_stream : c->stream);
+        cudaEventRecord(c->ev_main, c->copy_stream);
+        cudaStreamWaitEvent(c->stream, c->ev_main, 0);
+        for (size_t i = 0; i < count && !rc; i++) rc = hlapi::d2h_on(c, out.data() + i * n, d + i * n, n * 8, i % 3 ? c->stream : c->copy_stream);
+        if (!rc) rc = hlapi::sync(c, "areas");
+        hlapi::dev_free(c, d, a.size() * 8);
+        if (rc || a != out) bad("areas", "wrong bytes");
+    }
+    hl_b200_shutdown(c);
+}
+
 int main(int argc, char** argv) {
     if (argc == 3 && !strcmp(argv[1], "threads")) {
         g_threads = atol(argv[2]);
         sizes();
     } else if (argc == 2 && !strcmp(argv[1], "copies")) {
         sizes();
+        areas();
     } else {
         failures(false);
         failures(true);

@@ -18,7 +18,7 @@ def _words(n, seed):
     return np.random.default_rng(seed).integers(0, P, size=n, dtype=np.uint64)
 
 
-@pytest.mark.parametrize("n", [1, 8191, 8192, 8193, 24575, 24576, 24577, 131072, 131073, (1 << 20) + 5, (5 << 20) + 1])
+@pytest.mark.parametrize("n", [1, 8191, 8192, 8193, 16384, 16385, 32768, 32769, 49152, 49153, 24575, 24576, 24577, 131072, 131073, (1 << 20) + 5, (5 << 20) + 1])
 @pytest.mark.parametrize("locked", [False, True])
 def test_round_trip(n, locked):
     import torch
