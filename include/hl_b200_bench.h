@@ -1,6 +1,6 @@
-/* hl_b200_bench.h - measurement aids of the benchmark, exported by the same library but NOT part of the backend's interface.
+/* hl_b200_bench.h - measurement and test aids, exported by the same library but NOT part of the backend's interface.
  *
- * Nothing here has a counterpart in the reference and no prover calls it: bench.py uses these to put a measured integer
+ * Nothing here has a counterpart in the reference and no prover calls it: bench.py uses the first two to put a measured integer
  * ceiling beside the encoder and the column hash (the kernels are bound by integer issue, for which the machine has no
  * published peak).
  */
@@ -20,6 +20,9 @@ int hl_b200_compress_peak(hl_ctx* ctx, uint32_t iters, double* compressions_per_
 /* A/B switch of the sumcheck kernels' programmatic dependent launch (process-wide, on by default): with 0 every kernel of a
  * sumcheck is an ordinary stream launch again.  For measuring what the chained launch saves. */
 int hl_b200_set_dependent_launch(int on);
+/* How often the CTAs of the one-launch rounds of a sumcheck look for a round's sums and for its challenge before they give up (4,194,304
+ * each: some seconds).  A test makes a wait run out with a small number and sees HL_B200_ERR_TIMEOUT. */
+int hl_b200_set_wait_limits(hl_ctx* ctx, uint32_t sums, uint32_t challenge);
 
 #ifdef __cplusplus
 }

@@ -11,6 +11,7 @@
 
 #include "../../include/hl_b200.h"
 #include "kernels.h"
+#include "sumcheck.h"
 
 namespace hlapi { struct CopyRing; }
 
@@ -30,6 +31,7 @@ struct hl_ctx {
     std::string label, last_error;
     hl_stats stats{};
     bool timing = false;
+    hlk::ScWaits waits;      // of the sumchecks' resident CTAs
     struct Span { cudaEvent_t a, b; int cls; };
     std::vector<Span> spans;          // recorded, not yet read
     std::vector<cudaEvent_t> ev_pool;  // events ready for reuse

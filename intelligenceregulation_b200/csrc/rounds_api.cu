@@ -47,6 +47,7 @@ struct hl_rounds {
     u64* d_cfo = nullptr;      // its coefficients by occurrence
     u64* d_nonbase = nullptr;  // one word: bit t set when table t is extension-valued before the first fold
     u64 nonbase = ~0ull;
+    int failed = 0;            // the status of a batch that failed on the way: the tables are between two rounds, nothing goes on from there
     size_t out_row() const { return (2 * ((size_t)degree + 1) + 1) * 2; }
 };
 
@@ -60,6 +61,8 @@ void free_rounds(hl_rounds* r) {
     if (r->d_nonbase) dev_free(c, r->d_nonbase, 8);
     delete r;
 }
+
+int spent(hl_rounds* r) { return fail(r->ctx, r->failed, "rounds: an earlier batch of this evaluator failed"); }
 
 // What every round of a batch takes its step with; a plain round() leaves it as it is made.
 struct StepPlan {
@@ -332,6 +335,7 @@ void hl_b200_rounds_free(hl_rounds* r) {
 int hl_b200_rounds_round(hl_rounds* r, uint32_t j, int eval_one, uint64_t* sums) {
     if (!r || !sums) return HL_B200_ERR_ARG;
     hl_ctx* c = r->ctx;
+    if (r->failed) return spent(r);
     if (j != r->next || j >= r->n_vars) return fail(c, HL_B200_ERR_ARG, "rounds_round: round order (a round needs the preceding fold)");
     Call g(c);
     int rc;
@@ -347,6 +351,7 @@ int hl_b200_rounds_round(hl_rounds* r, uint32_t j, int eval_one, uint64_t* sums)
 int hl_b200_rounds_fold(hl_rounds* r, const uint64_t rr[2]) {
     if (!r || !rr) return HL_B200_ERR_ARG;
     hl_ctx* c = r->ctx;
+    if (r->failed) return spent(r);
     if (r->next >= r->n_vars) return fail(c, HL_B200_ERR_ARG, "rounds_fold: every variable is already folded");
     Call g(c);
     int rc = h2d(c, (char*)r->d_state + offsetof(hlk::ScState, r), rr, 16);
@@ -361,6 +366,7 @@ int hl_b200_rounds_fold(hl_rounds* r, const uint64_t rr[2]) {
 int hl_b200_rounds_finals(hl_rounds* r, uint64_t* out) {
     if (!r || !out) return HL_B200_ERR_ARG;
     hl_ctx* c = r->ctx;
+    if (r->failed) return spent(r);
     if (r->next != r->n_vars) return fail(c, HL_B200_ERR_ARG, "rounds_finals: finals need all folds");
     Call g(c);
     if (r->finals.empty()) {
@@ -381,11 +387,20 @@ int hl_b200_set_dependent_launch(int on) {
     return HL_B200_OK;
 }
 
+int hl_b200_set_wait_limits(hl_ctx* c, uint32_t sums, uint32_t challenge) {
+    if (!c) return HL_B200_ERR_ARG;
+    Call g(c);
+    c->waits.sums = sums;
+    c->waits.challenge = challenge;
+    return HL_B200_OK;
+}
+
 int hl_b200_rounds_batched(hl_rounds* r, uint32_t nd, hl_fs_state* fs, const uint64_t* mask_coeffs, uint32_t mask_vars,
                            const uint64_t mask_c[2], uint64_t* out) {
     if (!r || !fs || !out) return HL_B200_ERR_ARG;
     hl_ctx* c = r->ctx;
     if (nd == 0) return HL_B200_OK;
+    if (r->failed) return spent(r);
     if (r->next + nd > r->n_vars) return fail(c, HL_B200_ERR_ARG, "rounds_batched: more rounds than variables left");
     if (mask_coeffs && (r->next != 0 || !mask_c || mask_vars < r->n_vars || mask_vars > 63))
         return fail(c, HL_B200_ERR_ARG, "rounds_batched: a masked batch starts at round 0 and its mask covers every variable");
@@ -456,7 +471,7 @@ int hl_b200_rounds_batched(hl_rounds* r, uint32_t nd, hl_fs_state* fs, const uin
         if (!rc && i < nd) {  // the short rounds: one launch (sumcheck_run.cu)
             const u32 left = nd - i;
             cudaError_t e = hlk::sc_run(r->poly, r->ir, (int)r->k, r->d_tables, r->stride, (u32)r->len, r->d_coefs, step_of(r, r->next, 1, 0, plan), (int)left,
-                                        have_claim ? 1 : 0, r->d_sync, r->d_slots, r->d_other, c->sm_count, c->stream);
+                                        have_claim ? 1 : 0, r->d_sync, c->waits, r->d_slots, r->d_other, c->sm_count, c->stream);
             c->stats.kernel_launches++;
             if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "short rounds launch", e);
             r->len >>= left;
@@ -473,10 +488,10 @@ int hl_b200_rounds_batched(hl_rounds* r, uint32_t nd, hl_fs_state* fs, const uin
     std::vector<char> got(o_fin + r->k * 16);
     if (!rc) rc = d2h(c, got.data(), r->d_state, last ? got.size() : o_fin);
     if (!rc) rc = sync(c, "rounds_batched");
-    if (rc) return rc;
     hlk::ScSync sync_got;
     memcpy(&sync_got, got.data() + ((char*)r->d_sync - (char*)r->d_state), sizeof sync_got);
-    if (sync_got.failed) return fail(c, HL_B200_ERR_TIMEOUT, "rounds_batched: a device wait ran out");
+    if (!rc && sync_got.failed) rc = fail(c, HL_B200_ERR_TIMEOUT, "rounds_batched: a device wait ran out");
+    if (rc) return r->failed = rc;
     memcpy(out, got.data() + o_out + first * r->out_row() * 8, (size_t)nd * r->out_row() * 8);
     memcpy(&st, got.data(), sizeof st);
     if (last) {

@@ -67,6 +67,11 @@ struct ScSync {
     u64 sums[2][SC_MAX_POINTS][4];
 };
 
+// How often the CTAs of k_sc_run look for something before they give up: CTA 0 for a round's sums, the others for its challenge.
+struct ScWaits {
+    u32 sums = 1u << 22, challenge = 1u << 22;  // some seconds
+};
+
 void sc_set_dependent_launch(bool on);
 bool sc_dependent_launch();
 u32 sc_round_blocks(u32 half, int sm_count);
@@ -80,7 +85,7 @@ u32 sc_run_len(int poly, const IrDev& p);
 size_t sc_run_other_bytes(int k, u32 len);
 size_t sc_run_slot_bytes(int poly, const IrDev& p, int k, int eval_degree, int sm_count);
 cudaError_t sc_run(int poly, const IrDev& p, int k, u64* tables, size_t stride, u32 len, const u64* coefs, const ScStep& a, int nrounds, int have_claim,
-                   ScSync* sync, u64* slots, u64* other, int sm_count, cudaStream_t s);
+                   ScSync* sync, const ScWaits& waits, u64* slots, u64* other, int sm_count, cudaStream_t s);
 bool sc_supported(int poly, int k, int degree);
 // A round's sums and, by the CTA that finishes last, its step (sync: zero, and left ready for the next round)
 cudaError_t sc_round(int poly, int k, const u64* tables, size_t stride, u32 half, const u64* coefs, int eval_one, const ScStep& step, ScSync* sync,

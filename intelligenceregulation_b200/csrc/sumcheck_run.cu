@@ -11,7 +11,7 @@
 //   shrinking   a round with fewer units than CTAs lets the others go; once a single CTA is left it keeps the tables in shared memory
 //   the step    has a warp of its own, which prepares the mask before the sums arrive and updates the claim while the others fold and
 //               evaluate (sc_step.cuh): a round of two pairs is 5.5 k cycles of hashing and 4 k of everything else
-// Every wait is bounded: a CTA that waits too long records it and leaves, and the call returns HL_B200_ERR_TIMEOUT.
+// Every wait is bounded: a CTA that waits too long records it for the host and leaves, and the call returns HL_B200_ERR_TIMEOUT.
 #include "sc_poly.cuh"
 #include "sc_step.cuh"
 #include "slot_vm.cuh"
@@ -25,7 +25,6 @@ __device__ __forceinline__ u32 ld_acquire(const u32* p) {
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
-constexpr u32 POLL_LIMIT = 1u << 22;  // polls of one wait: some seconds
 constexpr u32 FLAG_FAILED = 0xFFFFFFFFu;
 
 struct RunArgs {
@@ -37,6 +36,7 @@ struct RunArgs {
     int have_claim;      // the first round's claim is known
     hlk::ScStep step;    // step.round: the first round's number
     hlk::ScSync* sync;   // zero at the launch
+    hlk::ScWaits waits;
 };
 
 // Shared memory: [evaluator's own][table chunk][its successor, half as long], the two swapping roles once one CTA is left.
@@ -204,9 +204,16 @@ __global__ void __launch_bounds__(RUN_MAX_T + 32) k_sc_run(RunArgs a, Eval ev) {
         if (!first) {
             if (tid == 0) {
                 u32 f = 0;
-                for (u32 n = 0; n < POLL_LIMIT && (f = ld_acquire(&a.sync->flag)) < rd + 1; n++) {}
-                if (f < rd + 1 || f == FLAG_FAILED) failed_s = 1;
-                else r_s = ld2(a.sync->r[rd & 1]);
+                for (u32 n = 0; n < a.waits.challenge && (f = ld_acquire(&a.sync->flag)) < rd + 1; n++) {}
+                if (f < rd + 1) {  // ran out: our entries stay unfolded, also when CTA 0 has nothing more to wait for
+                    failed_s = 1;
+                    a.sync->failed = 1;
+                    st_release(&a.sync->flag, FLAG_FAILED);
+                } else if (f == FLAG_FAILED) {
+                    failed_s = 1;
+                } else {
+                    r_s = ld2(a.sync->r[rd & 1]);
+                }
             }
             bar_workers(T);
             if (failed_s) return false;
@@ -329,8 +336,8 @@ __global__ void __launch_bounds__(RUN_MAX_T + 32) k_sc_run(RunArgs a, Eval ev) {
             if (ncta > 1) {
                 if (tid == 0) {
                     u32 n = 0;
-                    while (n < POLL_LIMIT && ld_acquire(&a.sync->arrived) < arrived) n++;
-                    if (n == POLL_LIMIT) {
+                    while (n < a.waits.sums && ld_acquire(&a.sync->arrived) < arrived) n++;
+                    if (n == a.waits.sums) {
                         failed_s = 1;
                         a.sync->failed = 1;
                         st_release(&a.sync->flag, FLAG_FAILED);
@@ -454,8 +461,9 @@ size_t sc_run_slot_bytes(int poly, const IrDev& p, int k, int eval_degree, int s
 }
 
 cudaError_t sc_run(int poly, const IrDev& p, int k, u64* tables, size_t stride, u32 len, const u64* coefs, const ScStep& step, int nrounds, int have_claim,
-                   ScSync* sync, u64* slots, u64* other, int sm_count, cudaStream_t st) {
+                   ScSync* sync, const ScWaits& waits, u64* slots, u64* other, int sm_count, cudaStream_t st) {
     RunArgs a;
+    a.waits = waits;
     a.tables = tables; a.other = other; a.stride = stride; a.len = len; a.k = (u32)k; a.nrounds = (u32)nrounds;
     a.have_claim = have_claim; a.step = step; a.sync = sync;
     const RunShape sh = run_shape(poly, p, k, step.eval_degree);

@@ -62,3 +62,37 @@ def test_programs(ctx, oracle, nodes, n, batches):
     c = p.coef_array()
     oracle.ir_set(p.words(), p.n_nodes, p.n_terms)
     _check(ctx, oracle, oracle.POLY_IR, tables, 3, n, batches, what=p, coefs=c if c.size else None)
+
+
+@pytest.mark.parametrize("limits,nd", [((0, 1 << 22), 13), ((1 << 12, 0), 13), ((1 << 12, 0), 1), ((1 << 12, 0), 2)])
+@pytest.mark.parametrize("parts", [False, True])
+def test_a_wait_that_runs_out_is_reported(ctx, oracle, limits, nd, parts):
+    """CTA 0's wait for a round's sums, or the others' for a challenge: in the middle of a batch, and for the last challenge of one that ends
+    before the last round, when CTA 0 has gone.  The evaluator then answers nothing but that status; the context goes on."""
+    from intelligenceregulation_b200 import backend
+
+    n, k, deg = 13, 4, 3
+    what = _program(oracle, 30) if parts else backend.POLY_ZC
+    tables = oracle.ZkRng(n, b"sc-run-wait").fp2_vec(k << n).reshape(k, 1 << n, 2)
+    if parts:
+        n, tables = 11, np.ascontiguousarray(tables[:, : 1 << 11])
+        nd = min(nd, n)
+    tr = oracle.Transcript(b"sc-run-wait")
+    ev = backend.B200Rounds(ctx, what, tables, deg)
+    ctx.check(ctx.lib.hl_b200_set_wait_limits(ctx.h, *limits))
+    try:
+        with pytest.raises(backend.DeviceError) as e:
+            ev.batched(nd, tr.state, tr.counter, None)
+        assert e.value.code == -4 and "wait" in str(e.value)
+        for again in (ev.finals, lambda: ev.batched(1, tr.state, tr.counter, None), lambda: ev.round(0), lambda: ev.fold((1, 2))):
+            with pytest.raises(backend.DeviceError) as e:
+                again()
+            assert e.value.code == -4
+        ev.free()
+    finally:
+        ctx.check(ctx.lib.hl_b200_set_wait_limits(ctx.h, 1 << 22, 1 << 22))
+    c = None
+    if parts:
+        c = what.coef_array()
+        oracle.ir_set(what.words(), what.n_nodes, what.n_terms)
+    _check(ctx, oracle, oracle.POLY_IR if parts else oracle.POLY_ZC, tables, deg, n, [n], what=what if parts else None, coefs=c)
