@@ -717,17 +717,18 @@ class SlotProgram:
         self.n_terms += 1
 
     def _arrays(self):
-        """(words, coefficients) as the C ABI takes them; a program only grows, so its sizes tell whether they still hold"""
-        now = (len(self._words), len(self.coefs))
-        if self._flat is None or self._flat[0] != now:
-            self._flat = now, np.array(self._words, dtype=np.uint32), np.array(self.coefs, dtype=np.uint64).reshape(-1, 2)
-        return self._flat[1:]
+        """(words, coefficients) as the C ABI takes them.  The words only grow; the coefficients may be replaced in place, as a challenge is
+        between two proofs, so they are taken as they are now (40 of them: 5 us)."""
+        if self._flat is None or self._flat.size != len(self._words):
+            self._flat = np.array(self._words, dtype=np.uint32)
+        cf = np.fromiter((x for c in self.coefs for x in c), dtype=np.uint64, count=2 * len(self.coefs)).reshape(-1, 2)
+        return self._flat, cf
 
     def words(self) -> np.ndarray:
         return self._arrays()[0].copy()
 
     def coef_array(self) -> np.ndarray:
-        return self._arrays()[1].copy()
+        return self._arrays()[1]
 
 
 class B200Rounds:

@@ -116,3 +116,19 @@ def test_every_node_uses_the_one_before_twice(emul, nodes):
         desc["terms"].append((c, [t, SP.node(prev)]))
     info = _within(60, lambda: _check(emul, prog, desc, 2, nodes))
     assert info[3] == 1
+
+
+def test_a_coefficient_replaced_in_place_counts():
+    from intelligenceregulation_b200 import backend
+
+    SP = backend.SlotProgram
+    prog = SP(2)
+    prog.term((5, 7), [0], [1])
+    prog.term((11, 0), [], [0])
+    w, cf = prog.words(), prog.coef_array()
+    assert cf.tolist() == [[5, 7], [11, 0]]
+    prog.coefs[0] = (1 << 63, 3)
+    assert prog.coef_array().tolist() == [[1 << 63, 3], [11, 0]] and prog._arrays()[1].tolist() == [[1 << 63, 3], [11, 0]]
+    assert (prog.words() == w).all()
+    prog.term((13, 0), [1], [])
+    assert prog.coef_array().tolist() == [[1 << 63, 3], [11, 0], [13, 0]] and prog.words().size > w.size
