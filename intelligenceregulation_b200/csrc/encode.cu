@@ -133,16 +133,23 @@ size_t encode_scratch_words(u32 logn, u32 T, int sm_count, u32 rows) {
 }
 
 // How many (row, residue) CTAs a launch of split rows takes at once: one per SM, or half of those that an SM holds where a CTA is far from
-// filling one (two of 256 threads take 1.2 times the time of one, four of them 2)
+// filling one
 size_t encode_split_units(u32 logn, int sm_count) {
     const u32 t = logn > 9 ? 1u << (logn - 4) : 32u;
     return (size_t)sm_count * (t > 512 ? 1 : 512 / t);
 }
-// Splitting rows by residue repeats their inverse transform: 2 transforms a CTA instead of 1 + R, R times the CTAs.  It pays when it
-// takes fewer turns of the machine (40 rows of 2^16 540 -> 386 us, 60 of 2^15 at rate 1/4 494 -> 410, 200 of 2^10 at rate 1/4 51 -> 29).
+// Splitting rows by residue repeats their inverse transform: 2 transforms a CTA instead of 1 + R, R times the CTAs.
+// Where a CTA has an SM to itself (2^13 words and more) a turn of the machine takes as long as a lone CTA, and splitting pays when it takes
+// fewer turns' transforms (38 rows of 2^14 103 -> 75 us, 74 of them 103 -> 74, 100 of them 103 -> 140; at rate 1/4 74
+// rows 189 -> 152, 100 rows 189 -> 224).  Smaller CTAs share an SM, and a full turn takes twice a lone CTA's time, in proportion to the
+// CTAs above that (measured for 2^8 .. 2^12 words at rates 1/2, 1/4, 1/8, and masks up to rate 1/64, as CTAs over the turn's CTAs where
+// both ways take the same time: 0.75 - 1, 1.1 - 1.4, 2 - 2.5, 16; the line: 0.75, 1.25, 2.25, 16.25).  296 rows of 2^11 at rate 1/4 62 -> 87 us
+// when split, 148 of them 58 -> 41.
 bool encode_split_pays(u32 logn, u32 logR, u32 rows, int sm_count) {
-    const u64 at_once = encode_split_units(logn, sm_count), units = (u64)rows << logR;
-    return logR >= 1 && (units + at_once - 1) / at_once * 2 < (rows + at_once - 1) / at_once * (1 + ((u64)1 << logR));
+    const u64 at_once = encode_split_units(logn, sm_count), units = (u64)rows << logR, whole = 1 + ((u64)1 << logR);
+    if (logR < 1) return false;
+    if (at_once > (u64)sm_count) return units * 4 < at_once * whole;
+    return (units + at_once - 1) / at_once * 2 < (rows + at_once - 1) / at_once * whole;
 }
 
 cudaError_t encode_rows(const enc::RowArgs& a, u32 logn, bool allow_fast, int sm_count, size_t scratch_words,

@@ -137,15 +137,16 @@ int hl_b200_mask_commit(hl_ctx* c, uint32_t log_msg, uint32_t log_dom, const uin
     u64 *d_msgs = nullptr, *d_pows = nullptr, *scratch = nullptr;
     uint32_t* d_key = nullptr;
     const u64* tw = nullptr;
-    // A block's masking commitment is some fifty rows of eight or more short transforms each: one CTA (a warp, at these sizes) per (row,
-    // residue), repeating the row's inverse transform, instead of one per row (24 masks: 219 us before, 45 us), while that fills the SMs
-    // no more than sixteen deep.
+    // A block's masking commitment is some fifty rows of eight or more short transforms each: by the encoder's rule one CTA (a warp, at
+    // these sizes) per (row, residue), repeating the row's inverse transform, instead of one per row (24 masks: 186 us before, 50 us).
     const u32 logr = log_dom - log_msg;
-    const size_t deep = (size_t)c->sm_count * 16;
-    const bool split_msg = (n_msg_rows << logr) <= deep, split_coef = (n_coef_rows << logr) <= deep;
-    size_t scratch_words = hlk::encode_scratch_words(log_msg, 2, c->sm_count, (u32)rows);
-    if (split_msg && (n_msg_rows << logr) * m > scratch_words) scratch_words = (n_msg_rows << logr) * m;
-    if (split_coef && (n_coef_rows << logr) * m2 > scratch_words) scratch_words = (n_coef_rows << logr) * m2;
+    const bool split_msg = hlk::encode_split_pays(log_msg, logr, (u32)n_msg_rows, c->sm_count), split_coef = hlk::encode_split_pays(log_msg, logr, (u32)n_coef_rows, c->sm_count);
+    auto words_of = [&](bool split, size_t n_rows, size_t per_cta) {  // scratch for the largest grid of a launch, 32 CTAs an SM
+        const size_t ctas = split ? n_rows << logr : n_rows, most = (size_t)c->sm_count * 32;
+        return (ctas < most ? ctas : most) * per_cta;
+    };
+    const size_t msg_words = words_of(split_msg, n_msg_rows, m), coef_words = words_of(split_coef, n_coef_rows, m2);
+    const size_t scratch_words = msg_words > coef_words ? msg_words : coef_words;
     int rc = root_powers(c, log_dom, &tw);
     if (!rc) rc = dev_alloc(c, (void**)&st->d_data, rows * m2 * 8);
     if (!rc) rc = dev_alloc(c, (void**)&st->d_enc, rows * dom * 8);

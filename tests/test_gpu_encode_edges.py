@@ -18,7 +18,8 @@ def dev():
 
 CASES = [(n, 2, rows, 33) for n in range(8, 15) for rows in (1, 74, 75)]
 CASES += [(9, 4, 38, 600), (14, 1, 2, 0), (15, 1, 2, 0), (16, 1, 1, 0), (15, 2, 3, 1), (16, 4, 1, 150000)]
-CASES += [(12, 2, 148, 5), (12, 2, 149, 5), (10, 4, 297, 5), (15, 2, 75, 70000 // 4), (15, 2, 149, 40)]  # where a row's residues stop being apart
+CASES += [(12, 2, 148, 5), (12, 2, 149, 5), (10, 4, 297, 5), (15, 2, 75, 70000 // 4), (15, 2, 149, 40)]
+CASES += [(12, 2, 110, 5), (12, 2, 111, 5), (11, 4, 184, 5), (11, 4, 185, 5), (10, 8, 332, 5), (10, 8, 333, 5), (8, 2, 887, 5), (8, 2, 888, 5)]  # where a row's residues stop being apart
 
 
 @pytest.mark.parametrize("log_cols,inv_rate,rows,q", CASES)

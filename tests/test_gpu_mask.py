@@ -33,6 +33,7 @@ def _functionals(o, mc, specs, count, seed):
 @pytest.mark.parametrize("specs,log_msg,log_dom,q", [
     ([(5, 3), (9, 2), (7, 5)], 9, 12, 256),                               # the reference's constants (zk.rs:391-393)
     ([(21, 3)] * 12 + [(19, 5)] * 8 + [(14, 2)] * 4, 9, 12, 256),         # 24 masks: a block's 52 rows
+    ([(4, 2)] * 166, 10, 13, 64), ([(4, 2)] * 167, 10, 13, 64),            # where a row's residues stop being apart
     ([(3, 2)], 8, 9, 100), ([(20, 4), (22, 7)], 10, 13, 256), ([(30, 6)] * 3, 11, 17, 512),
 ])
 def test_commit_and_open(ctx, oracle, specs, log_msg, log_dom, q):
