@@ -26,6 +26,7 @@ namespace ir {
 constexpr u32 IR_AFFINE = 0, IR_SUM = 1;
 constexpr u32 IR_NODE = 0x80000000u;
 constexpr u32 IR_ONE = 0xFFFFFFFFu, IR_NEG_ONE = 0xFFFFFFFEu, IR_ZERO = 0xFFFFFFFDu;
+constexpr u32 MAX_DEGREE = 1u << 20;  // degrees are counted up to here (64 factors of it do not wrap)
 constexpr u32 MAX_TABLES = 64, MAX_NODES = 128, MAX_WORDS = 4096, MAX_COEFS = 512;
 
 struct Shape {
@@ -212,6 +213,7 @@ inline u32 attained_degree(const Shape& s, const u32* w) {
         const u32 nf = w[pc + 1];
         u32 d = 0;
         for (u32 i = 0; i < nf; i++) d += (w[pc + 2 + i] & IR_NODE) ? deg[w[pc + 2 + i] & ~IR_NODE] : 1u;
+        if (d > MAX_DEGREE) d = MAX_DEGREE;  // a chain of products of the node before with itself doubles it per node
         pc += 2 + nf;
         return d;
     };

@@ -132,3 +132,21 @@ def test_a_coefficient_replaced_in_place_counts():
     assert (prog.words() == w).all()
     prog.term((13, 0), [1], [])
     assert prog.coef_array().tolist() == [[1 << 63, 3], [11, 0], [13, 0]] and prog.words().size > w.size
+
+
+@pytest.mark.parametrize("nodes", [2, 31, 32, 33, 120])
+def test_degrees_that_double_per_node_do_not_wrap(emul, nodes):
+    from intelligenceregulation_b200 import backend
+
+    SP = backend.SlotProgram
+    prog = SP(1)
+    prev = prog.affine((3, 0), [((5, 0), 0)])
+    for _ in range(nodes):
+        prev = prog.sum([((7, 1), [SP.node(prev), SP.node(prev)])])
+    prog.term(SP.ONE, [], [SP.node(prev)])
+    w, cf, info = prog.words(), prog.coef_array(), np.zeros(4, dtype=np.uint32)
+    tab, out = np.ones((1, 2), dtype=np.uint64), np.zeros((1, 2), dtype=np.uint64)
+    _within(60, lambda: [emul.emul_vm(w.ctypes.data_as(C.c_void_p), w.size, 1, prog.n_nodes, prog.n_terms, cf.ctypes.data_as(C.c_void_p), cf.shape[0],
+                                      tab.ctypes.data_as(C.c_void_p), tab.ctypes.data_as(C.c_void_p), 1, 0, 0, 1, out.ctypes.data_as(C.c_void_p),
+                                      info.ctypes.data_as(C.c_void_p))])
+    assert info[3] == min(2 ** nodes, 1 << 20)
