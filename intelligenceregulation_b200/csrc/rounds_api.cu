@@ -119,15 +119,6 @@ int launch_fold(hl_rounds* r) {
     return HL_B200_OK;
 }
 
-}  // namespace
-
-extern "C" {
-
-}  // extern "C"
-
-namespace {
-
-// the evaluator of either kind; `words` is the data form of the polynomial when poly == POLY_IR
 // A program of more than a dozen instructions is also cut into parts of about that many, for the rounds with few pairs.
 void compile(vm::Compiler& prog, const ir::Shape& sh, const uint32_t* words, const uint64_t* coefs) {
     const fp2* cf = reinterpret_cast<const fp2*>(coefs);
@@ -141,6 +132,7 @@ struct GenAsk {  // a slot program's generated kernel, looked up by the caller
     std::vector<fp2> cfo;
 };
 
+// the evaluator of either kind; `program` when poly == POLY_IR
 int rounds_build(hl_ctx* c, int poly, size_t k, uint32_t n_vars, uint32_t degree, const uint64_t* tables, const uint64_t* coefs,
                  size_t ncoefs, const vm::Program* program, hl_rounds** out, hl_tables* built = nullptr, const GenAsk* gen = nullptr) {
     Call g(c);

@@ -5,7 +5,7 @@
 //   * every value has a static type, base field or extension field, so no product tests its operands;
 //   * a sum of products is accumulated unreduced in 192 bits and reduced once;
 //   * table values are loaded where they are first used, so the live set is what the compiler can keep in registers.
-// A graph the generator has not seen runs through the interpreter (slot_ir.cuh); both return the reference's words,
+// A graph the generator has not seen runs through its program (slot_vm.cuh); both return the reference's words,
 // because field arithmetic is exact and the results are canonical.
 #pragma once
 #include "gl_field.cuh"

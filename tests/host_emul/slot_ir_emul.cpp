@@ -1,6 +1,6 @@
-// Runs the product's slot-polynomial interpreter and its program check (csrc/slot_ir.cuh) on the host,
-// so that the CPU test suite compares them with the oracle without a device.
-#include "../../intelligenceregulation_b200/csrc/slot_ir.cuh"
+// Runs the product's program check (csrc/slot_ir.cuh) and the tests' two evaluators of its word stream (slot_plan.h) on the host, so that the
+// CPU test suite compares them with the oracle without a device.
+#include "slot_plan.h"
 
 extern "C" int emul_ir_validate(const u32* words, u32 n_words, u32 n_tables, u32 n_nodes, u32 n_terms, u32 n_coefs) {
     ir::Shape s{n_tables, n_nodes, n_terms, n_coefs, n_words};

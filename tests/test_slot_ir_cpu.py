@@ -1,7 +1,7 @@
 """Slot polynomials as data, without a device: the structural fixture of the reference's 23 slot graphs is
 well formed, the oracle's interpreter (slot_ir.rs:352-377 restated in C) agrees with a pure-Python evaluation
-and with the closed-form families, and the product's interpreter and program check, compiled for the host,
-agree with the oracle.  Field work: bit-exact."""
+and with the closed-form families, and the product's program check with two evaluators of its word stream, compiled
+for the host, agree with the oracle.  Field work: bit-exact."""
 import ctypes as C
 import os
 import subprocess
@@ -19,7 +19,8 @@ def emul():
     src = os.path.join(ROOT, "tests", "host_emul", "slot_ir_emul.cpp")
     so = os.path.join(ROOT, "tests", "host_emul", "libslot_ir_emul.so")
     core = os.path.join(ROOT, "intelligenceregulation_b200", "csrc", "slot_ir.cuh")
-    if not os.path.exists(so) or max(os.path.getmtime(src), os.path.getmtime(core)) > os.path.getmtime(so):
+    plan = os.path.join(ROOT, "tests", "host_emul", "slot_plan.h")
+    if not os.path.exists(so) or max(os.path.getmtime(f) for f in (src, core, plan)) > os.path.getmtime(so):
         subprocess.check_call(["/usr/bin/g++", "-std=c++17", "-O2", "-shared", "-fPIC", "-o", so, src])
     return C.CDLL(so)
 
