@@ -446,9 +446,14 @@ cudaError_t launch_run(const RunArgs& a, const Eval& ev, const RunShape& sh, int
 
 namespace hlk {
 
-// From which length on a round is better off here than with launches of its own (a closed form over 2^21 points: from 2^14 entries 380 us,
-// 2^16 356, 2^18 351, all rounds 421; a short program over 2^14: 194 us from the start, 205 from 2^12; the width check's 246 instructions
-// over 2^19: from 2^14 2,311 us, 2^12 2,212, 2^11 2,185, 2^10 2,182: one point per thread costs a long program a third more).
+// From which length on a round is better off here than with launches of its own: one evaluation point per thread costs a long program a
+// third more, a launch costs a short one.  Whole sumchecks of the closed forms (products of two and six tables, the zero check, both LogUp
+// checks) over 2^14 .. 2^21 entries and of the 23 recorded programs over 2^12 .. 2^20, from 2^8 .. 2^21 entries on, in us:
+//   closed forms           2^18 is the best or within 2 % of it (LogUp over 2^21: 2^14 395, 2^16 376, 2^18 369, 2^20 395)
+//   24 instructions        2^13 .. 2^15 within 2 % of one another (over 2^18: 2^11 377, 2^14 365, 2^16 389)
+//   3 to 8 instructions    2^14 within 9 % of the best, which is 2^15 or 2^16 (5 over 2^20: 2^11 384, 2^14 372, 2^16 362; 3 over 2^18: 215, 211, 201)
+//   59 and more            2^11 within 2 % of the best (59 over 2^16: 347, 2^14 381, 2^16 480; 246 over 2^18: 1,399, 1,531, 1,938)
+// The code's length counts the program and its parts: 54 words for those 24 instructions, 125 for the 59.
 constexpr u32 RUN_SHORT_CODE = 64;
 u32 sc_run_len(int poly, const IrDev& p) { return poly != POLY_IR ? 1u << 18 : p.n_code <= RUN_SHORT_CODE ? 1u << 14 : 1u << 11; }
 
