@@ -28,9 +28,8 @@ def _n_vars(slot):
     return 13 if k <= 5 else 11 if k <= 25 else 10
 
 
-# every slot at a size that runs the point form, the warp form and the single-CTA tail; three slots at sizes whose first
-# rounds have more pairs than the machine has threads (the pair form); the D zero-check at its 8B size of 2^19 points and the
-# softmax zero-check at 2^20, the sizes the benchmark times
+# every slot at a size that the one launch takes (or nearly); three slots at sizes whose first rounds have launches of their own; the D
+# zero-check at its 8B size of 2^19 points and the softmax zero-check at 2^20, the sizes the benchmark times
 CASES = [(i, None) for i in range(23)] + [(14, 16), (3, 17), (5, 16), (14, 19), (17, 20)]
 
 
@@ -83,7 +82,7 @@ def test_every_known_graph_has_its_generated_kernel(ctx, oracle, golden_dir):
     o = oracle
     progs = [(U.build_program(backend, s, 7000 + i)[0], s["declared_degree"], len(s["table_fields"])) for i, s in enumerate(U.load_slots(golden_dir))]
     progs += [(l11_util.build_program(backend, s)[0], s["degree"], s["n_tabs"]) for s in l11_util.load(golden_dir)["slots"]]
-    n = 14  # above every program's one-CTA tail, so that at least two rounds run as grid launches
+    n = 14  # the generated rounds hand over to the one launch at 2^12 entries: two rounds run as grid launches
     for j, (prog, deg, k) in enumerate(progs):
         tables = o.ZkRng(600 + j, b"gen-any").fp2_vec(k << n).reshape(k, 1 << n, 2)  # every table extension-valued
         outs = []
@@ -98,11 +97,11 @@ def test_every_known_graph_has_its_generated_kernel(ctx, oracle, golden_dir):
     ctx.set_slot_kernels(False)
 
 
-def test_plan_beyond_the_all_points_form_runs_the_stepping_pair_form(ctx, oracle):
-    """A polynomial with more non-affine nodes than the all-points pair-per-thread kernel keeps (40) at 2^15 points: its long
-    rounds run the stepping form (`k_sc_round_irp`), which none of the recorded graphs reaches.  A chain of 44 sum nodes over
-    four tables, each node the product of the previous node's affine image and a table plus a second unit, so that every node
-    matters; compared with the oracle's masked prover word for word."""
+@pytest.mark.parametrize("chain", [False, True])
+def test_a_long_graph_at_a_size_with_long_rounds(ctx, oracle, chain):
+    """A polynomial of 44 sum nodes over four tables at 2^15 points: first the rounds with launches of their own (`k_sc_round_vm`), then the
+    one launch.  chain: every node is the node before times a constant plus a product, so that each of them matters, and some are used again at
+    the end; otherwise only the last four are, and the program drops the rest.  Compared with the oracle's masked prover word for word."""
     from intelligenceregulation_b200 import backend
 
     SP, o = backend.SlotProgram, oracle
@@ -112,10 +111,12 @@ def test_plan_beyond_the_all_points_form_runs_the_stepping_pair_form(ctx, oracle
     p = SP(4)
     a0 = p.affine(cf[0], [(cf[1], 1), (SP.NEG_ONE, 2)])
     prev = p.sum([(SP.ONE, [1, 2]), (cf[2], [3])])
-    for i in range(43):  # degree stays 2: each node is linear in the tables through one product of two affine-type factors
-        prev = p.sum([(cf[3 + i], [1 + (i % 3), SP.node(a0)]), (cf[50 + i], [1 + ((i + 1) % 3)]), (SP.ONE, [])] if i % 2 else
+    for i in range(43):  # degree stays 2
+        prev = p.sum([(cf[3 + i], [SP.node(prev)]), (cf[50 + i], [1 + i % 3, 1 + (i + 1) % 3])] if chain else
+                     [(cf[3 + i], [1 + (i % 3), SP.node(a0)]), (cf[50 + i], [1 + ((i + 1) % 3)]), (SP.ONE, [])] if i % 2 else
                      [(cf[3 + i], [2, 3]), (SP.NEG_ONE, [SP.node(a0)])])
-    mix = p.sum([(cf[90], [SP.node(prev)]), (cf[91], [SP.node(prev - 1)]), (cf[92], [SP.node(prev - 2)]), (cf[93], [SP.node(prev - 3)])])
+    back = (0, 7, 19, 40) if chain else (0, 1, 2, 3)
+    mix = p.sum([(cf[90 + j], [SP.node(prev - d)]) for j, d in enumerate(back)])
     p.term(SP.ONE, [0], [SP.node(mix)])
     tables = rng.fp2_vec(4 << n).reshape(4, 1 << n, 2)
     tables[2, :, 1] = 0
@@ -200,9 +201,8 @@ def test_l11_recorded_graphs_reach_the_reference_value_on_the_device(ctx, oracle
     """Each slot graph of the reference's real W16R2 block core, with its RECORDED coefficient values, evaluated by the device at
     the recorded terminal values `VALS`: the sums must be the reference's own `poly(vals)` (lean_l11_export_tests.rs:243,
     `RES`).  Three shapes per slot: one pair whose low entry is `VALS` (s(0) is the recorded value itself; s(1) is checked by
-    the independent Python walk), constant tables at a size that runs the warp form and the one-CTA tail (every s(d) is
-    2^(n-1) times the recorded value, and the finals after the folds are `VALS` again), and the same at 2^16 points, which
-    runs the pair-per-thread form."""
+    the independent Python walk), constant tables at a size that the one launch takes (every s(d) is 2^(n-1) times the recorded
+    value, and the finals after the folds are `VALS` again), and the same at 2^16 points, whose first rounds have launches of their own."""
     from intelligenceregulation_b200 import backend
     import l11_util
 
