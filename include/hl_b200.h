@@ -64,7 +64,7 @@ int hl_b200_set_alloc_cap(hl_ctx* ctx, size_t bytes);
  * register passes when 2^8 <= n <= 2^14 (default).  Same words either way. */
 int hl_b200_set_encoder(hl_ctx* ctx, int fast);
 /* Which evaluator runs a slot program whose graph the library has a generated kernel for (the CUDA counterpart of the
- * reference's generated Metal slot kernels, private_block/metal_slot.rs:115-497): 0 = the interpreter, which runs every
+ * reference's generated Metal slot kernels, private_block/metal_slot.rs:115-497): 0 = the program machine, which runs every
  * program (default: it is the faster one on this GPU for every recorded graph), 1 = the generated kernel.  Same words either
  * way; an A/B switch like the reference's HL_GPU_* switches (hashline/src/gpu/cuda.rs:74-125). */
 int hl_b200_set_slot_kernels(hl_ctx* ctx, int on);
@@ -296,8 +296,9 @@ typedef struct {
  * "sc-round", squeeze r_j, fold.  mask_coeffs NULL = no mask; otherwise mask_vars * degree + 2 Fp2 in
  * the layout of sumcheck.rs:199-200 and the batch must start at round 0.
  * out: per round (degree+1) unmasked sums, (degree+1) absorbed (masked) values, then r_j  (Fp2 each).
- * fs is updated to the position after the batch.  The caller replays the batch through its own
- * transcript and compares (metal.rs:4156-4171); nothing here is trusted blind. */
+ * fs is updated to the position after the batch.  A batch that fails on the way (a device wait that ran out, a device error) spends the
+ * evaluator: the tables are between two rounds, and every later call but hl_b200_rounds_free answers with the batch's status.
+ * The caller replays the batch through its own transcript and compares (metal.rs:4156-4171); nothing here is trusted blind. */
 int hl_b200_rounds_batched(hl_rounds* r, uint32_t nd, hl_fs_state* fs, const uint64_t* mask_coeffs, uint32_t mask_vars,
                            const uint64_t mask_c[2], uint64_t* out);
 

@@ -11,6 +11,7 @@ and raises instead when ``HL_GPU_REQUIRED=1`` (mod.rs:76-102).  Arrays are numpy
 from __future__ import annotations
 
 import ctypes as C
+import operator
 import os
 import struct
 from typing import List, Optional, Tuple
@@ -87,7 +88,7 @@ class Context:
         self.check(self.lib.hl_b200_set_encoder(self.h, 1 if fast else 0))
 
     def set_slot_kernels(self, on: bool) -> None:
-        """the generated per-graph round kernels, or (default) the interpreter, for slot programs with a known graph"""
+        """the generated per-graph round kernels, or (default) the program machine, for slot programs with a known graph"""
         self.check(self.lib.hl_b200_set_slot_kernels(self.h, 1 if on else 0))
 
     def set_dependent_launch(self, on: bool) -> None:
@@ -667,7 +668,7 @@ class SlotProgram:
         self._words: List[int] = []
         self.n_nodes = 0
         self.n_terms = 0
-        self._flat = None
+        self._flat = self._cf = self._cf_of = None
 
     @staticmethod
     def node(node_id: int) -> int:
@@ -717,18 +718,21 @@ class SlotProgram:
         self.n_terms += 1
 
     def _arrays(self):
-        """(words, coefficients) as the C ABI takes them.  The words only grow; the coefficients may be replaced in place, as a challenge is
-        between two proofs, so they are taken as they are now (40 of them: 5 us)."""
+        """(words, coefficients) as the C ABI takes them.  The words only grow; a coefficient may be replaced in place, as a challenge is
+        between two proofs, so their array is kept only while every one of them is the very tuple it was made from."""
         if self._flat is None or self._flat.size != len(self._words):
             self._flat = np.array(self._words, dtype=np.uint32)
-        cf = np.fromiter((x for c in self.coefs for x in c), dtype=np.uint64, count=2 * len(self.coefs)).reshape(-1, 2)
-        return self._flat, cf
+        c, of = self.coefs, self._cf_of
+        if of is None or len(c) != len(of) or not all(map(operator.is_, c, of)):
+            self._cf = np.array(c, dtype=np.uint64).reshape(-1, 2)
+            self._cf_of = list(c) if all(type(x) is tuple for x in c) else None
+        return self._flat, self._cf
 
     def words(self) -> np.ndarray:
         return self._arrays()[0].copy()
 
     def coef_array(self) -> np.ndarray:
-        return self._arrays()[1]
+        return self._arrays()[1].copy()
 
 
 class B200Rounds:

@@ -130,6 +130,10 @@ def test_a_coefficient_replaced_in_place_counts():
     prog.coefs[0] = (1 << 63, 3)
     assert prog.coef_array().tolist() == [[1 << 63, 3], [11, 0]] and prog._arrays()[1].tolist() == [[1 << 63, 3], [11, 0]]
     assert (prog.words() == w).all()
+    prog.coefs[1] = [17, 0]  # a list, which may change without being replaced
+    assert prog.coef_array()[1].tolist() == [17, 0]
+    prog.coefs[1][0] = 11
+    assert prog.coef_array()[1].tolist() == [11, 0]
     prog.term((13, 0), [1], [])
     assert prog.coef_array().tolist() == [[1 << 63, 3], [11, 0], [13, 0]] and prog.words().size > w.size
 
