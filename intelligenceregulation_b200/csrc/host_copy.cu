@@ -8,7 +8,7 @@
 //                            once.  The driver's own path for pageable memory stages and waits inside every single call.
 //   large, pageable          through a ring of page-locked slots, filled and emptied by a few host threads beside the copy engine.
 //                            One core moves about 18 GB/s (and far less into fresh pages, which it has to fault in), the bus 55 GB/s.
-//   page-locked or managed   one asynchronous copy.
+//   page-locked or managed   one asynchronous copy above SMALL_UP.
 //
 // A line that a helper's core still holds when it has gone to sleep again costs whoever touches it next a wake-up of that core: the
 // copy engine (1 MB into slots that helpers had read: 45 us instead of 18), and the caller, who reads the result or makes the next input
@@ -430,7 +430,7 @@ int d2h_on(hl_ctx* c, void* h, const void* d, size_t bytes, cudaStream_t s) {
     cudaError_t e;
     CopyRing* r;
     char* slot;
-    if (bytes <= SMALL_DOWN && (slot = bounce(c, c->down, bytes)) != nullptr) {
+    if (bytes <= SMALL_DOWN && (bytes <= SMALL_UP || pageable(h)) && (slot = bounce(c, c->down, bytes)) != nullptr) {
         e = bounce_down(c, slot, (char*)h, (const char*)d, bytes, s);
     } else if (pageable(h) && (r = ring_of(c)) != nullptr) {
         e = ring_down(r, (char*)h, (const char*)d, bytes, s);

@@ -135,12 +135,14 @@ static void failures(bool lock) {
 }
 
 // every size class of the copies and both sides of its limits, at every alignment that words have
-static void sizes() {
+static void sizes(bool lock) {
     hl_ctx* c = nullptr;
     hl_b200_init(0, &c);
     for (const size_t n : {1, 7, 8191, 8192, 8193, 16384, 16385, 21845, 32768, 32769, 43691, 49152, 49153, 65537, 100001, 3000001}) {
         std::vector<uint64_t> a(n + 8), b(n + 8), out(3 * n + 8);
         for (size_t i = 0; i < n + 8; i++) { a[i] = i * 0x9E3779B97F4A7C15ull; b[i] = ~a[i]; }
+        if (lock)
+            for (auto* v : {&a, &b, &out}) fake::locked[(const char*)v->data()] = v->size() * 8;
         for (size_t off = 0; off < (n > 1000000 ? 2u : 8u); off++) {
             std::fill(out.begin(), out.end(), 7);
             if (hl_b200_probe_field(c, a.data() + off, b.data() + off, n, out.data() + off)) bad("probe_field", "refused");
@@ -151,6 +153,8 @@ static void sizes() {
             for (size_t i = 3 * n + off; i < out.size(); i++) ok = ok && out[i] == 7;
             if (!ok) bad("probe_field", "wrong bytes at " + std::to_string(n) + " words, offset " + std::to_string(off));
         }
+        if (lock)
+            for (auto* v : {&a, &b, &out}) fake::locked.erase((const char*)v->data());
     }
     hl_b200_shutdown(c);
 }
@@ -180,9 +184,10 @@ static void areas() {
 int main(int argc, char** argv) {
     if (argc == 3 && !strcmp(argv[1], "threads")) {
         g_threads = atol(argv[2]);
-        sizes();
+        sizes(false);
     } else if (argc == 2 && !strcmp(argv[1], "copies")) {
-        sizes();
+        sizes(false);
+        sizes(true);
         areas();
     } else {
         failures(false);
