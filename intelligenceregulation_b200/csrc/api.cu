@@ -73,6 +73,32 @@ int root_powers(hl_ctx* c, u32 lognn, const u64** out) {
     return HL_B200_OK;
 }
 
+// the tensor-core encoder's tables for rows of 2^logn words at rate 2^-logr, made once per size, and its error word
+int encoder_tables(hl_ctx* c, u32 logn, u32 logr, const u64** out) {
+    if (!c->enc_flag) {
+        if (cudaHostAlloc((void**)&c->enc_flag, 4, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+            c->enc_flag = nullptr;
+            cudaGetLastError();
+            return fail(c, HL_B200_ERR_OOM, "encoder status word");
+        }
+        *c->enc_flag = 0;
+    }
+    const u32 key = logn + 64 * logr;
+    auto it = c->enc_tables.find(key);
+    if (it != c->enc_tables.end()) { *out = it->second; return HL_B200_OK; }
+    std::vector<u64> h(hlk::encode_tc_table_words(logn, logr));
+    hlk::encode_tc_build(logn, logr, h.data());
+    void* d = nullptr;
+    cudaError_t e = cudaMalloc(&d, h.size() * 8);
+    if (e != cudaSuccess) { cudaGetLastError(); return fail(c, HL_B200_ERR_OOM, "encoder tables", e); }
+    e = cudaMemcpyAsync(d, h.data(), h.size() * 8, cudaMemcpyHostToDevice, c->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);  // h dies at return
+    if (e != cudaSuccess) { cudaFree(d); return fail(c, HL_B200_ERR_DEVICE, "encoder table upload", e); }
+    c->enc_tables[key] = (u64*)d;
+    *out = (u64*)d;
+    return HL_B200_OK;
+}
+
 // a 32-byte key as eight device words; NULL stays NULL (unkeyed)
 int upload_key(hl_ctx* c, const uint8_t* key32, uint32_t** d_key) {
     *d_key = nullptr;
@@ -170,6 +196,8 @@ void hl_b200_shutdown(hl_ctx* c) {
     cudaStreamSynchronize(c->copy_stream);
     cudaStreamSynchronize(c->stream);
     for (auto& kv : c->tw) cudaFree(kv.second);
+    for (auto& kv : c->enc_tables) cudaFree(kv.second);
+    if (c->enc_flag) cudaFreeHost(c->enc_flag);
     if (c->wp_flag) cudaFreeHost(c->wp_flag);
     host_copy_release(c);
     if (c->up.mem) cudaFreeHost(c->up.mem);

@@ -28,6 +28,8 @@ struct hl_ctx {
     std::mutex mu;
     std::mutex err_mu;       // guards last_error and stats.declines: a decline may be recorded before `mu` is taken, from any thread
     std::map<u32, u64*> tw;  // log2 nn -> nn powers of the nn-th root
+    std::map<u32, u64*> enc_tables;  // log2 n + 64 log2 rate -> the tensor-core encoder's constants
+    int* enc_flag = nullptr;         // page-locked: the tensor-core encoder's error word (a bounded wait ran out): read at every synchronisation
     std::string label, last_error;
     hl_stats stats{};
     bool timing = false;
@@ -60,7 +62,8 @@ struct hl_store {
     bool fold_data = false;       // a plain store whose row fold reads d_data (a masking commitment's coefficient rows)
     u64* d_data = nullptr;        // rows x n
     u64* d_pads = nullptr;        // rows x q
-    u64* d_enc = nullptr;         // rows x nn
+    u64* d_enc = nullptr;         // rows x nn, the words of a row in `order`
+    ColOrder order;
     uint32_t* d_leaves = nullptr; // nn x 8 words, unsalted
     int encoder_path = -1;
     size_t n() const { return (size_t)1 << logn; }
@@ -104,6 +107,7 @@ struct Call {
     }
 };
 int root_powers(hl_ctx* c, u32 lognn, const u64** out);
+int encoder_tables(hl_ctx* c, u32 logn, u32 logr, const u64** out);
 int upload_key(hl_ctx* c, const uint8_t* key32, uint32_t** d_key);
 int log2_exact(size_t v);
 void store_release(hl_store* st);  // frees a store; the caller holds the context's lock

@@ -158,7 +158,18 @@ int commit_on_device(hl_ctx* c, hl_store* st, const u64* d_pows, const uint8_t* 
     uint32_t* cvs = nullptr;
     unsigned char *d_narrow = nullptr, *d_row_w = nullptr;
     u64* d_row_off = nullptr;
-    const size_t scratch_words = hlk::encode_scratch_words(logb, T, c->sm_count, st->rows);
+    size_t scratch_words = hlk::encode_scratch_words(logb, T, c->sm_count, st->rows);
+    const bool tc = c->fast_encoder && hlk::encode_tc_takes(logn, st->logr, st->rows, c->sm_count);
+    const u64* tc_tab = nullptr;
+    st->order = ColOrder();
+    if (tc) {
+        st->order.logn = logn;
+        st->order.logr = st->logr;
+        rc = encoder_tables(c, logn, st->logr, &tc_tab);
+        if (rc) return rc;
+        const size_t w = hlk::encode_tc_scratch_words(logn, st->logr, st->q, st->rows, c->sm_count);
+        if (w > scratch_words) scratch_words = w;
+    }
     const u32 nchunks = hlk::hash_chunks(st->rows);
     const size_t cvs_bytes = nchunks > 1 && leaves ? (size_t)nchunks * nn * 32 : 0;
     const size_t total_bytes = packed ? (size_t)hr.off[st->rows] : (size_t)st->rows * n * 8;
@@ -180,7 +191,7 @@ int commit_on_device(hl_ctx* c, hl_store* st, const u64* d_pows, const uint8_t* 
     // one before it when the device is the slower side - and the last two waves as pieces of their own, so that one wave's
     // encoding, not five, follows the last byte when the bus is the slower side.
     auto byte_at = [&](u32 r) { return packed ? (size_t)hr.off[r] : (size_t)r * n * 8; };
-    const u32 wave = (u32)c->sm_count;
+    const u32 wave = (u32)c->sm_count * (tc ? hlk::encode_tc_rows(logn) : 1u);
     const bool split = h_data && total_bytes >= ((size_t)32 << 20) && st->rows > 4u * wave;
     const bool bus_bound = total_bytes / st->rows >= n * 6;  // bytes per row near the 64-bit form
     const bool pieces = split;
@@ -256,7 +267,8 @@ int commit_on_device(hl_ctx* c, hl_store* st, const u64* d_pows, const uint8_t* 
             if (fused_widen) { a.narrow = d_narrow; a.row_off = d_row_off + r0; a.row_w = d_row_w + r0; }
             // a handful of rows (a boundary commitment, the last piece of an upload): one CTA per (row, residue)
             a.split = hlk::encode_split_pays(logb, st->logr, nr, c->sm_count) ? 1 : 0;
-            cudaError_t e = hlk::encode_rows(a, logb, c->fast_encoder || loga, c->sm_count, scratch_words, c->stream, &st->encoder_path);
+            cudaError_t e = tc ? hlk::encode_rows_tc(a, logn, tc_tab, c->sm_count, scratch_words, c->enc_flag, c->stream, &st->encoder_path)
+                               : hlk::encode_rows(a, logb, c->fast_encoder || loga, c->sm_count, scratch_words, c->stream, &st->encoder_path);
             c->stats.kernel_launches += 1;
             if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "row encoder launch", e);
             // the 128-row hash chunks that are complete now.  Launches of one or two chunks fill the machine badly (five such
@@ -265,7 +277,7 @@ int commit_on_device(hl_ctx* c, hl_store* st, const u64* d_pows, const uint8_t* 
             if (!rc && pieces) {
                 const u32 c1 = r0 + nr == st->rows ? nchunks : (r0 + nr) / 128u;
                 if (c1 > chunks_done && (bus_bound || c1 - chunks_done >= 4 || r0 + nr == st->rows)) {
-                    e = hlk::hash_column_chunks(st->d_enc, st->rows, (u32)nn, d_key, chunks_done, c1 - chunks_done, cvs, st->d_leaves, c->stream);
+                    e = hlk::hash_column_chunks(st->d_enc, st->rows, (u32)nn, d_key, chunks_done, c1 - chunks_done, cvs, st->d_leaves, c->stream, st->order);
                     c->stats.kernel_launches += 1;
                     if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "column hash launch", e);
                     chunks_done = c1;
@@ -275,13 +287,13 @@ int commit_on_device(hl_ctx* c, hl_store* st, const u64* d_pows, const uint8_t* 
     }
     if (!rc && pieces) {
         Timed t(c, HL_T_HASH);
-        cudaError_t e = hlk::hash_column_merge(st->rows, (u32)nn, d_key, cvs, st->d_leaves, c->stream);
+        cudaError_t e = hlk::hash_column_merge(st->rows, (u32)nn, d_key, cvs, st->d_leaves, c->stream, st->order);
         c->stats.kernel_launches += 1;
         if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "column hash merge launch", e);
     }
     if (!rc && !pieces && leaves) {
         Timed t(c, HL_T_HASH);
-        cudaError_t e = hlk::hash_columns(st->d_enc, st->rows, (u32)nn, d_key, cvs, st->d_leaves, c->stream);
+        cudaError_t e = hlk::hash_columns(st->d_enc, st->rows, (u32)nn, d_key, cvs, st->d_leaves, c->stream, st->order);
         c->stats.kernel_launches += nchunks > 1 ? 2 : 1;
         if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "column hash launch", e);
     }
@@ -475,7 +487,28 @@ int hl_b200_store_shape(hl_store* st, size_t* rows, size_t* n, size_t* nn, size_
     return HL_B200_OK;
 }
 
-const uint64_t* hl_b200_store_encoded_dev(hl_store* st) { return st ? (const uint64_t*)st->d_enc : nullptr; }
+// the words as the header promises them: an encoding that lies residue by residue is put into the columns' own order first, and stays in it
+const uint64_t* hl_b200_store_encoded_dev(hl_store* st) {
+    if (!st) return nullptr;
+    hl_ctx* c = st->ctx;
+    Call g(c);
+    if (st->order.logr) {
+        const u32 ctas = hlk::natural_order_rows(st->rows, c->sm_count);
+        const size_t bytes = (size_t)ctas * st->nn() * 8;
+        u64* d_rows = nullptr;
+        int rc = dev_alloc(c, (void**)&d_rows, bytes);
+        if (!rc) {
+            const cudaError_t e = hlk::natural_order(st->d_enc, st->rows, st->nn(), st->order, d_rows, ctas, c->stream);
+            c->stats.kernel_launches++;
+            if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "column order launch", e);
+        }
+        if (!rc) rc = sync(c, "store_encoded_dev");
+        dev_free(c, d_rows, bytes);
+        if (rc) return nullptr;
+        st->order = ColOrder();
+    }
+    return (const uint64_t*)st->d_enc;
+}
 const uint8_t* hl_b200_store_leaves_dev(hl_store* st) { return st ? (const uint8_t*)st->d_leaves : nullptr; }
 
 void hl_b200_store_free(hl_store* st) {
@@ -502,7 +535,7 @@ int hl_b200_store_fold(hl_store* st, const uint64_t* rhos, size_t k, int with_pa
     src.rows = rows; src.n = n; src.q = q;
     src.d = from_data ? st->d_data : st->d_enc;
     src.ld = from_data ? n : st->nn();
-    src.ir = from_data ? 1u : 1u << st->logr;
+    src.ir = from_data || st->order.logr ? 1u : 1u << st->logr;  // the systematic positions are residue 0
     src.pads = st->zk && q ? st->d_pads : nullptr;
     u64* d_out = nullptr;
     FoldPlan plan;
@@ -549,7 +582,7 @@ int hl_b200_store_columns(hl_store* st, const uint64_t* idx, size_t nidx, uint64
     if (!rc) rc = h2d(c, d_idx, idx, nidx * 8);
     if (!rc) {
         Timed t(c, HL_T_GATHER);
-        cudaError_t e = hlk::gather_columns(st->d_enc, st->rows, st->nn(), d_idx, (u32)nidx, d_out, c->stream);
+        cudaError_t e = hlk::gather_columns(st->d_enc, st->rows, st->nn(), d_idx, (u32)nidx, d_out, c->stream, st->order);
         c->stats.kernel_launches++;
         if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "gather launch", e);
     }

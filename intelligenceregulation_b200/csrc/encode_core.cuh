@@ -1,4 +1,5 @@
-// Row encoder of the Ligero commitment: the per-thread work of every phase.
+// Row encoder of the Ligero commitment in shared memory: the per-thread work of every phase.  (Rows of 2^14 words, and many shorter ones, go
+// through the tensor cores: encode_tc.cuh.)
 //
 // One CTA encodes one row at a time, entirely in shared memory:
 //

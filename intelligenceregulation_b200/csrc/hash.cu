@@ -16,7 +16,7 @@ namespace {
 
 __global__ void __launch_bounds__(128) k_hash_col_chunks(const u64* __restrict__ enc, u32 rows, u32 nn,
                                                          const uint32_t* __restrict__ key, u32 nchunks, u32 chunk0,
-                                                         uint32_t* __restrict__ cvs, uint32_t* __restrict__ leaves) {
+                                                         uint32_t* __restrict__ cvs, uint32_t* __restrict__ leaves, ColOrder order) {
     const u32 col = blockIdx.x * blockDim.x + threadIdx.x, chunk = chunk0 + blockIdx.y;
     if (col >= nn) return;
     const u32 r0 = chunk * 128u, r1 = min(rows, r0 + 128u);
@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(128) k_hash_col_chunks(const u64* __restrict__
         if (b == nb - 1) flags |= b3::CHUNK_END | (nchunks == 1 ? b3::ROOT : 0u);
         b3::compress(cv, m, chunk, cnt * 8u, flags);
     }
-    uint32_t* dst = nchunks == 1 ? leaves + (size_t)col * 8 : cvs + ((size_t)chunk * nn + col) * 8;
+    uint32_t* dst = nchunks == 1 ? leaves + order.column(col) * 8 : cvs + ((size_t)chunk * nn + col) * 8;
     reinterpret_cast<uint4*>(dst)[0] = make_uint4(cv[0], cv[1], cv[2], cv[3]);
     reinterpret_cast<uint4*>(dst)[1] = make_uint4(cv[4], cv[5], cv[6], cv[7]);
 }
@@ -55,7 +55,7 @@ __device__ __forceinline__ void parent(uint32_t (&out)[8], const uint32_t* l, co
 // soon as both halves exist (a binary counter over the chunks seen); what remains at the end
 // is joined from the right, and the last join carries the ROOT flag.
 __global__ void __launch_bounds__(128) k_hash_col_merge(const uint32_t* __restrict__ cvs, u32 nn, u32 nchunks,
-                                                        const uint32_t* __restrict__ key, uint32_t* __restrict__ leaves) {
+                                                        const uint32_t* __restrict__ key, uint32_t* __restrict__ leaves, ColOrder order) {
     const u32 col = blockIdx.x * blockDim.x + threadIdx.x;
     if (col >= nn) return;
     uint32_t stack[24][8];
@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(128) k_hash_col_merge(const uint32_t* __restri
 #pragma unroll
         for (int i = 0; i < 8; i++) stack[sp - 1][i] = out[i];
     }
-    uint32_t* dst = leaves + (size_t)col * 8;
+    uint32_t* dst = leaves + order.column(col) * 8;
 #pragma unroll
     for (int i = 0; i < 8; i++) dst[i] = stack[0][i];
 }
@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(128) k_hash_col_merge(const uint32_t* __restri
 // before, 6 us); above, lanes without a pair cost more than the chain.
 constexpr u32 MERGE_WARPS = 4, MERGE_MAX = 64;
 __global__ void __launch_bounds__(32 * MERGE_WARPS) k_hash_col_merge_few(const uint32_t* __restrict__ cvs, u32 nn, u32 nchunks, const uint32_t* __restrict__ key,
-                                                                         uint32_t* __restrict__ leaves) {
+                                                                         uint32_t* __restrict__ leaves, ColOrder order) {
     __shared__ __align__(16) uint32_t buf[MERGE_WARPS][MERGE_MAX * 8];
     const u32 warp = threadIdx.x >> 5, lane = threadIdx.x & 31, col = blockIdx.x * MERGE_WARPS + warp;
     if (col >= nn) return;
@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(32 * MERGE_WARPS) k_hash_col_merge_few(const u
             for (int i = 0; i < 8; i++) buf[warp][8 * lane + i] = out[i];
         __syncwarp();
     }
-    if (lane < 2) reinterpret_cast<uint4*>(leaves + (size_t)col * 8)[lane] = b[lane];
+    if (lane < 2) reinterpret_cast<uint4*>(leaves + order.column(col) * 8)[lane] = b[lane];
 }
 
 // dst[j] = H_key(a[j] || b[j]) for 32-byte a, b: salted leaves (a = leaves, b = salts) and
@@ -227,27 +227,27 @@ cudaError_t merkle_tree(const uint32_t* d_leaves, const uint32_t* d_salts, u32 n
 u32 hash_chunks(u32 rows) { return (rows + 127u) / 128u; }
 
 cudaError_t hash_columns(const u64* enc, u32 rows, u32 nn, const uint32_t* d_key, uint32_t* d_cvs, uint32_t* d_leaves,
-                         cudaStream_t st) {
+                         cudaStream_t st, ColOrder order) {
     const u32 nchunks = hash_chunks(rows);
-    cudaError_t e = hash_column_chunks(enc, rows, nn, d_key, 0, nchunks, d_cvs, d_leaves, st);
+    cudaError_t e = hash_column_chunks(enc, rows, nn, d_key, 0, nchunks, d_cvs, d_leaves, st, order);
     if (e != cudaSuccess || nchunks == 1) return e;
-    return hash_column_merge(rows, nn, d_key, d_cvs, d_leaves, st);
+    return hash_column_merge(rows, nn, d_key, d_cvs, d_leaves, st, order);
 }
 
 // the chunk values of the 1 KiB chunks [chunk0, chunk0 + count) of every column (rows 128 chunk0 .. of the encoding
 // must be complete); a commitment whose rows arrive in pieces hashes each piece as soon as it is encoded
 cudaError_t hash_column_chunks(const u64* enc, u32 rows, u32 nn, const uint32_t* d_key, u32 chunk0, u32 count, uint32_t* d_cvs,
-                               uint32_t* d_leaves, cudaStream_t st) {
+                               uint32_t* d_leaves, cudaStream_t st, ColOrder order) {
     if (count == 0) return cudaSuccess;
     dim3 grid((nn + 127u) / 128u, count);
-    k_hash_col_chunks<<<grid, 128, 0, st>>>(enc, rows, nn, d_key, hash_chunks(rows), chunk0, d_cvs, d_leaves);
+    k_hash_col_chunks<<<grid, 128, 0, st>>>(enc, rows, nn, d_key, hash_chunks(rows), chunk0, d_cvs, d_leaves, order);
     return cudaGetLastError();
 }
 
-cudaError_t hash_column_merge(u32 rows, u32 nn, const uint32_t* d_key, const uint32_t* d_cvs, uint32_t* d_leaves, cudaStream_t st) {
+cudaError_t hash_column_merge(u32 rows, u32 nn, const uint32_t* d_key, const uint32_t* d_cvs, uint32_t* d_leaves, cudaStream_t st, ColOrder order) {
     const u32 nchunks = hash_chunks(rows);
-    if (nn <= 4096u && nchunks >= 3u && nchunks <= MERGE_MAX) k_hash_col_merge_few<<<(nn + MERGE_WARPS - 1) / MERGE_WARPS, 32 * MERGE_WARPS, 0, st>>>(d_cvs, nn, nchunks, d_key, d_leaves);
-    else k_hash_col_merge<<<(nn + 127u) / 128u, 128, 0, st>>>(d_cvs, nn, nchunks, d_key, d_leaves);
+    if (nn <= 4096u && nchunks >= 3u && nchunks <= MERGE_MAX) k_hash_col_merge_few<<<(nn + MERGE_WARPS - 1) / MERGE_WARPS, 32 * MERGE_WARPS, 0, st>>>(d_cvs, nn, nchunks, d_key, d_leaves, order);
+    else k_hash_col_merge<<<(nn + 127u) / 128u, 128, 0, st>>>(d_cvs, nn, nchunks, d_key, d_leaves, order);
     return cudaGetLastError();
 }
 

@@ -4,6 +4,14 @@
 #include <stdint.h>
 #include "encode_core.cuh"
 
+// Where column j of an encoding of rows of n 2^logr words lies within a row: j itself (logr = 0), or residue by residue, j mod 2^logr first, as
+// the tensor-core encoder leaves it (whole sectors: a residue's words written R apart cost R writes of every sector).
+struct ColOrder {
+    u32 logn = 0, logr = 0;
+    GL_HD size_t at(size_t j) const { return ((j & (((size_t)1 << logr) - 1)) << logn) + (j >> logr); }
+    GL_HD size_t column(size_t at) const { return logr ? ((at & (((size_t)1 << logn) - 1)) << logr) + (at >> logn) : at; }
+};
+
 namespace hlk {
 
 // encode.cu
@@ -15,13 +23,21 @@ cudaError_t encode_rows(const enc::RowArgs& a, u32 logn, bool allow_fast, int sm
 cudaError_t widen_rows(const unsigned char* narrow, const u64* row_off, const unsigned char* row_w, u64* out, u32 rows, u32 n, int sm_count, cudaStream_t st);
 cudaError_t encode_rows_form(const enc::RowArgs& a, u32 logn, int form, int sm_count, size_t scratch_words, cudaStream_t st);
 
+// encode_tc.cu: the same rows on the tensor cores (rows of 2^10 words and more)
+size_t encode_tc_table_words(u32 logn, u32 logr);
+void encode_tc_build(u32 logn, u32 logr, u64* out);  // host
+bool encode_tc_takes(u32 logn, u32 logr, u32 rows, int sm_count);
+u32 encode_tc_rows(u32 logn);  // that one CTA takes at a time
+size_t encode_tc_scratch_words(u32 logn, u32 logr, u32 q, u32 rows, int sm_count);
+cudaError_t encode_rows_tc(enc::RowArgs a, u32 logn, const u64* tab, int sm_count, size_t scratch_words, int* err, cudaStream_t st, int* path_out);
+
 // hash.cu
 u32 hash_chunks(u32 rows);
 cudaError_t hash_column_chunks(const u64* enc, u32 rows, u32 nn, const uint32_t* d_key, u32 chunk0, u32 count, uint32_t* d_cvs,
-                               uint32_t* d_leaves, cudaStream_t st);
-cudaError_t hash_column_merge(u32 rows, u32 nn, const uint32_t* d_key, const uint32_t* d_cvs, uint32_t* d_leaves, cudaStream_t st);
+                               uint32_t* d_leaves, cudaStream_t st, ColOrder order = ColOrder());
+cudaError_t hash_column_merge(u32 rows, u32 nn, const uint32_t* d_key, const uint32_t* d_cvs, uint32_t* d_leaves, cudaStream_t st, ColOrder order = ColOrder());
 cudaError_t hash_columns(const u64* enc, u32 rows, u32 nn, const uint32_t* d_key, uint32_t* d_cvs, uint32_t* d_leaves,
-                         cudaStream_t st);
+                         cudaStream_t st, ColOrder order = ColOrder());
 cudaError_t salt_leaves(const uint32_t* d_leaves, const uint32_t* d_salts, u32 nn, const uint32_t* d_leaf_key,
                         uint32_t* d_out, cudaStream_t st);
 cudaError_t merkle_levels(uint32_t* d_levels, u32 nn, const uint32_t* d_node_key, cudaStream_t st);
@@ -42,7 +58,10 @@ cudaError_t fold_rows(const u64* src, u32 rows, u32 ncols, size_t ld, u32 ir, co
                       const u32* d_out_map, u64* d_out, u32 out_ld, cudaStream_t st, u32 splits = 1, u64* d_part = nullptr);
 cudaError_t fold_rows_sparse(const u64* src, u32 ncols, size_t ld, u32 ir, const u64* src2, u32 ncols2, size_t ld2, const u32* d_off,
                              const u32* d_rows, const u64* d_weights, u32 k, const u32* d_out_map, u64* d_out, u32 out_ld, cudaStream_t st);
-cudaError_t gather_columns(const u64* enc, u32 rows, size_t nn, const u64* d_idx, u32 nidx, u64* d_out, cudaStream_t st);
+cudaError_t gather_columns(const u64* enc, u32 rows, size_t nn, const u64* d_idx, u32 nidx, u64* d_out, cudaStream_t st, ColOrder order);
+// rows put into the columns' own order, in place; d_rows = natural_order_rows() x nn words of scratch
+u32 natural_order_rows(u32 rows, int sm_count);
+cudaError_t natural_order(u64* enc, u32 rows, size_t nn, ColOrder order, u64* d_rows, u32 ctas, cudaStream_t st);
 
 // misc.cu
 cudaError_t probe_field(const u64* d_a, const u64* d_b, size_t n, u64* d_out3, cudaStream_t st);

@@ -296,10 +296,22 @@ __global__ void __launch_bounds__(SPARSE_COLS) k_fold_sparse(FoldSeg seg0, FoldS
 
 // out[c * rows + i] = enc[i * nn + idx[c]]   (pcs.rs:1055-1067; order of idx, duplicates repeated)
 __global__ void k_gather_cols(const u64* __restrict__ enc, u32 rows, size_t nn, const u64* __restrict__ idx, u32 nidx,
-                              u64* __restrict__ out) {
+                              u64* __restrict__ out, ColOrder order) {
     const u32 i = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
     if (i >= rows || c >= nidx) return;
-    out[(size_t)c * rows + i] = enc[(size_t)i * nn + idx[c]];
+    out[(size_t)c * rows + i] = enc[(size_t)i * nn + order.at(idx[c])];
+}
+
+// a CTA takes a row into its scratch row and puts it back in the columns' own order
+__global__ void __launch_bounds__(1024) k_natural_order(u64* __restrict__ enc, u32 rows, size_t nn, ColOrder order, u64* __restrict__ scratch) {
+    u64* buf = scratch + blockIdx.x * nn;
+    for (u32 row = blockIdx.x; row < rows; row += gridDim.x) {
+        u64* r = enc + (size_t)row * nn;
+        for (size_t j = threadIdx.x; j < nn; j += blockDim.x) buf[j] = r[j];
+        __syncthreads();
+        for (size_t j = threadIdx.x; j < nn; j += blockDim.x) r[j] = buf[order.at(j)];
+        __syncthreads();
+    }
 }
 
 }  // namespace
@@ -369,10 +381,16 @@ cudaError_t fold_rows_sparse(const u64* src, u32 ncols, size_t ld, u32 ir, const
     return cudaGetLastError();
 }
 
-cudaError_t gather_columns(const u64* enc, u32 rows, size_t nn, const u64* d_idx, u32 nidx, u64* d_out, cudaStream_t st) {
+cudaError_t gather_columns(const u64* enc, u32 rows, size_t nn, const u64* d_idx, u32 nidx, u64* d_out, cudaStream_t st, ColOrder order) {
     if (nidx == 0) return cudaSuccess;
     dim3 grid((rows + 127u) / 128u, nidx);
-    k_gather_cols<<<grid, 128, 0, st>>>(enc, rows, nn, d_idx, nidx, d_out);
+    k_gather_cols<<<grid, 128, 0, st>>>(enc, rows, nn, d_idx, nidx, d_out, order);
+    return cudaGetLastError();
+}
+
+u32 natural_order_rows(u32 rows, int sm_count) { return rows < 2u * (u32)sm_count ? rows : 2u * (u32)sm_count; }
+cudaError_t natural_order(u64* enc, u32 rows, size_t nn, ColOrder order, u64* d_rows, u32 ctas, cudaStream_t st) {
+    k_natural_order<<<ctas, 1024, 0, st>>>(enc, rows, nn, order, d_rows);
     return cudaGetLastError();
 }
 

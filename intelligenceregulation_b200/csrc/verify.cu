@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(32 * VC_WARPS) k_verify_columns(const uint32_t
                                                         const uint32_t* __restrict__ paths, u32 depth, const u64* __restrict__ idx,
                                                         const uint32_t* __restrict__ root, const uint32_t* __restrict__ leaf_key,
                                                         const uint32_t* __restrict__ node_key, const u64* __restrict__ acc, u32 k,
-                                                        const u64* __restrict__ wants, const u64* __restrict__ enc, size_t nn, u32 ncols,
+                                                        const u64* __restrict__ wants, const u64* __restrict__ enc, size_t nn, ColOrder order, u32 ncols,
                                                         int32_t* __restrict__ verdict) {
     __shared__ uint32_t path_s[VC_WARPS][VC_DEPTH * 8];
     const u32 warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = blockIdx.x * VC_WARPS + warp;
@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(32 * VC_WARPS) k_verify_columns(const uint32_t
         const u64 a0 = acc[((size_t)g * ncols + c) * 2], a1 = acc[((size_t)g * ncols + c) * 2 + 1];
         u64 w0, w1;
         if (wants) { w0 = wants[((size_t)g * ncols + c) * 2]; w1 = wants[((size_t)g * ncols + c) * 2 + 1]; }
-        else { w0 = enc[(size_t)(2 * g) * nn + j]; w1 = enc[(size_t)(2 * g + 1) * nn + j]; }
+        else { w0 = enc[(size_t)(2 * g) * nn + order.at(j)]; w1 = enc[(size_t)(2 * g + 1) * nn + order.at(j)]; }
         if (a0 != w0 || a1 != w1) bad = g;
     }
     bad = __reduce_min_sync(0xffffffffu, bad);
@@ -176,7 +176,7 @@ static int verify_columns_locked(hl_ctx* c, const uint64_t* cols, size_t rows, s
         if (e == cudaSuccess && !rc) {
             k_verify_columns<<<(unsigned)((ncols + VC_WARPS - 1) / VC_WARPS), 32 * VC_WARPS, 0, c->stream>>>(
                 d_leaves, d_salts, d_paths, depth, d_idx, d_root, d_lk, d_nk, d_acc, (u32)k, d_wants, vec_store ? vec_store->d_enc : nullptr,
-                vec_store ? vec_store->nn() : 0, (u32)ncols, d_verdict);
+                vec_store ? vec_store->nn() : 0, vec_store ? vec_store->order : ColOrder(), (u32)ncols, d_verdict);
             e = cudaGetLastError();
         }
         c->stats.kernel_launches += 2 + (nchunks > 1 ? 2 : 1);

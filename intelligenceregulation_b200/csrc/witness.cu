@@ -15,6 +15,7 @@
 #include <cstdlib>
 
 #include "api_internal.h"
+#include "umma.cuh"
 
 using namespace hlapi;
 
@@ -126,58 +127,14 @@ __global__ void __launch_bounds__(256) k_wp_repack(const int8_t* __restrict__ sr
 // UM_SBO apart, a K step of 32 bytes is 32 bytes further along the row.
 // Every wait is bounded: a wait that runs out sets the error word, every thread leaves together and TMEM is freed.
 constexpr int UM_NT = 256, UM_KT = 128, UM_STAGES = 3, UM_THREADS = 256;
-constexpr u32 UM_SBO = 1024;
 constexpr u32 UM_A_BYTES = WP_MT * UM_KT, UM_B_BYTES = UM_NT * UM_KT, UM_STAGE_BYTES = 2 * UM_A_BYTES + UM_B_BYTES;
-constexpr u32 UM_SPIN_LIMIT = 1u << 22;
 
-__device__ __forceinline__ u64 um_desc(u32 smem_addr) {
-    // start address and stride byte offset in 16-byte units (the leading offset is not used by a swizzled K-major operand and is
-    // set to 1 as the canonical form has it); descriptor version 1; layout type 2 = 128-byte swizzle
-    return (u64)((smem_addr >> 4) & 0x3FFF) | (1ull << 16) | ((u64)(UM_SBO >> 4) << 32) | (1ull << 46) | (2ull << 61);
-}
-
-// instruction descriptor of kind::i8: D = s32, B = s8, A = s8 or u8, both K-major, N = 256, M = 128
-__host__ __device__ constexpr u32 um_idesc(bool a_signed) {
-    return (2u << 4) | ((a_signed ? 1u : 0u) << 7) | (1u << 10) | ((u32)(UM_NT >> 3) << 17) | ((u32)(WP_MT >> 4) << 24);
-}
-
-__device__ __forceinline__ void um_mma(u32 tmem_d, u64 a_desc, u64 b_desc, u32 idesc, u32 accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}\n" ::"r"(tmem_d),
-        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
-        : "memory");
-}
-__device__ __forceinline__ void um_commit(u32 mbar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(mbar) : "memory");
-}
-__device__ __forceinline__ bool um_wait(u32 mbar, u32 parity) {
-    for (u32 spin = 0; spin < UM_SPIN_LIMIT; spin++) {
-        u32 ok;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
-                     : "=r"(ok)
-                     : "r"(mbar), "r"(parity)
-                     : "memory");
-        if (ok) return true;
-    }
-    return false;
-}
 // one box of the tensor map into shared memory; its bytes are counted on the mbarrier
 __device__ __forceinline__ void um_tma_2d(u32 smem_dst, const CUtensorMap* map, u32 mbar, int x, int y) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n" ::"r"(smem_dst),
                  "l"((u64)map), "r"(mbar), "r"(x), "r"(y)
                  : "memory");
 }
-__device__ __forceinline__ void um_ld32(u32 taddr, u32 (&r)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, "
-        "%23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
-          "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
-          "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr));
-}
-
 __device__ __forceinline__ void um_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
 }
@@ -272,8 +229,8 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_wp_umma(const __grid_constant
             for (u32 kk = 0; kk < UM_KT / 32; kk++) {
                 const u64 bd = um_desc(sb + kk * 32);
                 const u32 accumulate = (it | kk) ? 1u : 0u;
-                um_mma(tmem, um_desc(sa + kk * 32), bd, um_idesc(true), accumulate);
-                um_mma(tmem + 256, um_desc(sa + UM_A_BYTES + kk * 32), bd, um_idesc(false), accumulate);
+                um_mma(tmem, um_desc(sa + kk * 32), bd, um_idesc(true, true, WP_MT, UM_NT), accumulate);
+                um_mma(tmem + 256, um_desc(sa + UM_A_BYTES + kk * 32), bd, um_idesc(false, true, WP_MT, UM_NT), accumulate);
             }
             um_commit(empty0 + 8 * st);  // arrives when the instructions above have read this stage
             // refill the stage read one iteration ago, once its instructions have completed
@@ -289,12 +246,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1) k_wp_umma(const __grid_constant
     bool ready = false;
     for (u32 round = 0; round < 1024 && !ready && !gave_up; round++) {
         for (u32 spin = 0; spin < (UM_SPIN_LIMIT >> 10) && !ready; spin++) {
-            u32 p;
-            asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
-                         : "=r"(p)
-                         : "r"(done), "r"(0u)
-                         : "memory");
-            ready = p != 0;
+            ready = um_try_wait(done, 0u);
             if (!ready) __nanosleep(128);  // the polling threads stay off the shared memory the tensor core is reading
         }
     }

@@ -27,18 +27,26 @@ static cudaError_t launch() { return fake::fails() ? cudaErrorUnknown : cudaSucc
 size_t encode_scratch_words(u32, u32, int, u32) { return 64; }
 bool encode_split_pays(u32, u32, u32, int) { return false; }
 cudaError_t encode_rows(const enc::RowArgs&, u32, bool, int, size_t, cudaStream_t, int*) { return launch(); }
+size_t encode_tc_table_words(u32, u32) { return 8; }
+void encode_tc_build(u32, u32, u64* out) { for (int i = 0; i < 8; i++) out[i] = 0; }
+bool encode_tc_takes(u32 logn, u32, u32, int) { return logn >= 10; }
+u32 encode_tc_rows(u32 logn) { return 16384u >> logn; }
+size_t encode_tc_scratch_words(u32, u32, u32, u32, int) { return 64; }
+cudaError_t encode_rows_tc(enc::RowArgs, u32, const u64*, int, size_t, int*, cudaStream_t, int*) { return launch(); }
+u32 natural_order_rows(u32, int) { return 1; }
+cudaError_t natural_order(u64*, u32, size_t, ColOrder, u64*, u32, cudaStream_t) { return launch(); }
 cudaError_t widen_rows(const unsigned char*, const u64*, const unsigned char*, u64*, u32, u32, int, cudaStream_t) { return launch(); }
 u32 hash_chunks(u32 rows) { return (rows + 127) / 128; }
-cudaError_t hash_column_chunks(const u64*, u32, u32, const uint32_t*, u32, u32, uint32_t*, uint32_t*, cudaStream_t) { return launch(); }
-cudaError_t hash_column_merge(u32, u32, const uint32_t*, const uint32_t*, uint32_t*, cudaStream_t) { return launch(); }
-cudaError_t hash_columns(const u64*, u32, u32, const uint32_t*, uint32_t*, uint32_t*, cudaStream_t) { return launch(); }
+cudaError_t hash_column_chunks(const u64*, u32, u32, const uint32_t*, u32, u32, uint32_t*, uint32_t*, cudaStream_t, ColOrder) { return launch(); }
+cudaError_t hash_column_merge(u32, u32, const uint32_t*, const uint32_t*, uint32_t*, cudaStream_t, ColOrder) { return launch(); }
+cudaError_t hash_columns(const u64*, u32, u32, const uint32_t*, uint32_t*, uint32_t*, cudaStream_t, ColOrder) { return launch(); }
 cudaError_t merkle_tree(const uint32_t*, const uint32_t*, u32, const uint32_t*, const uint32_t*, uint32_t*, cudaStream_t, int* n) { *n = 1; return launch(); }
 u32 fold_row_splits(u32, u32, u32, u32, int) { return 1; }
 u32 fold_few_ranges(u32, u32, u32, u32, u32, int) { return 0; }
 cudaError_t fold_rows_few(const u64*, u32, u32, size_t, const u64*, u32, size_t, const u64*, u32, const u32*, u64*, u32, u32, u64*, cudaStream_t) { return launch(); }
 cudaError_t fold_rows(const u64*, u32, u32, size_t, u32, const u64*, u32, size_t, const u64*, u32, const u32*, u64*, u32, cudaStream_t, u32, u64*) { return launch(); }
 cudaError_t fold_rows_sparse(const u64*, u32, size_t, u32, const u64*, u32, size_t, const u32*, const u32*, const u64*, u32, const u32*, u64*, u32, cudaStream_t) { return launch(); }
-cudaError_t gather_columns(const u64*, u32, size_t, const u64*, u32, u64*, cudaStream_t) { return launch(); }
+cudaError_t gather_columns(const u64*, u32, size_t, const u64*, u32, u64*, cudaStream_t, ColOrder) { return launch(); }
 // out: a + b, a - b, a b, three words a pair.  Here: a, b, 0, which shows that both arrays arrived and the results came back
 cudaError_t probe_field(const u64* a, const u64* b, size_t n, u64* out, cudaStream_t st) {
     cudaStreamSynchronize(st);

@@ -1,0 +1,99 @@
+"""The tensor-core row encoder at the edges of its forms: full and short batches of rows per 2^14 words, one residue or all of them a CTA, pads that
+reach most of a row and beyond it, rates 1, 1/2, 1/4, packed rows of every width, and rows that do not start on 32-byte boundaries; and
+what reads an encoding that lies residue by residue."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+P = 0xFFFFFFFF00000001
+
+
+@pytest.fixture(scope="module")
+def dev():
+    from intelligenceregulation_b200 import backend
+
+    d = backend.B200Backend(device=0)
+    yield d
+    d.ctx.close()
+
+
+# log_cols, inv_rate, rows, q: (10 .. 13) just above the line where the tensor cores take over, a last batch of one row
+CASES = [(10, 2, 2369, 33), (11, 2, 1185, 320), (12, 2, 593, 1), (12, 4, 601, 40), (13, 2, 149, 281), (13, 4, 41, 8000),
+         (14, 2, 3, 280), (14, 2, 149, 5), (14, 4, 38, 40001), (14, 4, 2, 1), (14, 1, 2, 0), (14, 2, 75, 0)]
+
+
+@pytest.mark.parametrize("log_cols,inv_rate,rows,q", CASES)
+def test_commitments_and_columns(dev, oracle, log_cols, inv_rate, rows, q):
+    n, nn = 1 << log_cols, inv_rate << log_cols
+    rng = np.random.default_rng(log_cols * 1000 + rows)
+    data = rng.integers(0, P, size=rows * n, dtype=np.uint64)
+    data[:n] = P - 1
+    data[-n:] = 0
+    if q:
+        pads, pows = rng.integers(0, P, size=rows * q, dtype=np.uint64), oracle.coset_powers(7, nn)
+        want = oracle.encode_rows_zk(data, rows, n, pads, q, pows, 18)
+        store, leaves = dev.try_commit_zk_keyed(log_cols, inv_rate, data, pads, pows, 18, None)
+    else:
+        want = oracle.encode_rows_plain(data, rows, n, nn, 18)
+        store, leaves = dev.try_commit(log_cols, inv_rate, data, 18)
+    assert (leaves == oracle.hash_columns(want, rows, nn)).all()
+    idx = np.array([0, nn - 1, nn // 2, 1 % nn, 5 % nn, nn // 3], dtype=np.uint64)
+    cols = oracle.gather_columns(want, rows, nn, idx)
+    assert (store.columns(idx) == cols).all()
+    if not q:  # a plain store folds the systematic positions of its encoding
+        rhos = rng.integers(0, P, size=(2, rows, 2), dtype=np.uint64)
+        assert (store.fold_rows(rhos) == oracle.fold_rows(np.ascontiguousarray(want.reshape(rows, nn)[:, ::inv_rate]).reshape(-1), rows, n, n, 1, rhos)).all()
+    if rows < 200:  # in the columns' own order, for callers on the device, and what reads it afterwards
+        import torch
+        from intelligenceregulation_b200 import backend
+
+        out = torch.empty((nn, 32), dtype=torch.uint8, device="cuda")
+        backend.hash_columns_static(store.encoded_dev(), rows, nn, None, out.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        assert (out.cpu().numpy() == leaves).all()
+        assert (store.columns(idx) == cols).all()
+    store.free()
+
+
+@pytest.mark.parametrize("log_cols,inv_rate,rows,q", [(12, 2, 593, 64), (13, 2, 150, 33), (14, 2, 40, 280), (14, 4, 75, 7)])
+def test_packed_rows_of_every_width(dev, oracle, log_cols, inv_rate, rows, q):
+    n, nn = 1 << log_cols, inv_rate << log_cols
+    rng = np.random.default_rng(rows)
+    widths = rng.choice(np.array([1, 2, 4, 8], dtype=np.uint8), size=rows)
+    parts, wide = [], []
+    for w in map(int, widths):
+        if w == 8:
+            row = rng.integers(0, P, size=n, dtype=np.uint64)
+            wide.append(row)
+        else:
+            row = rng.integers(-(1 << (8 * w - 1)), 1 << (8 * w - 1), size=n).astype({1: np.int8, 2: np.int16, 4: np.int32}[w])
+            row[:2] = [-(1 << (8 * w - 1)), (1 << (8 * w - 1)) - 1]
+            wide.append(np.where(row < 0, row.astype(np.int64).astype(np.uint64) + np.uint64(P), row.astype(np.uint64)))
+        parts.append(row.view(np.uint8))
+    data = np.concatenate(wide).astype(np.uint64)
+    pads, pows = rng.integers(0, P, size=rows * q, dtype=np.uint64), oracle.coset_powers(7, nn)
+    want = oracle.encode_rows_zk(data, rows, n, pads, q, pows, 18)
+    salts = rng.integers(0, 256, size=(nn, 32), dtype=np.uint8)
+    store, leaves, _ = dev.try_commit_zk_packed(log_cols, inv_rate, np.concatenate(parts), widths, pads, pows, 18, None, salts, None, None)
+    assert (leaves == oracle.hash_columns(want, rows, nn)).all()
+    rhos = rng.integers(0, P, size=(1, rows, 2), dtype=np.uint64)
+    assert (store.fold_rows(rhos) == oracle.fold_rows(data, rows, n, n, 1, rhos)).all()  # the widened rows
+    store.free()
+
+
+def test_rows_on_8_byte_boundaries(dev, oracle):
+    import torch
+
+    rows, q, n = 9, 31, 1 << 14
+    rng = np.random.default_rng(3)
+    data, pads = rng.integers(0, P, size=rows * n, dtype=np.uint64), rng.integers(0, P, size=rows * q, dtype=np.uint64)
+    pows = oracle.coset_powers(7, 2 * n)
+    up = lambda a, off: torch.from_numpy(np.concatenate([np.zeros(off, dtype=np.uint64), a]).view(np.int64)).cuda()
+    d, p, h = up(data, 1), up(pads, 1), up(pows, 1)
+    out = torch.empty((2 * n, 32), dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    store = dev.commit_zk_dev(14, 2, d.data_ptr() + 8, rows, p.data_ptr() + 8, q, h.data_ptr() + 8, None, d_leaves=out.data_ptr())
+    idx = np.arange(0, 2 * n, 4097, dtype=np.uint64)
+    want = oracle.encode_rows_zk(data, rows, n, pads, q, pows, 18)
+    assert (store.columns(idx) == oracle.gather_columns(want, rows, 2 * n, idx)).all()
+    assert (out.cpu().numpy() == oracle.hash_columns(want, rows, 2 * n)).all()
+    store.free()

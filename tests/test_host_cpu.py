@@ -60,8 +60,8 @@ def test_product_does_not_reach_the_oracle():
 def emul():
     src = os.path.join(ROOT, "tests", "host_emul", "encode_emul.cpp")
     so = os.path.join(ROOT, "tests", "host_emul", "libencode_emul.so")
-    core = os.path.join(ROOT, "intelligenceregulation_b200", "csrc", "encode_core.cuh")
-    if not os.path.exists(so) or max(os.path.getmtime(src), os.path.getmtime(core)) > os.path.getmtime(so):
+    core = [os.path.join(ROOT, "intelligenceregulation_b200", "csrc", f) for f in ("encode_core.cuh", "encode_tc.cuh", "gl_field.cuh")]
+    if not os.path.exists(so) or max(os.path.getmtime(f) for f in [src, *core]) > os.path.getmtime(so):
         subprocess.check_call(["/usr/bin/g++", "-std=c++17", "-O2", "-shared", "-fPIC", "-o", so, src])
     return C.CDLL(so)
 
@@ -89,3 +89,35 @@ def test_encoder_phases_on_the_host_match_the_oracle(emul, oracle, case):
     assert rc == 0
     want = oracle.encode_rows_zk(data, rows, n, pads, q, pows, 18) if zk else oracle.encode_rows_plain(data, rows, n, nn, 18)
     assert (out == want).all()
+
+
+TC_CASES = [  # log_n, inv_rate, rows, q, zk: every batch of rows per 2^14 words, full and short, both coset residues, pads above the row
+    (10, 2, 17, 40, 1), (10, 4, 3, 1500, 1), (11, 2, 8, 33, 1), (12, 2, 5, 64, 1), (12, 4, 4, 0, 0), (13, 2, 3, 280, 1),
+    (14, 2, 1, 280, 1), (14, 1, 1, 0, 0), (14, 4, 1, 33000, 1),
+]
+
+
+@pytest.mark.parametrize("logn,R,rows,q,zk", TC_CASES)
+def test_tensor_core_encoder_on_the_host_matches_the_oracle(emul, oracle, logn, R, rows, q, zk):
+    n, nn, logr = 1 << logn, (1 << logn) * R, R.bit_length() - 1
+    rng = np.random.default_rng(2000 + logn * 16 + R)
+    data = rng.integers(0, oracle.P, size=rows * n, dtype=np.uint64)
+    data[:n] = oracle.P - 1  # the largest bytes
+    pads = rng.integers(0, oracle.P, size=rows * max(q, 1), dtype=np.uint64)
+    pows = oracle.coset_powers(7, nn)
+    out = np.zeros(rows * nn, dtype=np.uint64)
+    rc = emul.emul_encode_tc(C.c_void_p(data.ctypes.data), rows, logn, logr, C.c_void_p(pads.ctypes.data), q, C.c_void_p(pows.ctypes.data), zk,
+                             C.c_void_p(out.ctypes.data))
+    assert rc == 0
+    want = oracle.encode_rows_zk(data, rows, n, pads, q, pows, 18) if zk else oracle.encode_rows_plain(data, rows, n, nn, 18)
+    assert (out.reshape(rows, R, n).transpose(0, 2, 1).reshape(-1) == want).all()  # residue by residue
+
+
+def test_the_join_of_eight_byte_sums(emul):
+    P, top = 0xFFFFFFFF00000001, 256 * 255 * 255
+    rng = np.random.default_rng(5)
+    rows = [[top] * 8, [0] * 8, [0] * 7 + [top], [top] * 4 + [0] * 4, [0] * 6 + [top, top], [255] * 8, [1] + [0] * 7]
+    sums = np.concatenate([np.array(rows, dtype=np.uint32), rng.integers(0, top + 1, size=(4000, 8), dtype=np.uint32), rng.choice([0, 1, top - 1, top], size=(4000, 8)).astype(np.uint32)])
+    out = np.zeros(len(sums), dtype=np.uint64)
+    emul.emul_join(C.c_void_p(sums.ctypes.data), len(sums), C.c_void_p(out.ctypes.data))
+    assert [int(x) for x in out] == [sum(int(v) << (8 * d) for d, v in enumerate(s)) % P for s in sums]
