@@ -36,20 +36,21 @@ __global__ void k_encode_generic(enc::RowArgs a, u32 logn) {
     }
 }
 
-template <int LOGN, int THREADS, int MINB, int FORM, bool NARROW, bool LONG, bool SPLIT>
-__global__ void __launch_bounds__(THREADS, MINB) k_encode_fast(enc::RowArgs a) {
+// CTA `cta` of `ctas`
+template <int LOGN, int THREADS, int FORM, bool NARROW, bool LONG, bool SPLIT>
+__device__ __forceinline__ void encode_fast(const enc::RowArgs& a, u32 cta, u32 ctas) {
     using F = enc::Fast<LOGN>;
     extern __shared__ u64 smem[];
     u64* S = smem;
     u64* TW = smem + F::N;
     const u32 tid = threadIdx.x;
-    u64* X = a.scratch + (size_t)blockIdx.x * a.T * F::N;
+    u64* X = a.scratch + (size_t)cta * a.T * F::N;
     F::load_twiddles(a, TW, tid, THREADS);
     __syncthreads();
     // a unit of work: a whole row, or (split) one output residue of a row with the row's inverse transform before it
     const u32 A = LONG ? 1u << a.loga : 1u, logR = LONG ? a.logr - a.loga : a.logr, R = 1u << logR;
     const u32 units = SPLIT ? a.rows << logR : a.rows;
-    for (u32 unit = blockIdx.x; unit < units; unit += gridDim.x) {
+    for (u32 unit = cta; unit < units; unit += ctas) {
         const u32 row = SPLIT ? unit >> logR : unit;
         if constexpr (FORM == enc::FORM_COEF) {
             F::row_given(a, row, X, tid, THREADS);
@@ -62,6 +63,20 @@ __global__ void __launch_bounds__(THREADS, MINB) k_encode_fast(enc::RowArgs a) {
             __syncthreads();  // the scratch slot is complete and shared memory is free again
         }
     }
+}
+
+template <int LOGN, int THREADS, int MINB, int FORM, bool NARROW, bool LONG, bool SPLIT>
+__global__ void __launch_bounds__(THREADS, MINB) k_encode_fast(enc::RowArgs a) {
+    encode_fast<LOGN, THREADS, FORM, NARROW, LONG, SPLIT>(a, blockIdx.x, gridDim.x);
+}
+
+// A masking commitment's two kinds of rows at once, a CTA for each (row, residue) of either: `a` messages by the first `ctas_a` CTAs, `b`
+// coefficient rows by the others.  Neither kind fills the machine, and each takes as long as its longest row: 27 us and then 32 for 24
+// masks in launches of their own.
+template <int LOGN, int THREADS, int MINB>
+__global__ void __launch_bounds__(THREADS, MINB) k_encode_mask(enc::RowArgs a, enc::RowArgs b, u32 ctas_a) {
+    if (blockIdx.x < ctas_a) encode_fast<LOGN, THREADS, enc::FORM_COSET, false, false, true>(a, blockIdx.x, ctas_a);
+    else encode_fast<LOGN, THREADS, enc::FORM_COEF, false, false, true>(b, blockIdx.x - ctas_a, gridDim.x - ctas_a);
 }
 
 // packed rows widened in a pass of their own: the shapes the fast path does not cover (rows below 2^8 or above 2^14 words)
@@ -109,6 +124,19 @@ cudaError_t launch_fast_as(const enc::RowArgs& a, int sm_count, size_t scratch_w
     if (grid < 1) return cudaErrorInvalidValue;
     *grid_out = (int)grid;
     kern<<<(unsigned)grid, T, smem, st>>>(a);
+    return cudaGetLastError();
+}
+
+template <int LOGN>
+cudaError_t launch_mask(const enc::RowArgs& a, const enc::RowArgs& b, cudaStream_t st) {
+    using F = enc::Fast<LOGN>;
+    constexpr int T = fast_threads<LOGN>();
+    auto kern = k_encode_mask<LOGN, T, (T > 256 ? 1 : 512 / T)>;
+    const size_t smem = (size_t)(F::N + F::TW_WORDS) * 8;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    const u32 ctas_a = a.rows << a.logr, ctas_b = b.rows << b.logr;
+    kern<<<ctas_a + ctas_b, T, smem, st>>>(a, b, ctas_a);
     return cudaGetLastError();
 }
 
@@ -209,6 +237,17 @@ cudaError_t widen_rows(const unsigned char* narrow, const u64* row_off, const un
     if (blocks < 1) blocks = 1;
     k_widen_rows<<<(unsigned)blocks, 256, 0, st>>>(narrow, row_off, row_w, out, rows, n);
     return cudaGetLastError();
+}
+
+// both kinds of rows of a masking commitment in one launch; a scratch slot of T x N words for each (row, residue) of either, a's first
+cudaError_t encode_rows_mask(const enc::RowArgs& a, const enc::RowArgs& b, u32 logn, cudaStream_t st) {
+    switch (logn) {
+        case 8: return launch_mask<8>(a, b, st);
+        case 9: return launch_mask<9>(a, b, st);
+        case 10: return launch_mask<10>(a, b, st);
+        case 11: return launch_mask<11>(a, b, st);
+    }
+    return cudaErrorInvalidValue;
 }
 
 // the rows of a masking commitment (messages of 2^8 .. 2^11 words): FORM_COSET or FORM_COEF, always the fast path

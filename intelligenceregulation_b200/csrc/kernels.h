@@ -21,6 +21,7 @@ bool encode_split_pays(u32 logn, u32 logR, u32 rows, int sm_count);
 cudaError_t encode_rows(const enc::RowArgs& a, u32 logn, bool allow_fast, int sm_count, size_t scratch_words,
                         cudaStream_t st, int* path_out);
 cudaError_t widen_rows(const unsigned char* narrow, const u64* row_off, const unsigned char* row_w, u64* out, u32 rows, u32 n, int sm_count, cudaStream_t st);
+cudaError_t encode_rows_mask(const enc::RowArgs& a, const enc::RowArgs& b, u32 logn, cudaStream_t st);
 cudaError_t encode_rows_form(const enc::RowArgs& a, u32 logn, int form, int sm_count, size_t scratch_words, cudaStream_t st);
 
 // encode_tc.cu: the same rows on the tensor cores (rows of 2^10 words and more)

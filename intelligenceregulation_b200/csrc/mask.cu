@@ -27,67 +27,67 @@ struct Tw {
     }
 };
 
-// natural order in, bit-reversed order out
-__device__ void ntt_dif(u64* x, u32 logl, const Tw& t, bool inv) {
-    const u32 half_n = 1u << (logl - 1);
-    for (u32 s = logl; s >= 1; s--) {
-        const u32 half = 1u << (s - 1);
-        for (u32 p = threadIdx.x; p < half_n; p += blockDim.x) {
-            const u32 j = p & (half - 1), i = ((p >> (s - 1)) << s) + j;
-            const u64 u = x[i], v = x[i + half];
-            x[i] = gl_add(u, v);
-            x[i + half] = gl_mul(gl_sub(u, v), t.at(j << (logl - s), logl, inv));
-        }
-        __syncthreads();
+// One stage of a transform of 2^logl words by `nt` threads: of an inverse-order one (decimation in frequency: natural order in, bit-reversed
+// out, stages logl .. 1) or the other way (bit-reversed in, natural out, stages 1 .. logl).  Several transforms run side by side, a
+// group of threads each, between the same barriers.
+__device__ __forceinline__ void dif_stage(u64* x, u32 logl, u32 s, const Tw& t, bool inv, u32 tid, u32 nt) {
+    const u32 half = 1u << (s - 1);
+    for (u32 p = tid; p < (1u << (logl - 1)); p += nt) {
+        const u32 j = p & (half - 1), i = ((p >> (s - 1)) << s) + j;
+        const u64 u = x[i], v = x[i + half];
+        x[i] = gl_add(u, v);
+        x[i + half] = gl_mul(gl_sub(u, v), t.at(j << (logl - s), logl, inv));
+    }
+}
+__device__ __forceinline__ void dit_stage(u64* x, u32 logl, u32 s, const Tw& t, bool inv, u32 tid, u32 nt) {
+    const u32 half = 1u << (s - 1);
+    for (u32 p = tid; p < (1u << (logl - 1)); p += nt) {
+        const u32 j = p & (half - 1), i = ((p >> (s - 1)) << s) + j;
+        const u64 u = x[i], v = gl_mul(x[i + half], t.at(j << (logl - s), logl, inv));
+        x[i] = gl_add(u, v);
+        x[i + half] = gl_sub(u, v);
     }
 }
 
-// bit-reversed order in, natural order out
-__device__ void ntt_dit(u64* x, u32 logl, const Tw& t, bool inv) {
-    const u32 half_n = 1u << (logl - 1);
-    for (u32 s = 1; s <= logl; s++) {
-        const u32 half = 1u << (s - 1);
-        for (u32 p = threadIdx.x; p < half_n; p += blockDim.x) {
-            const u32 j = p & (half - 1), i = ((p >> (s - 1)) << s) + j;
-            const u64 u = x[i], v = gl_mul(x[i + half], t.at(j << (logl - s), logl, inv));
-            x[i] = gl_add(u, v);
-            x[i + half] = gl_sub(u, v);
-        }
-        __syncthreads();
-    }
-}
-
-// CTA s: the two planes of p_{a_s} p_{W_s} at the 2m points of the product domain, bit-reversed order
-__global__ void __launch_bounds__(256) k_mask_products(const u64* __restrict__ coefs /* rows of 2m */, const u64* __restrict__ ws /* S x m Fp2 */,
-                                                       u32 logm, Tw t, u64 minv, u64* __restrict__ partial /* S x 2 x 2m */) {
+// CTA s: the two planes of p_{a_s} p_{W_s} at the 2m points of the product domain, bit-reversed order.
+// What bounds it: its barriers, one per stage.  So four groups of 256 threads work side by side: two bring W back to coefficients and forward
+// again, 2 log m + 1 stages, the other two transform a meanwhile (one transform after the other, 6 log m + 4 stages by 256 threads: 24 masks
+// of 2^9 33 us, now 12).
+constexpr u32 MP_GROUP = 256;
+__global__ void __launch_bounds__(4 * MP_GROUP) k_mask_products(const u64* __restrict__ coefs /* rows of 2m */, const u64* __restrict__ ws /* S x m Fp2 */,
+                                                                u32 logm, Tw t, u64 minv, u64* __restrict__ partial /* S x 2 x 2m */) {
     extern __shared__ u64 sm[];
-    const u32 m = 1u << logm, m2 = 2 * m, s = blockIdx.x;
-    u64 *are = sm, *aim = sm + m2, *wre = sm + 2 * m2, *wim = sm + 3 * m2;
-    for (u32 i = threadIdx.x; i < m2; i += blockDim.x) {
-        are[i] = coefs[(size_t)(2 * s) * m2 + i];
-        aim[i] = coefs[(size_t)(2 * s + 1) * m2 + i];
-        wre[i] = 0;
-        wim[i] = 0;
+    const u32 m = 1u << logm, m2 = 2 * m, s = blockIdx.x, grp = threadIdx.x / MP_GROUP, tid = threadIdx.x % MP_GROUP;
+    u64* x = sm + grp * m2;  // a_re, a_im, W_re, W_im
+    const bool is_w = grp >= 2;
+    if (is_w) {
+        // p_W interpolates W on G_m (zk.rs:596-602): the inverse transform, its input placed in bit-reversed order
+        for (u32 i = tid; i < m; i += MP_GROUP) {
+            x[__brev(i) >> (32 - logm)] = ws[((size_t)s * m + i) * 2 + (grp - 2)];
+            x[m + i] = 0;
+        }
+    } else {
+        for (u32 i = tid; i < m2; i += MP_GROUP) x[i] = coefs[(size_t)(2 * s + grp) * m2 + i];
     }
     __syncthreads();
-    // p_W interpolates W on G_m (zk.rs:596-602): the inverse transform, its input placed in bit-reversed order
-    for (u32 i = threadIdx.x; i < m; i += blockDim.x) {
-        const u32 r = __brev(i) >> (32 - logm);
-        wre[r] = ws[((size_t)s * m + i) * 2];
-        wim[r] = ws[((size_t)s * m + i) * 2 + 1];
+    const u32 stages = 2 * logm + 1;
+    for (u32 k = 0; k < stages; k++) {
+        if (!is_w) {
+            if (k <= logm) dif_stage(x, logm + 1, logm + 1 - k, t, false, tid, MP_GROUP);
+        } else if (k < logm) {
+            dit_stage(x, logm, k + 1, t, true, tid, MP_GROUP);
+        } else if (k == logm) {  // the first forward stage: its upper half is zero, and the division by m rides on it
+            for (u32 j = tid; j < m; j += MP_GROUP) {
+                const u64 u = gl_mul(x[j], minv);
+                x[j] = u;
+                x[m + j] = gl_mul(u, t.at(j, logm + 1, false));
+            }
+        } else {
+            dif_stage(x, logm + 1, stages - k, t, false, tid, MP_GROUP);
+        }
+        __syncthreads();
     }
-    __syncthreads();
-    ntt_dit(wre, logm, t, true);
-    ntt_dit(wim, logm, t, true);
-    for (u32 i = threadIdx.x; i < m; i += blockDim.x) {
-        wre[i] = gl_mul(wre[i], minv);
-        wim[i] = gl_mul(wim[i], minv);
-    }
-    __syncthreads();
-    ntt_dif(are, logm + 1, t, false);
-    ntt_dif(aim, logm + 1, t, false);
-    ntt_dif(wre, logm + 1, t, false);
-    ntt_dif(wim, logm + 1, t, false);
+    const u64 *are = sm, *aim = sm + m2, *wre = sm + 2 * m2, *wim = sm + 3 * m2;
     u64* out = partial + (size_t)s * 2 * m2;
     for (u32 k = threadIdx.x; k < m2; k += blockDim.x) {
         const fp2 p = f2_mul(f2(are[k], aim[k]), f2(wre[k], wim[k]));  // (a_re + U a_im)(W_re + U W_im), U^2 = 7
@@ -96,28 +96,36 @@ __global__ void __launch_bounds__(256) k_mask_products(const u64* __restrict__ c
     }
 }
 
-// one CTA: sum of the S products, back to coefficients, plus b
+// one CTA: sum of the S products, back to coefficients, plus b.  Two groups, a plane each (side by side and eight loads in flight: 23 -> 13 us)
 __global__ void __launch_bounds__(1024) k_mask_q(const u64* __restrict__ partial, u32 S, const u64* __restrict__ b_re, const u64* __restrict__ b_im,
                                                  u32 logm, Tw t, u64 m2inv, u64* __restrict__ q /* 2m Fp2 */) {
     extern __shared__ u64 sm[];
-    const u32 m2 = 2u << logm;
-    u64 *re = sm, *im = sm + m2;
-    for (u32 k = threadIdx.x; k < m2; k += blockDim.x) {
-        u64 a = 0, b = 0;
-        for (u32 s = 0; s < S; s++) {
-            a = gl_add(a, partial[(size_t)s * 2 * m2 + k]);
-            b = gl_add(b, partial[(size_t)s * 2 * m2 + m2 + k]);
+    const u32 m2 = 2u << logm, grp = threadIdx.x / 512, tid = threadIdx.x % 512;
+    u64* x = sm + grp * m2;
+    for (u32 k = tid; k < m2; k += 512) {
+        const u64* p = partial + grp * m2 + k;
+        u64 a = 0;
+        for (u32 s0 = 0; s0 < S; s0 += 8) {
+            u64 v[8];
+#pragma unroll
+            for (u32 e = 0; e < 8; e++) v[e] = s0 + e < S ? p[(size_t)(s0 + e) * 2 * m2] : 0;
+#pragma unroll
+            for (u32 e = 0; e < 8; e++) a = gl_add(a, v[e]);
         }
-        re[k] = a;
-        im[k] = b;
+        x[k] = a;
     }
     __syncthreads();
-    ntt_dit(re, logm + 1, t, true);
-    ntt_dit(im, logm + 1, t, true);
-    for (u32 i = threadIdx.x; i < m2; i += blockDim.x) {
-        q[2 * i] = gl_add(gl_mul(re[i], m2inv), b_re[i]);
-        q[2 * i + 1] = gl_add(gl_mul(im[i], m2inv), b_im[i]);
+    for (u32 s = 1; s <= logm + 1; s++) {
+        dit_stage(x, logm + 1, s, t, true, tid, 512);
+        __syncthreads();
     }
+    const u64* b = grp ? b_im : b_re;
+    for (u32 i = tid; i < m2; i += 512) q[2 * i + grp] = gl_add(gl_mul(x[i], m2inv), b[i]);
+}
+
+// the first m words of every row of 2m, side by side
+__global__ void __launch_bounds__(256) k_mask_coefs(const u64* __restrict__ rows, u32 logm, size_t words, u64* __restrict__ out) {
+    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < words; i += (size_t)gridDim.x * 256) out[i] = rows[((i >> logm) << (logm + 1)) + (i & ((1u << logm) - 1u))];
 }
 
 }  // namespace
@@ -146,7 +154,9 @@ int hl_b200_mask_commit(hl_ctx* c, uint32_t log_msg, uint32_t log_dom, const uin
         return (ctas < most ? ctas : most) * per_cta;
     };
     const size_t msg_words = words_of(split_msg, n_msg_rows, m), coef_words = words_of(split_coef, n_coef_rows, m2);
-    const size_t scratch_words = msg_words > coef_words ? msg_words : coef_words;
+    // rows of both kinds side by side where each (row, residue) has a CTA that is resident at once
+    const bool both = split_msg && split_coef && ((n_msg_rows + n_coef_rows) << logr) <= (size_t)c->sm_count * 32;
+    const size_t scratch_words = both ? msg_words + coef_words : msg_words > coef_words ? msg_words : coef_words;
     int rc = root_powers(c, log_dom, &tw);
     if (!rc) rc = dev_alloc(c, (void**)&st->d_data, rows * m2 * 8);
     if (!rc) rc = dev_alloc(c, (void**)&st->d_enc, rows * dom * 8);
@@ -169,11 +179,17 @@ int hl_b200_mask_commit(hl_ctx* c, uint32_t log_msg, uint32_t log_dom, const uin
         a.ninv = gl_inv((u64)m);
         // message rows: m evaluations -> coefficients (kept) -> the coset
         a.data = d_msgs; a.enc = st->d_enc; a.rows = (u32)n_msg_rows; a.q = 0; a.T = 1; a.logr = logr; a.coef_out = st->d_data;
-        cudaError_t e = hlk::encode_rows_form(a, log_msg, enc::FORM_COSET, c->sm_count, scratch_words, c->stream);
+        const enc::RowArgs msg_rows = a;
+        cudaError_t e = both ? cudaSuccess : hlk::encode_rows_form(a, log_msg, enc::FORM_COSET, c->sm_count, scratch_words, c->stream);
         // coefficient rows: 2m coefficients -> the coset
         a.data = st->d_data + n_msg_rows * m2; a.enc = st->d_enc + n_msg_rows * dom; a.rows = (u32)n_coef_rows; a.q = (u32)m; a.T = 2; a.coef_out = nullptr; a.split = split_coef;
-        if (e == cudaSuccess) e = hlk::encode_rows_form(a, log_msg, enc::FORM_COEF, c->sm_count, scratch_words, c->stream);
-        c->stats.kernel_launches += 2;
+        if (both) {
+            a.scratch = scratch + msg_words;
+            e = hlk::encode_rows_mask(msg_rows, a, log_msg, c->stream);
+        } else if (e == cudaSuccess) {
+            e = hlk::encode_rows_form(a, log_msg, enc::FORM_COEF, c->sm_count, scratch_words, c->stream);
+        }
+        c->stats.kernel_launches += both ? 1 : 2;
         if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "mask_commit: row encoder launch", e);
     }
     if (!rc) {
@@ -183,9 +199,14 @@ int hl_b200_mask_commit(hl_ctx* c, uint32_t log_msg, uint32_t log_dom, const uin
         if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "mask_commit: column hash launch", e);
     }
     if (!rc && a_coefs) {
-        cudaError_t e = cudaMemcpy2DAsync(a_coefs, m * 8, st->d_data, m2 * 8, m * 8, n_msg_rows, cudaMemcpyDeviceToHost, c->stream);
-        c->stats.bytes_d2h += n_msg_rows * m * 8;
-        if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "mask_commit: coefficient read", e);
+        // gathered in the messages' place, which nothing reads any more, so that one plain copy brings them (the strided one into pageable
+        // memory went row by row)
+        const size_t words = n_msg_rows * m, blocks = (words + 255) / 256, most = (size_t)c->sm_count * 8;
+        k_mask_coefs<<<(unsigned)(blocks < most ? blocks : most), 256, 0, c->stream>>>(st->d_data, log_msg, words, d_msgs);
+        c->stats.kernel_launches++;
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "mask_commit: coefficient launch", e);
+        if (!rc) rc = d2h(c, a_coefs, d_msgs, words * 8);
     }
     if (!rc) rc = d2h(c, leaves32, st->d_leaves, dom * 32);
     if (!rc) rc = sync(c, "mask_commit");
@@ -222,7 +243,7 @@ int hl_b200_mask_open_q(hl_store* st, size_t n_masks, const uint64_t* ws, uint64
         const size_t sm1 = 4 * m2 * 8, sm2 = 2 * m2 * 8;
         cudaError_t e = cudaFuncSetAttribute(k_mask_products, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm1);
         if (e == cudaSuccess) {
-            k_mask_products<<<(unsigned)n_masks, 256, sm1, c->stream>>>(st->d_data, d_ws, logm, T, gl_inv((u64)m), d_part);
+            k_mask_products<<<(unsigned)n_masks, 4 * MP_GROUP, sm1, c->stream>>>(st->d_data, d_ws, logm, T, gl_inv((u64)m), d_part);
             e = cudaGetLastError();
         }
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k_mask_q, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2);
