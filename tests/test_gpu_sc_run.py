@@ -96,3 +96,24 @@ def test_a_wait_that_runs_out_is_reported(ctx, oracle, limits, nd, parts):
         c = what.coef_array()
         oracle.ir_set(what.words(), what.n_nodes, what.n_terms)
     _check(ctx, oracle, oracle.POLY_IR if parts else oracle.POLY_ZC, tables, deg, n, [n], what=what if parts else None, coefs=c)
+
+
+@pytest.mark.parametrize("n", [6, 13])  # the one launch's evaluator, and the long rounds' before it
+def test_products_of_words_at_the_carries(ctx, oracle, n):
+    """Extension products whose partial sums carry, or do not, in every column: entries from the ends of the 32-bit halves."""
+    from intelligenceregulation_b200 import backend
+
+    P = 0xFFFFFFFF00000001
+    edge = np.array([0, 1, 7, 2**32 - 1, 2**32, 2**32 + 1, 2**63, P - 2**32, P - 2**32 + 1, P - 2, P - 1], dtype=np.uint64)
+    tables = np.random.default_rng(n).choice(edge, size=(4, 1 << n, 2))
+    p = backend.SlotProgram(4)
+    p.term((P - 1, P - 1), [0], [1, 2, 3])
+    o, tr = oracle, oracle.Transcript(b"sc-run")
+    scaled = tables.copy()  # the coefficient goes with the first table in the oracle
+    scaled[0] = np.array([o.fp2_mul((P - 1, P - 1), tuple(map(int, x))) for x in tables[0]], dtype=np.uint64)
+    t_cpu = tr.clone()
+    want = o.sc_prove(0, scaled, 4, t_cpu)
+    ev = backend.B200Rounds(ctx, p, tables, 4)
+    got = ev.batched(n, tr.state, tr.counter, None)
+    assert (got[0] == want.rounds).all() and got[3] == t_cpu.state
+    ev.free()
