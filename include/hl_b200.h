@@ -55,6 +55,8 @@ const char* hl_b200_label(hl_ctx* ctx);
 const char* hl_b200_last_error(hl_ctx* ctx);
 /* Run the context's work on the caller's CUDA stream (a cudaStream_t); NULL restores its own. */
 int hl_b200_set_stream(hl_ctx* ctx, void* cuda_stream);
+/* Waits for everything that is queued.  HL_B200_ERR_TIMEOUT, once: the row encoder of an asynchronous commitment (hl_b200_commit_zk_dev) gave
+ * up a bounded wait since this was last asked, whether its store still lives or not. */
 int hl_b200_sync(hl_ctx* ctx);
 /* Failure injection on the HOST side (hashline/src/gpu/mod.rs:121 set_alloc_cap_for_test): with a cap, a device
  * allocation that would bring the context's live bytes above `bytes` fails with HL_B200_ERR_OOM before the
@@ -114,7 +116,8 @@ int hl_b200_commit_zk_packed(hl_ctx* ctx, uint32_t log_cols, uint32_t inv_rate, 
 /* The same commitment for inputs that already live in device memory (the reference's
  * device-buffer commitment, pcs.rs:801-803 / metal.rs:3105 resident rows).  Asynchronous on
  * the context's stream; d_leaves32 (nn x 32 bytes, device) is ready when the stream reaches
- * this point.  The store BORROWS d_data and d_pads: keep them alive until it is freed. */
+ * this point.  The store BORROWS d_data and d_pads: keep them alive until it is freed.
+ * Where the encoder gives up a bounded wait, hl_b200_sync answers HL_B200_ERR_TIMEOUT, and so does every call on the store that waits. */
 int hl_b200_commit_zk_dev(hl_ctx* ctx, uint32_t log_cols, uint32_t inv_rate, const uint64_t* d_data, size_t rows,
                           const uint64_t* d_pads, size_t q, const uint64_t* d_pows, const uint8_t* key32,
                           hl_store** store, uint8_t* d_leaves32);

@@ -73,16 +73,34 @@ int root_powers(hl_ctx* c, u32 lognn, const u64** out) {
     return HL_B200_OK;
 }
 
-// the tensor-core encoder's tables for rows of 2^logn words at rate 2^-logr, made once per size, and its error word
-int encoder_tables(hl_ctx* c, u32 logn, u32 logr, const u64** out) {
-    if (!c->enc_flag) {
-        if (cudaHostAlloc((void**)&c->enc_flag, 4, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
-            c->enc_flag = nullptr;
+// a word in which the tensor-core encoder tells that it gave up on this store
+int encoder_word(hl_ctx* c, hl_store* st) {
+    if (c->enc_words.empty()) {
+        u32* block = nullptr;
+        if (cudaHostAlloc((void**)&block, 4096, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
             cudaGetLastError();
-            return fail(c, HL_B200_ERR_OOM, "encoder status word");
+            return fail(c, HL_B200_ERR_OOM, "encoder status words");
         }
-        *c->enc_flag = 0;
+        memset(block, 0, 4096);
+        c->enc_blocks.push_back(block);
+        for (u32 i = c->enc_later ? 0 : 1; i < 1024; i++) c->enc_words.push_back(block + i);
+        if (!c->enc_later) c->enc_later = block;
     }
+    st->enc_word = c->enc_words.back();
+    c->enc_words.pop_back();
+    if (++c->enc_mark == 0) c->enc_mark = 1;
+    st->enc_mark = c->enc_mark;
+    return HL_B200_OK;
+}
+
+static const char* const ENCODER_GAVE_UP = "row encoder: a bounded wait on the tensor-core pipeline ran out";
+int encoded_ok(hl_ctx* c, const hl_store* st) {
+    if (!st->enc_word || *reinterpret_cast<volatile u32*>(st->enc_word) != st->enc_mark) return HL_B200_OK;
+    return fail(c, HL_B200_ERR_TIMEOUT, ENCODER_GAVE_UP);
+}
+
+// the tensor-core encoder's tables for rows of 2^logn words at rate 2^-logr, made once per size
+int encoder_tables(hl_ctx* c, u32 logn, u32 logr, const u64** out) {
     const u32 key = logn + 64 * logr;
     auto it = c->enc_tables.find(key);
     if (it != c->enc_tables.end()) { *out = it->second; return HL_B200_OK; }
@@ -197,7 +215,7 @@ void hl_b200_shutdown(hl_ctx* c) {
     cudaStreamSynchronize(c->stream);
     for (auto& kv : c->tw) cudaFree(kv.second);
     for (auto& kv : c->enc_tables) cudaFree(kv.second);
-    if (c->enc_flag) cudaFreeHost(c->enc_flag);
+    for (u32* b : c->enc_blocks) cudaFreeHost(b);
     if (c->wp_flag) cudaFreeHost(c->wp_flag);
     host_copy_release(c);
     if (c->up.mem) cudaFreeHost(c->up.mem);
@@ -234,7 +252,12 @@ int hl_b200_set_stream(hl_ctx* c, void* s) {
 int hl_b200_sync(hl_ctx* c) {
     if (!c) return HL_B200_ERR_ARG;
     Call g(c);
-    return sync(c, "synchronize");
+    int rc = sync(c, "synchronize");
+    if (!rc && c->enc_later && *reinterpret_cast<volatile u32*>(c->enc_later)) {
+        *c->enc_later = 0;  // told once
+        rc = fail(c, HL_B200_ERR_TIMEOUT, ENCODER_GAVE_UP);
+    }
+    return rc;
 }
 
 int hl_b200_set_alloc_cap(hl_ctx* c, size_t bytes) {
@@ -247,6 +270,13 @@ int hl_b200_set_alloc_cap(hl_ctx* c, size_t bytes) {
 int hl_b200_set_encoder(hl_ctx* c, int fast) {
     if (!c) return HL_B200_ERR_ARG;
     c->fast_encoder = fast != 0;
+    return HL_B200_OK;
+}
+
+int hl_b200_set_encoder_wait_limit(hl_ctx* c, uint32_t looks) {
+    if (!c) return HL_B200_ERR_ARG;
+    Call g(c);
+    c->enc_limit = looks;
     return HL_B200_OK;
 }
 

@@ -29,7 +29,12 @@ struct hl_ctx {
     std::mutex err_mu;       // guards last_error and stats.declines: a decline may be recorded before `mu` is taken, from any thread
     std::map<u32, u64*> tw;  // log2 nn -> nn powers of the nn-th root
     std::map<u32, u64*> enc_tables;  // log2 n + 64 log2 rate -> the tensor-core encoder's constants
-    int* enc_flag = nullptr;         // page-locked: the tensor-core encoder's error word (a bounded wait ran out): read at every synchronisation
+    // Where the tensor-core encoder tells that a bounded wait ran out: a page-locked word for each of its stores, into which the store's own
+    // mark is written, so that a word can go on to the next store while the last one's kernels are still queued; and one that asynchronous
+    // commitments set as well, which hl_b200_sync reads
+    std::vector<u32*> enc_blocks, enc_words;  // 1,024 words each; those that no store has
+    u32* enc_later = nullptr;
+    u32 enc_mark = 0, enc_limit = 1u << 22;
     std::string label, last_error;
     hl_stats stats{};
     bool timing = false;
@@ -66,6 +71,8 @@ struct hl_store {
     ColOrder order;
     uint32_t* d_leaves = nullptr; // nn x 8 words, unsalted
     int encoder_path = -1;
+    u32* enc_word = nullptr;      // holds enc_mark: the encoder gave up, nothing of the encoding is valid (encoded_ok)
+    u32 enc_mark = 0;
     size_t n() const { return (size_t)1 << logn; }
     size_t nn() const { return (size_t)1 << (logn + logr); }
 };
@@ -108,6 +115,8 @@ struct Call {
 };
 int root_powers(hl_ctx* c, u32 lognn, const u64** out);
 int encoder_tables(hl_ctx* c, u32 logn, u32 logr, const u64** out);
+int encoder_word(hl_ctx* c, hl_store* st);
+int encoded_ok(hl_ctx* c, const hl_store* st);  // asked once the encoding has been waited for: HL_B200_ERR_TIMEOUT if the encoder gave up
 int upload_key(hl_ctx* c, const uint8_t* key32, uint32_t** d_key);
 int log2_exact(size_t v);
 void store_release(hl_store* st);  // frees a store; the caller holds the context's lock

@@ -161,12 +161,16 @@ int commit_on_device(hl_ctx* c, hl_store* st, const u64* d_pows, const uint8_t* 
     size_t scratch_words = hlk::encode_scratch_words(logb, T, c->sm_count, st->rows);
     const bool tc = c->fast_encoder && hlk::encode_tc_takes(logn, st->logr, st->rows, c->sm_count);
     const u64* tc_tab = nullptr;
+    hlk::TcReport report;
+    const bool later = !h_data && leaves;  // hl_b200_commit_zk_dev, which returns before its kernels have run
     st->order = ColOrder();
     if (tc) {
         st->order.logn = logn;
         st->order.logr = st->logr;
         rc = encoder_tables(c, logn, st->logr, &tc_tab);
+        if (!rc) rc = encoder_word(c, st);
         if (rc) return rc;
+        report = {st->enc_word, st->enc_mark, later ? c->enc_later : nullptr, c->enc_limit};
         const size_t w = hlk::encode_tc_scratch_words(logn, st->logr, st->q, st->rows, c->sm_count);
         if (w > scratch_words) scratch_words = w;
     }
@@ -270,7 +274,7 @@ int commit_on_device(hl_ctx* c, hl_store* st, const u64* d_pows, const uint8_t* 
             if (fused_widen) { a.narrow = d_narrow; a.row_off = d_row_off + r0; a.row_w = d_row_w + r0; }
             // a handful of rows (a boundary commitment, the last piece of an upload): one CTA per (row, residue)
             a.split = hlk::encode_split_pays(logb, st->logr, nr, c->sm_count) ? 1 : 0;
-            cudaError_t e = tc ? hlk::encode_rows_tc(a, logn, tc_tab, c->sm_count, scratch_words, c->enc_flag, c->stream, &st->encoder_path)
+            cudaError_t e = tc ? hlk::encode_rows_tc(a, logn, tc_tab, c->sm_count, scratch_words, report, c->stream, &st->encoder_path)
                                : hlk::encode_rows(a, logb, c->fast_encoder || loga, c->sm_count, scratch_words, c->stream, &st->encoder_path);
             c->stats.kernel_launches += 1;
             if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "row encoder launch", e);
@@ -328,6 +332,7 @@ int check_shape(hl_ctx* c, uint32_t log_cols, uint32_t inv_rate, size_t rows, si
 void free_store(hl_store* st) {
     hl_ctx* c = st->ctx;
     c->stores.erase(st);
+    if (st->enc_word) c->enc_words.push_back(st->enc_word);
     if (st->owns_inputs) {
         dev_free(c, st->d_data, (size_t)st->rows * st->n() * 8);
         dev_free(c, st->d_pads, (size_t)st->rows * st->q * 8);
@@ -366,6 +371,7 @@ int commit_host(hl_ctx* c, const Shape& s, const HostRows& data, const uint64_t*
     if (!rc && leaves32) rc = d2h(c, leaves32, st->d_leaves, nn * 32);
     if (!rc && tree) rc = d2h(c, tree->levels_out, d_levels, (2 * nn - 1) * 32);
     if (!rc) rc = sync(c, "commit");
+    if (!rc) rc = encoded_ok(c, st);
     if (!rc && tree) c->stats.merkles++;
     if (d_pows) dev_free(c, d_pows, nn * 8);
     if (d_salts) dev_free(c, d_salts, nn * 32);
@@ -509,6 +515,7 @@ const uint64_t* hl_b200_store_encoded_dev(hl_store* st) {
             if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "column order launch", e);
         }
         if (!rc) rc = sync(c, "store_encoded_dev");
+        if (!rc) rc = encoded_ok(c, st);
         dev_free(c, d_rows, bytes);
         if (rc) return nullptr;
         st->order = ColOrder();
@@ -566,6 +573,7 @@ int hl_b200_store_fold(hl_store* st, const uint64_t* rhos, size_t k, int with_pa
     if (!rc) rc = back(0, first, c->stream);
     if (!rc) rc = back(first + sparse_done, (u32)k, c->stream);
     if (!rc) rc = sync(c, "store_fold");
+    if (!rc) rc = encoded_ok(c, st);
     plan.release();
     if (d_out) dev_free(c, d_out, ob);
     if (!rc) c->stats.folds++;
@@ -594,6 +602,7 @@ int hl_b200_store_columns(hl_store* st, const uint64_t* idx, size_t nidx, uint64
     }
     if (!rc) rc = d2h(c, out, d_out, ob);
     if (!rc) rc = sync(c, "store_columns");
+    if (!rc) rc = encoded_ok(c, st);
     dev_free(c, d_idx, nidx * 8); dev_free(c, d_out, ob);
     if (!rc) c->stats.gathers++;
     return rc;
@@ -638,7 +647,8 @@ int hl_b200_store_merkle(hl_store* st, const uint8_t* salts32, const uint8_t* le
     if (!st || !levels_out) return HL_B200_ERR_ARG;
     hl_ctx* c = st->ctx;
     Call g(c);
-    return merkle_common(c, st->d_leaves, nullptr, salts32, st->nn(), leaf_key32, node_key32, levels_out);
+    const int rc = merkle_common(c, st->d_leaves, nullptr, salts32, st->nn(), leaf_key32, node_key32, levels_out);
+    return rc ? rc : encoded_ok(c, st);
 }
 
 int hl_b200_store_merkle_dev(hl_store* st, const uint8_t* d_salts32, const uint8_t* leaf_key32, const uint8_t* node_key32,
@@ -648,7 +658,8 @@ int hl_b200_store_merkle_dev(hl_store* st, const uint8_t* d_salts32, const uint8
     // the tree kernels move digests as 16-byte vectors: a misaligned caller pointer would be a device fault, not a status
     if (((uintptr_t)d_levels_out & 15) || ((uintptr_t)d_salts32 & 15)) return fail(c, HL_B200_ERR_ARG, "store_merkle_dev: device pointers must be 16-byte aligned");
     Call g(c);
-    int rc = merkle_on_device(c, st->d_leaves, (const uint32_t*)d_salts32, st->nn(), leaf_key32, node_key32, (uint32_t*)d_levels_out);
+    int rc = encoded_ok(c, st);  // where that is known already
+    if (!rc) rc = merkle_on_device(c, st->d_leaves, (const uint32_t*)d_salts32, st->nn(), leaf_key32, node_key32, (uint32_t*)d_levels_out);
     if (!rc) c->stats.merkles++;
     return rc;
 }

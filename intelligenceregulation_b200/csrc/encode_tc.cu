@@ -45,9 +45,9 @@ __device__ __forceinline__ void tc_arrive(u32 bar) { asm volatile("mbarrier.arri
 // the words 1,498; the later residues' words by asynchronous copies, twiddles asked for half a product ahead 1,479; residues apart in the output
 // 1,338.  Montgomery's reduction saves a seventh of the products' instructions and no time: they are not what it waits for.
 // Every wait is bounded: one that runs out sets `gave_up`, after which nobody waits and no product is issued; the CTA walks to its
-// end (all addresses are the same), waits for the products in flight and frees TMEM, and the host reads the error word.
+// end (all addresses are the same), waits for the products in flight and frees TMEM, and leaves the store's mark where the host reads it.
 template <int LOGN, bool NARROW>
-__global__ void __launch_bounds__(TC_THREADS, 1) k_encode_tc(RowArgs a, const u64* __restrict__ tab, int* __restrict__ err) {
+__global__ void __launch_bounds__(TC_THREADS, 1) k_encode_tc(RowArgs a, const u64* __restrict__ tab, const hlk::TcReport report) {
     using T = Tc<LOGN>;
     extern __shared__ __align__(16) unsigned char raw[];
     __shared__ __align__(8) u64 bars[BAR_COUNT];
@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_encode_tc(RowArgs a, const u6
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
     const u32 tmem = tmem_slot;
     auto wait = [&](u32 i, u32 parity) {
-        for (u32 spin = 0; spin < UM_SPIN_LIMIT; spin++) {
+        for (u32 spin = 0; spin < report.limit; spin++) {
             if (um_try_wait(bar(i), parity)) return;
             if ((spin & 63) == 63 && gave_up) return;
         }
@@ -426,7 +426,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_encode_tc(RowArgs a, const u6
     if (tid == 32 * TC_WORKERS) {
         um_commit(bar(BAR_DONE));
         if (!um_wait(bar(BAR_DONE), 0)) gave_up = 1;
-        if (gave_up) *reinterpret_cast<volatile int*>(err) = 1;
+        if (gave_up) {
+            *reinterpret_cast<volatile u32*>(report.word) = report.mark;
+            if (report.also) *reinterpret_cast<volatile u32*>(report.also) = 1;
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
     __syncthreads();
@@ -434,12 +437,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_encode_tc(RowArgs a, const u6
 }
 
 template <int LOGN, bool NARROW>
-cudaError_t launch_tc(const RowArgs& a, const u64* tab, unsigned grid, int* err, cudaStream_t st) {
+cudaError_t launch_tc(const RowArgs& a, const u64* tab, unsigned grid, const hlk::TcReport& report, cudaStream_t st) {
     auto kern = k_encode_tc<LOGN, NARROW>;
     const int smem = (int)TC_SMEM + 1024;
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    kern<<<grid, TC_THREADS, smem, st>>>(a, tab, err);
+    kern<<<grid, TC_THREADS, smem, st>>>(a, tab, report);
     return cudaGetLastError();
 }
 
@@ -477,7 +480,7 @@ size_t encode_tc_scratch_words(u32 logn, u32 logr, u32 q, u32 rows, int sm_count
     return (ctas < (size_t)sm_count ? ctas : (size_t)sm_count) * tc_slot_words(logn, 1u << logr, q);
 }
 
-cudaError_t encode_rows_tc(RowArgs a, u32 logn, const u64* tab, int sm_count, size_t scratch_words, int* err, cudaStream_t st, int* path_out) {
+cudaError_t encode_rows_tc(RowArgs a, u32 logn, const u64* tab, int sm_count, size_t scratch_words, TcReport report, cudaStream_t st, int* path_out) {
     const u64 batches = tc_batches(logn, a.rows), sms = (u64)sm_count, split_units = batches << a.logr;
     a.split = a.logr >= 1 && (split_units + sms - 1) / sms * 2 < (batches + sms - 1) / sms * (1 + ((u64)1 << a.logr));
     u64 grid = a.split ? split_units : batches;
@@ -488,11 +491,11 @@ cudaError_t encode_rows_tc(RowArgs a, u32 logn, const u64* tab, int sm_count, si
     if (path_out) *path_out = a.narrow ? 2 : 1;
     const unsigned gr = (unsigned)grid;
     switch (logn) {
-        case 10: return a.narrow ? launch_tc<10, true>(a, tab, gr, err, st) : launch_tc<10, false>(a, tab, gr, err, st);
-        case 11: return a.narrow ? launch_tc<11, true>(a, tab, gr, err, st) : launch_tc<11, false>(a, tab, gr, err, st);
-        case 12: return a.narrow ? launch_tc<12, true>(a, tab, gr, err, st) : launch_tc<12, false>(a, tab, gr, err, st);
-        case 13: return a.narrow ? launch_tc<13, true>(a, tab, gr, err, st) : launch_tc<13, false>(a, tab, gr, err, st);
-        case 14: return a.narrow ? launch_tc<14, true>(a, tab, gr, err, st) : launch_tc<14, false>(a, tab, gr, err, st);
+        case 10: return a.narrow ? launch_tc<10, true>(a, tab, gr, report, st) : launch_tc<10, false>(a, tab, gr, report, st);
+        case 11: return a.narrow ? launch_tc<11, true>(a, tab, gr, report, st) : launch_tc<11, false>(a, tab, gr, report, st);
+        case 12: return a.narrow ? launch_tc<12, true>(a, tab, gr, report, st) : launch_tc<12, false>(a, tab, gr, report, st);
+        case 13: return a.narrow ? launch_tc<13, true>(a, tab, gr, report, st) : launch_tc<13, false>(a, tab, gr, report, st);
+        case 14: return a.narrow ? launch_tc<14, true>(a, tab, gr, report, st) : launch_tc<14, false>(a, tab, gr, report, st);
     }
     return cudaErrorInvalidValue;
 }

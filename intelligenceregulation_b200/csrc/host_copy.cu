@@ -466,10 +466,6 @@ int sync(hl_ctx* c, const char* what) {
     drop_pending(c);
     c->up.off = c->down.off = 0;
     if (e != cudaSuccess) return fail(c, HL_B200_ERR_DEVICE, what, e);
-    if (c->enc_flag && *reinterpret_cast<volatile int*>(c->enc_flag)) {
-        *c->enc_flag = 0;  // told once
-        return fail(c, HL_B200_ERR_TIMEOUT, "row encoder: a bounded wait on the tensor-core pipeline ran out");
-    }
     return HL_B200_OK;
 }
 

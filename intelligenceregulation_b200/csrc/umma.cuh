@@ -4,7 +4,7 @@
 #include "gl_field.cuh"
 
 constexpr u32 UM_SBO = 1024;  // bytes between 8-row groups of an operand
-constexpr u32 UM_SPIN_LIMIT = 1u << 22;
+constexpr u32 UM_SPIN_LIMIT = 1u << 22;  // some seconds
 
 // K-major operand with the 128-byte swizzle: rows of 128 bytes, 8-row groups UM_SBO apart, a K step of 32 bytes is 32 bytes further
 // along the row.  Start address and stride byte offset in 16-byte units (the leading offset is not used by a swizzled K-major operand

@@ -184,6 +184,7 @@ static int verify_columns_locked(hl_ctx* c, const uint64_t* cols, size_t rows, s
     }
     if (!rc) rc = d2h(c, verdict, d_verdict, ncols * 4);
     if (!rc) rc = sync(c, "verify_columns");
+    if (!rc && vec_store) rc = encoded_ok(c, vec_store);
     if (!rc && first_bad) {
         *first_bad = -1;
         for (size_t i = 0; i < ncols; i++)

@@ -3,6 +3,7 @@
 //                              a copy uses it, no copy uses the caller's memory once the call is over, and nothing is lost
 //   host_api_emul copies       the bytes of copies of all sizes and alignments
 //   host_api_emul threads N    the same where the process can make only N threads
+//   host_api_emul timeouts     who is told that a row encoder's bounded wait ran out
 #include "fake_cuda.h"
 
 #include <dlfcn.h>
@@ -32,7 +33,14 @@ void encode_tc_build(u32, u32, u64* out) { for (int i = 0; i < 8; i++) out[i] = 
 bool encode_tc_takes(u32 logn, u32, u32, int) { return logn >= 10; }
 u32 encode_tc_rows(u32 logn) { return 16384u >> logn; }
 size_t encode_tc_scratch_words(u32, u32, u32, u32, int) { return 64; }
-cudaError_t encode_rows_tc(enc::RowArgs, u32, const u64*, int, size_t, int*, cudaStream_t, int*) { return launch(); }
+static bool g_gives_up = false;  // the encoder's waits run out
+cudaError_t encode_rows_tc(enc::RowArgs, u32, const u64*, int, size_t, TcReport r, cudaStream_t, int*) {
+    if (g_gives_up) {
+        *r.word = r.mark;
+        if (r.also) *r.also = 1;
+    }
+    return launch();
+}
 u32 natural_order_rows(u32, int) { return 1; }
 cudaError_t natural_order(u64*, u32, size_t, ColOrder, u64*, u32, cudaStream_t) { return launch(); }
 cudaError_t widen_rows(const unsigned char*, const u64*, const unsigned char*, u64*, u32, u32, int, cudaStream_t) { return launch(); }
@@ -190,6 +198,74 @@ static void areas() {
     hl_b200_shutdown(c);
 }
 
+// A wait of the encoder that runs out is told to the calls on that store, and for an asynchronous commitment to hl_b200_sync, once; never to
+// another call.
+static void timeouts() {
+    hl_ctx* c = nullptr;
+    hl_b200_init(0, &c);
+    const u32 rows = 6, lc = 12, q = 40;
+    const size_t n = (size_t)1 << lc, nn = 2 * n;
+    Host h(false);
+    uint64_t *data = h.words(rows * n), *pads = h.words(rows * q), *pows = h.words(nn), *idx = h.words(1), *got = h.words(rows), *rhos = h.words(rows * 2);
+    uint64_t *out = h.words((n + q) * 2);
+    uint8_t *leaves = h.bytes(nn * 32), *levels = h.bytes((2 * nn - 1) * 32);
+    idx[0] = 1;
+    auto host = [&](bool gives_up, hl_store** st) {
+        hlk::g_gives_up = gives_up;
+        return hl_b200_commit_zk(c, lc, 2, data, rows, pads, q, pows, lc + 1, nullptr, st, leaves);
+    };
+    auto dev = [&](bool gives_up, hl_store** st) {
+        hlk::g_gives_up = gives_up;
+        return hl_b200_commit_zk_dev(c, lc, 2, data, rows, pads, q, pows, nullptr, st, nullptr);
+    };
+    auto is = [&](int rc, int want, const char* what) {
+        if (rc != want) bad("timeouts", std::string(what) + " answers " + std::to_string(rc));
+    };
+    hl_store *lost = nullptr, *fine = nullptr, *none = nullptr;
+    is(dev(true, &lost), 0, "an asynchronous commitment that will give up");
+    is(host(false, &fine), 0, "another commitment");
+    is(hl_b200_store_columns(fine, idx, 1, got), 0, "the other store's columns");
+    for (int again = 0; again < 2; again++) {
+        is(hl_b200_store_columns(lost, idx, 1, got), HL_B200_ERR_TIMEOUT, "columns");
+        is(hl_b200_store_fold(lost, rhos, 1, 1, out), HL_B200_ERR_TIMEOUT, "fold");
+        is(hl_b200_store_merkle(lost, nullptr, nullptr, nullptr, levels), HL_B200_ERR_TIMEOUT, "tree");
+        if (hl_b200_store_encoded_dev(lost)) bad("timeouts", "the encoding is given out");
+    }
+    is(hl_b200_sync(c), HL_B200_ERR_TIMEOUT, "sync");
+    is(hl_b200_sync(c), 0, "sync, later");
+    hl_b200_store_free(lost);
+    is(dev(true, &lost), 0, "an asynchronous commitment that will give up");
+    hl_b200_store_free(lost);
+    is(host(false, &lost), 0, "a commitment after it");
+    is(hl_b200_store_columns(lost, idx, 1, got), 0, "its columns");
+    is(hl_b200_sync(c), HL_B200_ERR_TIMEOUT, "sync for a store that is gone");
+    hl_b200_store_free(lost);
+    is(host(true, &none), HL_B200_ERR_TIMEOUT, "a commitment that gives up");
+    if (none) bad("timeouts", "a failed commitment left a store");
+    is(hl_b200_sync(c), 0, "sync after a commitment that told it itself");
+    for (long at = 0; at < 200; at++) {  // whatever else fails in a call whose encoder gives up, the next call does not hear of it
+        fake::calls = 0;
+        fake::fail_at = at;
+        hl_store* st = nullptr;
+        host(true, &st);
+        fake::fail_at = -1;
+        is(hl_b200_store_columns(fine, idx, 1, got), 0, "another store's columns after a call that failed");
+        is(hl_b200_sync(c), 0, "sync after a call that failed");
+    }
+    for (int i = 0; i < 3000; i++) {  // more words than a block holds, given back in between
+        hl_store* st = nullptr;
+        is(dev(false, &st), 0, "a commitment");
+        hl_b200_store_free(st);
+    }
+    std::vector<hl_store*> many(2500);
+    for (auto& st : many) is(dev(false, &st), 0, "a commitment");
+    is(hl_b200_sync(c), 0, "sync");
+    for (auto& st : many) hl_b200_store_free(st);
+    hl_b200_store_free(fine);
+    hlk::g_gives_up = false;
+    hl_b200_shutdown(c);
+}
+
 int main(int argc, char** argv) {
     if (argc == 3 && !strcmp(argv[1], "threads")) {
         g_threads = atol(argv[2]);
@@ -198,6 +274,8 @@ int main(int argc, char** argv) {
         sizes(false);
         sizes(true);
         areas();
+    } else if (argc == 2 && !strcmp(argv[1], "timeouts")) {
+        timeouts();
     } else {
         failures(false);
         failures(true);

@@ -97,3 +97,44 @@ def test_rows_on_8_byte_boundaries(dev, oracle):
     assert (store.columns(idx) == oracle.gather_columns(want, rows, 2 * n, idx)).all()
     assert (out.cpu().numpy() == oracle.hash_columns(want, rows, 2 * n)).all()
     store.free()
+
+
+def test_a_wait_that_runs_out_is_told_to_its_own_store(dev, oracle):
+    """The kernel looks at its barriers no more than it is let: its CTAs give up, walk to their end and leave the machine as it was.  The store
+    answers nothing but that status, another store made beside it and one made afterwards are whole."""
+    from intelligenceregulation_b200 import backend
+
+    rows, n, ctx = 160, 1 << 14, dev.ctx
+    rng = np.random.default_rng(11)
+    data = rng.integers(0, P, size=rows * n, dtype=np.uint64)
+    idx = np.array([0, 5, 2 * n - 1], dtype=np.uint64)
+    want = oracle.gather_columns(oracle.encode_rows_plain(data, rows, n, 2 * n, 18), rows, 2 * n, idx)
+
+    import torch
+
+    d = torch.from_numpy(data.view(np.int64)).cuda()
+    p, h = torch.zeros(rows, dtype=torch.int64, device="cuda"), torch.ones(2 * n, dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    commit = lambda: dev.commit_zk_dev(14, 2, d.data_ptr(), rows, p.data_ptr(), 1, h.data_ptr(), None)
+    fine = commit()
+    ctx.check(ctx.lib.hl_b200_set_encoder_wait_limit(ctx.h, 0))
+    try:
+        lost, gone = commit(), commit()
+        gone.free()
+        assert dev.try_commit(14, 2, data, 18) is None and "wait" in dev.ctx.declines[-1][1]
+    finally:
+        ctx.check(ctx.lib.hl_b200_set_encoder_wait_limit(ctx.h, 1 << 22))
+    assert (fine.columns(idx) == want).all()
+    later, _ = dev.try_commit(14, 2, data, 18)
+    assert (later.columns(idx) == want).all()
+    for _ in range(2):
+        for ask in (lambda: lost.columns(idx), lambda: lost.merkle(None, None, None), lambda: lost.fold_rows(np.ones((1, rows, 2), dtype=np.uint64))):
+            with pytest.raises(backend.DeviceError) as e:
+                ask()
+            assert e.value.code == -4
+    with pytest.raises(backend.DeviceError) as e:
+        ctx.sync()
+    assert e.value.code == -4
+    ctx.sync()
+    for s in (fine, later, lost):
+        s.free()

@@ -29,6 +29,10 @@ def test_a_failing_call_leaves_no_copy_behind(emul):
     _ok(emul, "failures")
 
 
+def test_an_encoder_wait_that_runs_out_is_told_to_its_own_store(emul):
+    _ok(emul, "timeouts")
+
+
 def test_copies_of_all_sizes(emul):
     """the limits between the forms of a copy, unaligned ends, and more small copies in a call than the bounce areas hold"""
     _ok(emul, "copies")
