@@ -165,7 +165,8 @@ int hl_b200_store_columns(hl_store* store, const uint64_t* idx, size_t nidx, uin
 int hl_b200_store_shape(hl_store* store, size_t* rows, size_t* n, size_t* nn, size_t* q);
 /* device address of the encoding (rows x nn words, row-major, a row's words in the order of the columns) and of the leaves; for
  * device-side callers.  The encoding may lie in another order until it is asked for: the first call then puts it into this one and waits
- * for that (2,606 rows of 2^15 words: 0.3 ms), and answers NULL where there is no device memory for it. */
+ * for that (2,606 rows of 2^15 words: 0.3 ms).  NULL, with hl_b200_last_error's text, where that fails (it takes a row's words of device
+ * memory at the least) and where the row encoder has given up on this store. */
 const uint64_t* hl_b200_store_encoded_dev(hl_store* store);
 const uint8_t* hl_b200_store_leaves_dev(hl_store* store);
 void hl_b200_store_free(hl_store* store);

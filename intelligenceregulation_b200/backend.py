@@ -321,7 +321,10 @@ class B200Commit:
         self.ctx.check(self.ctx.lib.hl_b200_store_merkle_dev(self.h, C.c_void_p(d_salts), _ptr(leaf_key), _ptr(node_key), C.c_void_p(d_levels)))
 
     def encoded_dev(self) -> int:
-        return int(self.ctx.lib.hl_b200_store_encoded_dev(self.h) or 0)
+        p = self.ctx.lib.hl_b200_store_encoded_dev(self.h)
+        if not p:
+            raise DeviceError(-3, self.ctx.last_error())  # never an address of 0
+        return int(p)
 
     def leaves_dev(self) -> int:
         return int(self.ctx.lib.hl_b200_store_leaves_dev(self.h) or 0)

@@ -32,16 +32,25 @@ void settle(hl_ctx* c) {
 // Stream-ordered allocation from the device's default pool, whose release threshold is
 // lifted at init so that freed blocks are reused instead of returned to the driver.
 int dev_alloc(hl_ctx* c, void** p, size_t bytes) {
+    cudaError_t e = cudaSuccess;
+    if (dev_try(c, p, bytes, &e)) return HL_B200_OK;
+    return e == cudaSuccess ? fail(c, HL_B200_ERR_OOM, "allocation cap reached (test hook)") : fail(c, HL_B200_ERR_OOM, "cudaMallocAsync", e);
+}
+
+// The same for a caller that can do with less: not having it is no failure of the call.
+bool dev_try(hl_ctx* c, void** p, size_t bytes, cudaError_t* why) {
     *p = nullptr;
     if (bytes == 0) bytes = 16;
-    if (c->alloc_cap && c->alloc_live + bytes > c->alloc_cap) return fail(c, HL_B200_ERR_OOM, "allocation cap reached (test hook)");
-    cudaError_t e = cudaMallocAsync(p, bytes, c->stream);
+    if (c->alloc_cap && c->alloc_live + bytes > c->alloc_cap) return false;
+    const cudaError_t e = cudaMallocAsync(p, bytes, c->stream);
     if (e != cudaSuccess) {
         cudaGetLastError();
-        return fail(c, HL_B200_ERR_OOM, "cudaMallocAsync", e);
+        *p = nullptr;
+        if (why) *why = e;
+        return false;
     }
     c->alloc_live += bytes;
-    return HL_B200_OK;
+    return true;
 }
 
 void dev_free(hl_ctx* c, void* p, size_t bytes) {

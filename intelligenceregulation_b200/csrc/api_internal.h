@@ -80,6 +80,7 @@ struct hl_store {
 namespace hlapi {
 int fail(hl_ctx* c, int code, const char* what, cudaError_t e = cudaSuccess);
 int dev_alloc(hl_ctx* c, void** p, size_t bytes);
+bool dev_try(hl_ctx* c, void** p, size_t bytes, cudaError_t* why = nullptr);
 void dev_free(hl_ctx* c, void* p, size_t bytes);
 void settle(hl_ctx* c);  // waits for both streams if something of the present call has failed
 // host_copy.cu: uploads on the context's stream (h2d_on: on another one that the context's stream waits for before the call ends);

@@ -504,23 +504,24 @@ const uint64_t* hl_b200_store_encoded_dev(hl_store* st) {
     if (!st) return nullptr;
     hl_ctx* c = st->ctx;
     Call g(c);
+    int rc = HL_B200_OK;
     if (st->order.logr) {
-        const u32 ctas = hlk::natural_order_rows(st->rows, c->sm_count);
-        const size_t bytes = (size_t)ctas * st->nn() * 8;
+        // a CTA needs a row of scratch: fewer of them where memory is short, one at the least
+        u32 ctas = hlk::natural_order_rows(st->rows, c->sm_count);
         u64* d_rows = nullptr;
-        int rc = dev_alloc(c, (void**)&d_rows, bytes);
+        while (ctas > 1 && !dev_try(c, (void**)&d_rows, (size_t)ctas * st->nn() * 8)) ctas /= 2;
+        if (!d_rows) rc = dev_alloc(c, (void**)&d_rows, st->nn() * 8);
         if (!rc) {
             const cudaError_t e = hlk::natural_order(st->d_enc, st->rows, st->nn(), st->order, d_rows, ctas, c->stream);
             c->stats.kernel_launches++;
-            if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "column order launch", e);
+            if (e == cudaSuccess) st->order = ColOrder();  // for what is queued behind it, whatever becomes of this call
+            else rc = fail(c, HL_B200_ERR_DEVICE, "column order launch", e);
         }
         if (!rc) rc = sync(c, "store_encoded_dev");
-        if (!rc) rc = encoded_ok(c, st);
-        dev_free(c, d_rows, bytes);
-        if (rc) return nullptr;
-        st->order = ColOrder();
+        dev_free(c, d_rows, (size_t)ctas * st->nn() * 8);
     }
-    return (const uint64_t*)st->d_enc;
+    if (!rc) rc = encoded_ok(c, st);  // where that is known already
+    return rc ? nullptr : (const uint64_t*)st->d_enc;
 }
 const uint8_t* hl_b200_store_leaves_dev(hl_store* st) { return st ? (const uint8_t*)st->d_leaves : nullptr; }
 

@@ -22,6 +22,7 @@ inline std::vector<Stream*> streams;
 inline std::map<const char*, size_t> device, locked;  // start -> bytes
 inline std::vector<std::string> faults;
 inline long fail_at = -1, calls = 0;
+inline bool next_wait_fails = false;  // the next wait for a stream says that something on it went wrong
 
 inline bool fails() { return calls++ == fail_at; }
 inline bool inside(const std::map<const char*, size_t>& m, const void* p, size_t bytes) {
@@ -77,7 +78,12 @@ cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) {
     *s = (cudaStream_t)fake::streams.back();
     return cudaSuccess;
 }
-cudaError_t cudaStreamSynchronize(cudaStream_t s) { fake::run((fake::Stream*)s, ((fake::Stream*)s)->issued); return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t s) {
+    fake::run((fake::Stream*)s, ((fake::Stream*)s)->issued);
+    const bool bad = fake::next_wait_fails;
+    fake::next_wait_fails = false;
+    return bad ? cudaErrorUnknown : cudaSuccess;
+}
 cudaError_t cudaStreamDestroy(cudaStream_t s) {
     for (auto it = fake::streams.begin(); it != fake::streams.end(); ++it)
         if (*it == (fake::Stream*)s) { fake::streams.erase(it); break; }

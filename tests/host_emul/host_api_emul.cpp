@@ -4,6 +4,7 @@
 //   host_api_emul copies       the bytes of copies of all sizes and alignments
 //   host_api_emul threads N    the same where the process can make only N threads
 //   host_api_emul timeouts     who is told that a row encoder's bounded wait ran out
+//   host_api_emul reorder      the encoding's way into the columns' order: once, whatever fails, and with little memory
 #include "fake_cuda.h"
 
 #include <dlfcn.h>
@@ -41,8 +42,14 @@ cudaError_t encode_rows_tc(enc::RowArgs, u32, const u64*, int, size_t, TcReport 
     }
     return launch();
 }
-u32 natural_order_rows(u32, int) { return 1; }
-cudaError_t natural_order(u64*, u32, size_t, ColOrder, u64*, u32, cudaStream_t) { return launch(); }
+u32 natural_order_rows(u32 rows, int sms) { return rows < 2u * sms ? rows : 2u * sms; }
+static u32 g_reorders = 0, g_reorder_ctas = 0;
+cudaError_t natural_order(u64*, u32, size_t, ColOrder, u64*, u32 ctas, cudaStream_t) {
+    if (fake::fails()) return cudaErrorUnknown;
+    g_reorders++;
+    g_reorder_ctas = ctas;
+    return cudaSuccess;
+}
 cudaError_t widen_rows(const unsigned char*, const u64*, const unsigned char*, u64*, u32, u32, int, cudaStream_t) { return launch(); }
 u32 hash_chunks(u32 rows) { return (rows + 127) / 128; }
 u32 hash_chunks_at_once(u32, int) { return 5; }
@@ -266,6 +273,52 @@ static void timeouts() {
     hl_b200_shutdown(c);
 }
 
+static void reorder() {
+    hl_ctx* c = nullptr;
+    hl_b200_init(0, &c);
+    const u32 rows = 6, lc = 12, q = 40;
+    const size_t n = (size_t)1 << lc, nn = 2 * n;
+    Host h(false);
+    uint64_t *data = h.words(rows * n), *pads = h.words(rows * q), *pows = h.words(nn);
+    uint8_t* leaves = h.bytes(nn * 32);
+    hl_store* st = nullptr;
+    auto commit = [&] { return hl_b200_commit_zk(c, lc, 2, data, rows, pads, q, pows, lc + 1, nullptr, &st, leaves); };
+    // every fallible call of it in turn: the rows are never put in order a second time, and where they have not been the store says so
+    for (long at = 0;; at++) {
+        commit();
+        hlk::g_reorders = 0;
+        fake::calls = 0;
+        fake::fail_at = at;
+        hl_b200_store_encoded_dev(st);
+        fake::fail_at = -1;
+        const bool past = fake::calls <= at;
+        if ((st->order.logr == 0) != (hlk::g_reorders == 1)) bad("reorder", "the store's order is not that of its rows, call " + std::to_string(at));
+        if (!hl_b200_store_encoded_dev(st)) bad("reorder", "does not recover");
+        if (hlk::g_reorders != 1) bad("reorder", "the rows were put in order " + std::to_string(hlk::g_reorders) + " times, call " + std::to_string(at));
+        hl_b200_store_free(st);
+        if (past) break;
+    }
+    commit();
+    hlk::g_reorders = 0;
+    fake::next_wait_fails = true;  // behind the launch
+    if (hl_b200_store_encoded_dev(st)) bad("reorder", "a failed wait is not told");
+    if (!hl_b200_store_encoded_dev(st) || hlk::g_reorders != 1 || st->order.logr) bad("reorder", "after a failed wait the rows are put in order again");
+    hl_b200_store_free(st);
+    for (u32 fit = 0; fit <= 6; fit++) {  // memory for so many rows
+        commit();
+        const u64 declines = c->stats.declines;
+        hl_b200_set_alloc_cap(c, c->alloc_live + fit * nn * 8 + (fit ? 0 : 1));
+        hlk::g_reorder_ctas = 0;
+        const uint64_t* p = hl_b200_store_encoded_dev(st);
+        hl_b200_set_alloc_cap(c, 0);
+        const u32 want = fit >= 6 ? 6 : fit >= 3 ? 3 : fit >= 1 ? 1 : 0;
+        if ((p != nullptr) != (fit > 0) || hlk::g_reorder_ctas != want || (c->stats.declines != declines) != (fit == 0))
+            bad("reorder", "with memory for " + std::to_string(fit) + " rows " + std::to_string(hlk::g_reorder_ctas) + " at once");
+        hl_b200_store_free(st);
+    }
+    hl_b200_shutdown(c);
+}
+
 int main(int argc, char** argv) {
     if (argc == 3 && !strcmp(argv[1], "threads")) {
         g_threads = atol(argv[2]);
@@ -276,6 +329,8 @@ int main(int argc, char** argv) {
         areas();
     } else if (argc == 2 && !strcmp(argv[1], "timeouts")) {
         timeouts();
+    } else if (argc == 2 && !strcmp(argv[1], "reorder")) {
+        reorder();
     } else {
         failures(false);
         failures(true);

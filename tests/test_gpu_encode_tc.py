@@ -138,3 +138,29 @@ def test_a_wait_that_runs_out_is_told_to_its_own_store(dev, oracle):
     ctx.sync()
     for s in (fine, later, lost):
         s.free()
+
+
+@pytest.mark.parametrize("fit", [0, 1, 3, 40])
+def test_the_columns_order_with_little_memory(oracle, fit):
+    """the encoding is put into the columns' order with as many rows of scratch as there is memory for; with none that is an error, not an
+    address of 0, and the store stays as it was"""
+    import torch
+    from intelligenceregulation_b200 import backend
+
+    rows, n, q = 40, 1 << 14, 12
+    nn = 2 * n
+    dev = backend.B200Backend(device=0)
+    rng = np.random.default_rng(fit)
+    data, pads = rng.integers(0, P, size=rows * n, dtype=np.uint64), rng.integers(0, P, size=rows * q, dtype=np.uint64)
+    store, leaves = dev.try_commit_zk(14, 2, data, pads, oracle.coset_powers(7, nn), 18)
+    dev.ctx.set_alloc_cap((rows * (n + q + nn) + 4 * nn + fit * nn) * 8 + 64)  # what the store holds, and that many rows
+    out = torch.empty((nn, 32), dtype=torch.uint8, device="cuda")
+    if fit == 0:
+        with pytest.raises(backend.DeviceError):
+            store.encoded_dev()
+        dev.ctx.set_alloc_cap(0)
+    backend.hash_columns_static(store.encoded_dev(), rows, nn, None, out.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    assert (out.cpu().numpy() == leaves).all()
+    dev.ctx.set_alloc_cap(0)
+    store.free()
+    dev.ctx.close()

@@ -33,6 +33,11 @@ def test_an_encoder_wait_that_runs_out_is_told_to_its_own_store(emul):
     _ok(emul, "timeouts")
 
 
+def test_an_encoding_is_put_into_the_columns_order_once(emul):
+    """where a call fails behind the launch the rows are in order all the same; few rows of scratch are enough"""
+    _ok(emul, "reorder")
+
+
 def test_copies_of_all_sizes(emul):
     """the limits between the forms of a copy, unaligned ends, and more small copies in a call than the bounce areas hold"""
     _ok(emul, "copies")
