@@ -158,7 +158,7 @@ int commit_on_device(hl_ctx* c, hl_store* st, const u64* d_pows, const uint8_t* 
     uint32_t* cvs = nullptr;
     unsigned char *d_narrow = nullptr, *d_row_w = nullptr;
     u64* d_row_off = nullptr;
-    size_t scratch_words = hlk::encode_scratch_words(logb, T, c->sm_count, st->rows);
+    size_t scratch_words = 0;
     const bool tc = c->fast_encoder && hlk::encode_tc_takes(logn, st->logr, st->rows, c->sm_count);
     const u64* tc_tab = nullptr;
     hlk::TcReport report;
@@ -171,14 +171,11 @@ int commit_on_device(hl_ctx* c, hl_store* st, const u64* d_pows, const uint8_t* 
         if (!rc) rc = encoder_word(c, st);
         if (rc) return rc;
         report = {st->enc_word, st->enc_mark, later ? c->enc_later : nullptr, c->enc_limit};
-        const size_t w = hlk::encode_tc_scratch_words(logn, st->logr, st->q, st->rows, c->sm_count);
-        if (w > scratch_words) scratch_words = w;
     }
     const u32 nchunks = hlk::hash_chunks(st->rows);
     const size_t cvs_bytes = nchunks > 1 && leaves ? (size_t)nchunks * nn * 32 : 0;
     const size_t total_bytes = packed ? (size_t)hr.off[st->rows] : (size_t)st->rows * n * 8;
     rc = upload_key(c, key32, &d_key);
-    if (!rc) rc = dev_alloc(c, (void**)&scratch, scratch_words * 8);
     if (!rc && cvs_bytes) rc = dev_alloc(c, (void**)&cvs, cvs_bytes);
     if (!rc && packed) rc = dev_alloc(c, (void**)&d_narrow, total_bytes + 16);
     if (!rc && packed) rc = dev_alloc(c, (void**)&d_row_off, (size_t)st->rows * 8);
@@ -223,6 +220,16 @@ int commit_on_device(hl_ctx* c, hl_store* st, const u64* d_pows, const uint8_t* 
         }
         if (rem > 0) take(rem);
     }
+    if (!rc && tc) {
+        for (const u32 nr : piece_rows) {
+            const size_t w = hlk::encode_tc_scratch_words(logn, st->logr, st->q, nr, c->sm_count);
+            if (w > scratch_words) scratch_words = w;
+        }
+        if (!dev_try(c, (void**)&scratch, scratch_words * 8)) scratch_words = hlk::encode_tc_least_words(logn, st->logr, st->q, st->rows, c->sm_count);
+    } else if (!rc) {
+        scratch_words = hlk::encode_scratch_words(logb, T, c->sm_count, st->rows);
+    }
+    if (!rc && !scratch) rc = dev_alloc(c, (void**)&scratch, scratch_words * 8);
     if (!rc && pieces) {
         // the copy stream may touch the fresh allocations only after the main stream has made them
         cudaError_t e = cudaEventRecord(c->ev_main, c->stream);

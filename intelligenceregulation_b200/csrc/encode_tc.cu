@@ -450,6 +450,10 @@ u32 tc_batches(u32 logn, u32 rows) {
     const u32 per = TC_WORDS >> logn;
     return (rows + per - 1) / per;
 }
+// whether one residue a CTA, with the inverse transform before it, takes fewer turns of the machine than all of them after one inverse transform
+bool tc_splits(u32 logr, u64 batches, u64 sms) {
+    return logr >= 1 && ((batches << logr) + sms - 1) / sms * 2 < (batches + sms - 1) / sms * (1 + ((u64)1 << logr));
+}
 
 }  // namespace
 
@@ -474,16 +478,23 @@ bool encode_tc_takes(u32 logn, u32 logr, u32 rows, int sm_count) {
     return (whole < split ? whole : split) * 26000 < 12000 + 195 * (1 + ((u64)1 << logr)) * batches * 148 / sms;
 }
 
-// a slot for each CTA; never more CTAs than SMs
+// A slot for each CTA, never more CTAs than SMs.  Whole batches keep the words of all residues but one, so their slots come near the
+// encoding's own size where the machine holds every batch at once; split ones keep the pads' words alone.
 size_t encode_tc_scratch_words(u32 logn, u32 logr, u32 q, u32 rows, int sm_count) {
-    const size_t ctas = (size_t)tc_batches(logn, rows) << logr;
-    return (ctas < (size_t)sm_count ? ctas : (size_t)sm_count) * tc_slot_words(logn, 1u << logr, q);
+    const u64 batches = tc_batches(logn, rows), sms = (u64)sm_count;
+    if (tc_splits(logr, batches, sms)) return encode_tc_least_words(logn, logr, q, rows, sm_count);
+    return (size_t)(batches < sms ? batches : sms) * tc_slot_words(logn, 1u << logr, q);
+}
+size_t encode_tc_least_words(u32 logn, u32 logr, u32 q, u32 rows, int sm_count) {
+    const u64 units = (u64)tc_batches(logn, rows) << logr, sms = (u64)sm_count;
+    return (size_t)(units < sms ? units : sms) * tc_slot_words(logn, 1u, q);
 }
 
 cudaError_t encode_rows_tc(RowArgs a, u32 logn, const u64* tab, int sm_count, size_t scratch_words, TcReport report, cudaStream_t st, int* path_out) {
-    const u64 batches = tc_batches(logn, a.rows), sms = (u64)sm_count, split_units = batches << a.logr;
-    a.split = a.logr >= 1 && (split_units + sms - 1) / sms * 2 < (batches + sms - 1) / sms * (1 + ((u64)1 << a.logr));
-    u64 grid = a.split ? split_units : batches;
+    const u64 batches = tc_batches(logn, a.rows), sms = (u64)sm_count;
+    // split as well where the scratch is not what whole batches take: at rate 1/64 148 rows of 2^14 words would keep 1.2 GB
+    a.split = tc_splits(a.logr, batches, sms) || (a.logr && scratch_words < encode_tc_scratch_words(logn, a.logr, a.q, a.rows, sm_count));
+    u64 grid = a.split ? batches << a.logr : batches;
     if (grid > sms) grid = sms;
     const u64 per = tc_slot_words(logn, a.split ? 1u : 1u << a.logr, a.q);  // none for one residue without pads
     if (per && grid > scratch_words / per) grid = scratch_words / per;

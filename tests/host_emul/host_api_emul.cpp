@@ -34,6 +34,7 @@ void encode_tc_build(u32, u32, u64* out) { for (int i = 0; i < 8; i++) out[i] = 
 bool encode_tc_takes(u32 logn, u32, u32, int) { return logn >= 10; }
 u32 encode_tc_rows(u32 logn) { return 16384u >> logn; }
 size_t encode_tc_scratch_words(u32, u32, u32, u32, int) { return 64; }
+size_t encode_tc_least_words(u32, u32, u32, u32, int) { return 32; }
 static bool g_gives_up = false;  // the encoder's waits run out
 cudaError_t encode_rows_tc(enc::RowArgs, u32, const u64*, int, size_t, TcReport r, cudaStream_t, int*) {
     if (g_gives_up) {

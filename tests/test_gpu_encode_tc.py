@@ -140,6 +140,26 @@ def test_a_wait_that_runs_out_is_told_to_its_own_store(dev, oracle):
         s.free()
 
 
+# log_cols, inv_rate, rows, q, whole batches, the scratch they are left in MB: few rows never keep the other residues' words, and where there is no memory
+# for them many rows do without
+@pytest.mark.parametrize("log_cols,inv_rate,rows,q,left", [(14, 64, 4, 280, 2), (14, 256, 2, 5, 1), (14, 8, 140, 31, 16), (14, 2, 149, 7, 16), (13, 4, 296, 40, 16)])
+def test_scratch_does_not_grow_with_the_rate(oracle, log_cols, inv_rate, rows, q, left):
+    from intelligenceregulation_b200 import backend
+
+    n, nn = 1 << log_cols, inv_rate << log_cols
+    dev = backend.B200Backend(device=0)
+    rng = np.random.default_rng(rows)
+    data, pads = rng.integers(0, P, size=rows * n, dtype=np.uint64), rng.integers(0, P, size=rows * q, dtype=np.uint64)
+    pows = oracle.coset_powers(7, nn)
+    dev.ctx.set_alloc_cap((rows * (n + q + nn) + 5 * nn) * 8 + (rows + 127) // 128 * nn * 32 + (left << 20))  # what the call has to hold, and that
+    got = dev.try_commit_zk(log_cols, inv_rate, data, pads, pows, log_cols + inv_rate.bit_length() - 1)
+    assert got is not None, dev.ctx.declines
+    store, leaves = got
+    assert (leaves == oracle.hash_columns(oracle.encode_rows_zk(data, rows, n, pads, q, pows, log_cols + inv_rate.bit_length() - 1), rows, nn)).all()
+    store.free()
+    dev.ctx.close()
+
+
 @pytest.mark.parametrize("fit", [0, 1, 3, 40])
 def test_the_columns_order_with_little_memory(oracle, fit):
     """the encoding is put into the columns' order with as many rows of scratch as there is memory for; with none that is an error, not an
