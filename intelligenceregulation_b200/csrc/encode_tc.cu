@@ -469,6 +469,11 @@ void encode_tc_build(u32 logn, u32 logr, u64* out) { tc_build(logn, logr, out); 
 // takes 12 us + 0.195 us for each 2^14 words and transform of shorter ones (both fitted to rows of 2^10 .. 2^13 words, 4 to 2,606 times 2^14
 // words, rates 1/2 and 1/4): 592 rows of 2^11 58 -> 55, 600 of them 60 (74 here), 1,184 of them 96 -> 78; 888 of 2^12 148 (150 here), 2,368 of
 // them 346 -> 283; 148 of 2^13 62 -> 56, 74 of them 46 (54 here).
+// Measured at rates down to 1/64, 1 to 444 times 2^14 words (rows of 2^14: rate 1/8 38 rows 221 -> 146, 1,036 of them 3,204 -> 1,988; rate 1/16
+// 148 rows 1,121 -> 626; rate 1/64 4 rows 179 -> 121, 38 of them 1,407 -> 914; rows of 2^13 alike): what the line gives to this encoder is never
+// more than 8 % slower here (400 rows of 2^13 at 1/2 140, 151 here; 1,184 of 2^10 52, 56 here).  It is a cautious one: the other encoder's
+// scratch leaves L2 at rates of 1/16 and less, where its 0.195 us become 0.4 and more, and rows of 2^10 .. 2^12 that it keeps would take half
+// the time here (592 rows of 2^11 at 1/64 2,955, 1,370 here).
 bool encode_tc_takes(u32 logn, u32 logr, u32 rows, int sm_count) {
     if (logn < 10 || logn > 14) return false;
     if (logn == 14) return true;

@@ -1,5 +1,5 @@
 """The tensor-core row encoder at the edges of its forms: full and short batches of rows per 2^14 words, one residue or all of them a CTA, pads that
-reach most of a row and beyond it, rates 1, 1/2, 1/4, packed rows of every width, and rows that do not start on 32-byte boundaries; and
+reach most of a row and beyond it, rates 1 to 1/64, packed rows of every width, and rows that do not start on 32-byte boundaries; and
 what reads an encoding that lies residue by residue."""
 import numpy as np
 import pytest
@@ -19,23 +19,26 @@ def dev():
 
 # log_cols, inv_rate, rows, q: (10 .. 13) just above the line where the tensor cores take over, a last batch of one row
 CASES = [(10, 2, 2369, 33), (11, 2, 1185, 320), (12, 2, 593, 1), (12, 4, 601, 40), (13, 2, 149, 281), (13, 4, 41, 8000),
-         (14, 2, 3, 280), (14, 2, 149, 5), (14, 4, 38, 40001), (14, 4, 2, 1), (14, 1, 2, 0), (14, 2, 75, 0)]
+         (14, 2, 3, 280), (14, 2, 149, 5), (14, 4, 38, 40001), (14, 4, 2, 1), (14, 1, 2, 0), (14, 2, 75, 0),
+         # rates that keep many residues' words, whole batches and split ones
+         (14, 8, 3, 280), (14, 8, 79, 17), (14, 16, 75, 0), (14, 64, 2, 20001), (13, 8, 21, 9), (12, 8, 593, 12), (10, 16, 2353, 5)]
 
 
 @pytest.mark.parametrize("log_cols,inv_rate,rows,q", CASES)
 def test_commitments_and_columns(dev, oracle, log_cols, inv_rate, rows, q):
     n, nn = 1 << log_cols, inv_rate << log_cols
+    top = max(18, nn.bit_length() - 1)
     rng = np.random.default_rng(log_cols * 1000 + rows)
     data = rng.integers(0, P, size=rows * n, dtype=np.uint64)
     data[:n] = P - 1
     data[-n:] = 0
     if q:
         pads, pows = rng.integers(0, P, size=rows * q, dtype=np.uint64), oracle.coset_powers(7, nn)
-        want = oracle.encode_rows_zk(data, rows, n, pads, q, pows, 18)
-        store, leaves = dev.try_commit_zk_keyed(log_cols, inv_rate, data, pads, pows, 18, None)
+        want = oracle.encode_rows_zk(data, rows, n, pads, q, pows, top)
+        store, leaves = dev.try_commit_zk_keyed(log_cols, inv_rate, data, pads, pows, top, None)
     else:
-        want = oracle.encode_rows_plain(data, rows, n, nn, 18)
-        store, leaves = dev.try_commit(log_cols, inv_rate, data, 18)
+        want = oracle.encode_rows_plain(data, rows, n, nn, top)
+        store, leaves = dev.try_commit(log_cols, inv_rate, data, top)
     assert (leaves == oracle.hash_columns(want, rows, nn)).all()
     idx = np.array([0, nn - 1, nn // 2, 1 % nn, 5 % nn, nn // 3], dtype=np.uint64)
     cols = oracle.gather_columns(want, rows, nn, idx)
@@ -43,7 +46,7 @@ def test_commitments_and_columns(dev, oracle, log_cols, inv_rate, rows, q):
     if not q:  # a plain store folds the systematic positions of its encoding
         rhos = rng.integers(0, P, size=(2, rows, 2), dtype=np.uint64)
         assert (store.fold_rows(rhos) == oracle.fold_rows(np.ascontiguousarray(want.reshape(rows, nn)[:, ::inv_rate]).reshape(-1), rows, n, n, 1, rhos)).all()
-    if rows < 200:  # in the columns' own order, for callers on the device, and what reads it afterwards
+    if rows < 200 and nn <= 1 << 18:  # in the columns' own order, for callers on the device, and what reads it afterwards
         import torch
         from intelligenceregulation_b200 import backend
 

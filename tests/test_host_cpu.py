@@ -94,6 +94,7 @@ def test_encoder_phases_on_the_host_match_the_oracle(emul, oracle, case):
 TC_CASES = [  # log_n, inv_rate, rows, q, zk: every batch of rows per 2^14 words, full and short, both coset residues, pads above the row
     (10, 2, 17, 40, 1), (10, 4, 3, 1500, 1), (11, 2, 8, 33, 1), (12, 2, 5, 64, 1), (12, 4, 4, 0, 0), (13, 2, 3, 280, 1),
     (14, 2, 1, 280, 1), (14, 1, 1, 0, 0), (14, 4, 1, 33000, 1),
+    (14, 8, 1, 280, 1), (13, 16, 2, 9000, 1), (12, 64, 3, 5, 1), (10, 8, 17, 0, 0),
 ]
 
 
