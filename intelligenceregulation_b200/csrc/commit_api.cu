@@ -190,7 +190,7 @@ int commit_on_device(hl_ctx* c, hl_store* st, const u64* d_pows, const uint8_t* 
     // 25 us of its own.  1, 1, 2, 2, 3, 3, .. waves (1, 2, 3, 3, .. waited 57 us for the second piece and 110 for the third; five of one
     // and then twos cost more in launches), and the last two waves as one piece: no more than that follows the
     // last byte when several ranks share the bus and it is the slower side (90 MB take 1.6 ms alone and 2.5-3.7 ms beside seven other ranks).
-    // A block's A from the host 2,371 -> 2,320 us, and 2,375 -> 2,371 by the hash in whole multiples of what fills the machine.
+    // A block's A from the host 2,371 -> 2,320 us.
     auto byte_at = [&](u32 r) { return packed ? (size_t)hr.off[r] : (size_t)r * n * 8; };
     const u32 wave = (u32)c->sm_count * (tc ? hlk::encode_tc_rows(logn) : 1u);
     const bool split = h_data && total_bytes >= ((size_t)32 << 20) && st->rows > 4u * wave;
@@ -242,7 +242,6 @@ int commit_on_device(hl_ctx* c, hl_store* st, const u64* d_pows, const uint8_t* 
         Timed t(c, HL_T_ENCODE);
         size_t ev_i = 0;
         u32 nr = 0, chunks_done = 0;
-        const u32 at_once = pieces ? hlk::hash_chunks_at_once((u32)nn, c->sm_count) : 1u;
         size_t pk = 0;
         for (u32 r0 = 0; r0 < st->rows && !rc; r0 += nr) {
             nr = piece_rows[pk++];
@@ -285,14 +284,8 @@ int commit_on_device(hl_ctx* c, hl_store* st, const u64* d_pows, const uint8_t* 
                                : hlk::encode_rows(a, logb, c->fast_encoder || loga, c->sm_count, scratch_words, c->stream, &st->encoder_path);
             c->stats.kernel_launches += 1;
             if (e != cudaSuccess) rc = fail(c, HL_B200_ERR_DEVICE, "row encoder launch", e);
-            // The 128-row hash chunks that are complete now.  A launch takes as long as the next multiple of what fills the machine, 5 chunks
-            // of 2^15 columns: 3 of them 57 us, 4 of them 72, 6 of them 107, 7 of them 123, all twenty 290.  So narrow rows, whose encoding
-            // is as long as their upload, wait for whole multiples (twenty chunks as 6, 4, 7 and 3 359 us, as four times 5 300); the last
-            // launch takes what is left.  Where the bus is the slower side nothing is gained by waiting.
-            if (!rc && pieces) {
-                const bool last = r0 + nr == st->rows;
-                u32 c1 = last ? nchunks : (r0 + nr) / 128u;
-                if (!bus_bound && !last) c1 -= (c1 - chunks_done) % at_once;
+            if (!rc && pieces) {  // the 128-row hash chunks that are complete now
+                const u32 c1 = r0 + nr == st->rows ? nchunks : (r0 + nr) / 128u;
                 if (c1 > chunks_done) {
                     e = hlk::hash_column_chunks(st->d_enc, st->rows, (u32)nn, d_key, chunks_done, c1 - chunks_done, cvs, st->d_leaves, c->stream, st->order);
                     c->stats.kernel_launches += 1;

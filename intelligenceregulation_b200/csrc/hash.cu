@@ -226,16 +226,6 @@ cudaError_t merkle_tree(const uint32_t* d_leaves, const uint32_t* d_salts, u32 n
 
 u32 hash_chunks(u32 rows) { return (rows + 127u) / 128u; }
 
-u32 hash_chunks_at_once(u32 nn, int sm_count) {
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_hash_col_chunks, 128, 0) != cudaSuccess) {
-        cudaGetLastError();
-        per_sm = 0;
-    }
-    const u32 ctas = (nn + 127u) / 128u, chunks = (u32)(per_sm * sm_count) / ctas;
-    return chunks ? chunks : 1u;
-}
-
 cudaError_t hash_columns(const u64* enc, u32 rows, u32 nn, const uint32_t* d_key, uint32_t* d_cvs, uint32_t* d_leaves,
                          cudaStream_t st, ColOrder order) {
     const u32 nchunks = hash_chunks(rows);

@@ -38,7 +38,6 @@ cudaError_t encode_rows_tc(enc::RowArgs a, u32 logn, const u64* tab, int sm_coun
 
 // hash.cu
 u32 hash_chunks(u32 rows);
-u32 hash_chunks_at_once(u32 nn, int sm_count);  // that fill the machine once
 cudaError_t hash_column_chunks(const u64* enc, u32 rows, u32 nn, const uint32_t* d_key, u32 chunk0, u32 count, uint32_t* d_cvs,
                                uint32_t* d_leaves, cudaStream_t st, ColOrder order = ColOrder());
 cudaError_t hash_column_merge(u32 rows, u32 nn, const uint32_t* d_key, const uint32_t* d_cvs, uint32_t* d_leaves, cudaStream_t st, ColOrder order = ColOrder());

@@ -53,7 +53,6 @@ cudaError_t natural_order(u64*, u32, size_t, ColOrder, u64*, u32 ctas, cudaStrea
 }
 cudaError_t widen_rows(const unsigned char*, const u64*, const unsigned char*, u64*, u32, u32, int, cudaStream_t) { return launch(); }
 u32 hash_chunks(u32 rows) { return (rows + 127) / 128; }
-u32 hash_chunks_at_once(u32, int) { return 5; }
 cudaError_t hash_column_chunks(const u64*, u32, u32, const uint32_t*, u32, u32, uint32_t*, uint32_t*, cudaStream_t, ColOrder) { return launch(); }
 cudaError_t hash_column_merge(u32, u32, const uint32_t*, const uint32_t*, uint32_t*, cudaStream_t, ColOrder) { return launch(); }
 cudaError_t hash_columns(const u64*, u32, u32, const uint32_t*, uint32_t*, uint32_t*, cudaStream_t, ColOrder) { return launch(); }
