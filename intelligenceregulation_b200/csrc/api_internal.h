@@ -86,6 +86,7 @@ void settle(hl_ctx* c);  // waits for both streams if something of the present c
 // host_copy.cu: uploads on the context's stream (h2d_on: on another one that the context's stream waits for before the call ends);
 // h2d_owned: the caller's bytes are no longer needed when it returns, whatever kind of host memory they live in;
 // d2h: the bytes are in place after the next `sync`
+bool pageable(const void* h);
 int h2d(hl_ctx* c, void* d, const void* h, size_t bytes);
 int h2d_on(hl_ctx* c, void* d, const void* h, size_t bytes, cudaStream_t s);
 int h2d_owned(hl_ctx* c, void* d, const void* h, size_t bytes);

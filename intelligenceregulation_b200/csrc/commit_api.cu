@@ -1,4 +1,5 @@
 // C ABI: commitments (Backend::try_commit*), stores (EncodedStore), Merkle trees.
+#include <algorithm>
 #include <cstring>
 
 #include "api_internal.h"
@@ -136,6 +137,52 @@ struct HostRows {
     size_t tail_bytes = 0;
 };
 
+// The pieces of rows that come from the host: a piece is encoded and its complete 1 KiB hash chunks (128 rows) are hashed while the next one
+// is on the bus.  Sizes are turns of the machine, `sms` batches of 2^14 words; `bus` and `device` are what a turn takes on either side, in
+// us: 44 a byte of a word from page-locked memory and 58 from pageable (55 and 42 GB/s), 35 a transform with its share of the hash, 29 for
+// rows of 2^10 .. 2^13 words.
+// Where the bus is the slower side little must follow its last byte: pieces of two turns, one turn at the end, and where it is much slower half
+// a turn behind that, whose rows are split by residue.  1,000 rows of 2^13 64-bit words 1,741 us with no pieces below four turns, 1,469
+// now; 600 of 2^14 1,869 -> 1,737 (two turns and one); 9,000 of 2^9 1,597 -> 996 and 20,000 of 2^8 3,247 -> 1,276 (pieces of 296 rows);
+// 32-bit rows, 1,300 of 2^14 2,089 -> 1,987; 16-bit ones, 9,000 of 2^12 2,296 -> 2,177 (the growing pieces below), pageable ones, 1,777 of
+// 2^14 2,188 -> 2,023.
+// Where the device is (16-bit rows of 2^14 words from page-locked memory, 8-bit rows, lower rates) it should start early and have few
+// launches: 1, 1, 2, 2, 3, 3, .. turns and two at the end.  Twos ending in one: 2,504 rows of 2^14 2,304 -> 2,379 us, 2,000 of them 1,949 -> 1,979; the other
+// way round below ten turns, 1,200 of them 1,393 -> 1,324.  Rows written just before (their lines in the host's caches) keep these
+// differences and take 30 to 60 us more.
+std::vector<u32> row_pieces(u32 rows, u32 sms, u32 batch, double bus, double device) {
+    std::vector<u32> sizes;  // in batches
+    u32 left = (rows + batch - 1) / batch;
+    if (bus >= device) {
+        auto take = [&](u32 b) {
+            if (!left) return;
+            if (b > left) b = left;
+            if (b < sms / 4 && !sizes.empty()) sizes.back() += b;  // not worth a launch
+            else sizes.push_back(b);
+            left -= b;
+        };
+        if (bus >= 1.5 * device) take(sms / 2);
+        take(sms);
+        while (left) take(2 * sms);
+        std::reverse(sizes.begin(), sizes.end());
+    } else {
+        u32 turns = (left + sms - 1) / sms;
+        auto take = [&](u32 t) {
+            sizes.push_back(t * sms < left ? t * sms : left);
+            left -= sizes.back();
+            turns -= t;
+        };
+        for (u32 k = 0; turns > 2; k++) take(std::min(k < 2 ? 1u : k < 4 ? 2u : 3u, turns - 2));
+        if (turns) take(turns);
+    }
+    u32 at = 0;
+    for (u32& s : sizes) {
+        s = std::min(s * batch, rows - at);
+        at += s;
+    }
+    return sizes;
+}
+
 // Encode + column-hash.  With no host rows the data rows are already in st->d_data; otherwise they are
 // uploaded here in row chunks on the context's copy stream while the encoder works on the chunks that
 // have arrived (the upload of a block-sized matrix takes longer than its encoding).  Packed rows travel as
@@ -182,43 +229,13 @@ int commit_on_device(hl_ctx* c, hl_store* st, const u64* d_pows, const uint8_t* 
     if (!rc && packed) rc = dev_alloc(c, (void**)&d_row_w, st->rows);
     if (!rc && packed) rc = h2d_owned(c, d_row_off, hr.off.data(), (size_t)st->rows * 8);
     if (!rc && packed) rc = h2d_owned(c, d_row_w, hr.row_w, st->rows);
-    // Row pieces: a piece is encoded and its complete 1 KiB hash chunks (128 rows) are hashed while the next piece is still on
-    // the bus.  Piece sizes are whole waves of the encoder (one row per SM per wave).  When the bytes per row make the bus the
-    // slower side (64-bit words) the pieces are two waves and the last one a single wave, so that little follows the upload.
-    // With narrow rows a wave's encoding takes as long as its upload (148 rows of 2^14 int16 words: 95 us each), so a piece that is larger
-    // than the one before it leaves the device waiting, until the hash launches between them have put it behind the bus; and a piece costs
-    // 25 us of its own.  1, 1, 2, 2, 3, 3, .. waves (1, 2, 3, 3, .. waited 57 us for the second piece and 110 for the third; five of one
-    // and then twos cost more in launches), and the last two waves as one piece: no more than that follows the
-    // last byte when several ranks share the bus and it is the slower side (90 MB take 1.6 ms alone and 2.5-3.7 ms beside seven other ranks).
-    // A block's A from the host 2,371 -> 2,320 us.
     auto byte_at = [&](u32 r) { return packed ? (size_t)hr.off[r] : (size_t)r * n * 8; };
-    const u32 wave = (u32)c->sm_count * (tc ? hlk::encode_tc_rows(logn) : 1u);
-    const bool split = h_data && total_bytes >= ((size_t)32 << 20) && st->rows > 4u * wave;
-    const bool bus_bound = total_bytes / st->rows >= n * 6;  // bytes per row near the 64-bit form
-    const bool pieces = split;
-    std::vector<u32> piece_rows;
-    if (!pieces) {
-        piece_rows.push_back(st->rows);
-    } else if (bus_bound) {
-        for (u32 r0 = 0; r0 < st->rows;) {
-            u32 nr = st->rows - r0 < 2u * wave ? st->rows - r0 : 2u * wave;
-            if (r0 + nr == st->rows && nr > wave) nr -= wave;  // leave one wave or less for the end
-            piece_rows.push_back(nr);
-            r0 += nr;
-        }
-    } else {
-        u32 rem = (st->rows + wave - 1) / wave, r0 = 0;  // waves left, the last one possibly short
-        auto take = [&](u32 w) {
-            const u32 nr = st->rows - r0 < w * wave ? st->rows - r0 : w * wave;
-            piece_rows.push_back(nr);
-            r0 += nr;
-            rem -= w;
-        };
-        for (u32 k = 0; rem > 2; k++) {
-            const u32 w = k < 2 ? 1u : k < 4 ? 2u : 3u;
-            take(w < rem - 2 ? w : rem - 2);
-        }
-        if (rem > 0) take(rem);
+    const u32 batch = logn < 14 ? 16384u >> logn : 1u;
+    const bool pieces = h_data && total_bytes >= ((size_t)32 << 20) && st->rows > (u32)c->sm_count * batch;
+    std::vector<u32> piece_rows{st->rows};
+    if (pieces) {
+        const double bus = (double)total_bytes / ((double)st->rows * n) * (pageable(h_data) ? 58 : 44), device = (1 + (1u << st->logr)) * (tc && logn < 14 ? 29 : 35);
+        piece_rows = row_pieces(st->rows, (u32)c->sm_count, batch, bus, device);
     }
     if (!rc && tc) {
         for (const u32 nr : piece_rows) {

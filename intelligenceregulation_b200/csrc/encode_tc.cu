@@ -459,7 +459,6 @@ bool tc_splits(u32 logr, u64 batches, u64 sms) {
 
 namespace hlk {
 
-u32 encode_tc_rows(u32 logn) { return TC_WORDS >> logn; }
 size_t encode_tc_table_words(u32 logn, u32 logr) { return tc_table_words(logn, logr); }
 void encode_tc_build(u32 logn, u32 logr, u64* out) { tc_build(logn, logr, out); }
 

@@ -161,14 +161,14 @@ Helpers& helpers() {
 std::mutex g_ctx_mu;
 int g_contexts = 0;
 
+}  // namespace
+
 bool pageable(const void* h) {
     cudaPointerAttributes attr;
     const bool yes = cudaPointerGetAttributes(&attr, h) != cudaSuccess || attr.type == cudaMemoryTypeUnregistered;
     cudaGetLastError();  // an unregistered pointer is not an error here
     return yes;
 }
-
-}  // namespace
 
 // A ring of page-locked slots.  Use number i of the ring takes slot i % SLOTS.  The host's side of a use (an upload: fill the slot; a
 // download: empty it) is SHARES shares of the slot, so that several threads work on the piece that the copy engine or the caller is

@@ -28,7 +28,6 @@ cudaError_t encode_rows_form(const enc::RowArgs& a, u32 logn, int form, int sm_c
 size_t encode_tc_table_words(u32 logn, u32 logr);
 void encode_tc_build(u32 logn, u32 logr, u64* out);  // host
 bool encode_tc_takes(u32 logn, u32 logr, u32 rows, int sm_count);
-u32 encode_tc_rows(u32 logn);  // that one CTA takes at a time
 // what these rows ask for, and what is enough for any number of them up to that, in the form that needs less
 size_t encode_tc_scratch_words(u32 logn, u32 logr, u32 q, u32 rows, int sm_count);
 size_t encode_tc_least_words(u32 logn, u32 logr, u32 q, u32 rows, int sm_count);

@@ -4,6 +4,7 @@
 //   host_api_emul copies       the bytes of copies of all sizes and alignments
 //   host_api_emul threads N    the same where the process can make only N threads
 //   host_api_emul timeouts     who is told that a row encoder's bounded wait ran out
+//   host_api_emul pieces       the row pieces of uploads
 //   host_api_emul reorder      the encoding's way into the columns' order: once, whatever fails, and with little memory
 #include "fake_cuda.h"
 
@@ -28,15 +29,16 @@ namespace hlk {
 static cudaError_t launch() { return fake::fails() ? cudaErrorUnknown : cudaSuccess; }
 size_t encode_scratch_words(u32, u32, int, u32) { return 64; }
 bool encode_split_pays(u32, u32, u32, int) { return false; }
-cudaError_t encode_rows(const enc::RowArgs&, u32, bool, int, size_t, cudaStream_t, int*) { return launch(); }
+static std::vector<u32> g_pieces;  // the rows of every encoder launch
+cudaError_t encode_rows(const enc::RowArgs& a, u32, bool, int, size_t, cudaStream_t, int*) { g_pieces.push_back(a.rows); return launch(); }
 size_t encode_tc_table_words(u32, u32) { return 8; }
 void encode_tc_build(u32, u32, u64* out) { for (int i = 0; i < 8; i++) out[i] = 0; }
 bool encode_tc_takes(u32 logn, u32, u32, int) { return logn >= 10; }
-u32 encode_tc_rows(u32 logn) { return 16384u >> logn; }
 size_t encode_tc_scratch_words(u32, u32, u32, u32, int) { return 64; }
 size_t encode_tc_least_words(u32, u32, u32, u32, int) { return 32; }
 static bool g_gives_up = false;  // the encoder's waits run out
-cudaError_t encode_rows_tc(enc::RowArgs, u32, const u64*, int, size_t, TcReport r, cudaStream_t, int*) {
+cudaError_t encode_rows_tc(enc::RowArgs a, u32, const u64*, int, size_t, TcReport r, cudaStream_t, int*) {
+    g_pieces.push_back(a.rows);
     if (g_gives_up) {
         *r.word = r.mark;
         if (r.also) *r.also = 1;
@@ -319,6 +321,40 @@ static void reorder() {
     hl_b200_shutdown(c);
 }
 
+// Every row in one piece, whole batches but for the last; 64-bit rows of every length come in pieces from 32 MB on, no more than two turns of
+// the machine each and no more than one at the end, and small or resident ones whole.
+static void pieces() {
+    hl_ctx* c = nullptr;
+    hl_b200_init(0, &c);
+    struct { u32 lc, rows, bytes; bool lock; u32 last; } all[] = {  // last: batches of 2^14 words behind which nothing is on the bus
+        {14, 300, 8, true, 74}, {14, 1000, 8, false, 74}, {13, 520, 8, true, 74}, {13, 1000, 8, true, 74}, {13, 1001, 8, true, 74}, {12, 1500, 8, false, 74},
+        {12, 2301, 8, true, 74}, {11, 3001, 8, true, 74}, {10, 4097, 8, true, 74}, {9, 9000, 8, true, 74}, {8, 20001, 8, true, 74}, {14, 600, 4, true, 74}, {12, 4500, 2, true, 148},
+        {14, 1100, 2, false, 148}, {14, 1100, 2, true, 296}, {10, 34000, 1, true, 296}, {14, 2605, 1, true, 296}, {15, 161, 8, true, 74}, {14, 255, 8, true, 0}, {12, 900, 8, true, 0}};
+    for (auto& k : all) {
+        const size_t n = (size_t)1 << k.lc, nn = 2 * n;
+        const u32 batch = k.lc < 14 ? 16384u >> k.lc : 1u;
+        Host h(k.lock);
+        uint64_t *data = h.words(k.rows * n * k.bytes / 8), *pads = h.words(k.rows), *pows = h.words(nn);
+        uint8_t *leaves = h.bytes(nn * 32), *widths = h.bytes(k.rows);
+        memset(widths, k.bytes, k.rows);
+        hlk::g_pieces.clear();
+        hl_store* st = nullptr;
+        if (hl_b200_commit_zk_packed(c, k.lc, 2, data, widths, k.rows, pads, 1, pows, 0, nullptr, nullptr, nullptr, nullptr, &st, leaves, nullptr)) bad("pieces", "refused");
+        hl_b200_store_free(st);
+        const std::vector<u32> p = hlk::g_pieces;
+        std::string how = "2^" + std::to_string(k.lc) + ":";
+        u32 sum = 0;
+        bool ok = !p.empty() && (p.size() > 1) == (k.last > 0);
+        for (size_t i = 0; i < p.size(); i++) {
+            how += " " + std::to_string(p[i]);
+            sum += p[i];
+            ok = ok && p[i] > 0 && (i + 1 == p.size() || p[i] % batch == 0) && (p.size() == 1 || p[i] <= 3 * 148 * batch);
+        }
+        if (!ok || sum != k.rows || (k.last && (p.back() + batch - 1) / batch > k.last)) bad("pieces", how);
+    }
+    hl_b200_shutdown(c);
+}
+
 int main(int argc, char** argv) {
     if (argc == 3 && !strcmp(argv[1], "threads")) {
         g_threads = atol(argv[2]);
@@ -331,6 +367,8 @@ int main(int argc, char** argv) {
         timeouts();
     } else if (argc == 2 && !strcmp(argv[1], "reorder")) {
         reorder();
+    } else if (argc == 2 && !strcmp(argv[1], "pieces")) {
+        pieces();
     } else {
         failures(false);
         failures(true);

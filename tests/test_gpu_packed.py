@@ -139,16 +139,26 @@ def test_block_shape_from_pageable_and_page_locked_packed_rows(dev, oracle):
 
 @pytest.mark.parametrize("rows", [593, 1185, 1777, 2369])
 def test_piecewise_upload_at_row_counts_around_the_piece_boundaries(dev, oracle, rows):
-    """The narrow upload goes in pieces of 1, 2, 3, 5, 8 waves (a wave = one row per SM), the pads of each piece and the salts with
-    them.  Row counts one above a piece boundary on a 148-SM device (4 x 148 + 1, 8 x 148 + 1, ..), where the last piece is a single
-    row: the packed call from page-locked and from pageable memory, the wide call, and a commitment of the same rows already on the
-    device (no pieces at all) give one tree, and the pads and widened rows left resident give the same opening combination."""
+    """The upload goes in pieces of 1, 1, 2, 2, 3, .. turns of the machine (148 rows of 2^14 words), or of two with one or a half behind them, the
+    pads of each piece and the salts with them.  Row counts one above a multiple of a turn: see `same_in_pieces`."""
+    same_in_pieces(dev, oracle, 14, rows)
+
+
+# rows of which several share 2^14 words, the last batch of a piece and of the commitment not full; more than 32 MB of 16-bit and of 64-bit words
+@pytest.mark.parametrize("log_cols,rows", [(13, 1187), (13, 3999), (12, 2307), (12, 5001), (10, 9003), (9, 9001)])
+def test_piecewise_upload_of_shorter_rows(dev, oracle, log_cols, rows):
+    same_in_pieces(dev, oracle, log_cols, rows)
+
+
+def same_in_pieces(dev, oracle, log_cols, rows):
+    """The packed call from page-locked and from pageable memory, the wide call, and a commitment of the same rows already on the device (no
+    pieces at all) give one tree, and the pads and widened rows left resident give the same opening combination."""
     import torch
 
     from intelligenceregulation_b200 import backend
 
     o = oracle
-    log_cols, ir, q = 14, 2, 280
+    ir, q = 2, 280
     n, nn = 1 << log_cols, ir << log_cols
     rng = np.random.default_rng(rows)
     data = to_fp(rng.integers(-32768, 32768, rows * n)).reshape(rows, n)

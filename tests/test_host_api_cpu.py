@@ -38,6 +38,10 @@ def test_an_encoding_is_put_into_the_columns_order_once(emul):
     _ok(emul, "reorder")
 
 
+def test_rows_of_every_length_come_in_pieces(emul):
+    _ok(emul, "pieces")
+
+
 def test_copies_of_all_sizes(emul):
     """the limits between the forms of a copy, unaligned ends, and more small copies in a call than the bounce areas hold"""
     _ok(emul, "copies")
