@@ -250,9 +250,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_encode_tc(RowArgs a, const u6
                     const u32 to = S + at_i2(4 * t + q, 8 * g, lane);
                     ask(w1 + t * 128 + 2048, 512, wb);
                     product_done(t);
-                    half(t, 0, [&](u32 e, u64 v) { tc_sts(go_i2(to, e), tc_mul(v, wa[e])); });
+                    half(t, 0, [&](u32 e, u64 v) { tc_sts(go_i2(to, e), gl_mul_lazy(v, wa[e])); });
                     if (t < 3) ask(w1 + (t + 1) * 128, 512, wa);
-                    half(t, 1, [&](u32 e, u64 v) { tc_sts(go_i2(to, 4 + e), tc_mul(v, wb[e])); });
+                    half(t, 1, [&](u32 e, u64 v) { tc_sts(go_i2(to, 4 + e), gl_mul_lazy(v, wb[e])); });
                     arrive(4 + t, 1);
                 }
             }
@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_encode_tc(RowArgs a, const u6
                     for (u32 h = 0; h < 2; h++)
                         half(4 + t, h, [&](u32 e, u64 v) {
                             const u32 r = 4 * h + e;
-                            v = tc_mul(v, tc_lds(tw + r * 128 + t * 32));
+                            v = gl_mul_lazy(v, tc_lds(tw + r * 128 + t * 32));
                             if (t == 3) tc_sts(go_c(tile_i2(to, 3), r), v);
                             else hold[8 * (t % 3) + r] = v;
                         });
@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_encode_tc(RowArgs a, const u6
                         for (u32 e = 0; e < 4; e++) z[e] = tc_ldg(tab + TC_TWIST + ((index(t, 4 * h + e) * s) & (nn - 1)));
                     };
                     if (later || s0) twists(later ? 1u : s0);
-                    half(8 + t, h, [&](u32 e, u64 v) { x[e] = tc_mul(v, w[e]); });
+                    half(8 + t, h, [&](u32 e, u64 v) { x[e] = gl_mul_lazy(v, w[e]); });
                     const bool padded = pad_words(t, h, 0, d);
                     if (padded) {
 #pragma unroll
@@ -328,7 +328,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_encode_tc(RowArgs a, const u6
                         }
                         if (s) {
 #pragma unroll
-                            for (u32 e = 0; e < 4; e++) y[e] = tc_mul(y[e], z[e]);
+                            for (u32 e = 0; e < 4; e++) y[e] = gl_mul_lazy(y[e], z[e]);
                         }
                         if (f == 0) break;
 #pragma unroll
@@ -374,7 +374,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_encode_tc(RowArgs a, const u6
                         for (u32 h = 0; h < 2; h++) {
                             half(t, h, [&](u32 e, u64 v) {
                                 const u32 r = 4 * h + e;
-                                v = tc_mul(v, h ? wb[e] : wa[e]);
+                                v = gl_mul_lazy(v, h ? wb[e] : wa[e]);
                                 if (t == 3) tc_sts(go_f2(tile_f1(to, 3), r), v);
                                 else hold[8 * (t % 3) + r] = v;
                             });
@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_encode_tc(RowArgs a, const u6
                     const u32 tw = S + TC_S_SMALL + (TC_F2 + 8 * g * 32 + lane) * 8, to = S + at_f3(4 * t + q, 8 * g, lane);
                     product_done(4 + t);
 #pragma unroll
-                    for (u32 h = 0; h < 2; h++) half(4 + t, h, [&](u32 e, u64 v) { tc_sts(go_f3(to, 4 * h + e), tc_mul(v, tc_lds(tw + (4 * h + e) * 256))); });
+                    for (u32 h = 0; h < 2; h++) half(4 + t, h, [&](u32 e, u64 v) { tc_sts(go_f3(to, 4 * h + e), gl_mul_lazy(v, tc_lds(tw + (4 * h + e) * 256))); });
                     arrive(8 + t, 1);
                 }
                 // ---- F3 ----

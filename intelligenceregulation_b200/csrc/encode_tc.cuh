@@ -102,35 +102,6 @@ GL_HD u64 tc_join(const u32* s) {
 #endif
 }
 
-// a b / 2^64 mod p (lazy; canonical where b is) with Montgomery's reduction: 1 / p = 2^32 + 1 mod 2^64, so with lo + (lo << 32) = m + e 2^64 the
-// word is hi - (m - (m >> 32) - e).  Nine instructions where the plain reduction takes eleven; every table here holds its constants
-// times 2^64.
-GL_HD u64 tc_mul(u64 a, u64 b) {
-#ifdef __CUDA_ARCH__
-    u32 p0, p1, p2, p3, r0, r1;
-    gl_product(a, b, p0, p1, p2, p3);
-    asm("{\n\t"
-        ".reg .u32 h,t,b0,b1,m;\n\t"
-        "add.cc.u32 h, %3, %2;\n\t"
-        "addc.u32 t, h, 0;\n\t"  // no carry: h + e <= 2^32 - 1
-        "sub.cc.u32 b0, %2, t;\n\t"
-        "subc.u32 b1, h, 0;\n\t"
-        "sub.cc.u32 %0, %4, b0;\n\t"
-        "subc.cc.u32 %1, %5, b1;\n\t"
-        "subc.u32 m, 0, 0;\n\t"
-        "sub.cc.u32 %0, %0, m;\n\t"
-        "subc.u32 %1, %1, 0;\n\t"
-        "}"
-        : "=&r"(r0), "=&r"(r1)
-        : "r"(p0), "r"(p1), "r"(p2), "r"(p3));
-    return ((u64)r1 << 32) | r0;
-#else
-    const unsigned __int128 x = (unsigned __int128)a * b;
-    const u64 lo = (u64)x, hi = (u64)(x >> 64), m = lo + (lo << 32), e = m < lo ? 1 : 0, t = m - (m >> 32) - e;
-    return hi >= t ? hi - t : hi - t - GL_EPS;
-#endif
-}
-
 template <int LOGN>
 struct Tc {
     static_assert(LOGN >= 10 && LOGN <= 14, "tensor-core path sizes");
@@ -203,29 +174,28 @@ struct Tc {
 };
 
 // The tables of rows of 2^logn words at rate 2^-logr; `out` holds tc_table_words words: those above, and then the residues' twists
-// w_nn^j, j < nn.  All twiddles times 2^64 (`tc_mul`); I2's carry 2^64 / n beside that: an inverse transform's results are then 2^64 c, and
-// their product with a power of the coset, which is the caller's and a plain word, is a plain word.
+// w_nn^j, j < nn.  I2's twiddles carry 1 / n.
 constexpr u32 TC_TWIST = TC_TABLE_WORDS;
 inline size_t tc_table_words(u32 logn, u32 logr) { return TC_TABLE_WORDS + ((size_t)1 << (logn + logr)); }
 inline void tc_build(u32 logn, u32 logr, u64* out) {
     const u32 g = logn - 10, cm = (1u << g) - 1u, N = 1u << logn;
-    const u64 root = gl_pow(gl_pow(7, (GL_P - 1) >> 32), 1ull << (32 - logn)), ninv = gl_inv(N), mont = GL_EPS;  // 2^64 = 2^32 - 1
-    u64 *w = new u64[N], *wm = new u64[N];
+    const u64 root = gl_pow(gl_pow(7, (GL_P - 1) >> 32), 1ull << (32 - logn)), ninv = gl_inv(N);
+    u64* w = new u64[N];
     u64 x = 1;
-    for (u32 i = 0; i < N; i++) { w[i] = x; wm[i] = gl_mul(x, mont); x = gl_mul(x, root); }
+    for (u32 i = 0; i < N; i++) { w[i] = x; x = gl_mul(x, root); }
     const u64 root_nn = gl_pow(gl_pow(7, (GL_P - 1) >> 32), 1ull << (32 - logn - logr));
-    x = mont;
+    x = 1;
     for (size_t j = 0; j < (size_t)1 << (logn + logr); j++) { out[TC_TWIST + j] = x; x = gl_mul(x, root_nn); }
     for (u32 k = 0; k < 32; k++) {
         for (u32 c = 0; c < 16; c++) {
-            for (u32 b = 0; b < 32; b++) out[TC_I1 + (k * 16 + c) * 32 + b] = wm[(k * ((b << g) + (c & cm))) & (N - 1)];
-            out[TC_SMALL + k * 16 + c] = gl_mul(gl_mul(wm[(32 * k * (c & cm)) & (N - 1)], ninv), mont);
+            for (u32 b = 0; b < 32; b++) out[TC_I1 + (k * 16 + c) * 32 + b] = w[(k * ((b << g) + (c & cm))) & (N - 1)];
+            out[TC_SMALL + k * 16 + c] = gl_mul(w[(32 * k * (c & cm)) & (N - 1)], ninv);
         }
-        for (u32 b = 0; b < 32; b++) out[TC_SMALL + TC_F2 + k * 32 + b] = wm[(k * b * (N / 1024)) & (N - 1)];
+        for (u32 b = 0; b < 32; b++) out[TC_SMALL + TC_F2 + k * 32 + b] = w[(k * b * (N / 1024)) & (N - 1)];
     }
     for (u32 c = 0; c < 16; c++)
         for (u32 tile = 0; tile < 8; tile++)
-            for (u32 row = 0; row < 128; row++) out[TC_F1 + (c * 8 + tile) * 128 + row] = wm[((c & cm) * tc_k_of(tile, row)) & (N - 1)];
+            for (u32 row = 0; row < 128; row++) out[TC_F1 + (c * 8 + tile) * 128 + row] = w[((c & cm) * tc_k_of(tile, row)) & (N - 1)];
     unsigned char* bm = reinterpret_cast<unsigned char*>(out + TC_B);
     for (u32 i = 0; i < 32; i++)
         for (u32 j = 0; j < 32; j++)
@@ -241,7 +211,6 @@ inline void tc_build(u32 logn, u32 logr, u64* out) {
                 for (u32 d = 0; d < 8; d++) b3[tc_swizzled(8 * i + d, j * 8 + b)] = (unsigned char)(v >> (8 * d));
             }
     delete[] w;
-    delete[] wm;
 }
 
 }  // namespace enc

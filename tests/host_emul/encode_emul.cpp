@@ -136,14 +136,14 @@ static int run_tc(const RowArgs& a) {
         for (u32 t = 0; t < 4; t++) {
             product(false, t, [&](u32 m, u32 k, u64 v) {
                 const u32 b = m & 31, c = 4 * t + (m >> 5);
-                to(go_i2(S0 + at_i2(c, k & ~7u, b), k & 7), at_i2(c, k, b), tc_mul(v, tab[TC_I1 + (k * 16 + c) * 32 + b]));
+                to(go_i2(S0 + at_i2(c, k & ~7u, b), k & 7), at_i2(c, k, b), gl_mul_lazy(v, tab[TC_I1 + (k * 16 + c) * 32 + b]));
             });
             flush(t);
         }
         for (u32 t = 0; t < 4; t++)
             product(false, t, [&](u32 m, u32 k, u64 v) {
                 const u32 ka = (m >> 1) & 31, c = 4 * t + (m & 1) + ((m >> 6) << 1);
-                to(go_c(tile_i2(S0 + at_c(ka, k & ~7u, c & 3), t), k & 7), at_c(ka, k, c), tc_mul(v, tab[TC_SMALL + k * 16 + c]));
+                to(go_c(tile_i2(S0 + at_c(ka, k & ~7u, c & 3), t), k & 7), at_c(ka, k, c), gl_mul_lazy(v, tab[TC_SMALL + k * 16 + c]));
             });
         flush(-1);
         for (u32 s = 0; s < (1u << a.logr); s++) {
@@ -152,7 +152,7 @@ static int run_tc(const RowArgs& a) {
                     product(true, t, [&](u32 m, u32 o, u64 v) {
                         const u32 i = (T::N - tc_k_of(t, m) - 1024 * (o & T::CMASK)) & (T::N - 1), row = row0 + (o >> T::G), at = t * 16384 + tc_swizzled(m, 8 * o);
                         const bool pad = row < a.rows && i < tc_pad_words(LOGN, a.q) / T::ROWS;
-                        u64 x = tc_mul(v, a.zk ? a.pows[i] : 1);
+                        u64 x = gl_mul_lazy(v, a.zk ? a.pows[i] : 1);
                         if (pad) x = gl_add_lazy(x, T::pad_below(a, row, i));
                         keep[at / 8] = x;
                         if (pad) x = gl_add_lazy(x, T::pad_above(a, row, i, 0));
@@ -167,19 +167,19 @@ static int run_tc(const RowArgs& a) {
                             const u32 i = (T::N - tc_k_of(t, m) - 1024 * (o & T::CMASK)) & (T::N - 1), row = row0 + (o >> T::G), at = t * 16384 + tc_swizzled(m, 8 * o);
                             u64 x = keep[at / 8];
                             if (row < a.rows && i < tc_pad_words(LOGN, a.q) / T::ROWS) x = gl_add_lazy(x, T::pad_above(a, row, i, s));
-                            word(at) = tc_mul(x, tab[TC_TWIST + ((i * s) & (nn - 1))]);
+                            word(at) = gl_mul_lazy(x, tab[TC_TWIST + ((i * s) & (nn - 1))]);
                         }
             }
             for (u32 t = 0; t < 8; t++)
                 product(true, t, [&](u32 m, u32 c, u64 v) {
                     const u32 ka = tc_k_of(t, m) & 31, kb = tc_k_of(t, m) >> 5;
-                    to(go_f2(tile_f1(S0 + at_f2(c & ~7u, ka, kb & 7), t >> 1), c & 7), at_f2(c, ka, kb), tc_mul(v, tab[TC_F1 + (c * 8 + t) * 128 + m]));
+                    to(go_f2(tile_f1(S0 + at_f2(c & ~7u, ka, kb & 7), t >> 1), c & 7), at_f2(c, ka, kb), gl_mul_lazy(v, tab[TC_F1 + (c * 8 + t) * 128 + m]));
                 });
             flush(-1);
             for (u32 t = 0; t < 4; t++) {
                 product(false, t, [&](u32 m, u32 k, u64 v) {
                     const u32 ka = m & 31, c = 4 * t + (m >> 5);
-                    to(go_f3(S0 + at_f3(c, k & ~7u, ka), k & 7), at_f3(c, k, ka), tc_mul(v, tab[TC_SMALL + TC_F2 + k * 32 + ka]));
+                    to(go_f3(S0 + at_f3(c, k & ~7u, ka), k & 7), at_f3(c, k, ka), gl_mul_lazy(v, tab[TC_SMALL + TC_F2 + k * 32 + ka]));
                 });
                 flush(t);
             }
