@@ -23,7 +23,8 @@ int hl_b200_set_dependent_launch(int on);
 /* How often the CTAs of the one-launch rounds of a sumcheck look for a round's sums and for its challenge before they give up (4,194,304
  * each: some seconds).  A test makes a wait run out with a small number and sees HL_B200_ERR_TIMEOUT. */
 int hl_b200_set_wait_limits(hl_ctx* ctx, uint32_t sums, uint32_t challenge);
-/* The same for the waits of the tensor-core row encoder (4,194,304), in the commitments that follow. */
+/* The same for the waits of the tensor-core row encoder (4,194,304, looked at every 64 times), in the commitments that follow; with 0 they all
+ * run out. */
 int hl_b200_set_encoder_wait_limit(hl_ctx* ctx, uint32_t looks);
 
 #ifdef __cplusplus

@@ -31,7 +31,7 @@ bool encode_tc_takes(u32 logn, u32 logr, u32 rows, int sm_count);
 // what these rows ask for, and what is enough for any number of them up to that, in the form that needs less
 size_t encode_tc_scratch_words(u32 logn, u32 logr, u32 q, u32 rows, int sm_count);
 size_t encode_tc_least_words(u32 logn, u32 logr, u32 q, u32 rows, int sm_count);
-// A wait of the kernel that runs out writes `mark` into `word` and, where it is not null, 1 into `also` (page-locked); it looks `limit` times
+// A wait of the kernel that runs out writes `mark` into `word` and, where it is not null, 1 into `also` (page-locked); it looks `limit` times, with 0 in vain
 struct TcReport { u32 *word = nullptr, mark = 0, *also = nullptr, limit = 0; };
 cudaError_t encode_rows_tc(enc::RowArgs a, u32 logn, const u64* tab, int sm_count, size_t scratch_words, TcReport report, cudaStream_t st, int* path_out);
 
