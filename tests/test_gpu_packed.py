@@ -104,7 +104,7 @@ def test_packed_rows_commit_to_the_same_leaves_tree_and_opening(dev, oracle, sha
 
 def test_block_shape_from_pageable_and_page_locked_packed_rows(dev, oracle):
     """2,504 rows of 2^14 words (the Llama-3-8B block `A` shape), int16-valued except eight full-width rows: the upload goes in
-    wave-sized pieces (82 MB of narrow bytes instead of 328 MB), from pageable memory through the context's staging buffers and from
+    pieces (82 MB of narrow bytes instead of 328 MB), from pageable memory through the context's staging buffers and from
     page-locked memory directly; leaves and tree equal the wide call's."""
     import torch
     from intelligenceregulation_b200 import backend
@@ -144,9 +144,10 @@ def test_piecewise_upload_at_row_counts_around_the_piece_boundaries(dev, oracle,
     same_in_pieces(dev, oracle, 14, rows)
 
 
-# rows of which several share 2^14 words, the last batch of a piece and of the commitment not full; more than 32 MB of 16-bit and of 64-bit words
-@pytest.mark.parametrize("log_cols,rows", [(13, 1187), (13, 3999), (12, 2307), (12, 5001), (10, 9003), (9, 9001)])
-def test_piecewise_upload_of_shorter_rows(dev, oracle, log_cols, rows):
+# rows of which several share 2^14 words, the last batch of a piece and of the commitment not full, and longer ones, whose last piece is split
+# by residue; more than 32 MB of 16-bit and of 64-bit words
+@pytest.mark.parametrize("log_cols,rows", [(13, 1187), (13, 3999), (12, 2307), (12, 5001), (10, 9003), (9, 9001), (8, 17001), (15, 201), (15, 801), (16, 163)])
+def test_piecewise_upload_of_shorter_and_longer_rows(dev, oracle, log_cols, rows):
     same_in_pieces(dev, oracle, log_cols, rows)
 
 
@@ -158,8 +159,8 @@ def same_in_pieces(dev, oracle, log_cols, rows):
     from intelligenceregulation_b200 import backend
 
     o = oracle
-    ir, q = 2, 280
-    n, nn = 1 << log_cols, ir << log_cols
+    ir, n, nn = 2, 1 << log_cols, 2 << log_cols
+    q = min(280, n)
     rng = np.random.default_rng(rows)
     data = to_fp(rng.integers(-32768, 32768, rows * n)).reshape(rows, n)
     data[::97] = rng.integers(0, P, (len(range(0, rows, 97)), n), dtype=np.uint64)
@@ -176,14 +177,14 @@ def same_in_pieces(dev, oracle, log_cols, rows):
     st_r.merkle_dev(ds.data_ptr(), tag.leaf, tag.node, dl.data_ptr())
     dev.ctx.sync()
     want = dl.cpu().numpy().reshape(2 * nn - 1, 32)
-    st_w, _, levels_w = dev.try_commit_zk_tree(log_cols, ir, data, pads, pows, 15, tag.column, salts, tag.leaf, tag.node, want_leaves=False)
+    st_w, _, levels_w = dev.try_commit_zk_tree(log_cols, ir, data, pads, pows, 17, tag.column, salts, tag.leaf, tag.node, want_leaves=False)
     assert (levels_w == want).all()
-    st_p, _, levels_p = dev.try_commit_zk_packed(log_cols, ir, packed, widths, pads, pows, 15, tag.column, salts, tag.leaf, tag.node, want_leaves=False)
+    st_p, _, levels_p = dev.try_commit_zk_packed(log_cols, ir, packed, widths, pads, pows, 17, tag.column, salts, tag.leaf, tag.node, want_leaves=False)
     assert (levels_p == want).all()
     pin = torch.empty(packed.size, dtype=torch.uint8, pin_memory=True)
     pin.numpy()[...] = packed
     pin_pads = torch.from_numpy(pads.view(np.int64)).pin_memory()
-    st_q, _, levels_q = dev.try_commit_zk_packed(log_cols, ir, pin.numpy(), widths, pin_pads.numpy().view(np.uint64), pows, 15, tag.column, salts, tag.leaf, tag.node,
+    st_q, _, levels_q = dev.try_commit_zk_packed(log_cols, ir, pin.numpy(), widths, pin_pads.numpy().view(np.uint64), pows, 17, tag.column, salts, tag.leaf, tag.node,
                                                   want_leaves=False)
     assert (levels_q == want).all()
     rhos = rng.integers(0, P, (2, rows, 2), dtype=np.uint64)
