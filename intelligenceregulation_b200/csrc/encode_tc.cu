@@ -37,13 +37,14 @@ __device__ __forceinline__ void tc_arrive(u32 bar) { asm volatile("mbarrier.arri
 // product runs beside them.
 // Barriers: FULL[2] an accumulator holds its product; FREE[2] the workers have read it; READY[j] the operand of product j is in place, once a
 // transform each.
-// What bounds it: a row of 2^14 words at rate 1/2 takes 141 k cycles, 65 k of them instructions of each scheduler (a third of them moves
+// What bounds it: a row of 2^14 words at rate 1/2 takes some 140 k cycles, 65 k of them instructions of each scheduler (a third of them moves
 // and addresses around the 8 products and 9 joins of a word), the rest waits of its four workers on each other's passes (20 k), stores (8,192
-// sectors, which the L2 takes in bursts) and the twiddles' way from L2; the tensor pipe is busy 22 %.  2,606 rows: 1,338 us, the
+// sectors, which the L2 takes in bursts) and the twiddles' way from L2; the tensor pipe is busy 22 %.  2,606 rows: 1,326 us, the
 // shared-memory encoder 1,901.  Steps that brought it there, 2,606 rows each time: both transforms through a scratch row and one order of passes
 // 2,105; the forward transform's passes reversed, so that its words stay where they are 1,674; the pads worked out ahead, no branches among
 // the words 1,498; the later residues' words by asynchronous copies, twiddles asked for half a product ahead 1,479; residues apart in the output
-// 1,338.  Montgomery's reduction saves a seventh of the products' instructions and no time: they are not what it waits for.
+// 1,338; a shorter test in the polling loop 1,326.  Montgomery's reduction saves a seventh of the products' instructions and 0.6 % of the time, and is
+// not worth a second product and tables in its form.  96 registers a thread, with 96 to 156 bytes of them spilled (`-Xptxas -v`).
 // Every wait is bounded: one that runs out sets `gave_up`, after which nobody waits and no product is issued; the CTA walks to its
 // end (all addresses are the same), waits for the products in flight and frees TMEM, and leaves the store's mark where the host reads it.
 template <int LOGN, bool NARROW>
@@ -462,17 +463,17 @@ namespace hlk {
 size_t encode_tc_table_words(u32 logn, u32 logr) { return tc_table_words(logn, logr); }
 void encode_tc_build(u32 logn, u32 logr, u64* out) { tc_build(logn, logr, out); }
 
-// Rows of 2^14 words always: 2,606 of them 1,901 -> 1,338 us, 74 of them 74 -> 61, 4 of them 72 -> 56; at rate 1/4 1,184 rows 1,625 -> 1,135.
+// Rows of 2^14 words always: 2,606 of them 1,901 -> 1,326 us, 74 of them 74 -> 56, 4 of them 72 -> 55; at rate 1/4 1,184 rows 1,625 -> 1,146.
 // Shorter rows where a CTA that takes 2^14 words' worth of them is not the longer chain: a transform takes one 26 us and a machine full of
 // them no longer.  The shared-memory encoder gives rows of 2^13 words a CTA each per residue (44 us) while they fit the SMs, and
 // takes 12 us + 0.195 us for each 2^14 words and transform of shorter ones (both fitted to rows of 2^10 .. 2^13 words, 4 to 2,606 times 2^14
-// words, rates 1/2 and 1/4): 592 rows of 2^11 58 -> 55, 600 of them 60 (74 here), 1,184 of them 96 -> 78; 888 of 2^12 148 (150 here), 2,368 of
-// them 346 -> 283; 148 of 2^13 62 -> 56, 74 of them 46 (54 here).
-// Measured at rates down to 1/64, 1 to 444 times 2^14 words (rows of 2^14: rate 1/8 38 rows 221 -> 146, 1,036 of them 3,204 -> 1,988; rate 1/16
-// 148 rows 1,121 -> 626; rate 1/64 4 rows 179 -> 121, 38 of them 1,407 -> 914; rows of 2^13 alike): what the line gives to this encoder is never
-// more than 8 % slower here (400 rows of 2^13 at 1/2 140, 151 here; 1,184 of 2^10 52, 56 here).  It is a cautious one: the other encoder's
-// scratch leaves L2 at rates of 1/16 and less, where its 0.195 us become 0.4 and more, and rows of 2^10 .. 2^12 that it keeps would take half
-// the time here (592 rows of 2^11 at 1/64 2,955, 1,370 here).
+// words, rates 1/2 and 1/4): 592 rows of 2^11 56 -> 52, 1,184 of them 95 -> 74, 720 of them 65 (72 here); 2,368 of 2^12 346 -> 283, 800 of them
+// 131 (142 here); 148 of 2^13 63 -> 56, 74 of them 47 (54 here).
+// Measured at rates down to 1/64, 1 to 444 times 2^14 words (rows of 2^14: rate 1/8 38 rows 221 -> 143, 1,036 of them 3,204 -> 1,903; rate 1/16
+// 148 rows 1,121 -> 596; rate 1/64 4 rows 179 -> 119, 38 of them 1,407 -> 866; rows of 2^13 alike): what the line gives to this encoder is never
+// more than 3 % slower here (400 rows of 2^13 at 1/2 142, 146 here).  It is a cautious one: the other encoder's scratch leaves L2 at rates of
+// 1/16 and less, where its 0.195 us become 0.4 and more, and rows of 2^10 .. 2^12 that it keeps would take half the time here (592 rows of
+// 2^11 at 1/64 2,885, 1,301 here).
 bool encode_tc_takes(u32 logn, u32 logr, u32 rows, int sm_count) {
     if (logn < 10 || logn > 14) return false;
     if (logn == 14) return true;
